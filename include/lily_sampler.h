@@ -260,6 +260,17 @@ typedef struct lily_sample_args {
 int32_t lily_sample_batch(lily_sampler_t *h, void *stream, const lily_sample_args_t *args);
 
 /*
+ * src/kernels/sample.rs:373-387 sample_f32 as the reference calls it: one draw from
+ * logits[0, logits_len >= vocab) on draw index `step`, with the penalties over
+ * history_ids[0, history_len) (device ids, a HOST length). `params` is a HOST
+ * pointer. Equal to lily_sample_batch with one row; nothing but the kernel is
+ * enqueued, no length has to be brought to the device first.
+ */
+int32_t lily_sample_one(lily_sampler_t *h, void *stream, const void *logits, uint32_t logits_dtype,
+                        uint64_t logits_len, const lily_sampling_params_t *params, uint32_t step,
+                        const uint32_t *history_ids, uint32_t history_len, uint32_t *out_id);
+
+/*
  * The same draw for callers that cannot allocate device memory. (No
  * counterpart in the reference.)
  *

@@ -16,7 +16,7 @@
 #include "../../include/lily_sampler.h"
 #include "sample_kernel.cuh"
 #include "stream_kernel.cuh"
-#include "cluster_kernel.cuh"
+#include "split_args.cuh"
 #include "lmhead_kernel.cuh"
 
 namespace {
@@ -57,8 +57,7 @@ struct lily_sampler {
     uint32_t *part_n = nullptr;
     uint32_t *tickets = nullptr;
     uint32_t *status_word = nullptr;
-    char *spill = nullptr;  // parameters of rows the small-batch kernel hands to the general code
-    int max_clusters = -1;  // clusters of the small-batch kernel the GPU runs at once (-1: not asked yet)
+    char *spill = nullptr;  // inline parameters of rows the row kernel hands to the general code
     uint32_t *counts_scratch = nullptr;
     uint32_t *counts_table = nullptr;
     uint32_t *seen_table = nullptr;
@@ -109,17 +108,18 @@ int32_t cuda_fail(lily_sampler *h, cudaError_t e, const char *what) {
 
 struct DeviceGuard {
     int prev = -1;
-    bool ok = true;
+    bool ok = true, moved = false;
     explicit DeviceGuard(int dev) {
         if (cudaGetDevice(&prev) != cudaSuccess) {
             prev = -1;
         }
         if (prev != dev) {
+            moved = true;
             ok = cudaSetDevice(dev) == cudaSuccess;
         }
     }
     ~DeviceGuard() {
-        if (prev >= 0) {
+        if (moved && prev >= 0) {
             cudaSetDevice(prev);
         }
     }
@@ -256,109 +256,120 @@ int32_t launch_one(lily_sampler *h, cudaStream_t stream_, const lily::KArgs &a, 
     return launch_serialised(h, stream_, kernel, dim3(a.n_slices, rows, 1), smem, a);
 }
 
-// Whether a call goes to the small-batch kernel (a cluster of eight blocks per
-// row): few enough rows for every cluster to have SMs of its own, aligned logits,
-// a vocabulary whose eighth fits a block's shared memory, a plain draw.
-size_t cluster_launch_smem(uint32_t vocab) {
-    const size_t own = lily::cluster_smem_bytes(vocab);
-    const size_t general = smem_bytes(vocab, 1);  // the leader may run the general row code
-    return own > general ? own : general;
+// How the row kernel is launched: the blocks a row is split over, and how each
+// keeps the history ids of its share.
+struct SplitPlan {
+    bool take = false;
+    bool sole = false;   // at most one block per SM
+    bool share = false;  // the blocks of a row share its history list
+    uint32_t log_blocks = 0, mark_mode = lily::MARK_BITS, mark_words = 0;
+    size_t smem = 0;
+};
+
+using lily::INLINE_ROWS;
+using lily::INLINE_ROWS_MAX;
+
+// `lists`: rows may bring a list of ids (history, bias, ban, or ids drawn earlier
+// in the step); `counts`: a history list with a frequency penalty.
+SplitPlan split_plan(const lily_sampler *h, const lily::KArgs &a, uint32_t rows, uint32_t dtype, bool lists,
+                     bool counts) {
+    SplitPlan p;
+    if (a.cand_out != nullptr || a.merge_in != nullptr) {
+        return p;
+    }
+    const uint32_t per = dtype == LILY_F32 ? lily::Piece<float>::PER : lily::Piece<__nv_bfloat16>::PER;
+    const uint32_t logits = 32u * per;
+    if (a.vocab / logits < lily::SPL_MIN_TILES) {
+        return p;
+    }
+    const uint32_t pieces = lily::split_pieces(a.vocab, per - 1u, per);
+    const size_t general = smem_bytes(a.vocab, 1);  // the first block may run the general row code
+    const uint32_t slots = (uint32_t)h->sm_count;
+    uint32_t lb = 3;
+    while (lb > 0u && ((rows << lb) > slots || (a.vocab / logits) >> lb < lily::SPL_MIN_TILES)) {
+        --lb;
+    }
+    p.sole = (rows << lb) <= (uint32_t)h->sm_count;
+    const uint32_t here = (pieces + (1u << lb) - 1u) >> lb, entries = here * logits;
+    const size_t fixed = sizeof(lily::SmemFixed) + sizeof(lily::SplitSmem) +
+                         (size_t)lily::split_buckets(here, lily::split_u(p.sole ? 1 : 2)) * lily::SPL_NT * 4u;
+    p.log_blocks = lb;
+    if (lists) {
+        const size_t limit = p.sole ? (size_t)h->max_smem : 113u * 1024u;
+        if (counts && fixed + (size_t)entries * 2u <= limit) {
+            p.mark_mode = lily::MARK_COUNTS;
+            p.mark_words = entries / 2u;
+        } else if (fixed + entries <= limit) {
+            p.mark_mode = lily::MARK_BYTES;
+            p.mark_words = entries / 4u;
+        } else {
+            p.mark_mode = lily::MARK_BITS;
+            p.mark_words = (entries / 32u + 3u) & ~3u;
+        }
+    }
+    // (Below some thousands of ids looking at all of them costs less than the blocks' meeting.)
+    p.share = lists && lb > 0u && a.history_ids != nullptr && (p.mark_mode == lily::MARK_COUNTS || a.history_ld > 4096u);
+    p.smem = fixed + (size_t)p.mark_words * 4u;
+    p.smem = p.smem > general ? p.smem : general;
+    p.take = p.smem <= (size_t)h->max_smem && p.sole;
+    return p;
 }
 
-// How many clusters of the small-batch kernel run at once: a launch of more
-// rows than that would take its rows in turns, which the kernel of one block per
-// row does not. (A cluster needs eight free SMs of one GPC.)
-int max_active_clusters(lily_sampler *h) {
-    if (h->max_clusters < 0) {
-        h->max_clusters = 0;
-        auto kernel = lily::cluster_rows_kernel<__nv_bfloat16>;
-        const size_t smem = cluster_launch_smem(h->vocab);
-        if (smem <= (size_t)h->max_smem &&
-            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, h->max_smem) == cudaSuccess) {
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3(lily::CL, 64, 1);
-            cfg.blockDim = dim3(lily::NT, 1, 1);
-            cfg.dynamicSmemBytes = smem;
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeClusterDimension;
-            attr[0].val.clusterDim.x = lily::CL;
-            attr[0].val.clusterDim.y = 1;
-            attr[0].val.clusterDim.z = 1;
-            cfg.attrs = attr;
-            cfg.numAttrs = 1;
-            int n = 0;
-            if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess) {
-                h->max_clusters = n;
-            }
-        }
-        (void)cudaGetLastError();
-    }
-    return h->max_clusters;
-}
-
-bool cluster_call(lily_sampler *h, const void *logits, uint64_t logits_ld, uint32_t dtype,
-                  uint32_t rows, bool plain) {
-    const size_t esize = dtype == LILY_F32 ? 4 : 2;
-    const bool vec = (reinterpret_cast<uintptr_t>(logits) % 16u == 0u) && ((logits_ld * esize) % 16u == 0u);
-    return plain && vec && lily::cluster_slice_len(h->vocab) <= lily::CL_SLICE_MAX && h->vocab >= 4096u &&
-           (int)rows <= max_active_clusters(h);
-}
-
-int32_t launch_cluster(lily_sampler *h, cudaStream_t stream, const lily::ClusterArgs &ca_, uint32_t rows,
-                       uint32_t dtype) {
-    const size_t smem = cluster_launch_smem(ca_.a.vocab);
-    if (smem > (size_t)h->max_smem) {
-        return fail(h, LILY_ERR_CAPACITY, "vocabulary too large for the small-batch kernel");
-    }
-    lily::ClusterArgs ca = ca_;
-    ca.spill_params = reinterpret_cast<lily_sampling_params_t *>(h->spill);
-    ca.spill_steps = reinterpret_cast<uint32_t *>(h->spill + lily::CL_MAX_ROWS * sizeof(lily_sampling_params_t));
-    ca.spill_slots = ca.spill_steps + lily::CL_MAX_ROWS;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(lily::CL, rows, 1);
-    cfg.blockDim = dim3(lily::NT, 1, 1);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = lily::CL;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 2;
-    if (dtype == LILY_F32) {
-        auto kernel = lily::cluster_rows_kernel<float>;
-        const int32_t st = raise_smem_limit(h, kernel, 1u << 8);
-        if (st != LILY_OK) {
-            return st;
-        }
-        CU(h, cudaLaunchKernelEx(&cfg, kernel, ca));
-    } else {
-        auto kernel = lily::cluster_rows_kernel<__nv_bfloat16>;
-        const int32_t st = raise_smem_limit(h, kernel, 1u << 9);
-        if (st != LILY_OK) {
-            return st;
-        }
-        CU(h, cudaLaunchKernelEx(&cfg, kernel, ca));
-    }
+template <uint32_t MAXR>
+int32_t launch_split(lily_sampler *h, cudaStream_t stream, lily::SplitArgs<MAXR> &sa, const SplitPlan &p,
+                     uint32_t rows, uint32_t dtype) {
+    sa.log_blocks = p.log_blocks;
+    sa.mark_mode = p.mark_mode;
+    sa.mark_words = p.mark_words;
+    sa.share = p.share ? 1u : 0u;
+    sa.spill_params = reinterpret_cast<lily_sampling_params_t *>(h->spill);
+    sa.spill_steps = reinterpret_cast<uint32_t *>(h->spill + INLINE_ROWS_MAX * sizeof(lily_sampling_params_t));
+    sa.spill_slots = sa.spill_steps + INLINE_ROWS_MAX;
+    sa.spill_history = sa.spill_slots + INLINE_ROWS_MAX;
+    CU(h, lily::split_launch<MAXR>(sa, rows, dtype, p.smem, h->max_smem, &h->attr_mask, stream));
     return LILY_OK;
 }
 
+// The row kernel with host parameters in its arguments. sa.a is complete but for
+// params, steps and slots, which come as host arrays.
+template <uint32_t MAXR>
+int32_t launch_split_inline(lily_sampler *h, cudaStream_t stream, const lily::KArgs &a, const SplitPlan &p,
+                            uint32_t rows, uint32_t dtype, const lily_sampling_params_t *params,
+                            const uint32_t *steps, const uint32_t *slots, uint32_t inline_history = 0,
+                            uint32_t grid_rows = 0) {
+    lily::SplitArgs<MAXR> sa;
+    sa.a = a;
+    sa.a.params = nullptr;
+    sa.a.steps = nullptr;
+    sa.a.count_slots = nullptr;
+    sa.inline_params = 1;
+    sa.inline_slots = slots != nullptr ? 1u : 0u;
+    sa.inline_history = inline_history;
+    for (uint32_t r = 0; r < rows; ++r) {
+        sa.in[r] = lily::row_in(params[r], steps != nullptr ? steps[r] : 0u);
+    }
+    if (slots != nullptr) {
+        std::memcpy(sa.slots, slots, sizeof(uint32_t) * rows);
+    }
+    return launch_split(h, stream, sa, p, grid_rows ? grid_rows : rows, dtype);
+}
+
 int32_t launch(lily_sampler *h, cudaStream_t stream, const lily::KArgs &a, uint32_t rows,
-               uint32_t dtype) {
+               uint32_t dtype, bool slices = false) {
     const size_t smem = smem_bytes(a.vocab, a.n_slices);
     if (smem > (size_t)h->max_smem) {
         return fail(h, LILY_ERR_CAPACITY, "vocabulary too large for the shared-memory bitmap");
     }
-    const bool plain = a.cand_out == nullptr && a.merge_in == nullptr && a.spec.n_spec == 0u &&
-                       a.extra_len == 0u;
-    if (cluster_call(h, a.logits, a.logits_ld, dtype, rows, plain)) {
-        lily::ClusterArgs ca;
-        std::memset(&ca, 0, sizeof(ca));
-        ca.a = a;
-        return launch_cluster(h, stream, ca, rows, dtype);
+    // (Parameters on the device: their penalties are not known here.)
+    const SplitPlan plan = split_plan(h, a, rows, dtype,
+                                      (a.history_ids != nullptr && a.count_slots == nullptr) || a.extra_len != 0u ||
+                                          a.bias_ids != nullptr || a.ban_ids != nullptr,
+                                      !a.force_greedy);
+    if (plan.take && !slices) {
+        lily::SplitArgs<INLINE_ROWS> sa;
+        sa.a = a;
+        sa.inline_params = sa.inline_slots = sa.inline_history = 0;
+        return launch_split(h, stream, sa, plan, rows, dtype);
     }
     const size_t esize = dtype == LILY_F32 ? 4 : 2;
     const bool vec = (reinterpret_cast<uintptr_t>(a.logits) % 16u == 0u) &&
@@ -515,8 +526,8 @@ int32_t lily_sampler_create(int32_t device, uint32_t vocab, uint32_t max_rows,
     if ((e = cudaMemset(h->tickets, 0, (size_t)max_rows * 4)) != cudaSuccess) {
         return bail(e, "tickets");
     }
-    if ((e = cudaMalloc(&h->spill, lily::CL_MAX_ROWS * (sizeof(lily_sampling_params_t) + 8))) != cudaSuccess) {
-        return bail(e, "parameter words of the small-batch kernel");
+    if ((e = cudaMalloc(&h->spill, INLINE_ROWS_MAX * (sizeof(lily_sampling_params_t) + 12))) != cudaSuccess) {
+        return bail(e, "parameter words of the row kernel");
     }
     if ((e = cudaMalloc(&h->status_word, 4)) != cudaSuccess ||
         (e = cudaMemset(h->status_word, 0, 4)) != cudaSuccess) {
@@ -844,10 +855,29 @@ int32_t lily_sample_batch(lily_sampler_t *h, void *stream_, const lily_sample_ar
     const uint32_t *d_steps = g.steps;
     const uint32_t *d_slots = nullptr;
     int slot = -1;
-    // A small batch's host parameters (and slots) travel in the kernel's own
-    // arguments: nothing is staged, no copy sits in front of the launch.
-    const bool in_args = !g.params_on_device && g.rows <= lily::CL_MAX_ROWS &&
-                         cluster_call(h, g.logits, g.logits_ld, g.logits_dtype, g.rows, true);
+    a.logits = g.logits;
+    a.logits_ld = g.logits_ld;
+    a.rows = g.rows;
+    // Host parameters (and slots) of up to INLINE_ROWS_MAX rows travel in the
+    // kernel's own arguments: nothing is staged, no copy sits in front of the launch.
+    SplitPlan plan;
+    bool raises_few = false;
+    if (!g.params_on_device && g.rows <= INLINE_ROWS_MAX) {
+        const bool history = g.history_ids != nullptr && g.count_slots == nullptr;
+        bool counts = false, raises = false;
+        for (uint32_t r = 0; r < g.rows; ++r) {
+            const lily_sampling_params_t &p = g.params[r];
+            counts = counts || p.frequency_penalty != 0.0f;
+            raises = raises || p.repetition_penalty < 1.0f || p.presence_penalty < 0.0f || p.frequency_penalty < 0.0f;
+        }
+        plan = split_plan(h, a, g.rows, g.logits_dtype, history || g.bias_ids != nullptr || g.ban_ids != nullptr,
+                          history && counts);
+        // (A few rows whose penalties can raise a logit, which the row kernel leaves to one
+        // block: the general kernel cuts them into slices.)
+        raises_few = raises && g.rows <= 16u;
+        plan.take = plan.take && !raises_few;
+    }
+    const bool in_args = plan.take;
     if (!in_args && (!g.params_on_device || g.count_slots != nullptr)) {
         st = next_stage(h, &slot);
         if (st != LILY_OK) {
@@ -888,9 +918,6 @@ int32_t lily_sample_batch(lily_sampler_t *h, void *stream_, const lily_sample_ar
         CU(h, cudaMemcpyAsync(h->d_stage[slot], h->h_stage[slot], h->layout.total,
                               cudaMemcpyHostToDevice, stream));
     }
-    a.logits = g.logits;
-    a.logits_ld = g.logits_ld;
-    a.rows = g.rows;
     a.params = d_params;
     a.uniforms = g.uniforms;
     a.steps = d_steps;
@@ -914,26 +941,69 @@ int32_t lily_sample_batch(lily_sampler_t *h, void *stream_, const lily_sample_ar
     a.kept_ld = g.kept_ld;
     a.n_slices = choose_slices(h, g.rows);
     if (in_args) {
-        lily::ClusterArgs ca;
-        std::memset(&ca, 0, sizeof(ca));
-        ca.a = a;
-        ca.a.params = nullptr;
-        ca.a.steps = nullptr;
-        ca.inline_params = 1;
-        std::memcpy(ca.params, g.params, sizeof(lily_sampling_params_t) * g.rows);
-        if (g.steps != nullptr) {
-            std::memcpy(ca.steps, g.steps, sizeof(uint32_t) * g.rows);
-        }
-        if (g.count_slots != nullptr) {
-            ca.inline_slots = 1;
-            std::memcpy(ca.slots, g.count_slots, sizeof(uint32_t) * g.rows);
-        }
-        return launch_cluster(h, stream, ca, g.rows, g.logits_dtype);
+        return g.rows <= INLINE_ROWS
+                   ? launch_split_inline<INLINE_ROWS>(h, stream, a, plan, g.rows, g.logits_dtype, g.params, g.steps,
+                                                      g.count_slots)
+                   : launch_split_inline<INLINE_ROWS_MAX>(h, stream, a, plan, g.rows, g.logits_dtype, g.params,
+                                                          g.steps, g.count_slots);
     }
-    st = launch(h, stream, a, g.rows, g.logits_dtype);
+    st = launch(h, stream, a, g.rows, g.logits_dtype, raises_few);
     if (slot >= 0) {
         CU(h, cudaEventRecord(h->ev[slot], stream));
     }
+    return st;
+}
+
+int32_t lily_sample_one(lily_sampler_t *h, void *stream_, const void *logits, uint32_t logits_dtype,
+                        uint64_t logits_len, const lily_sampling_params_t *params, uint32_t step,
+                        const uint32_t *history_ids, uint32_t history_len, uint32_t *out_id) {
+    int32_t st = check_handle(h);
+    if (st != LILY_OK) {
+        return st;
+    }
+    if (logits == nullptr || out_id == nullptr || params == nullptr || logits_len < h->vocab ||
+        logits_dtype > LILY_BF16) {
+        return fail(h, LILY_ERR_ARG, "logits must be F32 or BF16 [ld >= vocab]; out and params set");
+    }
+    if (history_len > 0u && history_ids == nullptr) {
+        return fail(h, LILY_ERR_ARG, "history_len without history_ids");
+    }
+    if (!params_ok(*params)) {
+        return fail(h, LILY_ERR_PARAMS, "row 0: invalid sampling parameters");
+    }
+    DeviceGuard guard(h->device);
+    cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+    lily::KArgs a;
+    base_args(h, &a);
+    a.logits = logits;
+    a.logits_ld = logits_len;
+    a.rows = 1;
+    a.history_ids = history_ids;
+    a.history_ld = history_len;
+    a.out_ids = out_id;
+    a.n_slices = choose_slices(h, 1u);
+    const bool raises = params->repetition_penalty < 1.0f || params->presence_penalty < 0.0f ||
+                        params->frequency_penalty < 0.0f;
+    const SplitPlan plan = split_plan(h, a, 1u, logits_dtype, history_ids != nullptr, params->frequency_penalty != 0.0f);
+    if (plan.take && !raises) {
+        return launch_split_inline<INLINE_ROWS>(h, stream, a, plan, 1u, logits_dtype, params, &step, nullptr,
+                                                1u + history_len);
+    }
+    int slot = -1;
+    st = next_stage(h, &slot);
+    if (st != LILY_OK) {
+        return st;
+    }
+    char *hs = h->h_stage[slot], *ds = h->d_stage[slot];
+    std::memcpy(hs + h->layout.params, params, sizeof(*params));
+    std::memcpy(hs + h->layout.steps, &step, 4);
+    std::memcpy(hs + h->layout.hist_len, &history_len, 4);
+    CU(h, cudaMemcpyAsync(ds, hs, h->layout.total, cudaMemcpyHostToDevice, stream));
+    a.params = reinterpret_cast<const lily_sampling_params_t *>(ds + h->layout.params);
+    a.steps = reinterpret_cast<const uint32_t *>(ds + h->layout.steps);
+    a.history_len = history_ids ? reinterpret_cast<const uint32_t *>(ds + h->layout.hist_len) : nullptr;
+    st = launch(h, stream, a, 1u, logits_dtype, true);
+    CU(h, cudaEventRecord(h->ev[slot], stream));
     return st;
 }
 
@@ -1533,39 +1603,14 @@ int32_t lily_spec_verify(lily_sampler_t *h, void *stream_, const lily_spec_args_
     }
     DeviceGuard guard(h->device);
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-    int slot = -1;
-    st = next_stage(h, &slot);
-    if (st != LILY_OK) {
-        return st;
-    }
-    char *hs = h->h_stage[slot];
-    auto *sp = reinterpret_cast<lily_sampling_params_t *>(hs + h->layout.params);
-    auto *ss = reinterpret_cast<uint32_t *>(hs + h->layout.steps);
-    auto *sl = reinterpret_cast<uint32_t *>(hs + h->layout.slots);
-    auto *sh = reinterpret_cast<uint32_t *>(hs + h->layout.hist_len);
-    for (uint32_t j = 0; j < g.m; ++j) {
-        sp[j] = p;
-        ss[j] = g.step0 + j;
-        sl[j] = g.count_slot ? *g.count_slot : 0u;
-        sh[j] = g.history_len;
-    }
-    CU(h, cudaMemcpyAsync(h->d_stage[slot], hs, h->layout.total, cudaMemcpyHostToDevice, stream));
-    char *ds = h->d_stage[slot];
-
     lily::KArgs a;
     base_args(h, &a);
     a.logits = g.target_logits;
     a.logits_ld = g.logits_ld;
     a.rows = g.m;
-    a.params = reinterpret_cast<const lily_sampling_params_t *>(ds + h->layout.params);
     a.uniforms = g.u_accept;
-    a.steps = reinterpret_cast<const uint32_t *>(ds + h->layout.steps);
     a.history_ids = g.history_ids;
-    a.history_len = g.history_ids ? reinterpret_cast<const uint32_t *>(ds + h->layout.hist_len)
-                                  : nullptr;
     a.history_ld = 0;  // every row of the step reads the same list
-    a.count_slots = g.count_slot ? reinterpret_cast<const uint32_t *>(ds + h->layout.slots)
-                                 : nullptr;
     a.out_ids = g.out_ids;
     a.out_status = g.out_status;
     if (spec_rows) {
@@ -1578,23 +1623,51 @@ int32_t lily_spec_verify(lily_sampler_t *h, void *stream_, const lily_spec_args_
         a.spec.u_resid = g.u_resid;
         a.spec.n_spec = g.m - 1u;
     }
-    if (!pen) {
-        // Without penalties the rows do not depend on one another.
-        a.n_slices = choose_slices(h, g.m);
-        st = launch(h, stream, a, g.m, g.logits_dtype);
-    } else {
-        // Row j's penalties see the draws of rows < j (the reference's rows
-        // share one histogram, src/qwen4exp/model.rs:3008-3012): one launch
-        // per row, in stream order.
-        a.n_slices = choose_slices(h, 1u);
-        for (uint32_t j = 0; j < g.m && st == LILY_OK; ++j) {
-            a.row0 = j;
-            if (g.count_slot == nullptr) {
-                a.extra_ids = g.out_ids;
-                a.extra_len = j;
-            }
-            st = launch(h, stream, a, 1u, g.logits_dtype);
+    // Without penalties the rows do not depend on one another. With them row j's see
+    // the draws of rows < j (the reference's rows share one histogram,
+    // src/qwen4exp/model.rs:3008-3012): one launch per row, in stream order.
+    const uint32_t launches = pen ? g.m : 1u, rows = pen ? 1u : g.m;
+    a.n_slices = choose_slices(h, rows);
+    const bool listed = g.count_slot == nullptr && pen;
+    const bool raises = p.repetition_penalty < 1.0f || p.presence_penalty < 0.0f || p.frequency_penalty < 0.0f;
+    const SplitPlan plan = split_plan(h, a, rows, g.logits_dtype, listed, p.frequency_penalty != 0.0f);
+    const bool in_args = plan.take && !raises;
+    lily_sampling_params_t params[8];
+    uint32_t steps[8], slots[8];
+    for (uint32_t j = 0; j < g.m; ++j) {
+        params[j] = p;
+        steps[j] = g.step0 + j;
+        slots[j] = g.count_slot ? *g.count_slot : 0u;
+    }
+    int slot = -1;
+    if (!in_args) {
+        st = next_stage(h, &slot);
+        if (st != LILY_OK) {
+            return st;
         }
+        char *hs = h->h_stage[slot], *ds = h->d_stage[slot];
+        auto *sh = reinterpret_cast<uint32_t *>(hs + h->layout.hist_len);
+        std::memcpy(hs + h->layout.params, params, sizeof(params[0]) * g.m);
+        std::memcpy(hs + h->layout.steps, steps, 4u * g.m);
+        std::memcpy(hs + h->layout.slots, slots, 4u * g.m);
+        for (uint32_t j = 0; j < g.m; ++j) {
+            sh[j] = g.history_len;
+        }
+        CU(h, cudaMemcpyAsync(ds, hs, h->layout.total, cudaMemcpyHostToDevice, stream));
+        a.params = reinterpret_cast<const lily_sampling_params_t *>(ds + h->layout.params);
+        a.steps = reinterpret_cast<const uint32_t *>(ds + h->layout.steps);
+        a.history_len = g.history_ids ? reinterpret_cast<const uint32_t *>(ds + h->layout.hist_len) : nullptr;
+        a.count_slots = g.count_slot ? reinterpret_cast<const uint32_t *>(ds + h->layout.slots) : nullptr;
+    }
+    for (uint32_t j = 0; j < launches && st == LILY_OK; ++j) {
+        a.row0 = j;
+        if (listed) {
+            a.extra_ids = g.out_ids;
+            a.extra_len = j;
+        }
+        st = in_args ? launch_split_inline<INLINE_ROWS>(h, stream, a, plan, pen ? j + 1u : g.m, g.logits_dtype, params,
+                                                        steps, g.count_slot ? slots : nullptr, 1u + g.history_len, rows)
+                     : launch(h, stream, a, rows, g.logits_dtype, true);
     }
     if (st == LILY_OK) {
         if (g.m > 1u) {
@@ -1605,7 +1678,9 @@ int32_t lily_spec_verify(lily_sampler_t *h, void *stream_, const lily_spec_args_
         }
         CU(h, cudaGetLastError());
     }
-    CU(h, cudaEventRecord(h->ev[slot], stream));
+    if (slot >= 0) {
+        CU(h, cudaEventRecord(h->ev[slot], stream));
+    }
     return st;
 }
 

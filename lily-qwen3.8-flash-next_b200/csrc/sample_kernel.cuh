@@ -164,12 +164,14 @@ struct RowCtx {
     const uint32_t *ban_ids;
     uint32_t ban_len;
     bool sp_in_smem;
+    bool count_draw;         // the draw is added to a histogram slot (src/kernels/metal/sample.metal:509-511)
+    uint32_t slot;
 };
 
 struct alignas(16) SmemFixed {
     uint32_t key[CAP];    // candidates: adjusted keys below n_adj, raw logit bits above;
     uint32_t id[CAP];     //   during the first round key+id hold the 8192-bin histogram
-    uint32_t tkey[KCAP];  // select's histogram / staging; later the candidates' p
+    alignas(16) uint32_t tkey[KCAP];  // select's histogram / staging; later the candidates' p
     uint32_t tid[KCAP];   // select's histogram / staging; later the prefix sums
     uint32_t thist[TH_BINS];
     uint32_t warp_sums[NT / 32];
@@ -202,9 +204,10 @@ struct alignas(16) SmemFixed {
     uint32_t *cid;
     uint32_t ccap;
     float u_draw;         // the row's uniform, fetched (or derived) when the block starts
+    uint32_t step_draw;   // the row's draw index (0 when the uniforms are given)
     uint32_t lean_abort;  // stream_rows_kernel: a thread saw a NaN before the threshold was taken
     alignas(8) unsigned long long mbar[2];  // stream_rows_kernel: history marked; thread maxima written
-    uint32_t lkey[LCAP];
+    alignas(16) uint32_t lkey[LCAP];
     uint32_t lid[LCAP];
     RowCtx ctx;  // the row's parameters, for the out-of-line helpers
 };
@@ -288,7 +291,7 @@ __device__ __forceinline__ bool is_special(const SmemFixed *sm, const RowCtx &c,
 // ban, division by the temperature, monotone key. `special`: the id is on
 // the bias / ban list (the up-front pass only; the stream skips those ids).
 // A NaN marks the row as failed.
-__device__ __noinline__ uint32_t adjusted_key(SmemFixed *sm, uint32_t id, float l, bool special) {
+static __device__ __noinline__ uint32_t adjusted_key(SmemFixed *sm, uint32_t id, float l, bool special) {
     const RowCtx &c = sm->ctx;
     float x = l;
     bool banned = false;
@@ -328,7 +331,7 @@ __device__ __noinline__ uint32_t adjusted_key(SmemFixed *sm, uint32_t id, float 
 // The stream pushes raw logits; before a selection looks at the buffer, the
 // entries pushed since the last one, [n_adj, n), become adjusted keys, all
 // threads at once.
-__device__ __noinline__ void adjust_pending(SmemFixed *sm) {
+static __device__ __noinline__ void adjust_pending(SmemFixed *sm) {
     const uint32_t n = min(sm->n, CAP);
     const uint32_t from = sm->n_adj;
     for (uint32_t i = from + threadIdx.x; i < n; i += NT) {
@@ -344,7 +347,7 @@ __device__ __noinline__ void adjust_pending(SmemFixed *sm) {
 // End of the stream: adjusts what is still raw and keeps only the entries
 // whose key reaches the threshold (at least k of them do), compacted to the
 // front in chunks so that no entry is overwritten before it is read.
-__device__ __noinline__ void filter_adjust(SmemFixed *sm) {
+static __device__ __noinline__ void filter_adjust(SmemFixed *sm) {
     const uint32_t tid = threadIdx.x;
     const uint32_t n = min(sm->n, sm->ccap);
     const uint32_t from = sm->n_adj;
@@ -458,7 +461,7 @@ __device__ __forceinline__ void find_bin(SmemFixed *sm, const uint32_t *hist, ui
 // is the rank wanted inside that value's ties, *count_eq_out how many
 // entries hold the value.
 template <bool BY_ID>
-__device__ __noinline__ uint32_t adaptive_select(SmemFixed *sm, uint32_t n, uint32_t remaining, uint32_t kstar,
+static __device__ __noinline__ uint32_t adaptive_select(SmemFixed *sm, uint32_t n, uint32_t remaining, uint32_t kstar,
                                     uint32_t *remaining_out, uint32_t *count_eq_out) {
     const uint32_t tid = threadIdx.x;
     uint32_t *hist = sm->tkey;  // SEL_BINS words: tkey and tid are adjacent
@@ -535,7 +538,7 @@ __device__ __noinline__ uint32_t adaptive_select(SmemFixed *sm, uint32_t n, uint
 
 // Keeps the best k of the n buffered candidates (n > k), by key descending
 // then id ascending, in slots [0, k) in any order; records the k-th key.
-__device__ __noinline__ void select_topk(SmemFixed *sm, uint32_t n, uint32_t k) {
+static __device__ __noinline__ void select_topk(SmemFixed *sm, uint32_t n, uint32_t k) {
     const uint32_t tid = threadIdx.x;
     uint32_t remaining = 0, count_eq = 0;
     const uint32_t kstar = adaptive_select<false>(sm, n, k, 0u, &remaining, &count_eq);
@@ -591,7 +594,7 @@ __device__ __noinline__ void select_topk(SmemFixed *sm, uint32_t n, uint32_t k) 
 
 // The largest raw logit c whose plain key does not beat kstar: an untouched
 // logit l beats the k-th candidate exactly when l > c. Thread 0 only.
-__device__ __noinline__ float raw_threshold(uint32_t kstar, float T, bool argmax_mode) {
+static __device__ __noinline__ float raw_threshold(uint32_t kstar, float T, bool argmax_mode) {
     const float tq = float_of_key(kstar);
     if (tq != tq) {
         return tq;
@@ -640,7 +643,7 @@ struct Team {
 
 // Bitonic sort of slots [0, n) by (key descending, id ascending).
 template <bool SMALL>
-__device__ __noinline__ void sort_candidates(SmemFixed *sm, uint32_t n) {
+static __device__ __noinline__ void sort_candidates(SmemFixed *sm, uint32_t n) {
     const uint32_t me = Team<SMALL>::rank(), team = Team<SMALL>::size();
     uint32_t P = 1;
     while (P < n) {
@@ -685,7 +688,7 @@ __device__ __forceinline__ unsigned long long sort_exchange(unsigned long long v
     return keep_first ? (v > other ? v : other) : (v < other ? v : other);
 }
 
-__device__ __noinline__ void sort_block_2k(SmemFixed *sm, uint32_t n) {
+static __device__ __noinline__ void sort_block_2k(SmemFixed *sm, uint32_t n) {
     const uint32_t t = threadIdx.x;
     unsigned long long *buf = reinterpret_cast<unsigned long long *>(sm->key);
     unsigned long long v[4];
@@ -769,7 +772,7 @@ __device__ __forceinline__ void pick(SmemFixed *sm, const float *cum, uint32_t n
 // Steps 6-8 on the sorted candidates [0, n): softmax weights, sequential
 // prefix, cut, draw (plain or speculative), outputs.
 template <bool SMALL>
-__device__ __noinline__ void finalize(SmemFixed *sm, const KArgs &a, uint32_t row, uint32_t n,
+static __device__ __noinline__ void finalize(SmemFixed *sm, const KArgs &a, uint32_t row, uint32_t n,
                                       uint64_t seed) {
     const RowCtx &c = sm->ctx;
     const uint32_t me = Team<SMALL>::rank(), team = Team<SMALL>::size();
@@ -808,15 +811,8 @@ __device__ __noinline__ void finalize(SmemFixed *sm, const KArgs &a, uint32_t ro
         }
         return;
     }
-    // The uniform is fetched early: its latency hides behind the prefix sums.
-    float u;
-    uint32_t step = 0;
-    if (a.uniforms) {
-        u = a.uniforms[row];
-    } else {
-        step = a.steps ? a.steps[row] : 0u;
-        u = uniform_for(seed, step);
-    }
+    const float u = sm->u_draw;
+    const uint32_t step = sm->step_draw;
     for (uint32_t i = me; i < n; i += team) {
         p[i] = exp_f32(__fsub_rn(float_of_key(sm->key[i]), top));
     }
@@ -936,14 +932,10 @@ __device__ __noinline__ void finalize(SmemFixed *sm, const KArgs &a, uint32_t ro
         if (a.out_status) {
             a.out_status[out_row] = LILY_ROW_OK;
         }
-        if (c.use_pen && a.count_slots) {
+        if (c.count_draw && chosen_id < a.vocab) {
             // src/kernels/metal/sample.metal:509-511: the draw is counted.
-            const uint32_t slot = a.count_slots[row];
-            if (chosen_id < a.vocab) {
-                atomicAdd(a.counts_table + (uint64_t)slot * a.vocab + chosen_id, 1u);
-                atomicOr(a.seen_table + (uint64_t)slot * a.seen_words + (chosen_id >> 5),
-                         1u << (chosen_id & 31u));
-            }
+            atomicAdd(a.counts_table + (uint64_t)c.slot * a.vocab + chosen_id, 1u);
+            atomicOr(a.seen_table + (uint64_t)c.slot * a.seen_words + (chosen_id >> 5), 1u << (chosen_id & 31u));
         }
     }
 }
@@ -954,7 +946,7 @@ __device__ __noinline__ void finalize(SmemFixed *sm, const KArgs &a, uint32_t ro
 // reference (tests/unit/kernels/sample.rs:37-46): every lane runs the same
 // chain of adds over values handed round by shuffles, which do not sit on the
 // chain.
-__device__ __noinline__ void finalize_warp(SmemFixed *sm, const KArgs &a, uint32_t row, uint32_t n,
+static __device__ __noinline__ void finalize_warp(SmemFixed *sm, const KArgs &a, uint32_t row, uint32_t n,
                                            uint64_t seed) {
     const RowCtx &c = sm->ctx;
     const uint32_t lane = threadIdx.x & 31u;
@@ -1060,14 +1052,10 @@ __device__ __noinline__ void finalize_warp(SmemFixed *sm, const KArgs &a, uint32
         if (a.out_status) {
             a.out_status[row] = LILY_ROW_OK;
         }
-        if (c.use_pen && a.count_slots) {
+        if (c.count_draw && chosen_id < a.vocab) {
             // src/kernels/metal/sample.metal:509-511: the draw is counted.
-            const uint32_t slot = a.count_slots[row];
-            if (chosen_id < a.vocab) {
-                atomicAdd(a.counts_table + (uint64_t)slot * a.vocab + chosen_id, 1u);
-                atomicOr(a.seen_table + (uint64_t)slot * a.seen_words + (chosen_id >> 5),
-                         1u << (chosen_id & 31u));
-            }
+            atomicAdd(a.counts_table + (uint64_t)c.slot * a.vocab + chosen_id, 1u);
+            atomicOr(a.seen_table + (uint64_t)c.slot * a.seen_words + (chosen_id >> 5), 1u << (chosen_id & 31u));
         }
     }
 }
@@ -1109,7 +1097,7 @@ __device__ __forceinline__ void set_raw_edge(SmemFixed *sm, uint32_t edge_key) {
 // One warp tightens the threshold from the histogram of the raw keys pushed
 // so far: the highest bin edge that at least k counted (untouched) logits
 // reach. Only the bins at and above the current threshold can matter.
-__device__ __noinline__ void tighten(SmemFixed *sm) {
+static __device__ __noinline__ void tighten(SmemFixed *sm) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t k = sm->ctx.k;
     const uint32_t base = sm->th_base;
@@ -1160,7 +1148,7 @@ __device__ __noinline__ void tighten(SmemFixed *sm) {
 
 // Exact best-k of n <= RANKSORT_MAX buffered candidates by counting, for
 // each, how many others come before it: the best k land sorted in [0, k).
-__device__ __noinline__ void rank_sort(SmemFixed *sm, uint32_t n, uint32_t k) {
+static __device__ __noinline__ void rank_sort(SmemFixed *sm, uint32_t n, uint32_t k) {
     const uint32_t tid = threadIdx.x;
     uint32_t rank = 0xFFFFFFFFu, mk = 0, mi = 0;
     if (tid < n) {
@@ -1390,7 +1378,7 @@ __device__ __forceinline__ uint32_t process_frag(SmemFixed *sm, const RowCtx &c,
 
 // Block-wide: adjusts what the stream pushed, keeps the exact best k and
 // raises the threshold to the k-th key.
-__device__ __noinline__ void compact(SmemFixed *sm) {
+static __device__ __noinline__ void compact(SmemFixed *sm) {
     adjust_pending(sm);
     const uint32_t n = min(sm->n, CAP);
     const uint32_t k = sm->ctx.k;
@@ -1451,7 +1439,7 @@ __device__ __forceinline__ void lean_write_slot(uint32_t at, const Frag &f) {
 // m2, m3, m4, r2 | r3 << 16): pass 2 then needs the row again only where a
 // second or further fragment of a thread also beats the threshold.
 template <typename T>
-__device__ __noinline__ Pass1 lean_pass1(uint32_t slot_a, uint32_t slot_b, const char *src0, uint32_t nfull,
+static __device__ __noinline__ Pass1 lean_pass1(uint32_t slot_a, uint32_t slot_b, const char *src0, uint32_t nfull,
                                          const uint4 *h4, uint32_t fused4, uint32_t *seen, uint32_t lo,
                                          uint32_t width, uint32_t tab) {
     constexpr uint32_t NONE = 0xFFFFFFFFu;
@@ -1560,7 +1548,7 @@ __device__ __forceinline__ void lean_take(SmemFixed *sm, const Frag &cur, uint32
 // Returns which of the steps the thread took (bit 0: second fragment read,
 // bit 1: third, bit 2: the walk over all rounds), for the phase trace.
 template <typename T>
-__device__ __noinline__ uint32_t lean_pass2(SmemFixed *sm, const char *src0, uint32_t nfull, uint32_t base0,
+static __device__ __noinline__ uint32_t lean_pass2(SmemFixed *sm, const char *src0, uint32_t nfull, uint32_t base0,
                                             float c_fix, uint32_t slot_keep, uint32_t tab, float m1,
                                             uint32_t r1) {
     constexpr uint32_t NONE = 0xFFFFFFFFu;
@@ -1826,6 +1814,8 @@ __device__ __forceinline__ void sample_row(const KArgs &a, const uint32_t row, c
     c.seen = seen;
     const bool table_mode = a.count_slots != nullptr;
     const uint32_t slot = table_mode ? slot_row : 0u;
+    c.count_draw = c.use_pen && table_mode;
+    c.slot = slot;
     uint32_t *counts_rw = nullptr;
     if (c.need_counts) {
         counts_rw = table_mode ? a.counts_table + (uint64_t)slot * a.vocab
@@ -1969,6 +1959,7 @@ __device__ __forceinline__ void sample_row(const KArgs &a, const uint32_t row, c
         sm->cid = sm->id;
         sm->ccap = CAP;
         sm->u_draw = a.uniforms ? u_row : uniform_for(P.seed, step_row);
+        sm->step_draw = step_row;
         sm->lean_abort = 0;
     }
     if (c.use_pen) {
@@ -2761,9 +2752,9 @@ __global__ void __launch_bounds__(NT, 2) sample_rows_kernel(const __grid_constan
 
 // The whole row in one block, out of line: what stream_rows_kernel calls for a
 // row it does not take itself.
-template <typename T>
-__device__ __noinline__ void sample_whole_row(const KArgs &a, uint32_t row) {
-    sample_row<T, true>(a, row, 0u);
+template <typename T, bool VEC = true>
+static __device__ __noinline__ void sample_whole_row(const KArgs &a, uint32_t row) {
+    sample_row<T, VEC>(a, row, 0u);
 }
 
 // The draw of a vocabulary-sharded row: the shards' records hold every
@@ -2772,7 +2763,7 @@ __device__ __noinline__ void sample_whole_row(const KArgs &a, uint32_t row) {
 // what one pass over the whole vocabulary gives. One block per row.
 __device__ __forceinline__ void peer_exchange_row(const KArgs &a, uint32_t row);
 
-__global__ void __launch_bounds__(NT, 2) merge_rows_kernel(const __grid_constant__ KArgs a) {
+static __global__ void __launch_bounds__(NT, 2) merge_rows_kernel(const __grid_constant__ KArgs a) {
     extern __shared__ uint4 smem_raw[];
     SmemFixed *sm = reinterpret_cast<SmemFixed *>(smem_raw);
     const uint32_t tid = threadIdx.x;
@@ -2801,10 +2792,13 @@ __global__ void __launch_bounds__(NT, 2) merge_rows_kernel(const __grid_constant
         c.bias_vals = nullptr;
         c.bias_len = c.ban_len = 0;
         c.sp_in_smem = true;
+        c.count_draw = false;
+        c.slot = 0;
         sm->ctx = c;
         sm->n = 0;
         sm->err = 0;
         sm->u_draw = a.uniforms ? a.uniforms[row] : uniform_for(P.seed, a.steps ? a.steps[row] : 0u);
+        sm->step_draw = 0;
         sm->ckey = sm->key;
         sm->cid = sm->id;
         sm->ccap = CAP;
@@ -2987,7 +2981,7 @@ __device__ __forceinline__ void peer_raise(void *buffer, uint32_t max_rows, uint
 // every row there. (The merge kernel does the same for its own row when it is
 // given the records; this kernel serves a rank that publishes apart from its
 // merge, and one GPU that plays several ranks in a test.)
-__global__ void __launch_bounds__(256) shard_publish_kernel(const __grid_constant__ PeerArgs p) {
+static __global__ void __launch_bounds__(256) shard_publish_kernel(const __grid_constant__ PeerArgs p) {
     void *buffer = p.buffers[blockIdx.x];
     const uint2 *src = reinterpret_cast<const uint2 *>(p.records);
     uint2 *dst = reinterpret_cast<uint2 *>(peer_slot(buffer, p.n_shards, p.max_rows, p.step, p.rank));
@@ -3047,7 +3041,7 @@ __device__ __forceinline__ void peer_exchange_row(const KArgs &a, uint32_t row) 
 }
 
 // src/kernels/metal/spec.metal:14-38, one thread.
-__global__ void spec_accept_kernel(const uint32_t *draws, const uint32_t *ids, uint32_t id_offset,
+static __global__ void spec_accept_kernel(const uint32_t *draws, const uint32_t *ids, uint32_t id_offset,
                                    uint32_t m, uint32_t *ctrl, uint32_t pos0, uint32_t ratio,
                                    uint32_t chain, uint32_t stride) {
     if (blockIdx.x != 0 || threadIdx.x != 0) {
@@ -3074,7 +3068,7 @@ __global__ void spec_accept_kernel(const uint32_t *draws, const uint32_t *ids, u
 }
 
 // Histogram-slot maintenance (src/kernels/sample.rs:145-174).
-__global__ void uncount_kernel(uint32_t *counts, uint32_t *seen, uint32_t vocab, uint32_t token) {
+static __global__ void uncount_kernel(uint32_t *counts, uint32_t *seen, uint32_t vocab, uint32_t token) {
     if (blockIdx.x != 0 || threadIdx.x != 0 || token >= vocab) {
         return;
     }
@@ -3087,7 +3081,7 @@ __global__ void uncount_kernel(uint32_t *counts, uint32_t *seen, uint32_t vocab,
     }
 }
 
-__global__ void rebuild_seen_kernel(const uint32_t *counts, uint32_t *seen, uint32_t vocab) {
+static __global__ void rebuild_seen_kernel(const uint32_t *counts, uint32_t *seen, uint32_t vocab) {
     const uint32_t w = blockIdx.x * blockDim.x + threadIdx.x;
     if (w * 32u >= vocab) {
         return;
@@ -3102,7 +3096,7 @@ __global__ void rebuild_seen_kernel(const uint32_t *counts, uint32_t *seen, uint
     seen[w] = bits;
 }
 
-__global__ void exp_kernel(const float *in, float *out, uint64_t n) {
+static __global__ void exp_kernel(const float *in, float *out, uint64_t n) {
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (uint64_t)gridDim.x * blockDim.x) {
         out[i] = exp_f32(in[i]);

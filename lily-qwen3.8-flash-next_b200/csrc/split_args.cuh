@@ -1,0 +1,145 @@
+// What the row kernel (split_kernel.cuh) and its host side share: constants, the
+// kernel's arguments, the sizes of its shared memory.
+#pragma once
+
+#include <math.h>
+
+#include "sample_kernel.cuh"
+
+namespace lily {
+
+constexpr uint32_t SPL_NT = 256;         // threads at work; the other half of the block waits for a row of the general code
+constexpr uint32_t SPL_WARPS = SPL_NT / 32;
+// Vectors of a bucket: a thread's loads in flight (with two blocks per SM as many
+// as 64 registers a thread hold).
+__host__ __device__ constexpr uint32_t split_u(int bps) { return bps == 1 ? 10u : 6u; }
+constexpr uint32_t SPL_MAX_BLOCKS = 8;   // blocks of a cluster (the portable size)
+constexpr uint32_t SPL_SMALL_K = 64;     // up to here a block's bound is its own; finalize_warp's limit
+constexpr uint32_t SPL_POOL = 256;       // keys in the pool a narrow row's bound is taken from
+constexpr uint32_t SPL_HITS = 512;       // vectors of a block that may reach the bound
+constexpr uint32_t SPL_FLAGGED = 2048;   // buckets that may reach the bound
+constexpr uint32_t SPL_SORTED = 2048;    // candidates of a wide row
+constexpr uint32_t SPL_MIN_TILES = SPL_WARPS;  // a block has at least a piece per warp
+constexpr uint32_t SPL_COUNT_MAX = 32767;      // of an id in a history list (a mark's top bit says "on a list")
+constexpr uint32_t SPL_NAN_KEY = 0xFFFFFFFFu;  // a candidate that came out a NaN
+
+// How a block keeps the history ids of its share.
+enum { MARK_BITS = 0, MARK_BYTES = 1, MARK_COUNTS = 2 };
+
+template <typename T>
+struct Piece {
+    static constexpr uint32_t PER = 16u / (uint32_t)sizeof(T);    // logits per vector
+    static constexpr uint32_t SHIFT = sizeof(T) == 4 ? 7u : 8u;   // log2 of the logits per piece (32 vectors)
+    static constexpr uint32_t LOGITS = 1u << SHIFT;
+};
+
+// A row's parameters as the kernel uses them.
+struct RowIn {
+    float temp, rep, presence, frequency, top_p, min_p;
+    uint32_t k, flags;
+    float u;        // the row's uniform, unless the caller gave an array of them
+    uint32_t step;
+    uint64_t seed;
+};
+enum { ROW_GREEDY = 1, ROW_PEN = 2, ROW_COUNTS = 4, ROW_RAISES = 8, ROW_BAD = 16 };
+
+__host__ __device__ inline bool split_finite(float x) { return x - x == 0.0f; }
+
+__host__ __device__ inline RowIn row_in(const lily_sampling_params_t &P, uint32_t step) {
+    RowIn r;
+    // src/kernels/sample.rs:57-79 validate, :83-94 effective.
+    const bool ok = split_finite(P.temperature) && split_finite(P.top_p) && split_finite(P.min_p) &&
+                    split_finite(P.repetition_penalty) && split_finite(P.presence_penalty) &&
+                    split_finite(P.frequency_penalty) && P.temperature >= 0.0f && P.top_p > 0.0f &&
+                    P.top_p <= 1.0f && P.min_p >= 0.0f && P.min_p <= 1.0f && P.repetition_penalty > 0.0f;
+    const bool greedy = P.temperature <= 0.0f || P.top_k == 1u;
+    const bool pen = P.presence_penalty != 0.0f || P.frequency_penalty != 0.0f || P.repetition_penalty != 1.0f;
+    // (A negative zero counts as "can raise", as the general code has it.)
+    const bool raises = P.repetition_penalty < 1.0f || signbit(P.presence_penalty) || signbit(P.frequency_penalty);
+    r.temp = greedy ? 1.0f : P.temperature;
+    r.rep = P.repetition_penalty;
+    r.presence = P.presence_penalty;
+    r.frequency = P.frequency_penalty;
+    r.top_p = P.top_p;
+    r.min_p = P.min_p;
+    r.k = greedy ? 1u : (P.top_k == 0u || P.top_k > KCAP ? KCAP : P.top_k);
+    r.flags = (greedy ? ROW_GREEDY : 0) | (pen ? ROW_PEN : 0) | (P.frequency_penalty != 0.0f ? ROW_COUNTS : 0) |
+              (pen && raises ? ROW_RAISES : 0) | (ok ? 0 : ROW_BAD);
+    r.u = uniform_for(P.seed, step);
+    r.step = step;
+    r.seed = P.seed;
+    return r;
+}
+
+struct alignas(16) SplitSmem {
+    unsigned long long mbar_pool;    // every block's keys have arrived
+    unsigned long long mbar_cand;    // first block: every block's candidates have arrived
+    uint4 head[SPL_MAX_BLOCKS];      // first block: a block's number of candidates, flag, bound
+    union {
+        alignas(16) uint32_t pool[SPL_POOL];     // the best keys of every warp of the cluster
+        uint32_t tmax[SPL_MAX_BLOCKS * SPL_NT];  // wide rows: the keys of all its threads
+    };
+    uint32_t hit_at[SPL_HITS];       // vectors that reach the bound: the id of their first logit (mod 2^32)
+    uint16_t flagged[SPL_FLAGGED];
+    uint32_t n_flagged;
+    uint32_t n_hits;
+    uint32_t n_listed;               // ids on the row's bias list that are this block's
+    uint32_t n_sent;
+    uint32_t n_live;
+    uint32_t hard;                   // the row goes to the general code
+    uint32_t bin;
+    uint32_t verdict[2];             // what the waiting warps of the first block learn
+    uint32_t bound_key;
+    uint32_t pad;
+};
+static_assert(sizeof(SplitSmem) % 16u == 0u, "the arrays behind it are 16-byte aligned");
+
+// Parameters of up to MAXR rows travel in the kernel's own arguments: no staging
+// copy sits in front of the launch.
+template <uint32_t MAXR>
+struct SplitArgs {
+    KArgs a;
+    uint32_t log_blocks;      // log2 of the blocks per row
+    uint32_t mark_mode;
+    uint32_t mark_words;      // 32-bit words of the marks, a multiple of four
+    uint32_t share;           // the blocks of a row share its history list (else each looks at all of it)
+    uint32_t inline_params;   // `in` below is valid (else a.params / a.steps)
+    uint32_t inline_slots;
+    uint32_t inline_history;  // 1 + the history length of every row (0: a.history_len)
+    // Device words of the handle: where the first block puts what travelled here
+    // when it hands a row to the general code.
+    lily_sampling_params_t *spill_params;
+    uint32_t *spill_steps, *spill_slots, *spill_history;
+    RowIn in[MAXR];
+    // Keys that a warp gives to the pool of a row that keeps k: so much above its share
+    // that all but some three of the best k are in the pool. (What is missing there
+    // lowers the bound by as many places.)
+    __device__ __forceinline__ uint32_t rounds_of(uint32_t k) const {
+        const uint32_t share10 = (k * 10u) >> (3u + log_blocks);  // tenths
+        static_assert(SPL_WARPS == 8u, "");
+        return min((share10 * 13u + 170u) / 100u, SPL_POOL / (SPL_WARPS << log_blocks));
+    }
+    uint32_t slots[MAXR];
+};
+
+// Pieces of a row, and the most of them a block has.
+__host__ __device__ inline uint32_t split_pieces(uint32_t vocab, uint32_t skip, uint32_t per) {
+    const uint32_t piece = 32u * per;
+    return (vocab + skip + piece - 1u) / piece;
+}
+
+__host__ __device__ inline uint32_t split_buckets(uint32_t pieces_of_block, uint32_t u) {
+    return (pieces_of_block + SPL_WARPS * u - 1u) / (SPL_WARPS * u);
+}
+
+// Launches the kernel for a.a.rows rows from row0 on: logits of `dtype`, `smem` bytes of
+// dynamic shared memory (at most max_smem). `attr_mask`: bits of the kernels whose
+// limit has been raised, the caller's to keep per device. Instantiated for INLINE_ROWS
+// and INLINE_ROWS_MAX rows in split.cu.
+template <uint32_t MAXR>
+cudaError_t split_launch(const SplitArgs<MAXR> &a, uint32_t rows, uint32_t dtype, size_t smem, int max_smem,
+                         uint32_t *attr_mask, cudaStream_t stream);
+
+constexpr uint32_t INLINE_ROWS = 8, INLINE_ROWS_MAX = 64;  // rows whose parameters travel in the kernel's arguments
+
+}  // namespace lily

@@ -196,7 +196,7 @@ __device__ __forceinline__ float running_sum_total(SmemFixed *sm, const RunningS
 // The same sum by a second look at the row, for a row that went to the general
 // code (which leaves sum_exp at 0): every thread its strided share.
 template <typename T>
-__device__ __noinline__ float reread_sum(SmemFixed *sm, const T *row_ptr, uint32_t vocab, float scale, float top2) {
+static __device__ __noinline__ float reread_sum(SmemFixed *sm, const T *row_ptr, uint32_t vocab, float scale, float top2) {
     RunningSum rs{top2, 0.0f};
     for (uint32_t i = threadIdx.x; i < vocab; i += NT) {
         const float t = exp2f(fmaf(widen(row_ptr[i]), scale, -top2));
@@ -814,6 +814,11 @@ __global__ void __launch_bounds__(NT, StreamDepth<AHEAD>::BLOCKS) stream_rows_ke
         return;
     }
     if (tid < 32u) {
+        if (tid == 0) {
+            sm->ctx.count_draw = a.count_slots != nullptr && sm->ctx.use_pen;
+            sm->ctx.slot = a.count_slots ? a.count_slots[row] : 0u;
+        }
+        __syncwarp();
         finalize_warp(sm, a, row, n, P.seed);
         if (stamps && tid == 0) {
             stamps[PH_END] = global_ns();

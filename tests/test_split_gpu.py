@@ -1,0 +1,49 @@
+"""The row kernel (csrc/split_kernel.cuh) at the sizes where its cut of a row can
+go wrong, against the CPU oracle: vocabularies around a whole number of pieces
+and of buckets, rows that do not start on 16 bytes, every number of blocks per row,
+and every way of keeping the history. Ids and kept sets are exact, as everywhere."""
+import numpy as np
+import pytest
+
+from test_sampler_gpu import check, make_batch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def W(lily):
+    import workloads as w
+    return w
+
+
+# 8 pieces per block at least (2048 bf16, 1024 f32 logits); a bucket is 80 pieces.
+EDGES = [2047, 2048, 2049, 16383, 16384, 16385, 20480 * 2 - 1, 20480 * 2 + 8, 60001]
+
+
+@pytest.mark.parametrize("bf16", [False, True])
+@pytest.mark.parametrize("vocab", EDGES)
+def test_edges_of_the_cut(cuda, lily, W, vocab, bf16):
+    rng = np.random.default_rng(vocab * 2 + bf16)
+    for rows, k, kw in ((1, 1, {}), (2, 20, dict(history=300, rep=1.1)), (3, 64, dict(history=7, presence=0.4)),
+                        (4, 0, dict(history=500, presence=0.5, frequency=0.2, n_bias=9, n_ban=3)),
+                        (2, 65, dict(n_ban=5)), (1, 2, dict(history=4099, frequency=0.1))):
+        b = make_batch(W, rng, rows, vocab, k, bf16, kind="zipf", **kw)
+        check(cuda, lily, W, b, vocab, f"V={vocab} k={k} B={rows}")
+
+
+@pytest.mark.parametrize("rows", [1, 18, 19, 37, 38, 74, 75, 148, 149])
+def test_every_number_of_blocks_per_row(cuda, lily, W, rows):
+    vocab = 20_011  # (odd: only every eighth bf16 row starts on 16 bytes)
+    rng = np.random.default_rng(rows)
+    for bf16, k, kw in ((True, 40, dict(history=5000, rep=1.2)), (False, 50, dict(history=600, frequency=0.3, n_bias=6))):
+        b = make_batch(W, rng, rows, vocab, k, bf16, kind="zipf", **kw)
+        check(cuda, lily, W, b, vocab, f"B={rows} bf16={bf16}")
+
+
+def test_ties_fill_the_candidates(cuda, lily, W):
+    # Coarse values: more logits reach the bound than one warp, then than the buffers
+    # take (the general code draws those rows).
+    rng = np.random.default_rng(5)
+    for quantise in (16, 4, 1, 0.25):
+        b = make_batch(W, rng, 2, 30_000, 50, True, kind="uniform", quantise=quantise, history=50, rep=1.1)
+        check(cuda, lily, W, b, 30_000, f"steps of 1/{quantise}")
