@@ -18,6 +18,7 @@ import os
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "liblily_sampler.so")
+CALLS_PATH = os.path.join(_HERE, "_lily_calls.so")
 
 K_CAP = 1024
 F32, BF16 = 0, 1
@@ -190,6 +191,8 @@ def lib():
                                        C.c_uint32, C.c_void_p, C.c_uint32, C.c_uint32,
                                        C.c_uint32, C.c_uint32]
         L.lily_debug_exp.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_uint64]
+        L.lily_sample_one.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_uint32, C.c_uint64,
+                                      C.POINTER(SamplingParams), C.c_uint32, C.c_void_p, C.c_uint32, C.c_void_p]
         L.lily_sample_batch_noalloc.argtypes = [C.c_void_p, C.c_uint32, C.POINTER(SampleArgs),
                                                 C.c_char_p, C.c_uint32]
         L.lily_sampler_read_phase_clocks.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p]
@@ -215,6 +218,30 @@ def lib():
                                            C.c_uint32, C.POINTER(SampleArgs), C.c_void_p]
         _lib = L
     return _lib
+
+
+_calls = None
+
+
+def calls():
+    """The extension module that fills the library's argument blocks from torch
+    tensors (csrc/python_ext.cpp); raises if it has not been built. Its functions
+    return None for a call they do not know how to read."""
+    global _calls
+    if _calls is None:
+        import importlib.machinery
+
+        import torch  # noqa: F401  (its libraries are what the module links to)
+
+        lib()
+        if not os.path.exists(CALLS_PATH):
+            raise LilyError(ERR_CUDA, f"{CALLS_PATH} is missing: run build.py")
+        loader = importlib.machinery.ExtensionFileLoader("_lily_calls", CALLS_PATH)
+        mod = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_lily_calls", CALLS_PATH, loader=loader))
+        loader.exec_module(mod)
+        mod.bind(SamplingParams)
+        _calls = mod
+    return _calls
 
 
 def debug_exp(x, stream=None):
@@ -303,11 +330,13 @@ class SamplerScratch:
                                        C.byref(self._h))
         if st != OK:
             raise LilyError(st, "lily_sampler_create failed (is a CUDA device present?)")
+        self._calls = calls()
+        self._addr = self._h.value
 
     def close(self):
         if getattr(self, "_h", None) is not None and self._h:
             lib().lily_sampler_destroy(self._h)
-            self._h = None
+            self._h = self._addr = None
 
     def __del__(self):
         try:
@@ -382,8 +411,12 @@ class SamplerScratch:
     def sample_batch(self, logits, params, out_ids, *, stream=None, **kw):
         """lily_sample_batch: `params` is a list of SamplingParams (host), or with
         params_on_device a uint8 tensor holding the 40-byte structs."""
-        a, keep = self._sample_args(logits, params, out_ids, **kw)
-        self._check(lib().lily_sample_batch(self._h, _stream_ptr(stream), C.byref(a)))
+        st = self._calls.sample_batch(self._addr, stream, logits, params, out_ids, kw)
+        if st is None:
+            a, keep = self._sample_args(logits, params, out_ids, **kw)
+            st = lib().lily_sample_batch(self._h, _stream_ptr(stream), C.byref(a))
+        if st:
+            self._check(st)
 
     def prepare_sample_batch(self, logits, params, out_ids, **kw):
         """The argument block of a sample_batch call, built once: a decode loop
@@ -392,7 +425,11 @@ class SamplerScratch:
         return self._sample_args(logits, params, out_ids, **kw)
 
     def sample_prepared(self, prepared, stream=None):
-        self._check(lib().lily_sample_batch(self._h, _stream_ptr(stream), C.byref(prepared[0])))
+        st = self._calls.sample_prepared(self._addr, stream, prepared[0])
+        if st is None:
+            st = lib().lily_sample_batch(self._h, _stream_ptr(stream), C.byref(prepared[0]))
+        if st:
+            self._check(st)
 
     def _sample_args(self, logits, params, out_ids, *, uniforms=None, steps=None,
                      history_ids=None, history_len=None, bias_ids=None, bias_vals=None,
@@ -475,6 +512,11 @@ class SamplerScratch:
         With bf16 `biases` [rows, hidden/64] the head is in MLX affine 8-bit
         storage: `weights` are unsigned bytes, w = scale * q + bias; with
         code_bits=4 they are the 4-bit codes as bytes [rows, hidden/2]."""
+        st = self._calls.lmhead_logits(self._addr, stream, weights, scales, hidden, out_logits, biases, code_bits)
+        if st is not None:
+            if st:
+                self._check(st)
+            return
         hd = self._head(weights, scales, biases, code_bits=code_bits)
         self._check(lib().lily_lmhead_logits(self._h, _stream_ptr(stream), C.byref(hd), _ptr(hidden),
                                              _ld(hidden), int(hidden.shape[0]), _ptr(out_logits),
@@ -494,6 +536,12 @@ class SamplerScratch:
                                 want_sums: bool = False, stream=None, biases=None, code_bits: int = 8):
         """lily_lmhead_shard_candidates: head projection into the handle's own
         logits, then this shard's records (needs lmhead=True at creation)."""
+        st = self._calls.lmhead_shard_candidates(self._addr, stream, weights, scales, hidden, params, records, first_id,
+                                                 want_sums, biases, code_bits)
+        if st is not None:
+            if st:
+                self._check(st)
+            return
         rows = int(hidden.shape[0])
         keep = []
         a = self._shard_args(rows, params, None, keep)
@@ -505,6 +553,13 @@ class SamplerScratch:
     def merge_draw(self, gathered, params, out_ids, *, uniforms=None, steps=None, out_status=None,
                    kept_n=None, kept_ids=None, kept_probs=None, out_lse=None, stream=None):
         """lily_merge_draw over `gathered` (uint8 [n_shards, rows, 520])."""
+        st = self._calls.merge_draw(self._addr, stream, gathered, params, out_ids,
+                                    {"uniforms": uniforms, "steps": steps, "out_status": out_status, "kept_n": kept_n,
+                                     "kept_ids": kept_ids, "kept_probs": kept_probs, "out_lse": out_lse})
+        if st is not None:
+            if st:
+                self._check(st)
+            return
         n_shards, rows = int(gathered.shape[0]), int(gathered.shape[1])
         keep = []
         a = self._shard_args(rows, params, steps, keep)
@@ -542,15 +597,28 @@ class SamplerScratch:
 
     def argmax_batch(self, logits, out_ids, stream=None):
         """src/kernels/elementwise.rs:297-308 argmax_f32 for each row."""
+        st = self._calls.argmax_batch(self._addr, stream, logits, out_ids)
+        if st is not None:
+            if st:
+                self._check(st)
+            return
         rows = logits.shape[0] if logits.dim() == 2 else 1
         ld = _ld(logits)
         self._check(lib().lily_argmax_batch(self._h, _stream_ptr(stream), _ptr(logits),
                                             _dtype_code(logits), ld, rows, _ptr(out_ids)))
 
-    def spec_verify(self, target_logits, params: SamplingParams, draft_ids, out_ids,
-                    out_accepted, *, mode=SPEC_REJECTION, q_dense=None, q_ids=None,
-                    q_probs=None, q_n=None, u_accept=None, u_resid=None, step0=0,
-                    history_ids=None, count_slot=None, out_status=None, stream=None):
+    def spec_verify(self, target_logits, params: SamplingParams, draft_ids, out_ids, out_accepted, *, stream=None, **kw):
+        """lily_spec_verify; keywords: mode, q_dense or q_ids / q_probs / q_n, u_accept,
+        u_resid, step0, history_ids, count_slot, out_status."""
+        st = self._calls.spec_verify(self._addr, stream, target_logits, params, draft_ids, out_ids, out_accepted, kw)
+        if st is None:
+            st = self._spec_verify(target_logits, params, draft_ids, out_ids, out_accepted, stream=stream, **kw)
+        if st:
+            self._check(st)
+
+    def _spec_verify(self, target_logits, params, draft_ids, out_ids, out_accepted, *, mode=SPEC_REJECTION,
+                     q_dense=None, q_ids=None, q_probs=None, q_n=None, u_accept=None, u_resid=None, step0=0,
+                     history_ids=None, count_slot=None, out_status=None, stream=None):
         a = SpecArgs()
         a.struct_size = C.sizeof(SpecArgs)
         a.m = target_logits.shape[0]
@@ -574,7 +642,7 @@ class SamplerScratch:
             slot = C.c_uint32(count_slot)
             a.count_slot = C.cast(C.pointer(slot), C.c_void_p)
         a.out_ids, a.out_accepted, a.out_status = _ptr(out_ids), _ptr(out_accepted), _ptr(out_status)
-        self._check(lib().lily_spec_verify(self._h, _stream_ptr(stream), C.byref(a)))
+        return lib().lily_spec_verify(self._h, _stream_ptr(stream), C.byref(a))
 
     def spec_accept(self, draws, ids, ctrl, pos0: int, ratio: int, chain: int, stride: int = 4,
                     stream=None):
@@ -636,6 +704,11 @@ def sample_batch_noalloc(vocab, logits, params, out_ids, *, uniforms=None, steps
 def sample_f32(logits, scratch: SamplerScratch, params: SamplingParams, step: int, out,
                history_ids=None, stream=None):
     """src/kernels/sample.rs:373-387: one draw from `logits` [V] into `out` [1]."""
+    st = scratch._calls.sample_one(scratch._addr, stream, logits, params, step, out, history_ids)
+    if st is not None:
+        if st:
+            scratch._check(st)
+        return
     import torch
 
     hl = None

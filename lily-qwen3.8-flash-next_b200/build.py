@@ -1,47 +1,80 @@
-"""Builds the CUDA library in-tree with nvcc for sm_100a.
+"""Builds the CUDA library and the Python call layer in-tree for sm_100a.
 
     python lily-qwen3.8-flash-next_b200/build.py [--force]
 
-The result, liblily_sampler.so beside this file, exports the C ABI of
-include/lily_sampler.h. nvcc cross-compiles without a GPU.
+liblily_sampler.so beside this file exports the C ABI of include/lily_sampler.h
+(nvcc cross-compiles without a GPU); _lily_calls.so is the extension module that fills
+its argument blocks from torch tensors (csrc/python_ext.cpp). One compiler process per
+source file, side by side; a file is compiled again when it or a header is newer.
 """
 from __future__ import annotations
 
 import os
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
+OBJ = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "liblily_sampler.so")
+CALLS = os.path.join(HERE, "_lily_calls.so")
+CALLS_SOURCE = os.path.join(CSRC, "python_ext.cpp")
 
-NVCC_FLAGS = [
-    "-gencode", "arch=compute_100a,code=sm_100a",
-    "-lineinfo", "-O3", "-std=c++17",
-    "-shared", "-Xcompiler", "-fPIC",
-]
+ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
+NVCC_FLAGS = [*ARCH_FLAGS, "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC"]
 
 
 def sources():
     out = []
     for name in sorted(os.listdir(CSRC)):
-        if name.endswith((".cu", ".cpp")):
-            out.append(os.path.join(CSRC, name))
+        path = os.path.join(CSRC, name)
+        if name.endswith((".cu", ".cpp")) and path != CALLS_SOURCE:
+            out.append(path)
     return out
 
 
-def _deps():
+def _headers():
     deps = [os.path.join(INCLUDE, n) for n in os.listdir(INCLUDE)]
-    deps += [os.path.join(CSRC, n) for n in os.listdir(CSRC)]
-    return deps
+    return deps + [os.path.join(CSRC, n) for n in os.listdir(CSRC) if n.endswith((".cuh", ".h"))]
+
+
+def _newest(paths) -> float:
+    return max(os.path.getmtime(p) for p in paths)
+
+
+def _older(target: str, t: float) -> bool:
+    return not os.path.exists(target) or os.path.getmtime(target) < t
 
 
 def stale() -> bool:
-    if not os.path.exists(LIB):
-        return True
-    t = os.path.getmtime(LIB)
-    return any(os.path.getmtime(d) > t for d in _deps())
+    headers = _newest(_headers())
+    return _older(LIB, max(headers, _newest(sources()))) or _older(CALLS, max(headers, os.path.getmtime(CALLS_SOURCE)))
+
+
+def _run(cmd, verbose=False):
+    proc = subprocess.run(cmd, capture_output=True, text=True)
+    if proc.returncode != 0:
+        raise RuntimeError(" ".join(cmd[:1]) + " failed:\n" + proc.stdout + proc.stderr)
+    if verbose:
+        sys.stderr.write(proc.stderr)
+
+
+def _calls_command():
+    """g++ for the extension module: torch's headers and libraries, the library beside it."""
+    import sysconfig
+
+    import torch
+
+    root = os.path.dirname(torch.__file__)
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    abi = int(torch._C._GLIBCXX_USE_CXX11_ABI)
+    return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={abi}",
+            "-I", os.path.join(root, "include"), "-I", os.path.join(root, "include", "torch", "csrc", "api", "include"),
+            "-I", os.path.join(cuda, "include"), "-I", sysconfig.get_paths()["include"], CALLS_SOURCE,
+            "-L", os.path.join(root, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda", LIB,
+            "-Wl,-rpath,$ORIGIN", "-o", CALLS]
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -49,15 +82,23 @@ def build(force: bool = False, verbose: bool = False) -> str:
         return LIB
     nvcc = os.environ.get("NVCC", "nvcc")
     extra = os.environ.get("LILY_NVCC_EXTRA", "").split()  # extra nvcc flags, e.g. -Xptxas -v
-    cmd = [nvcc, *NVCC_FLAGS, *extra, "-I", INCLUDE, "-o", LIB, *sources()]
     if verbose:
-        cmd.insert(1, "-Xptxas")
-        cmd.insert(2, "-v")
-    proc = subprocess.run(cmd, capture_output=True, text=True)
-    if proc.returncode != 0:
-        raise RuntimeError("nvcc failed:\n" + proc.stdout + proc.stderr)
-    if verbose:
-        sys.stderr.write(proc.stderr)
+        extra += ["-Xptxas", "-v"]
+    os.makedirs(OBJ, exist_ok=True)
+    headers = _newest(_headers())
+    jobs, objects = [], []
+    for src in sources():
+        obj = os.path.join(OBJ, os.path.basename(src) + ".o")
+        objects.append(obj)
+        if force or _older(obj, max(headers, os.path.getmtime(src))):
+            jobs.append([nvcc, *NVCC_FLAGS, *extra, "-I", INCLUDE, "-c", "-o", obj, src])
+    with ThreadPoolExecutor(max_workers=max(1, len(jobs))) as pool:
+        list(pool.map(lambda cmd: _run(cmd, verbose), jobs))
+    _run([nvcc, *ARCH_FLAGS, "-shared", "-Xcompiler", "-fPIC", "-o", LIB, *objects])
+    if force or _older(CALLS, max(headers, os.path.getmtime(CALLS_SOURCE))):
+        _run(_calls_command())
+    else:
+        os.utime(CALLS)
     return LIB
 
 
