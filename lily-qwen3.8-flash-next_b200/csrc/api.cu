@@ -261,7 +261,6 @@ int32_t launch_one(lily_sampler *h, cudaStream_t stream_, const lily::KArgs &a, 
 struct SplitPlan {
     bool take = false;
     bool sole = false;   // at most one block per SM
-    bool share = false;  // the blocks of a row share its history list
     uint32_t log_blocks = 0, mark_mode = lily::MARK_BITS, mark_words = 0;
     size_t smem = 0;
 };
@@ -307,8 +306,6 @@ SplitPlan split_plan(const lily_sampler *h, const lily::KArgs &a, uint32_t rows,
             p.mark_words = (entries / 32u + 3u) & ~3u;
         }
     }
-    // (Below some thousands of ids looking at all of them costs less than the blocks' meeting.)
-    p.share = lists && lb > 0u && a.history_ids != nullptr && (p.mark_mode == lily::MARK_COUNTS || a.history_ld > 4096u);
     p.smem = fixed + (size_t)p.mark_words * 4u;
     p.smem = p.smem > general ? p.smem : general;
     p.take = p.smem <= (size_t)h->max_smem && p.sole;
@@ -321,7 +318,6 @@ int32_t launch_split(lily_sampler *h, cudaStream_t stream, lily::SplitArgs<MAXR>
     sa.log_blocks = p.log_blocks;
     sa.mark_mode = p.mark_mode;
     sa.mark_words = p.mark_words;
-    sa.share = p.share ? 1u : 0u;
     sa.spill_params = reinterpret_cast<lily_sampling_params_t *>(h->spill);
     sa.spill_steps = reinterpret_cast<uint32_t *>(h->spill + INLINE_ROWS_MAX * sizeof(lily_sampling_params_t));
     sa.spill_slots = sa.spill_steps + INLINE_ROWS_MAX;

@@ -19,7 +19,7 @@ constexpr uint32_t SPL_POOL = 256;       // keys in the pool a narrow row's boun
 constexpr uint32_t SPL_HITS = 512;       // vectors of a block that may reach the bound
 constexpr uint32_t SPL_FLAGGED = 2048;   // buckets that may reach the bound
 constexpr uint32_t SPL_SORTED = 2048;    // candidates of a wide row
-constexpr uint32_t SPL_MIN_TILES = SPL_WARPS;  // a block has at least a piece per warp
+constexpr uint32_t SPL_MIN_TILES = SPL_WARPS / 2u;  // pieces of a block, at least
 constexpr uint32_t SPL_COUNT_MAX = 32767;      // of an id in a history list (a mark's top bit says "on a list")
 constexpr uint32_t SPL_NAN_KEY = 0xFFFFFFFFu;  // a candidate that came out a NaN
 
@@ -74,6 +74,7 @@ __host__ __device__ inline RowIn row_in(const lily_sampling_params_t &P, uint32_
 struct alignas(16) SplitSmem {
     unsigned long long mbar_pool;    // every block's keys have arrived
     unsigned long long mbar_cand;    // first block: every block's candidates have arrived
+    unsigned long long mbar_list;    // wide rows: the sorted lists of all blocks have arrived
     uint4 head[SPL_MAX_BLOCKS];      // first block: a block's number of candidates, flag, bound
     union {
         alignas(16) uint32_t pool[SPL_POOL];     // the best keys of every warp of the cluster
@@ -90,7 +91,7 @@ struct alignas(16) SplitSmem {
     uint32_t bin;
     uint32_t verdict[2];             // what the waiting warps of the first block learn
     uint32_t bound_key;
-    uint32_t pad;
+    uint32_t n_slots;                // candidates whose ids are counted in the history
 };
 static_assert(sizeof(SplitSmem) % 16u == 0u, "the arrays behind it are 16-byte aligned");
 
@@ -102,7 +103,6 @@ struct SplitArgs {
     uint32_t log_blocks;      // log2 of the blocks per row
     uint32_t mark_mode;
     uint32_t mark_words;      // 32-bit words of the marks, a multiple of four
-    uint32_t share;           // the blocks of a row share its history list (else each looks at all of it)
     uint32_t inline_params;   // `in` below is valid (else a.params / a.steps)
     uint32_t inline_slots;
     uint32_t inline_history;  // 1 + the history length of every row (0: a.history_len)

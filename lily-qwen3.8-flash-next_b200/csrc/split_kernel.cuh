@@ -129,131 +129,15 @@ static __device__ __noinline__ uint4 edge_vec(const T *row_ptr, uint32_t vocab, 
 }
 
 
-// The best k of the candidates in the blocks' regions, sorted into key[] / id[]
-// [0, k): for rows that keep many. A histogram over the distance from the top puts
-// each near its place, the few that share a bin are ranked by counting. Returns how
-// many there are (at most k), 0 if they do not fit. Keys below `kmin` are not
-// wanted. `room`: SPL_SORTED words of 8 bytes. All SPL_NT threads.
-static __device__ __noinline__ uint32_t split_sort_bins(SmemFixed *sm, SplitSmem *ss, unsigned long long *room,
-                                                 uint32_t log_blocks, uint32_t k, uint32_t kmin) {
-    constexpr unsigned FULL = 0xFFFFFFFFu;
-    constexpr uint32_t BPT = TH_BINS / SPL_NT;
-    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    const uint2 *cand = reinterpret_cast<const uint2 *>(sm->key);  // over key and id: CAP of them
-    const uint32_t cap = CAP >> log_blocks, team = SPL_NT >> log_blocks;
-    const uint32_t region = tid / team, n_region = ss->head[region].x;
-    const uint2 *mine = cand + region * cap;
-    uint32_t best = 0;
-    for (uint32_t i = tid % team; i < n_region; i += team) {
-        best = max(best, mine[i].x);
-    }
-    best = __reduce_max_sync(FULL, best);
-    for (uint32_t b = tid; b < TH_BINS; b += SPL_NT) {
-        sm->thist[b] = 0;
-        sm->tkey[b] = 0;
-    }
-    if (lane == 0) {
-        sm->warp_sums[warp] = best;
-    }
-    spl_sync();
-    best = __reduce_max_sync(FULL, sm->warp_sums[lane & (SPL_WARPS - 1u)]);
-    const float top = float_of_key(best), low = float_of_key(kmin);
-    const float range = __fsub_rn(top, low);
-    const float scale = range > 0.0f ? __fdiv_rn((float)(TH_BINS - 1u), range) : 0.0f;
-    // (Falls with the key: every step is monotone. A NaN or an infinity lands in bin 0 or the last.)
-    auto bin_of = [&](uint32_t x) -> uint32_t {
-        const float d = __fmul_rn(__fsub_rn(top, float_of_key(x)), scale);
-        return d > 0.0f ? min((uint32_t)d, TH_BINS - 1u) : 0u;
-    };
-    for (uint32_t i = tid % team; i < n_region; i += team) {
-        const uint32_t x = mine[i].x;
-        if (x >= kmin) {
-            atomicAdd(&sm->thist[bin_of(x)], 1u);
-        }
-    }
-    spl_sync();
-    // Candidates in the bins before each.
-    uint32_t c[BPT], sum = 0;
-#pragma unroll
-    for (uint32_t j = 0; j < BPT; ++j) {
-        c[j] = sm->thist[tid * BPT + j];
-        sum += c[j];
-    }
-    uint32_t incl = sum;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t t = __shfl_up_sync(FULL, incl, o);
-        if (lane >= (uint32_t)o) {
-            incl += t;
-        }
-    }
-    if (lane == 31u) {
-        sm->warp_sums[SPL_WARPS + warp] = incl;
-    }
-    if (tid == 0) {
-        ss->bin = 0;  // the end of the last bin that is needed
-    }
-    spl_sync();
-    uint32_t before = incl - sum, total = 0;
-#pragma unroll
-    for (uint32_t w = 0; w < SPL_WARPS; ++w) {
-        const uint32_t s = sm->warp_sums[SPL_WARPS + w];
-        before += w < warp ? s : 0u;
-        total += s;
-    }
-    uint32_t end = 0;
-#pragma unroll
-    for (uint32_t j = 0; j < BPT; ++j) {
-        sm->tid[tid * BPT + j] = before;
-        if (before < k) {
-            end = before + c[j];
-        }
-        before += c[j];
-    }
-    end = __reduce_max_sync(FULL, end);
-    if (lane == 0) {
-        atomicMax(&ss->bin, end);
-    }
-    spl_sync();
-    end = ss->bin;
-    if (end > SPL_SORTED) {
-        return 0u;
-    }
-    // To the bin's part of the array (bins that begin past rank k are not needed).
-    for (uint32_t i = tid % team; i < n_region; i += team) {
-        const uint2 e = mine[i];
-        if (e.x >= kmin) {
-            const uint32_t b = bin_of(e.x), first = sm->tid[b];
-            if (first < k) {
-                room[first + atomicAdd(&sm->tkey[b], 1u)] = ((unsigned long long)e.x << 32) | (uint32_t)~e.y;
-            }
-        }
-    }
-    spl_sync();
-    for (uint32_t i = tid; i < end; i += SPL_NT) {
-        const unsigned long long me = room[i];
-        const uint32_t b = bin_of((uint32_t)(me >> 32)), first = sm->tid[b], last = first + sm->thist[b];
-        uint32_t place = first;
-        for (uint32_t j = first; j < last; ++j) {
-            place += room[j] > me ? 1u : 0u;
-        }
-        if (place < k) {
-            sm->key[place] = (uint32_t)(me >> 32);
-            sm->id[place] = ~(uint32_t)me;
-        }
-    }
-    spl_sync();
-    return min(total, k);
-}
-
-// The draw of a row that keeps more than 64 candidates, sorted in key[] / id[]: the
+// The draw of a row that keeps more than 64 candidates, sorted in `best`: the
 // softmax weights, the prefix sums in rank order with one rounding per add
 // (tests/unit/kernels/sample.rs:37-46), the cut, the draw. All SPL_NT threads.
-static __device__ __noinline__ void split_finalize_wide(SmemFixed *sm, SplitSmem *ss, const KArgs &a, uint32_t row, uint32_t n,
+static __device__ __noinline__ void split_finalize_wide(SmemFixed *sm, SplitSmem *ss, const unsigned long long *best,
+                                                       const KArgs &a, uint32_t row, uint32_t n,
                                                  float top_p, float min_p, float u, bool counts_draw, uint32_t slot) {
     const uint32_t tid = threadIdx.x;
     float *p = reinterpret_cast<float *>(sm->tkey), *cum = reinterpret_cast<float *>(sm->tid);
-    const float top = float_of_key(sm->key[0]);
+    const float top = float_of_key((uint32_t)(best[0] >> 32));
     if (top == neg_inf() || top == -neg_inf()) {
         if (tid == 0) {
             a.out_ids[row] = 0xFFFFFFFFu;
@@ -268,7 +152,7 @@ static __device__ __noinline__ void split_finalize_wide(SmemFixed *sm, SplitSmem
         return;
     }
     for (uint32_t i = tid; i < KCAP; i += SPL_NT) {
-        p[i] = i < n ? exp_f32(__fsub_rn(float_of_key(sm->key[i]), top)) : 0.0f;
+        p[i] = i < n ? exp_f32(__fsub_rn(float_of_key((uint32_t)(best[i] >> 32)), top)) : 0.0f;
     }
     if (tid == 0) {
         ss->n_live = n;   // the first rank that is not kept
@@ -276,29 +160,33 @@ static __device__ __noinline__ void split_finalize_wide(SmemFixed *sm, SplitSmem
     }
     spl_sync();
     if (tid == 0) {
-        // A chain of n dependent adds; the loads run one step ahead of it. (Ranks past
-        // n weigh 0, and s + 0 is s.)
+        // A chain of n dependent adds (4 clocks each); the loads run 32 ranks ahead of it.
+        // (Ranks past n weigh 0, and s + 0 is s.)
         const float4 *p4 = reinterpret_cast<const float4 *>(p);
         float4 *c4 = reinterpret_cast<float4 *>(cum);
-        const uint32_t steps = (n + 7u) / 8u;
+        constexpr uint32_t A = 8;
         float s = 0.0f;
-        float4 v0 = p4[0], v1 = p4[1];
-        for (uint32_t i = 0; i < steps; ++i) {
-            const uint32_t nx = min(i + 1u, KCAP / 8u - 1u);
-            const float4 w0 = p4[2u * nx], w1 = p4[2u * nx + 1u];
-            float4 o0, o1;
-            o0.x = s = __fadd_rn(s, v0.x);
-            o0.y = s = __fadd_rn(s, v0.y);
-            o0.z = s = __fadd_rn(s, v0.z);
-            o0.w = s = __fadd_rn(s, v0.w);
-            o1.x = s = __fadd_rn(s, v1.x);
-            o1.y = s = __fadd_rn(s, v1.y);
-            o1.z = s = __fadd_rn(s, v1.z);
-            o1.w = s = __fadd_rn(s, v1.w);
-            c4[2u * i] = o0;
-            c4[2u * i + 1u] = o1;
-            v0 = w0;
-            v1 = w1;
+        float4 v[A], w[A];
+#pragma unroll
+        for (uint32_t h = 0; h < A; ++h) {
+            v[h] = p4[h];
+        }
+        for (uint32_t i = 0; i < n; i += 4u * A) {
+            const uint32_t next = min(i / 4u + A, KCAP / 4u - A);
+#pragma unroll
+            for (uint32_t h = 0; h < A; ++h) {
+                w[h] = p4[next + h];
+            }
+#pragma unroll
+            for (uint32_t h = 0; h < A; ++h) {
+                float4 o;
+                o.x = s = __fadd_rn(s, v[h].x);
+                o.y = s = __fadd_rn(s, v[h].y);
+                o.z = s = __fadd_rn(s, v[h].z);
+                o.w = s = __fadd_rn(s, v[h].w);
+                c4[i / 4u + h] = o;
+                v[h] = w[h];
+            }
         }
     }
     spl_sync();
@@ -322,13 +210,13 @@ static __device__ __noinline__ void split_finalize_wide(SmemFixed *sm, SplitSmem
     }
     if (a.kept_n) {
         for (uint32_t i = tid; i < n_keep; i += SPL_NT) {
-            a.kept_ids[(uint64_t)row * a.kept_ld + i] = sm->id[i];
+            a.kept_ids[(uint64_t)row * a.kept_ld + i] = ~(uint32_t)best[i];
             a.kept_probs[(uint64_t)row * a.kept_ld + i] = __fdiv_rn(p[i], mass);
         }
     }
     spl_sync();
     if (tid == 0) {
-        const uint32_t id = sm->id[min(ss->bin, n_keep - 1u)];
+        const uint32_t id = ~(uint32_t)best[min(ss->bin, n_keep - 1u)];
         a.out_ids[row] = id;
         if (a.out_status) {
             a.out_status[row] = LILY_ROW_OK;
@@ -565,6 +453,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         ss->n_hits = 0;
         ss->n_listed = 0;
         ss->n_sent = 0;
+        ss->n_slots = 0;
         ss->n_live = 0;
         ss->hard = 0;
         ss->bound_key = 0;
@@ -573,6 +462,8 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
             const uint32_t cand_bar = (uint32_t)__cvta_generic_to_shared(&ss->mbar_cand);
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(pool_bar) : "memory");
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(cand_bar), "r"(blocks) : "memory");
+            const uint32_t list_bar = (uint32_t)__cvta_generic_to_shared(&ss->mbar_list);
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(list_bar), "r"(blocks) : "memory");
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
     }
@@ -656,19 +547,14 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
             asm volatile("bar.arrive 2, %0;" ::"n"(NT) : "memory");
         }
     };
-    if (tid >= SPL_NT) {
-        if (rank == 0u) {
-            if (ca.share && blocks > 1u) {
-                // (Threads that stay have to come to the cluster's second meeting as well.)
-                asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-                asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-            }
-            if (wait_verdict(0u)) {
-                wait_verdict(1u);
-            }
+    // The upper half of the block marks the row's history while the lower half reads
+    // its logits; then it waits (in the first block) for the verdict.
+    const bool marker = tid >= SPL_NT;
+    auto marker_ends = [&]() {
+        if (rank == 0u && wait_verdict(0u)) {
+            wait_verdict(1u);
         }
-        return;
-    }
+    };
     // ---- the first bucket is asked for before anything is known about the row
     const uint4 *vec0 = reinterpret_cast<const uint4 *>(row_ptr - skip) + lane;
     const uint32_t pieces = split_pieces(vocab, skip, PER);
@@ -684,25 +570,25 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
     };
     // The row's first history ids go first. (Their number is not known yet; the row
     // has room for history_ld of them.)
-    constexpr uint32_t HU = BPS == 1 ? 4u : 2u;
+    constexpr uint32_t HU = 8u;
     const uint32_t *hist = a.history_ids + (uint64_t)row * a.history_ld;
-    const bool hist_vec = a.history_ids != nullptr && (reinterpret_cast<uintptr_t>(hist) & 15u) == 0u;
-    const uint4 *h4 = reinterpret_cast<const uint4 *>(hist);
-    const uint4 no_ids = make_uint4(NONE, NONE, NONE, NONE);
-    // Either every block looks at the whole list for the ids of its share, or (a long
-    // list, or one that is counted) a part of the list each, for all blocks.
-    const uint32_t h_step = ca.share ? SPL_NT << log_blocks : SPL_NT, h_first = ca.share ? rank * SPL_NT + tid : tid;
-    uint4 hx[HU];
-    const uint32_t room4 = hist_vec ? (uint32_t)min(a.history_ld, (uint64_t)a.max_history) >> 2 : 0u;
-#pragma unroll
-    for (uint32_t i = 0; i < HU; ++i) {
-        const uint32_t at = h_first + i * h_step;
-        hx[i] = at < room4 ? __ldg(h4 + at) : no_ids;
-    }
+    const uint32_t lead = (4u - ((uint32_t)(reinterpret_cast<uintptr_t>(hist) >> 2) & 3u)) & 3u;  // ids before the first 16-byte boundary
+    const uint4 *h4 = reinterpret_cast<const uint4 *>(hist + lead);
+    const uint32_t room = a.history_ids ? (uint32_t)min(a.history_ld, (uint64_t)a.max_history) : 0u;
+    const uint32_t room4 = room > lead ? (room - lead) >> 2 : 0u;
     uint4 q[SPL_U];
+    if (marker) {
+        const uint4 no_ids = make_uint4(NONE, NONE, NONE, NONE);
 #pragma unroll
-    for (uint32_t i = 0; i < SPL_U; ++i) {
-        q[i] = load_piece(warp + SPL_WARPS * i);
+        for (uint32_t i = 0; i < HU; ++i) {
+            const uint32_t at = tid - SPL_NT + i * SPL_NT;
+            q[i] = at < room4 ? __ldg(h4 + at) : no_ids;
+        }
+    } else {
+#pragma unroll
+        for (uint32_t i = 0; i < SPL_U; ++i) {
+            q[i] = load_piece(warp + SPL_WARPS * i);
+        }
     }
 
     // ---- the row's parameters
@@ -769,8 +655,8 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
     // Decided alike by every block of the cluster: rows that end here.
     const bool general = (in.flags & ROW_RAISES) || n_sp > SP_SMEM ||
                          (n_sp != 0u && mark_mode == MARK_BITS) ||
-                         (list_mode && need_counts && (mark_mode != MARK_COUNTS || hist_len + extra_len > SPL_COUNT_MAX)) ||
-                         (wide && (row < a.spec.n_spec || blocks * SPL_NT < 2u * k));
+                         (list_mode && need_counts && mark_mode != MARK_COUNTS) ||
+                         (wide && (row < a.spec.n_spec || min(vocab / PER, blocks * SPL_NT) * 8u < 9u * k));
     if (status != LILY_ROW_OK || general) {
         if (status != LILY_ROW_OK && rank == 0u && tid == 0) {
             a.out_ids[row] = status == LILY_ROW_FORCED ? (uint32_t)forced : 0xFFFFFFFFu;
@@ -784,7 +670,9 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
                 atomicOr(a.status_word, 1u << (status & 31u));
             }
         }
-        if (rank == 0u) {
+        if (marker) {
+            marker_ends();
+        } else if (rank == 0u) {
             verdict(0u, status == LILY_ROW_OK ? ALONE : DONE);
         }
         return;
@@ -795,6 +683,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
     ahead.draft = draws && row < a.spec.n_spec ? __ldg(a.spec.draft_ids + row) : 0u;
     const float u_row = !draws ? 0.0f : a.uniforms ? __ldg(a.uniforms + row) : in.u;
 
+    LILY_STAMP(14);
     // ---- 1. the stream: maxima and marks
     // Which block an id belongs to, and its place in that block's marks.
     auto place_of = [&](uint32_t id, uint32_t &at) -> uint32_t {
@@ -804,122 +693,158 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
     };
     uint8_t *mark8 = reinterpret_cast<uint8_t *>(marks);
     uint16_t *mark16 = reinterpret_cast<uint16_t *>(marks);
-    const uint32_t marks_at = (uint32_t)__cvta_generic_to_shared(marks);
-    // One id of the history; `WAY` says how (chosen once per row, not per id). Rows
-    // that need no multiplicity: any thread may write the same.
-    enum { OWN_BYTE, OWN_SHORT, OWN_BIT, OWN_COUNT, ANY_BYTE, ANY_SHORT, ANY_BIT, ANY_COUNT };
-    auto mark_id = [&](auto way, uint32_t id) {
-        constexpr int WAY = decltype(way)::value;
-        uint32_t at, to;
-        const uint32_t owner = place_of(id, at);
-        if (WAY < ANY_BYTE) {
-            if (owner == rank) {
-                if (WAY == OWN_BYTE) {
-                    mark8[at] = 1;
-                } else if (WAY == OWN_SHORT) {
-                    mark16[at] = 1;
-                } else if (WAY == OWN_BIT) {
-                    atomicOr(marks + (at >> 5), 1u << (at & 31u));
-                } else {
-                    atomicAdd(marks + (at >> 1), 1u << (16u * (at & 1u)));
+    const bool marked = hist_len + extra_len != 0u;
+    const bool counted = marked && need_counts;  // (a list whose multiplicities matter)
+    if (marker) {
+        // Every block looks at the whole list for the ids of its share. (Sharing the list
+        // out and marking in the owner's memory was measured slower from 2000 ids on:
+        // a remote store costs an SM some 4 clocks, looking at an id a fraction of one.)
+        const uint32_t t = tid - SPL_NT;
+        const uint32_t n4 = hist_len > lead ? (hist_len - lead) >> 2 : 0u;
+        const uint32_t loose = hist_len - n4 * 4u, more = loose + extra_len;  // what the 16-byte loads leave out, and
+                                                                              // ids drawn earlier in this step
+        bool loaded = n4 <= room4;  // q holds the list's first part
+        auto each_four = [&](auto f) {  // f(four ids) over the list (NONE where there are no four)
+            for (uint32_t h_at = 0; h_at < n4; h_at += HU * SPL_NT) {
+                if (!loaded) {
+#pragma unroll
+                    for (uint32_t i = 0; i < HU; ++i) {
+                        const uint32_t at = h_at + i * SPL_NT + t;
+                        q[i] = at < n4 ? __ldg(h4 + at) : make_uint4(NONE, NONE, NONE, NONE);
+                    }
+                }
+                loaded = false;
+#pragma unroll
+                for (uint32_t i = 0; i < HU; ++i) {
+                    if (h_at + i * SPL_NT < n4) {
+                        f(h_at + i * SPL_NT + t < n4 ? q[i] : make_uint4(NONE, NONE, NONE, NONE));
+                    }
                 }
             }
-        } else if (WAY != ANY_COUNT) {
-            if (owner != NONE) {
-                const uint32_t off = WAY == ANY_BYTE ? at : WAY == ANY_SHORT ? at * 2u : (at >> 5) * 4u;
-                asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(marks_at + off), "r"(owner));
-                if (WAY == ANY_BYTE) {
-                    asm volatile("st.shared::cluster.u8 [%0], %1;" ::"r"(to), "h"((unsigned short)1) : "memory");
-                } else if (WAY == ANY_SHORT) {
-                    asm volatile("st.shared::cluster.u16 [%0], %1;" ::"r"(to), "h"((unsigned short)1) : "memory");
-                } else {
-                    asm volatile("red.shared::cluster.or.b32 [%0], %1;" ::"r"(to), "r"(1u << (at & 31u)) : "memory");
-                }
+            loaded = n4 <= HU * SPL_NT;
+            const uint32_t first = min(lead, loose);
+            for (uint32_t i0 = 0; i0 < more; i0 += SPL_NT) {
+                const uint32_t i = i0 + t;
+                const uint32_t id = i < loose ? __ldg(hist + (i < first ? i : n4 * 4u + i))
+                                    : i < more ? __ldcg(a.extra_ids + (i - loose)) : NONE;
+                f(make_uint4(id, NONE, NONE, NONE));
             }
-        } else {
-            // Real histories repeat a few ids very often: the lanes that hold the same id as
-            // the first of a warp add up to one atomic. Every lane of the warp is here.
-            const uint32_t first = __shfl_sync(FULL, id, 0);
-            const bool same = id == first;
-            const uint32_t n = (uint32_t)__popc(__ballot_sync(FULL, same));
-            if (owner != NONE && (!same || lane == 0u)) {
-                asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(marks_at + (at >> 1) * 4u), "r"(owner));
-                asm volatile("red.shared::cluster.add.u32 [%0], %1;" ::"r"(to), "r"((same ? n : 1u) << (16u * (at & 1u)))
-                             : "memory");
-            }
+        };
+        for (uint32_t j = t; j < n_sp; j += SPL_NT) {
+            sm->sp_ids[j] = j < n_bias ? a.bias_ids[(uint64_t)row * a.bias_ld + j]
+                                       : a.ban_ids[(uint64_t)row * a.ban_ld + (j - n_bias)];
+            sm->sp_vals[j] = j < n_bias ? a.bias_vals[(uint64_t)row * a.bias_ld + j] : 0.0f;
         }
-    };
-    // Calls f with the row's way of marking.
-    auto with_way = [&](bool own, auto f) {
-        if (own) {
-            if (mark_mode == MARK_BYTES) {
-                f(std::integral_constant<int, OWN_BYTE>());
-            } else if (mark_mode == MARK_BITS) {
-                f(std::integral_constant<int, OWN_BIT>());
-            } else if (need_counts) {
-                f(std::integral_constant<int, OWN_COUNT>());
-            } else {
-                f(std::integral_constant<int, OWN_SHORT>());
-            }
+        if (t < 4u) {
+            sm->sp_ids[min(n_sp, SP_SMEM) + t] = NONE;
+        }
+        // (Any thread may write the same mark: how often an id occurs is counted later, and
+        // only for the candidates. Counting every id here took 6 us for 8192 ids: real
+        // histories repeat a few ids very often, and all in one block's share.)
+        auto mark_all = [&](auto mark) {
+            each_four([&](const uint4 &x) {
+                uint32_t at;
+                if (place_of(x.x, at) == rank) {
+                    mark(at);
+                }
+                if (place_of(x.y, at) == rank) {
+                    mark(at);
+                }
+                if (place_of(x.z, at) == rank) {
+                    mark(at);
+                }
+                if (place_of(x.w, at) == rank) {
+                    mark(at);
+                }
+            });
+        };
+        if (!marked) {
         } else if (mark_mode == MARK_BYTES) {
-            f(std::integral_constant<int, ANY_BYTE>());
-        } else if (mark_mode == MARK_BITS) {
-            f(std::integral_constant<int, ANY_BIT>());
-        } else if (need_counts) {
-            f(std::integral_constant<int, ANY_COUNT>());
+            mark_all([&](uint32_t at) { mark8[at] = 1; });
+        } else if (mark_mode == MARK_COUNTS) {
+            mark_all([&](uint32_t at) { mark16[at] = 1; });
         } else {
-            f(std::integral_constant<int, ANY_SHORT>());
+            mark_all([&](uint32_t at) { atomicOr(marks + (at >> 5), 1u << (at & 31u)); });
         }
-    };
-    const uint32_t n4 = hist_vec ? hist_len >> 2 : 0u;
-    const uint32_t h_rounds = (n4 + h_step - 1u) / h_step;  // 16-byte loads of ids per thread
-    const uint32_t h_per = buckets == 1u ? h_rounds : (h_rounds + buckets - 1u) / buckets;  // ... per bucket
-    const bool shared_list = ca.share != 0u && n4 != 0u;
-    if (shared_list) {
-        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");  // the other blocks' marks are cleared
-    }
-    for (uint32_t j = tid; j < n_sp; j += SPL_NT) {
-        sm->sp_ids[j] = j < n_bias ? a.bias_ids[(uint64_t)row * a.bias_ld + j]
-                                   : a.ban_ids[(uint64_t)row * a.ban_ld + (j - n_bias)];
-        sm->sp_vals[j] = j < n_bias ? a.bias_vals[(uint64_t)row * a.bias_ld + j] : 0.0f;
+        if (n_sp != 0u) {
+            // The ids on the bias or ban list that are this block's, each by the thread of
+            // its first entry: marked, so that the stream's candidates leave them out, and
+            // a candidate of its own with its bias entries added in list order (a banned
+            // id is none).
+            asm volatile("bar.sync 6, %0;" ::"n"(SPL_NT) : "memory");  // the lists and the marks are there
+            for (uint32_t j = t; j < n_sp; j += SPL_NT) {
+                const uint32_t id = sm->sp_ids[j];
+                uint32_t at;
+                if (place_of(id, at) != rank) {
+                    continue;
+                }
+                float x = widen(row_ptr[id]);
+                // (Four entries per load; the padding never matches an id of the vocabulary.)
+                uint32_t before = 0, bans = 0, same = 0;
+                const uint4 *v4 = reinterpret_cast<const uint4 *>(sm->sp_ids);
+#pragma unroll 4
+                for (uint32_t e = 0; e < n_sp; e += 4u) {
+                    const uint4 v = v4[e >> 2];
+                    const uint32_t m = (v.x == id ? 1u : 0u) | (v.y == id ? 2u : 0u) | (v.z == id ? 4u : 0u) | (v.w == id ? 8u : 0u);
+                    same += __popc(m);
+                    before |= e >= j ? 0u : m & ((1u << min(j - e, 4u)) - 1u);
+                    bans |= e + 4u <= n_bias ? 0u : m & ~((1u << (n_bias > e ? n_bias - e : 0u)) - 1u);
+                }
+                const bool first = before == 0u, banned = bans != 0u;
+                if (same == 1u) {
+                    x = j < n_bias ? __fadd_rn(x, sm->sp_vals[j]) : x;
+                } else {
+                    for (uint32_t e = 0; e < n_bias; ++e) {
+                        x = sm->sp_ids[e] == id ? __fadd_rn(x, sm->sp_vals[e]) : x;
+                    }
+                }
+                if (first) {
+                    if (mark_mode == MARK_BYTES) {
+                        mark8[at] |= 0x80u;
+                    } else {
+                        mark16[at] |= 0x8000u;
+                    }
+                    if (!banned) {
+                        const uint32_t to = atomicAdd(&ss->n_listed, 1u);
+                        sm->tkey[to] = __float_as_uint(x);
+                        sm->tid[to] = id;
+                    }
+                }
+            }
+        }
+        if (marked || n_sp != 0u) {
+            asm volatile("bar.arrive 3, %0;" ::"n"(NT) : "memory");
+        }
+        if (counted) {
+            asm volatile("bar.sync 4, %0;" ::"n"(NT) : "memory");
+            if (ss->n_slots != 0u) {
+                // The candidates' marks name their counters.
+                each_four([&](const uint4 &x) {
+                    uint32_t at, m[4] = {0, 0, 0, 0};
+                    m[0] = place_of(x.x, at) == rank ? mark16[at] & 0x7FFFu : 0u;
+                    m[1] = place_of(x.y, at) == rank ? mark16[at] & 0x7FFFu : 0u;
+                    m[2] = place_of(x.z, at) == rank ? mark16[at] & 0x7FFFu : 0u;
+                    m[3] = place_of(x.w, at) == rank ? mark16[at] & 0x7FFFu : 0u;
+                    if (max(max(m[0], m[1]), max(m[2], m[3])) >= 2u) {
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            if (m[e] >= 2u) {
+                                atomicAdd(&sm->thist[m[e] - 2u], 1u);
+                            }
+                        }
+                    }
+                });
+                asm volatile("bar.arrive 5, %0;" ::"n"(NT) : "memory");
+            }
+        }
+        marker_ends();
+        return;
     }
     float best = neg_inf(), bm = neg_inf();
     uint32_t best_j = NONE;
     bool bad = false;
     uint4 best_v = make_uint4(0, 0, 0, 0);
     for (uint32_t b = 0;;) {
-        const uint32_t h_end = min(h_rounds, (b + 1u) * h_per);
-        for (uint32_t h_at = min(h_rounds, b * h_per); h_at < h_end; h_at += HU) {
-            if (h_at != 0u) {
-#pragma unroll
-                for (uint32_t i = 0; i < HU; ++i) {
-                    const uint32_t at = (h_at + i) * h_step + h_first;
-                    hx[i] = (at < n4 && h_at + i < h_end) ? __ldg(h4 + at) : no_ids;
-                }
-            } else {
-#pragma unroll
-                for (uint32_t i = 0; i < HU; ++i) {
-                    const uint32_t at = i * h_step + h_first;
-                    if (at >= n4 || i >= h_end) {
-                        hx[i] = no_ids;
-                    } else if (at >= room4) {
-                        hx[i] = __ldg(h4 + at);
-                    }
-                }
-            }
-            with_way(ca.share == 0u, [&](auto way) {
-#pragma unroll
-                for (uint32_t i = 0; i < HU; ++i) {
-                    mark_id(way, hx[i].x);
-                    mark_id(way, hx[i].y);
-                    mark_id(way, hx[i].z);
-                    mark_id(way, hx[i].w);
-                }
-            });
-        }
-        if (shared_list && b + 1u == buckets) {
-            asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-        }
         bm = neg_inf();
 #pragma unroll
         for (uint32_t i = 0; i < SPL_U; ++i) {
@@ -942,7 +867,6 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
             break;
         }
     }
-    bool joined = shared_list;  // the other blocks of the cluster are known to be running
     if (argmax_mode) {
         // Nothing adjusts a logit: every warp sends its best, equal values in favour of
         // the lowest id (within a thread the ids rise).
@@ -963,9 +887,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         const uint32_t m = __reduce_max_sync(FULL, key);
         const uint32_t mi = __reduce_min_sync(FULL, key == m ? id : NONE);
         if (blocks > 1u) {
-            if (!joined) {
-                asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-            }
+            asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
             if (lane == 0) {
                 put_2u32(peer_smem(&ss->pool[2u * (rank * SPL_WARPS + warp)], 0), m, mi, peer_smem(&ss->mbar_pool, 0));
             }
@@ -1021,18 +943,9 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         LILY_STAMP(PH_END);
         return;
     }
-    const bool marked = hist_len + extra_len != 0u;
-    if (marked) {
-        // What the 16-byte loads left out, and ids drawn earlier in this step.
-        const uint32_t rest = hist_len - n4 * 4u, more = rest + extra_len;
-        for (uint32_t i = tid; i < more; i += SPL_NT) {
-            const uint32_t id = i < rest ? __ldg(hist + n4 * 4u + i) : __ldcg(a.extra_ids + (i - rest));
-            with_way(true, [&](auto way) { mark_id(way, id); });
-        }
-        if (shared_list) {
-            asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");  // every block's marks have arrived
-        }
-        spl_sync();
+    LILY_STAMP(15);
+    if (marked || n_sp != 0u) {
+        asm volatile("bar.sync 3, %0;" ::"n"(NT) : "memory");
     }
     if (draws && row < a.spec.n_spec) {
         spec_ahead(a.spec, row, vocab, ahead);
@@ -1076,48 +989,6 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         }
         return m;
     };
-    if (n_sp != 0u) {
-        // The ids on the bias or ban list that are this block's, each by the thread of
-        // its first entry: marked, so that the stream's candidates leave them out, and
-        // a candidate of its own with its bias entries added in list order (a banned
-        // id is none).
-        if (!marked) {
-            spl_sync();  // (the lists are in shared memory)
-        }
-        for (uint32_t j = tid; j < n_sp; j += SPL_NT) {
-            const uint32_t id = sm->sp_ids[j];
-            uint32_t at;
-            if (place_of(id, at) != rank) {
-                continue;
-            }
-            float x = widen(row_ptr[id]);
-            bool first = true, banned = false;
-#pragma unroll 4
-            for (uint32_t e = 0; e < n_sp; ++e) {
-                if (sm->sp_ids[e] == id) {
-                    first = first && e >= j;
-                    banned = banned || e >= n_bias;
-                    if (e < n_bias) {
-                        x = __fadd_rn(x, sm->sp_vals[e]);
-                    }
-                }
-            }
-            if (first) {
-                if (mark_mode == MARK_BYTES) {
-                    mark8[at] |= 0x80u;
-                } else {
-                    mark16[at] |= 0x8000u;
-                }
-                if (!banned) {
-                    const uint32_t to = atomicAdd(&ss->n_listed, 1u);
-                    sm->tkey[to] = __float_as_uint(x);
-                    sm->tid[to] = id;
-                }
-            }
-        }
-        spl_sync();
-    }
-
     // ---- 2. the bound
     auto id_at = [&](uint32_t j, uint32_t e) -> uint32_t {  // element e of this lane's vector of piece j of the block
         return ((((j << log_blocks) | rank) * 32u + lane) * PER + e) - skip;
@@ -1133,14 +1004,15 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
                 e = vec_get<T>(best_v, (uint32_t)i) == best ? (uint32_t)i : e;
             }
             const uint32_t m = mark_of(id_at(warp + SPL_WARPS * best_j, e));
-            x = (m & LISTED) ? neg_inf() : penalised(x, m);
+            // (Not yet counted: left out, which can only lower the bound.)
+            x = (m & LISTED) || (counted && m != 0u) ? neg_inf() : penalised(x, m);
         }
         key = key_of(__fadd_rn(x, 0.0f));
     }
     if (bad) {
         ss->hard = 1;  // (read after the next barrier)
     }
-    if (blocks > 1u && !joined) {
+    if (blocks > 1u) {
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     }
     uint32_t bound_key = 0;
@@ -1341,15 +1213,28 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         if (n_flagged > SPL_FLAGGED) {
             ss->hard = 1;
         } else {
-            // (Each of them again, from L2: a vector per thread.)
-            for (uint32_t i = tid; i < n_flagged * SPL_U; i += SPL_NT) {
-                const uint32_t f = ss->flagged[i / SPL_U], owner = f % SPL_NT;
-                const uint32_t j = (owner >> 5) + SPL_WARPS * ((f / SPL_NT) * SPL_U + i % SPL_U);
-                const uint32_t t = (j << log_blocks) | rank, v = t * 32u + (owner & 31u);
-                const uint4 x = (t < whole_end && (t != 0u || skip == 0u)) ? __ldg(vec0 - lane + v)
-                                                                           : edge_vec<T>(row_ptr, vocab, skip, v);
-                if (vec_max<T>(x) >= least) {
-                    hit(x, v * PER - skip);
+            // (Each of them again, from L2: four vectors per thread at a time.)
+            for (uint32_t i0 = tid; i0 < n_flagged * SPL_U; i0 += 4u * SPL_NT) {
+                uint4 x[4];
+                uint32_t v[4];
+#pragma unroll
+                for (uint32_t h = 0; h < 4u; ++h) {
+                    const uint32_t i = i0 + h * SPL_NT;
+                    v[h] = NONE;
+                    if (i < n_flagged * SPL_U) {
+                        const uint32_t f = ss->flagged[i / SPL_U], owner = f % SPL_NT;
+                        const uint32_t j = (owner >> 5) + SPL_WARPS * ((f / SPL_NT) * SPL_U + i % SPL_U);
+                        const uint32_t t = (j << log_blocks) | rank;
+                        v[h] = t * 32u + (owner & 31u);
+                        x[h] = (t < whole_end && (t != 0u || skip == 0u)) ? __ldg(vec0 - lane + v[h])
+                                                                           : edge_vec<T>(row_ptr, vocab, skip, v[h]);
+                    }
+                }
+#pragma unroll
+                for (uint32_t h = 0; h < 4u; ++h) {
+                    if (v[h] != NONE && vec_max<T>(x[h]) >= least) {
+                        hit(x[h], v[h] * PER - skip);
+                    }
                 }
             }
         }
@@ -1363,47 +1248,197 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
     uint2 *cand = reinterpret_cast<uint2 *>(sm->key);  // over key and id: CAP of them, a region per block
     const uint32_t bar = blocks > 1u ? peer_smem(&ss->mbar_cand, 0) : 0u;
     const uint32_t cand_at = blocks > 1u ? peer_smem(cand + rank * cap, 0) : 0u;
-    if (n_hits <= SPL_HITS && ss->hard == 0u) {
-        const uint32_t n_elem = n_hits * PER, n_all = n_elem + ss->n_listed;
+    // (Wide rows: first here, over the pool, which has served.)
+    constexpr uint32_t OWN = SPL_MAX_BLOCKS * SPL_NT / 2u;
+    unsigned long long *own = reinterpret_cast<unsigned long long *>(ss->tmax);
+    const uint32_t most = wide ? min(cap, OWN) : cap;
+    // f(id, logit, whether it comes from the bias list) for every one that may be among
+    // the best: a thread per vector, mostly with one such logit.
+    const uint32_t n_vecs = n_hits <= SPL_HITS && ss->hard == 0u ? n_hits : 0u;
+    const uint32_t n_all = n_vecs + (ss->hard == 0u ? ss->n_listed : 0u);
+    auto each_logit = [&](auto f) {
         for (uint32_t i = tid; i < n_all; i += SPL_NT) {
-            uint32_t id;
-            float x;
-            if (i < n_elem) {
-                const T l = reinterpret_cast<const T *>(hits)[i];
-                x = widen(l);
-                id = ss->hit_at[i / PER] + i % PER;
-                if (!(x >= least) || id >= vocab) {
-                    continue;
+            if (i < n_vecs) {
+                const uint4 x = hits[i];
+                const uint32_t first_id = ss->hit_at[i];
+                uint32_t pass = 0;
+#pragma unroll
+                for (uint32_t e = 0; e < PER; ++e) {
+                    pass |= vec_get<T>(x, e) >= least ? 1u << e : 0u;
+                }
+                for (; pass != 0u; pass &= pass - 1u) {
+                    const uint32_t e = (uint32_t)__ffs(pass) - 1u;
+                    if (first_id + e < vocab) {
+                        f(first_id + e, vec_get<T>(x, e), false);
+                    }
                 }
             } else {
-                x = __uint_as_float(sm->tkey[i - n_elem]);
-                id = sm->tid[i - n_elem];
+                f(sm->tid[i - n_vecs], __uint_as_float(sm->tkey[i - n_vecs]), true);
             }
-            if (use_pen || n_sp != 0u) {
-                const uint32_t m = mark_of(id);
-                if ((m & LISTED) && i < n_elem) {
-                    continue;  // (its own entry stands for it)
+        }
+    };
+    uint32_t n_slots = 0;
+    if (counted) {
+        // The markers count the candidates' ids in the history: a counter each.
+        each_logit([&](uint32_t id, float, bool listed) {
+            const uint32_t m = mark_of(id);
+            if ((m & ~LISTED) != 0u && (listed || !(m & LISTED))) {
+                const uint32_t to = atomicAdd(&ss->n_slots, 1u);
+                if (to < TH_BINS) {
+                    uint32_t at;
+                    place_of(id, at);
+                    sm->thist[to] = 0;
+                    mark16[at] = (uint16_t)((mark16[at] & 0x8000u) | (to + 2u));
                 }
-                x = penalised(x, m & ~LISTED);
             }
-            const float quot = __fdiv_rn(x, in.temp);
-            if (x >= least || quot != quot) {
-                const uint32_t to = atomicAdd(&ss->n_sent, 1u);
-                if (to < cap) {
-                    const uint32_t key_q = quot != quot ? SPL_NAN_KEY : key_of(quot);
-                    if (blocks > 1u) {
-                        put_2u32(cand_at + to * 8u, key_q, id, bar);
-                    } else {
-                        cand[to] = make_uint2(key_q, id);
-                    }
+        });
+        asm volatile("bar.sync 1, %0;\n bar.arrive 4, %1;" ::"n"(SPL_NT), "n"(NT) : "memory");
+        n_slots = ss->n_slots;
+        if (n_slots != 0u) {
+            asm volatile("bar.sync 5, %0;" ::"n"(NT) : "memory");
+        }
+    }
+    each_logit([&](uint32_t id, float x, bool listed) {
+        if (use_pen || n_sp != 0u) {
+            uint32_t m = mark_of(id);
+            if ((m & LISTED) && !listed) {
+                return;  // (its own entry stands for it)
+            }
+            m &= ~LISTED;
+            if (counted && m != 0u) {
+                m = m >= 2u ? sm->thist[m - 2u] : 0u;
+            }
+            x = penalised(x, m);
+        }
+        const float quot = __fdiv_rn(x, in.temp);
+        if (x >= least || quot != quot) {
+            const uint32_t to = atomicAdd(&ss->n_sent, 1u);
+            if (to < most) {
+                if (quot != quot) {
+                    ss->hard = 1;
+                }
+                const uint32_t key_q = key_of(quot);
+                if (wide) {
+                    own[to] = ((unsigned long long)key_q << 32) | (uint32_t)~id;
+                } else if (blocks > 1u) {
+                    put_2u32(cand_at + to * 8u, key_q, id, bar);
+                } else {
+                    cand[to] = make_uint2(key_q, id);
                 }
             }
         }
-    }
+    });
     spl_sync();
+    const uint32_t sent = min(ss->n_sent, most);
+    const uint32_t hard = (ss->hard != 0u || n_hits > SPL_HITS || ss->n_sent > most || n_slots > TH_BINS) ? 1u : 0u;
+    const bool counts_draw = use_pen && table_mode;
+    if (wide) {
+        // Every block sorts its list and sends it to all blocks; then each knows its
+        // entries' ranks in the row (their places in the eight lists, by bisection) and
+        // sends them to the first block, to where they belong. (Merged by the first block
+        // alone, 1300 entries took 6 to 9 us: gathers from one SM's shared memory.)
+        unsigned long long *lists = reinterpret_cast<unsigned long long *>(sm->key);  // over key and id: CAP
+        unsigned long long *best_of = reinterpret_cast<unsigned long long *>(ss + 1);  // SPL_SORTED (the marks have served)
+        if (tid == 0 && sent < OWN) {
+            own[sent] = 0ull;  // (they are counted in pairs)
+        }
+        spl_sync();
+        const ulonglong2 *pairs = reinterpret_cast<const ulonglong2 *>(own);
+        for (uint32_t i = tid; i < sent; i += SPL_NT) {
+            const unsigned long long mine = own[i];
+            uint32_t place = 0;
+#pragma unroll 8
+            for (uint32_t j = 0; j < (sent + 1u) / 2u; ++j) {
+                const ulonglong2 o = pairs[j];
+                place += (o.x > mine ? 1u : 0u) + (o.y > mine ? 1u : 0u);
+            }
+            (blocks > 1u ? lists + rank * cap : best_of)[place] = mine;
+        }
+        uint32_t total = sent;
+        bool lost = hard != 0u;
+        if (blocks > 1u) {
+            // (One copy per block: stores of a thread each cost the SM some 4 clocks a piece.)
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            spl_sync();
+            if (tid < blocks) {
+                const uint32_t list_bar = peer_smem(&ss->mbar_list, tid);
+                const uint32_t bytes = tid != rank ? (sent * 8u + 15u) & ~15u : 0u;
+                put_4u32(peer_smem(&ss->head[rank], tid), sent, hard, 0u, 0u, list_bar);
+                if (bytes != 0u) {
+                    asm volatile(
+                        "cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                            peer_smem(lists + rank * cap, tid)),
+                        "r"((uint32_t)__cvta_generic_to_shared(lists + rank * cap)), "r"(bytes), "r"(list_bar)
+                        : "memory");
+                }
+                arrive_expect(list_bar, bytes + 16u);
+            }
+            lost = !wait_first_phase(&ss->mbar_list);
+            const uint4 head = lane < blocks ? ss->head[lane] : make_uint4(0, 0, 0, 0);
+            total = __reduce_add_sync(FULL, head.x);
+            lost = __any_sync(FULL, lost || head.y != 0u);
+        }
+        LILY_STAMP(PH_LOCAL_SELECT);
+        if (lost || total == 0u || total > SPL_SORTED) {  // (every block decides alike)
+            if (rank == 0u) {
+                verdict(0u, ALONE);
+            }
+            return;
+        }
+        if (blocks > 1u) {
+            uint32_t n_of[SPL_MAX_BLOCKS], longest = 1;  // (its own list counts for nothing)
+#pragma unroll
+            for (uint32_t r = 0; r < SPL_MAX_BLOCKS; ++r) {
+                n_of[r] = r < blocks && r != rank ? ss->head[r].x : 0u;
+                longest = max(longest, n_of[r]);
+            }
+            for (uint32_t i = tid; i < sent; i += SPL_NT) {
+                const unsigned long long x = lists[rank * cap + i];
+                uint32_t low[SPL_MAX_BLOCKS], place = i;
+#pragma unroll
+                for (uint32_t r = 0; r < SPL_MAX_BLOCKS; ++r) {
+                    low[r] = 0;
+                }
+                // (Steps of falling powers of two: low counts the entries known to be larger.
+                // Eight independent chains of loads, no branches: that is what makes it fast.)
+                for (uint32_t step = 1u << (31 - __clz(longest)); step != 0u; step >>= 1) {
+#pragma unroll
+                    for (uint32_t r = 0; r < SPL_MAX_BLOCKS; ++r) {
+                        const uint32_t to = low[r] + step;
+                        const unsigned long long at = lists[(r * cap + min(to, cap) - 1u) & (CAP - 1u)];
+                        low[r] = (uint32_t)(to <= n_of[r]) & (uint32_t)(at > x) ? to : low[r];
+                    }
+                }
+#pragma unroll
+                for (uint32_t r = 0; r < SPL_MAX_BLOCKS; ++r) {
+                    place += low[r];
+                }
+                put_2u32(peer_smem(best_of + place, 0), (uint32_t)x, (uint32_t)(x >> 32), bar);
+            }
+            if (tid == 0) {
+                arrive_expect(bar, sent * 8u);
+            }
+            if (rank != 0u) {
+                return;
+            }
+            LILY_STAMP(PH_MERGE);
+            if (!wait_first_phase(&ss->mbar_cand)) {
+                ss->hard = 2;
+            }
+        }
+        spl_sync();
+        if (ss->hard != 0u) {
+            verdict(0u, ALONE);
+            return;
+        }
+        verdict(0u, DONE);
+        LILY_STAMP(PH_SORT);
+        split_finalize_wide(sm, ss, best_of, a, row, min(total, k), in.top_p, in.min_p,
+                            a.uniforms ? __ldg(a.uniforms + row) : in.u, counts_draw, slot);
+        LILY_STAMP(PH_END);
+        return;
+    }
     if (tid == 0) {
-        const uint32_t sent = min(ss->n_sent, cap);
-        const uint32_t hard = (ss->hard != 0u || n_hits > SPL_HITS || ss->n_sent > cap) ? 1u : 0u;
         if (blocks > 1u) {
             put_4u32(peer_smem(&ss->head[rank], 0), sent, hard, __float_as_uint(least), 0u, bar);
             arrive_expect(bar, sent * 8u + 16u);
@@ -1417,7 +1452,6 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
     }
 
     // ---- 4. ranks and the draw
-    const bool counts_draw = use_pen && table_mode;
     auto draw = [&](uint32_t n) {  // (n candidates sorted in key[] / id[]; the warp that draws)
         split_finalize(sm, a, row, n, in.top_p, in.min_p, u_row, a.uniforms ? 0u : in.step, in.seed, counts_draw, slot,
                        ahead);
@@ -1425,76 +1459,68 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
     if (blocks == 1u) {
         spl_sync();  // (head[0] and the candidates are this block's own)
     }
-    uint32_t second = 0;
-    if (!wide) {
-        // Hardly more candidates than the row keeps: one warp does the rest.
-        if (warp != 0u) {
-            if (!wait_verdict(0u)) {
-                return;
-            }
-        } else {
-            const bool late = blocks > 1u && !wait_first_phase(&ss->mbar_cand);
-            LILY_STAMP(PH_MERGE);
-            const uint4 head = lane < blocks ? ss->head[lane] : make_uint4(0, 0, 0, 0);
-            const uint32_t n = __reduce_add_sync(FULL, head.x);
-            if (__any_sync(FULL, head.y != 0u || late) || n == 0u) {
-                verdict(0u, ALONE);
-                return;
-            }
-            if (n <= SPL_SMALL_K) {
-                // Candidates `lane` and `lane + 32`: the first ends of the regions add up to places.
-                uint32_t end = head.x;
-#pragma unroll
-                for (int o = 1; o < (int)SPL_MAX_BLOCKS; o <<= 1) {
-                    const uint32_t t = __shfl_up_sync(FULL, end, o);
-                    end += lane >= (uint32_t)o ? t : 0u;
-                }
-                uint32_t r0 = 0, r1 = 0, b0 = 0, b1 = 0;
-                for (uint32_t r = 0; r + 1u < blocks; ++r) {
-                    const uint32_t e = __shfl_sync(FULL, end, (int)r);
-                    r0 = lane >= e ? r + 1u : r0;
-                    b0 = lane >= e ? e : b0;
-                    r1 = lane + 32u >= e ? r + 1u : r1;
-                    b1 = lane + 32u >= e ? e : b1;
-                }
-                const uint2 c0 = lane < n ? cand[r0 * cap + (lane - b0)] : make_uint2(0u, 0u);
-                const uint2 c1 = lane + 32u < n ? cand[r1 * cap + (lane + 32u - b1)] : make_uint2(0u, 0u);
-                if (__any_sync(FULL, c0.x == SPL_NAN_KEY || c1.x == SPL_NAN_KEY)) {
-                    verdict(0u, ALONE);
-                    return;
-                }
-                const unsigned long long m0 = lane < n ? ((unsigned long long)c0.x << 32) | (uint32_t)~c0.y : 0ull;
-                const unsigned long long m1 = lane + 32u < n ? ((unsigned long long)c1.x << 32) | (uint32_t)~c1.y : 0ull;
-                unsigned long long *packed = reinterpret_cast<unsigned long long *>(sm->tkey);
-                packed[lane] = m0;
-                packed[lane + 32u] = m1;
-                __syncwarp();
-                uint32_t p0 = 0, p1 = 0;
-                const ulonglong2 *pairs = reinterpret_cast<const ulonglong2 *>(packed);
-#pragma unroll 4
-                for (uint32_t j = 0; j < (n + 1u) / 2u; ++j) {
-                    const ulonglong2 o = pairs[j];
-                    p0 += (o.x > m0 ? 1u : 0u) + (o.y > m0 ? 1u : 0u);
-                    p1 += (o.x > m1 ? 1u : 0u) + (o.y > m1 ? 1u : 0u);
-                }
-                if (lane < n) {
-                    sm->key[p0] = c0.x;
-                    sm->id[p0] = c0.y;
-                }
-                if (lane + 32u < n) {
-                    sm->key[p1] = c1.x;
-                    sm->id[p1] = c1.y;
-                }
-                __syncwarp();
-                LILY_STAMP(PH_SORT);
-                draw(min(n, k));
-                LILY_STAMP(PH_END);
-                verdict(0u, DONE);
-                return;
-            }
-            verdict(0u, HANDS);
+    // Hardly more candidates than the row keeps: one warp does the rest.
+    if (warp != 0u) {
+        if (!wait_verdict(0u)) {
+            return;
         }
-        second = 1u;
+    } else {
+        const bool late = blocks > 1u && !wait_first_phase(&ss->mbar_cand);
+        LILY_STAMP(PH_MERGE);
+        const uint4 head = lane < blocks ? ss->head[lane] : make_uint4(0, 0, 0, 0);
+        const uint32_t n = __reduce_add_sync(FULL, head.x);
+        if (__any_sync(FULL, head.y != 0u || late) || n == 0u) {
+            verdict(0u, ALONE);
+            return;
+        }
+        if (n <= SPL_SMALL_K) {
+            // Candidates `lane` and `lane + 32`: the first ends of the regions add up to places.
+            uint32_t end = head.x;
+#pragma unroll
+            for (int o = 1; o < (int)SPL_MAX_BLOCKS; o <<= 1) {
+                const uint32_t t = __shfl_up_sync(FULL, end, o);
+                end += lane >= (uint32_t)o ? t : 0u;
+            }
+            uint32_t r0 = 0, r1 = 0, b0 = 0, b1 = 0;
+            for (uint32_t r = 0; r + 1u < blocks; ++r) {
+                const uint32_t e = __shfl_sync(FULL, end, (int)r);
+                r0 = lane >= e ? r + 1u : r0;
+                b0 = lane >= e ? e : b0;
+                r1 = lane + 32u >= e ? r + 1u : r1;
+                b1 = lane + 32u >= e ? e : b1;
+            }
+            const uint2 c0 = lane < n ? cand[r0 * cap + (lane - b0)] : make_uint2(0u, 0u);
+            const uint2 c1 = lane + 32u < n ? cand[r1 * cap + (lane + 32u - b1)] : make_uint2(0u, 0u);
+            const unsigned long long m0 = lane < n ? ((unsigned long long)c0.x << 32) | (uint32_t)~c0.y : 0ull;
+            const unsigned long long m1 = lane + 32u < n ? ((unsigned long long)c1.x << 32) | (uint32_t)~c1.y : 0ull;
+            unsigned long long *packed = reinterpret_cast<unsigned long long *>(sm->tkey);
+            packed[lane] = m0;
+            packed[lane + 32u] = m1;
+            __syncwarp();
+            uint32_t p0 = 0, p1 = 0;
+            const ulonglong2 *pairs = reinterpret_cast<const ulonglong2 *>(packed);
+#pragma unroll 4
+            for (uint32_t j = 0; j < (n + 1u) / 2u; ++j) {
+                const ulonglong2 o = pairs[j];
+                p0 += (o.x > m0 ? 1u : 0u) + (o.y > m0 ? 1u : 0u);
+                p1 += (o.x > m1 ? 1u : 0u) + (o.y > m1 ? 1u : 0u);
+            }
+            if (lane < n) {
+                sm->key[p0] = c0.x;
+                sm->id[p0] = c0.y;
+            }
+            if (lane + 32u < n) {
+                sm->key[p1] = c1.x;
+                sm->id[p1] = c1.y;
+            }
+            __syncwarp();
+            LILY_STAMP(PH_SORT);
+            draw(min(n, k));
+            LILY_STAMP(PH_END);
+            verdict(0u, DONE);
+            return;
+        }
+        verdict(0u, HANDS);
     }
     if (blocks > 1u && !wait_first_phase(&ss->mbar_cand)) {
         ss->hard = 2;
@@ -1504,21 +1530,20 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
     // Every block's bound holds for the row: what does not reach the largest is out.
     const uint32_t least_key = __reduce_max_sync(FULL, lane < blocks ? key_of(__uint_as_float(head.z)) : 0u);
     const uint32_t kmin = key_of(__fdiv_rn(float_of_key(least_key), in.temp));
-    unsigned long long *packed = reinterpret_cast<unsigned long long *>(sm->tkey);  // (key, ~id), over tkey and tid
     if (__any_sync(FULL, head.y != 0u)) {
         ss->hard = 2;
-    } else {
-        // A region to each of as many teams of warps: NaNs, and in narrow rows the live ones.
+    }
+    unsigned long long *packed = reinterpret_cast<unsigned long long *>(sm->tkey);  // (key, ~id), over tkey and tid
+    {
+        // A region to each of as many teams of whole warps: the live ones.
         const uint32_t team = SPL_NT >> log_blocks, first = tid & (team - 1u);
         const uint32_t region = tid / team, n_region = __shfl_sync(FULL, head.x, (int)region);
         const uint2 *mine = cand + region * cap;
-        bool nan = false;
-        for (uint32_t i = first; i - lane < n_region; i += team) {  // (a team is whole warps)
+        for (uint32_t i = first; i - lane < n_region; i += team) {
             const uint2 e = i < n_region ? mine[i] : make_uint2(0u, 0u);
-            nan = nan || e.x == SPL_NAN_KEY;
             const bool live = e.x >= kmin && i < n_region;
             const unsigned who = __ballot_sync(FULL, live);
-            if (who != 0u && !wide) {
+            if (who != 0u) {
                 uint32_t at = 0;
                 if (lane == 0) {
                     at = atomicAdd(&ss->n_live, (uint32_t)__popc(who));
@@ -1529,48 +1554,30 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
                 }
             }
         }
-        if (nan) {
-            ss->hard = 2;
-        }
     }
     spl_sync();
     const uint32_t n_live = ss->n_live;
-    if (ss->hard != 0u || (!wide && (n_live == 0u || n_live > KCAP))) {
-        verdict(second, ALONE);
+    if (ss->hard != 0u || n_live == 0u || n_live > KCAP) {
+        verdict(1u, ALONE);
         return;
     }
-    uint32_t n;
-    if (!wide) {
-        for (uint32_t c = tid; c < n_live; c += SPL_NT) {
-            const unsigned long long mine = packed[c];
-            uint32_t before = 0;
+    for (uint32_t c = tid; c < n_live; c += SPL_NT) {
+        const unsigned long long mine = packed[c];
+        uint32_t before = 0;
 #pragma unroll 8
-            for (uint32_t j = 0; j < n_live; ++j) {
-                before += packed[j] > mine ? 1u : 0u;
-            }
-            if (before < k) {
-                sm->key[before] = (uint32_t)(mine >> 32);
-                sm->id[before] = ~(uint32_t)mine;
-            }
+        for (uint32_t j = 0; j < n_live; ++j) {
+            before += packed[j] > mine ? 1u : 0u;
         }
-        spl_sync();
-        n = min(n_live, k);
-    } else {
-        n = split_sort_bins(sm, ss, reinterpret_cast<unsigned long long *>(ss + 1), log_blocks, k, kmin);
-        if (n == 0u) {
-            verdict(second, ALONE);
-            return;
+        if (before < k) {
+            sm->key[before] = (uint32_t)(mine >> 32);
+            sm->id[before] = ~(uint32_t)mine;
         }
     }
-    verdict(second, DONE);
+    spl_sync();
+    verdict(1u, DONE);
     LILY_STAMP(PH_SORT);
-    if (n <= SPL_SMALL_K) {
-        if (draws) {
-            draw(n);
-        }
-    } else {
-        split_finalize_wide(sm, ss, a, row, n, in.top_p, in.min_p, a.uniforms ? __ldg(a.uniforms + row) : in.u, counts_draw,
-                            slot);
+    if (draws) {
+        draw(min(n_live, k));
     }
     LILY_STAMP(PH_END);
 }
