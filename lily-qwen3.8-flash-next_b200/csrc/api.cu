@@ -10,6 +10,7 @@
 #include <mutex>
 #include <new>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/lily_batch.h"
@@ -17,7 +18,7 @@
 #include "sample_kernel.cuh"
 #include "stream_kernel.cuh"
 #include "split_args.cuh"
-#include "lmhead_kernel.cuh"
+#include "lmhead_args.cuh"
 
 namespace {
 
@@ -57,6 +58,7 @@ struct lily_sampler {
     uint32_t *part_n = nullptr;
     uint32_t *tickets = nullptr;
     uint32_t *status_word = nullptr;
+    char *arena = nullptr;  // the device workspaces below are places in it, the staging ring's host side lies behind h_status
     char *spill = nullptr;  // inline parameters of rows the row kernel hands to the general code
     uint32_t *counts_scratch = nullptr;
     uint32_t *counts_table = nullptr;
@@ -78,8 +80,13 @@ struct lily_sampler {
     std::vector<char> shard_bytes;
     float *lm_logits = nullptr;  // LILY_FLAG_LMHEAD: F32 [64, lm_ld]
     uint64_t lm_ld = 0;
-    float *lm_hsum = nullptr;    // affine heads: sums of hidden values, F32 [BIAS_MAX_GROUPS, 64]
-    bool lm_attr = false, lm_attr_affine = false, lm_attr_q4 = false, lm_attr_bias = false, merge_attr = false;
+    // The LM head's workspaces: the hidden states' images, the sums of tiles that two
+    // blocks work on (for lm_tokens padded tokens) and the flags that say they are there.
+    char *lm_prepared = nullptr;
+    float *lm_part = nullptr;
+    uint32_t *lm_flags = nullptr;
+    uint32_t lm_tokens = 0;
+    bool merge_attr = false;
 };
 
 namespace {
@@ -510,69 +517,60 @@ int32_t lily_sampler_create(int32_t device, uint32_t vocab, uint32_t max_rows,
                                     device)) != cudaSuccess) {
         return bail(e, "shared memory limit");
     }
-    if ((e = cudaMalloc(&h->part, (size_t)max_rows * lily::CAP * sizeof(uint2))) != cudaSuccess) {
-        return bail(e, "candidate scratch");
-    }
-    if ((e = cudaMalloc(&h->part_n, (size_t)max_rows * lily::MAX_SLICES * 4)) != cudaSuccess) {
-        return bail(e, "slice counters");
-    }
-    if ((e = cudaMalloc(&h->tickets, (size_t)max_rows * 4)) != cudaSuccess) {
-        return bail(e, "tickets");
-    }
-    if ((e = cudaMemset(h->tickets, 0, (size_t)max_rows * 4)) != cudaSuccess) {
-        return bail(e, "tickets");
-    }
-    if ((e = cudaMalloc(&h->spill, INLINE_ROWS_MAX * (sizeof(lily_sampling_params_t) + 12))) != cudaSuccess) {
-        return bail(e, "parameter words of the row kernel");
-    }
-    if ((e = cudaMalloc(&h->status_word, 4)) != cudaSuccess ||
-        (e = cudaMemset(h->status_word, 0, 4)) != cudaSuccess) {
-        return bail(e, "status word");
-    }
-    if ((e = cudaMallocHost(&h->h_status, 4)) != cudaSuccess) {
-        return bail(e, "status word (host)");
-    }
-    if ((e = cudaMalloc(&h->lm_hsum, (size_t)lily_head::BIAS_MAX_GROUPS * lily_head::TOK * sizeof(float))) !=
-        cudaSuccess) {
-        return bail(e, "LM head group sums");
-    }
-    if (max_history > 0u) {
-        // A row with a frequency penalty over a history LIST counts the list's ids
-        // into this table and clears it again before the launch ends: all zero
-        // between launches. Made here, never inside a draw.
-        const size_t bytes = (size_t)max_rows * vocab * sizeof(uint32_t);
-        if ((e = cudaMalloc(&h->counts_scratch, bytes)) != cudaSuccess ||
-            (e = cudaMemset(h->counts_scratch, 0, bytes)) != cudaSuccess) {
-            return bail(e, "count table of the history lists");
+    // One device allocation, one pinned one: an allocation takes some 0.3 ms, whatever
+    // its size. What has to start from zero comes first, cleared by one call.
+    size_t bytes = 0, cleared = 0;
+    h->lm_ld = ((uint64_t)vocab + 3u) & ~uint64_t(3);
+    h->lm_tokens = lily_head::padded_tokens(max_rows < lily_head::TOK ? max_rows : lily_head::TOK);
+    for (int pass = 0; pass < 2; ++pass) {  // sizes, then addresses
+        if (pass == 1) {
+            if ((e = cudaMalloc(&h->arena, bytes)) != cudaSuccess || (e = cudaMemset(h->arena, 0, cleared)) != cudaSuccess) {
+                return bail(e, "device workspaces");
+            }
         }
-    }
-    if (flags & LILY_FLAG_COUNTS_TABLE) {
-        const size_t cb = (size_t)max_rows * vocab * 4, sb = (size_t)max_rows * h->seen_words * 4;
-        if ((e = cudaMalloc(&h->counts_table, cb)) != cudaSuccess ||
-            (e = cudaMemset(h->counts_table, 0, cb)) != cudaSuccess ||
-            (e = cudaMalloc(&h->seen_table, sb)) != cudaSuccess ||
-            (e = cudaMemset(h->seen_table, 0, sb)) != cudaSuccess) {
-            return bail(e, "histogram slots");
+        size_t at = 0;
+        auto place = [&](auto *&p, size_t n) {
+            if (pass == 1) {
+                p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(h->arena + at);
+            }
+            at += (n + 255u) & ~size_t(255);
+        };
+        place(h->status_word, 4);
+        place(h->tickets, (size_t)max_rows * 4);
+        if (max_history > 0u) {
+            // A row with a frequency penalty over a history LIST counts the list's ids
+            // into this table and clears it again before the launch ends: all zero
+            // between launches. Made here, never inside a draw.
+            place(h->counts_scratch, (size_t)max_rows * vocab * sizeof(uint32_t));
         }
-    }
-    if (flags & LILY_FLAG_LMHEAD) {
-        h->lm_ld = ((uint64_t)vocab + 3u) & ~uint64_t(3);
-        if ((e = cudaMalloc(&h->lm_logits, (size_t)lily_head::TOK * h->lm_ld * sizeof(float))) !=
-            cudaSuccess) {
-            return bail(e, "LM head logits");
+        if (flags & LILY_FLAG_COUNTS_TABLE) {
+            place(h->counts_table, (size_t)max_rows * vocab * 4);
+            place(h->seen_table, (size_t)max_rows * h->seen_words * 4);
         }
-    }
-    if (flags & LILY_FLAG_PHASE_CLOCKS) {
-        const size_t pb = (size_t)max_rows * LILY_MAX_SLICES * LILY_PHASES * sizeof(long long);
-        if ((e = cudaMalloc(&h->phase_clocks, pb)) != cudaSuccess ||
-            (e = cudaMemset(h->phase_clocks, 0, pb)) != cudaSuccess) {
-            return bail(e, "phase clocks");
+        if (flags & LILY_FLAG_PHASE_CLOCKS) {
+            place(h->phase_clocks, (size_t)max_rows * LILY_MAX_SLICES * LILY_PHASES * sizeof(long long));
         }
+        cleared = at;
+        place(h->part, (size_t)max_rows * lily::CAP * sizeof(uint2));
+        place(h->part_n, (size_t)max_rows * lily::MAX_SLICES * 4);
+        place(h->spill, INLINE_ROWS_MAX * (sizeof(lily_sampling_params_t) + 12));
+        place(h->lm_prepared, lily_head::prepared_bytes());
+        place(h->lm_part, lily_head::part_bytes(h->lm_tokens, (uint32_t)h->sm_count));
+        place(h->lm_flags, lily_head::flag_bytes((uint32_t)h->sm_count));
+        if (flags & LILY_FLAG_LMHEAD) {
+            place(h->lm_logits, (size_t)lily_head::TOK * h->lm_ld * sizeof(float));
+        }
+        for (int i = 0; i < RING; ++i) {
+            place(h->d_stage[i], h->layout.total);
+        }
+        bytes = at;
+    }
+    if ((e = cudaMallocHost(&h->h_status, 256 + RING * h->layout.total)) != cudaSuccess) {
+        return bail(e, "pinned workspaces");
     }
     for (int i = 0; i < RING; ++i) {
-        if ((e = cudaMallocHost(&h->h_stage[i], h->layout.total)) != cudaSuccess ||
-            (e = cudaMalloc(&h->d_stage[i], h->layout.total)) != cudaSuccess ||
-            (e = cudaEventCreateWithFlags(&h->ev[i], cudaEventDisableTiming)) != cudaSuccess) {
+        h->h_stage[i] = reinterpret_cast<char *>(h->h_status) + 256 + i * h->layout.total;
+        if ((e = cudaEventCreateWithFlags(&h->ev[i], cudaEventDisableTiming)) != cudaSuccess) {
             return bail(e, "staging ring");
         }
     }
@@ -589,25 +587,11 @@ void lily_sampler_destroy(lily_sampler_t *h) {
     }
     DeviceGuard guard(h->device);
     cudaDeviceSynchronize();
-    cudaFree(h->part);
-    cudaFree(h->part_n);
-    cudaFree(h->tickets);
-    cudaFree(h->status_word);
-    cudaFree(h->spill);
-    cudaFree(h->counts_scratch);
-    cudaFree(h->counts_table);
-    cudaFree(h->seen_table);
-    cudaFree(h->phase_clocks);
-    cudaFree(h->lm_logits);
-    cudaFree(h->lm_hsum);
+    cudaFree(h->arena);
     if (h->h_status) {
         cudaFreeHost(h->h_status);
     }
     for (int i = 0; i < RING; ++i) {
-        if (h->h_stage[i]) {
-            cudaFreeHost(h->h_stage[i]);
-        }
-        cudaFree(h->d_stage[i]);
         if (h->ev[i]) {
             cudaEventDestroy(h->ev[i]);
         }
@@ -1077,7 +1061,7 @@ int32_t lmhead_launch(lily_sampler *h, cudaStream_t stream, const lily_lmhead_t 
         return fail(h, LILY_ERR_ARG, "weights, scales, biases and hidden rows must be 16-byte aligned");
     }
     const bool affine = head->biases_bf16 != nullptr;
-    if (affine && head->hidden / lily_head::GROUP_K > lily_head::BIAS_MAX_GROUPS) {
+    if (affine && head->hidden > lily_head::CHUNK_K) {
         return fail(h, LILY_ERR_CAPACITY, "an affine head takes a hidden size of at most 8192");
     }
     if (head->code_bits != 0u && head->code_bits != 8u && head->code_bits != 4u) {
@@ -1087,78 +1071,53 @@ int32_t lmhead_launch(lily_sampler *h, cudaStream_t stream, const lily_lmhead_t 
     if (q4 && !affine) {
         return fail(h, LILY_ERR_ARG, "4-bit codes are the affine storage: biases must be set");
     }
-    auto kernel = q4 ? lily_head::lmhead_int8_kernel<lily_head::VARIANT_AFFINE | lily_head::VARIANT_Q4>
-                     : affine ? lily_head::lmhead_int8_kernel<lily_head::VARIANT_AFFINE>
-                              : lily_head::lmhead_int8_kernel<0>;
-    bool &attr_set = q4 ? h->lm_attr_q4 : affine ? h->lm_attr_affine : h->lm_attr;
-    if (!attr_set) {
-        CU(h, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)lily_head::Smem::BYTES));
-        attr_set = true;
-    }
     EncodeTiledFn encode = tensor_map_encoder();
     if (encode == nullptr) {
         return fail(h, LILY_ERR_CUDA, "the driver does not offer cuTensorMapEncodeTiled");
     }
     lily_head::Args a;
     {
-        // Weights: uint8 [rows, hidden] (4-bit codes: [rows, hidden / 2]), boxes of 256 rows x 128 bytes.
+        // Weights: uint8 [rows, hidden] (4-bit codes: [rows, hidden / 2]), boxes of 256 rows x
+        // 128 bytes, fetched 256 bytes at a time: the next box along the row finds its half in
+        // L2 (262144 x 4096, 16 tokens: 214 us with promotion to 128 bytes, 190 with this).
         const cuuint64_t row_bytes = q4 ? head->hidden / 2u : head->hidden;
         const cuuint64_t dims[2] = {row_bytes, head->rows};
         const cuuint64_t strides[1] = {row_bytes};
-        const cuuint32_t box[2] = {(cuuint32_t)(lily_head::GROUP_K * lily_head::RAW_GROUPS),
-                                   (cuuint32_t)lily_head::TILE_ROWS};
+        const cuuint32_t box[2] = {128, (cuuint32_t)lily_head::TILE_ROWS};
         const cuuint32_t estr[2] = {1, 1};
         if (encode(&a.w_map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<int8_t *>(head->weights), dims,
                    strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                   CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) {
+                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) {
             return fail(h, LILY_ERR_CUDA, "cuTensorMapEncodeTiled refused the weights");
         }
     }
-    {
-        // Hidden states: bf16 [tokens, hidden], boxes of 64 rows x 64 columns.
-        const cuuint64_t dims[2] = {head->hidden, tokens};
-        const cuuint64_t strides[1] = {hidden_ld * 2u};
-        const cuuint32_t box[2] = {(cuuint32_t)lily_head::GROUP_K, (cuuint32_t)lily_head::TOK};
-        const cuuint32_t estr[2] = {1, 1};
-        if (encode(&a.h_map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(hidden), dims, strides,
-                   box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                   CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) {
-            return fail(h, LILY_ERR_CUDA, "cuTensorMapEncodeTiled refused the hidden states");
-        }
-    }
-    a.scales = static_cast<const __nv_bfloat16 *>(head->scales_bf16);
-    if (affine) {
-        const uint32_t head_groups = head->hidden / lily_head::GROUP_K;
-        lily_head::hidden_group_sums_kernel<<<head_groups, lily_head::TOK, 0, stream>>>(
-            static_cast<const __nv_bfloat16 *>(hidden), hidden_ld, tokens, h->lm_hsum);
-        if (!h->lm_attr_bias) {
-            CU(h, cudaFuncSetAttribute(lily_head::affine_bias_term_kernel,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)lily_head::bias_smem_bytes(lily_head::BIAS_MAX_GROUPS)));
-            h->lm_attr_bias = true;
-        }
-        lily_head::affine_bias_term_kernel<<<(head->rows + lily_head::BIAS_ROWS - 1) / lily_head::BIAS_ROWS,
-                                             lily_head::BIAS_THREADS, lily_head::bias_smem_bytes(head_groups),
-                                             stream>>>(
-            h->lm_hsum, tokens, static_cast<const __nv_bfloat16 *>(head->scales_bf16),
-            static_cast<const __nv_bfloat16 *>(head->biases_bf16), head_groups, head->rows, out, out_ld,
-            q4 ? 0.0f : 128.0f);
-        CU(h, cudaGetLastError());
-    }
+    const lily_head::Format format = q4 ? lily_head::FMT_U4 : affine ? lily_head::FMT_U8 : lily_head::FMT_S8;
+    a.scale_ld = head->hidden / lily_head::GROUP_K;
     a.tokens = tokens;
-    a.k = head->hidden;
     a.rows = head->rows;
     a.out = out;
     a.ldo = out_ld;
+    a.prep = lily_head::prepared_at(h->lm_prepared);
+    a.part = h->lm_part;
+    a.flags = h->lm_flags;
+    // (The sums' place is laid out for the handle's rows; a call of more gives every block whole tiles.)
+    a.whole_tiles = lily_head::padded_tokens(tokens) > h->lm_tokens ? 1u : 0u;
     a.status_word = h->status_word;
     a.wait_ns = h->wait_ns;
     a.lost_stage = h->lost_stage;
     h->lost_stage = 0xFFFFFFFFu;  // one launch only
-    const uint32_t tiles = (head->rows + lily_head::TILE_ROWS - 1) / lily_head::TILE_ROWS;
-    const uint32_t grid = tiles < (uint32_t)h->sm_count ? tiles : (uint32_t)h->sm_count;
-    kernel<<<grid, lily_head::THREADS, lily_head::Smem::BYTES, stream>>>(a);
-    CU(h, cudaGetLastError());
+    for (uint32_t k0 = 0; k0 < head->hidden; k0 += lily_head::CHUNK_K) {
+        const uint32_t columns = head->hidden - k0 < lily_head::CHUNK_K ? head->hidden - k0 : lily_head::CHUNK_K;
+        a.groups = columns / lily_head::GROUP_K;
+        a.byte0 = q4 ? k0 / 2u : k0;
+        a.scales = static_cast<const __nv_bfloat16 *>(head->scales_bf16) + k0 / lily_head::GROUP_K;
+        a.biases = affine ? static_cast<const __nv_bfloat16 *>(head->biases_bf16) + k0 / lily_head::GROUP_K : nullptr;
+        a.accumulate = k0 != 0u ? 1u : 0u;
+        CU(h, lily_head::launch_prepare(a.prep, static_cast<const __nv_bfloat16 *>(hidden) + k0, hidden_ld, tokens,
+                                        a.groups, format, a.flags, (uint32_t)h->sm_count, stream));
+        CU(h, lily_head::launch_head(a, format, (uint32_t)h->sm_count, stream));
+        a.lost_stage = 0xFFFFFFFFu;
+    }
     return LILY_OK;
 }
 

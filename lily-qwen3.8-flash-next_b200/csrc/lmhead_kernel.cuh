@@ -1,130 +1,112 @@
-// The 8-bit LM head that feeds the sampler: logits[t, n] = sum over column
-// groups g of scale[n, g] * (sum over the group's 64 columns of w[n, c] * h[t, c]),
-// w int8 (symmetric), scale bf16 per 64 columns, h bf16, everything summed in
-// binary32. It stands where the reference projects the hidden state through
-// its quantised head before sampling (gemv_quant, src/kernels/quant.rs:141-175,
-// called from src/qwen4exp/model.rs:2999-3006); the reference's format is
-// affine 4/8-bit, this one is the symmetric int8 layout of the vocab-sharded
-// configuration, so parity here is by tolerance against a binary32 CPU sum.
-// The same kernel (VARIANT bit 5) takes the reference's own 8-bit storage, MLX
-// affine (src/weights.rs:21-36; gemv_q8, src/kernels/metal/quant.metal:
-// 124-160): w = scale * q + bias with q an unsigned byte. The converters widen
-// q - 128 (again exact in bf16, and for the same three instructions); the
-// term that leaves out, (128 * scale + bias) * (sum of the group's 64 hidden
-// values) summed over the groups, is written to the output by a small kernel
-// that runs first (affine_bias_term_kernel); the epilogue's sums start from it.
+// The quantised LM head that feeds the sampler: logits[t, n] = sum over column groups g
+// of scale[n, g] * (sum over the group's 64 columns of w[n, c] * h[t, c]), w int8
+// (symmetric), scale bf16 per 64 columns, h bf16, everything summed in binary32. It
+// stands where the reference projects the hidden state through its quantised head
+// before sampling (gemv_quant, src/kernels/quant.rs:141-175, called from
+// src/qwen4exp/model.rs:2999-3006). The reference's own storage, MLX affine
+// (src/weights.rs:21-36; gemv_q8, src/kernels/metal/quant.metal:124-160; 4 bits:
+// :44-66), is w = scale * q + bias: the converters widen q - 128 (4 bits: q), and the
+// epilogue adds (128 * scale + bias) * (sum of the group's hidden values).
 //
-// sm_100a only. The weights are the only large operand (1 byte per
-// multiply-add), so the kernel is a stream of them through the tensor cores,
-// one persistent block per SM, warps specialised:
+// The weights are the only large operand, so the kernel is a stream of them through
+// the tensor cores, one persistent block per SM, warps specialised:
 //
-//   * a tile is 256 vocabulary rows. One thread asks the copy engine (TMA,
-//     128-byte swizzle) for 256 rows x 128 bytes of int8 per stage, four
-//     stages deep, and for each group's 64 x 64 slice of the hidden states,
-//     which lands in the swizzled K-major layout the multiplier's B operand
-//     descriptor names;
-//   * eight warps own one tile row per thread: per 64-column group a thread
-//     widens its row's 64 bytes to bf16 exactly (every int8 is a bf16) and
-//     stores them with tcgen05.st into TENSOR MEMORY, where the multiplier
-//     reads its A operand (lane = row, two bf16 per column): the widened
-//     weights never touch shared memory;
-//   * two threads (one per 128 rows) issue, per group, 4 tcgen05.mma each
-//     (M = 128 rows, N = 64 tokens, K = 16) into a TMEM accumulator that
-//     starts from zero: products of two bf16 are exact in binary32, so only
-//     the order of the 64 adds differs from a sequential sum. One commit per
-//     thread and group completes the group's "done" barrier, which frees the
-//     group's operand slots and hands its sums to the epilogue;
-//   * sixteen warps read each group's sums back with tcgen05.ld, multiply by
-//     the row's scale of that group and add into registers: the group sums
-//     cannot stay in TMEM across groups because each has its own scale;
-//   * after the last group the tile's 256 x 64 logits go to global memory.
+//   * one thread asks the copy engine (TMA, 128-byte swizzle) for 256 rows x 128 bytes
+//     of weights per stage, another for each group's slice of the hidden states (a
+//     ready image, see prepare_hidden_kernel);
+//   * converter warps own one tile row per thread: they widen a group's 64 weights
+//     exactly to 16 bits and store them with tcgen05.st into TENSOR MEMORY, where the
+//     multiplier reads its A operand (lane = row, two values per column);
+//   * two threads, one per 128 rows, issue 4 tcgen05.mma each per group (M = 128, N =
+//     tokens, K = 16) into an accumulator that starts from zero: products of two
+//     8-bit significands are exact in binary32;
+//   * epilogue warps read each group's sums back with tcgen05.ld, multiply by the
+//     row's scale of that group and add into registers: the sums cannot stay in
+//     tensor memory across groups because each has its own scale.
 //
-// Tensor memory: 3 accumulators of 128 columns, 2 operand slots of 64.
+// The two halves of a tile are pipelines of their own (barriers, accumulators, operand
+// slots): one converts while the other multiplies.
+//
+// Binary16 or bf16. Widening a byte to binary16 costs two or three integer
+// instructions per four weights, to bf16 (whose significand does not hold 128 + 255)
+// six; the integer pipe was the busiest one. A bf16 hidden value times a power of two
+// per token fits binary16 exactly if it lies within 2^32 of the token's largest, which
+// hidden states do; a call in which one does not is multiplied in bf16, same results.
+//
+// Measured at 262144 x 4096, 64 tokens (before: bf16 only, one pipeline for both
+// halves, N = 64 always, the affine term in a kernel of its own): see the figures at
+// launch_head.
 //
 // Every wait on an mbarrier is bounded in time; a wait that runs out sets an
 // abort word, after which no wait blocks any more: the block runs to its end
 // (results are garbage, TMEM is freed) and the status word tells the host.
 #pragma once
 
-#include <cuda.h>
-#include <cuda_bf16.h>
-#include <cuda_runtime.h>
-#include <stdint.h>
+#include <cuda_fp16.h>
+
+#include <type_traits>
+
+#include "lmhead_args.cuh"
 
 namespace lily_head {
 
-constexpr int TILE_ROWS = 256;   // two M = 128 accumulators
-constexpr int TOK = 64;          // MMA N: the most hidden rows per launch
-constexpr int GROUP_K = 64;      // columns per scale group = one 128-byte bf16 atom
-constexpr int RAW_GROUPS = 2;    // groups per stage of int8 bytes
-constexpr int RAW_STAGES = 4;
-constexpr int H_SLOTS = 8;       // hidden slices in shared memory: as many groups as the stages hold
-static_assert(H_SLOTS == 8, "the hidden ring and the done ring share their indexing");
-constexpr int A_SLOTS = 2;       // bf16 weight tiles in tensor memory
-constexpr int ACC_BUFS = 3;      // accumulators in tensor memory
-constexpr uint32_t RAW_STAGE_BYTES = TILE_ROWS * GROUP_K * RAW_GROUPS;  // 32 KB
-constexpr uint32_t H_BYTES = TOK * 128;                                 // 8 KB
+// Warps: four that multiply, two that load (two idle), then converters, then the epilogue.
+constexpr int MMA_WARPS = 4;
+constexpr int WARP_LOAD_W = 4;
+constexpr int WARP_LOAD_H = 5;
+constexpr int WARP_CONV0 = 8;
+
+constexpr uint32_t RAW_STAGE_BYTES = TILE_ROWS * 128u;  // 32 KB
+constexpr uint32_t H_SLOTS = 8;    // hidden slices in shared memory
+constexpr uint32_t SUM_SLOTS = 16; // their sums: read by the epilogue, at most that far behind
+constexpr uint32_t DONE_SLOTS = 8; // ring of "group q has been multiplied" barriers
 constexpr uint32_t TMEM_COLS = 512;
-constexpr uint32_t ACC_COLS = 128;           // two row halves x 64 tokens, binary32
-constexpr uint32_t A_COLS = 64;              // two row halves x 64 bf16 = 32 columns each
-constexpr uint32_t A_COL0 = ACC_BUFS * ACC_COLS;
-static_assert(A_COL0 + A_SLOTS * A_COLS <= TMEM_COLS, "tensor memory columns");
 
-constexpr int WARP_MMA = 0;
-constexpr int WARP_LOAD = 1;
-constexpr int WARP_CONV0 = 2;
-constexpr int N_CONV_WARPS = 8;
-constexpr int WARP_EPI0 = WARP_CONV0 + N_CONV_WARPS;
-constexpr int N_EPI_WARPS = 16;  // a row's 64 tokens are split between two warps
-constexpr int WARP_MMA1 = WARP_EPI0 + N_EPI_WARPS;  // issues the multiplies of rows 128..255
-constexpr int THREADS = 32 * (WARP_MMA1 + 1);  // 864 (registers are granted as for 896)
-constexpr int DONE_SLOTS = 8;    // ring of "group q has been multiplied" barriers
-constexpr int CONV_THREADS = 32 * N_CONV_WARPS;
-constexpr int EPI_THREADS = 32 * N_EPI_WARPS;
-static_assert(CONV_THREADS == TILE_ROWS && EPI_THREADS == 2 * TILE_ROWS, "threads per tile row");
-static_assert(WARP_CONV0 % 2 == 0 && WARP_EPI0 % 2 == 0, "warp % 4 must cover all four lane quarters");
+// What depends on the (padded) number of tokens and the format. Tensor memory per half:
+// ACC_BUFS accumulators of N columns, A_SLOTS operand tiles of 32. The converters are one
+// codes is two weights to widen: two teams of converter warps.
+template <uint32_t N, int FMT>
+struct Shape {
+    static constexpr uint32_t TEAMS = N == 64u && FMT != FMT_S8 ? 1u : 2u;
+    static constexpr bool LEAN = TEAMS == 2u;  // converters of few registers
+    static constexpr uint32_t CONV_WARPS = 8u * TEAMS;
+    static constexpr uint32_t EPI_WARPS = EPILOGUE_WARPS;
+    static constexpr uint32_t THREADS = 32u * (8u + CONV_WARPS + EPI_WARPS);
+    // Registers a thread: at launch, then as the roles share them out (setmaxnreg; the
+    // shares add up to what the block was launched with, launch_one checks that).
+    static constexpr uint32_t REGS = TEAMS == 2u ? 64u : 80u;
+    static constexpr uint32_t REGS_CTRL = 40u;
+    static constexpr uint32_t REGS_CONV = TEAMS == 1u ? 64u : N == 64u ? 48u : 56u;
+    static constexpr uint32_t REGS_EPI = TEAMS == 1u ? 136u : N == 64u ? 120u : 104u;
+    static_assert(32u * (8u * REGS_CTRL + CONV_WARPS * REGS_CONV + EPI_WARPS * REGS_EPI) <= THREADS * REGS, "register shares");
+    static constexpr uint32_t ACC_BUFS = N == 64u ? 2u : 4u;
+    static constexpr uint32_t A_SLOTS = 4u;
+    static constexpr uint32_t RAW_STAGES = N == 64u ? 4u : N == 32u ? 5u : 6u;
+    static constexpr uint32_t H_BYTES = N * 128u;
+    static constexpr uint32_t A_COL0 = ACC_BUFS * N;                    // within a half's 256 columns
+    static_assert(A_COL0 + A_SLOTS * 32u <= TMEM_COLS / 2u, "tensor memory columns of a half");
+    static_assert(ACC_BUFS <= DONE_SLOTS && A_SLOTS <= DONE_SLOTS, "the rings' phases");
+    static constexpr int WARP_EPI0 = WARP_CONV0 + (int)CONV_WARPS;
 
-constexpr uint32_t STATUS_TIMEOUT_BIT = 30;  // bit of the handle's status word
-
-struct Smem {
     // Offsets from a 1024-byte aligned base.
     static constexpr uint32_t HID = 0;
     static constexpr uint32_t RAW = HID + H_SLOTS * H_BYTES;
-    static constexpr uint32_t BARS = RAW + RAW_STAGES * RAW_STAGE_BYTES;
-    static constexpr uint32_t RAW_FULL = BARS;                      // [RAW_STAGES]
-    static constexpr uint32_t RAW_EMPTY = RAW_FULL + 8 * RAW_STAGES;  // [RAW_STAGES]
-    static constexpr uint32_t A_FULL = RAW_EMPTY + 8 * RAW_STAGES;  // [A_SLOTS]
-    static constexpr uint32_t H_FULL = A_FULL + 8 * A_SLOTS;        // [H_SLOTS]
-    // DONE[q % 8] completes when both halves of group q have been multiplied:
-    // one commit per issuing thread tells the converters (slot of q free for
-    // q + 2), the loader (slot free for q + 8) and the epilogue (sums ready).
-    static constexpr uint32_t DONE = H_FULL + 8 * H_SLOTS;          // [DONE_SLOTS]
-    static constexpr uint32_t ACC_EMPTY = DONE + 8 * DONE_SLOTS;    // [ACC_BUFS]
-    static constexpr uint32_t FINAL = ACC_EMPTY + 8 * ACC_BUFS;     // [2] an issuing thread's last commit
-    static constexpr uint32_t TMEM_ADDR = FINAL + 8 * 2;
+    static constexpr uint32_t SUMS = RAW + RAW_STAGES * RAW_STAGE_BYTES;
+    static constexpr uint32_t UNSCALE = SUMS + SUM_SLOTS * N * 4u;
+    static constexpr uint32_t BARS = UNSCALE + N * 4u;
+    static constexpr uint32_t RAW_FULL = BARS;                          // [RAW_STAGES]
+    static constexpr uint32_t RAW_EMPTY = RAW_FULL + 8 * RAW_STAGES;
+    static constexpr uint32_t H_FULL = RAW_EMPTY + 8 * RAW_STAGES;      // [H_SLOTS / 2]
+    static constexpr uint32_t A_FULL = H_FULL + 8 * H_SLOTS;            // [2][A_SLOTS]
+    // DONE[half][q % 8]: a half of group q has been multiplied. One commit tells the
+    // converters (slot free), the hidden loader and the epilogue (sums ready).
+    static constexpr uint32_t DONE = A_FULL + 2 * 8 * A_SLOTS;          // [2][DONE_SLOTS]
+    static constexpr uint32_t ACC_EMPTY = DONE + 2 * 8 * DONE_SLOTS;    // [2][ACC_BUFS]
+    static constexpr uint32_t FINAL = ACC_EMPTY + 2 * 8 * ACC_BUFS;     // [MMA_WARPS] an issuing warp's last commit
+    static constexpr uint32_t TMEM_ADDR = FINAL + 8 * MMA_WARPS;
     static constexpr uint32_t ABORT = TMEM_ADDR + 4;
-    static constexpr uint32_t END = ABORT + 4;
-    static constexpr uint32_t BYTES = END + 1024;  // room to align the base
-};
-static_assert(Smem::BYTES <= 227 * 1024, "shared memory of one block");
-
-struct Args {
-    // Tiled copies (TMA), both with the 128-byte swizzle: the weights as uint8
-    // [rows, k] in boxes of 256 rows x 128 bytes, the hidden states as bf16
-    // [tokens, k] in boxes of 64 rows x 64 columns. Rows past the end read 0.
-    CUtensorMap w_map;
-    CUtensorMap h_map;
-    const __nv_bfloat16 *scales;  // [rows, hidden / 64]
-    uint32_t tokens;            // <= 64
-    uint32_t k;                 // hidden size, a multiple of 512
-    uint32_t rows;              // vocabulary rows of this shard
-    float *out;                 // [tokens, ldo]
-    uint64_t ldo;
-    uint32_t *status_word;
-    uint64_t wait_ns;           // the bound of every wait inside the kernel
-    // Test hook: block 0 does not ask for the weights of this stage (~0: none),
-    // so that the wait of their consumers runs out.
-    uint32_t lost_stage;
+    static constexpr uint32_t BYTES = ABORT + 4 + 1024;                  // room to align the base
+    static_assert(BYTES <= 227u * 1024u, "shared memory of one block");
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
@@ -217,10 +199,6 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map
         : "memory");
 }
 
-__device__ __forceinline__ void fence_async_proxy() {
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-
 // K-major operand in shared memory, 128-byte swizzle, rows 128 bytes apart,
 // 8-row groups 1024 bytes apart; the start address may be advanced by 32
 // bytes per K = 16 step inside the (1024-byte aligned) atom.
@@ -229,19 +207,49 @@ __device__ __forceinline__ uint64_t operand_desc(uint32_t addr) {
            (1ull << 46) | (2ull << 61);
 }
 
-// kind::f16: D binary32, A and B bf16, both K-major, N = 64, M = 128.
-constexpr uint32_t INSTR_DESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TOK >> 3) << 17) |
-                                ((128u >> 4) << 24);
+// Every warp of a warpgroup gives registers back or takes more.
+template <uint32_t REGS, bool MORE>
+__device__ __forceinline__ void set_registers() {
+    if (MORE) {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS));
+    } else {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS));
+    }
+}
+
+// A plain copy into shared memory (addresses and size multiples of 16 bytes); its bytes complete `bar`.
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"(src), "r"(bytes), "r"(bar)
+                 : "memory");
+}
+
+// kind::f16: D binary32, A and B both binary16 or both bf16, both K-major, M = 128.
+template <uint32_t N>
+__device__ __forceinline__ uint32_t instr_desc(bool bf16) {
+    return (1u << 4) | (bf16 ? (1u << 7) | (1u << 10) : 0u) | ((N >> 3) << 17) | ((128u >> 4) << 24);
+}
 
 // D[tmem] (+)= A[tmem] * B[smem]^T.
-__device__ __forceinline__ void mma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc,
-                                            uint32_t accumulate) {
+__device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
+                                       uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(INSTR_DESC), "r"(accumulate)
+        ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
+}
+
+// One lane of the (converged) warp.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t is;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xFFFFFFFF;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(is));
+    return is != 0u;
 }
 
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
@@ -269,6 +277,18 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16
         : "memory");
 }
 
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+        "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
+        ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
+          "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]),
+          "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]),
+          "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
+        : "memory");
+}
+
 __device__ __forceinline__ void tmem_ld_wait() {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
@@ -283,33 +303,6 @@ __device__ __forceinline__ void tc_fence_before() {
 
 __device__ __forceinline__ void tc_fence_after() {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-}
-
-// Four int8 in a word -> two words of bf16 pairs, exactly. With c = 0x43 in
-// the high byte, (0x4300 | b) & 0xFF7F is 128 + (b & 127) and
-// (0x4300 | b) & 0xFF80 is 128 or 256: their difference is the signed byte.
-// (A variant that trades the two masks for two bf16 fused multiply-adds and a
-// minimum was measured slower.)
-template <bool UNSIGNED>
-__device__ __forceinline__ void widen4(uint32_t x, uint32_t &lo, uint32_t &hi) {
-    const uint32_t t01 = __byte_perm(x, 0x43434343u, 0x5140);
-    const uint32_t t23 = __byte_perm(x, 0x43434343u, 0x5342);
-    // An unsigned byte q widens to q - 128: the same subtraction with the
-    // byte's top bit flipped in the subtrahend.
-    constexpr uint32_t FLIP = UNSIGNED ? 0x00800080u : 0u;
-    const uint32_t a01 = t01 & 0xFF7FFF7Fu, b01 = (t01 ^ FLIP) & 0xFF80FF80u;
-    const uint32_t a23 = t23 & 0xFF7FFF7Fu, b23 = (t23 ^ FLIP) & 0xFF80FF80u;
-    asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(lo) : "r"(a01), "r"(b01));
-    asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(hi) : "r"(a23), "r"(b23));
-}
-
-// The same for four bytes below 128 (4-bit codes): 0x4300 | b is 128 + b as it
-// stands, and one subtraction of 128 per pair is all that is left.
-__device__ __forceinline__ void widen4_small(uint32_t x, uint32_t &lo, uint32_t &hi) {
-    const uint32_t t01 = __byte_perm(x, 0x43434343u, 0x5140);
-    const uint32_t t23 = __byte_perm(x, 0x43434343u, 0x5342);
-    asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(lo) : "r"(t01), "r"(0x43004300u));
-    asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(hi) : "r"(t23), "r"(0x43004300u));
 }
 
 // Two binary32 values in one 64-bit register, and the packed fused
@@ -329,68 +322,195 @@ __device__ __forceinline__ void unpack2(uint64_t v, float &lo, float &hi) {
     hi = __uint_as_float(b);
 }
 
-#define LM_T0() do {} while (0)
-#define LM_ACC(var) do {} while (0)
+// 16 bytes in registers -> 64 weights' worth of A operand words (two values each).
+// Bytes: word w gives columns (4w, 4w + 2), (4w + 1, 4w + 3); nibbles: columns
+// (0, 4), (1, 5), (2, 6), (3, 7) of the word's eight. The hidden states' image has its
+// columns in the same order.
+//
+// Binary16: a byte b under the exponent of 1024 (0x6400 | b) is 1024 + b; the even
+// bytes take one masking, the odd ones one byte permute, and a subtraction makes
+// the value exact. Signed bytes have their top bit flipped first: (b ^ 0x80) - 128.
+// bf16: with c = 0x43 in the high byte, (0x4300 | b) & 0xFF7F is 128 + (b & 127) and
+// (0x4300 | b) & 0xFF80 is 128 or 256: their difference is the signed byte, and with the
+// subtrahend's top bit flipped q - 128.
+template <int FMT, bool BF16>
+__device__ __forceinline__ void widen_bytes(uint32_t x, uint32_t &even, uint32_t &odd) {
+    if (!BF16) {
+        const uint32_t y = FMT == FMT_S8 ? x ^ 0x80808080u : x;
+        const uint32_t e = (y & 0x00FF00FFu) | 0x64006400u, o = __byte_perm(y, 0x64646464u, 0x4341);
+        asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(even) : "r"(e), "r"(0x64806480u));
+        asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(odd) : "r"(o), "r"(0x64806480u));
+    } else {
+        constexpr uint32_t FLIP = FMT == FMT_S8 ? 0u : 0x00800080u;
+        const uint32_t e = (x & 0x00FF00FFu) | 0x43004300u, o = __byte_perm(x, 0x43434343u, 0x4341);
+        asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(even) : "r"(e & 0xFF7FFF7Fu), "r"((e ^ FLIP) & 0xFF80FF80u));
+        asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(odd) : "r"(o & 0xFF7FFF7Fu), "r"((o ^ FLIP) & 0xFF80FF80u));
+    }
+}
 
-// VARIANT is 0 in the product; debug builds instantiate others that leave
-// out the epilogue's math (bit 0), the conversion (bit 1), the hidden-state
-// copies (bit 3) or the weight copies (bit 4) to time the rest. Bit 5 selects
-// the affine storage (unsigned bytes, a bias per group).
-constexpr int VARIANT_AFFINE = 32;
-// Bit 6 (with bit 5): the affine storage in 4 bits, eight codes to a 32-bit word,
-// low nibble first (src/kernels/metal/quant.metal:44-66, src/weights.rs:20-36). A
-// stage's 128 bytes per row are then four groups, not two; a thread splits a word
-// into its low and high nibbles, interleaves them back into code order with two
-// byte permutes and widens the eight small bytes as it widens int8 (a code is at
-// most 15: no shift by 128, the bias term is bias * sum of the hidden values).
-constexpr int VARIANT_Q4 = 64;
-template <int VARIANT>
-__global__ void __launch_bounds__(THREADS, 1) lmhead_int8_kernel(const __grid_constant__ Args a) {
-    constexpr bool AFFINE = (VARIANT & VARIANT_AFFINE) != 0;
-    constexpr bool Q4 = (VARIANT & VARIANT_Q4) != 0;
-    static_assert(!Q4 || AFFINE, "4-bit codes come with a bias per group");
-    constexpr uint32_t RG = Q4 ? 2u * RAW_GROUPS : (uint32_t)RAW_GROUPS;  // groups per stage
+template <bool BF16>
+__device__ __forceinline__ void widen_nibbles(uint32_t x, uint32_t &a, uint32_t &b, uint32_t &c, uint32_t &d) {
+    if (!BF16) {
+        // (A nibble in the upper half of a byte stands for 16 times its value.)
+        const uint32_t y = x >> 8;
+        asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(a) : "r"((x & 0x000F000Fu) | 0x64006400u), "r"(0x64006400u));
+        asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(b) : "r"((x & 0x00F000F0u) | 0x64006400u), "r"(0x2C002C00u), "r"(0xD400D400u));
+        asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(c) : "r"((y & 0x000F000Fu) | 0x64006400u), "r"(0x64006400u));
+        asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"((y & 0x00F000F0u) | 0x64006400u), "r"(0x2C002C00u), "r"(0xD400D400u));
+    } else {
+        asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(a) : "r"((x & 0x000F000Fu) | 0x43004300u), "r"(0x43004300u));
+        asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(b) : "r"(((x >> 4) & 0x000F000Fu) | 0x43004300u), "r"(0x43004300u));
+        asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(c) : "r"(((x >> 8) & 0x000F000Fu) | 0x43004300u), "r"(0x43004300u));
+        asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(((x >> 12) & 0x000F000Fu) | 0x43004300u), "r"(0x43004300u));
+    }
+}
+
+// Grid (padded tokens): a token's images and sums. Padded tokens are zeros.
+__global__ void __launch_bounds__(256) prepare_hidden_kernel(const Prepared p, const __nv_bfloat16 *hidden, uint64_t ld,
+                                                             uint32_t tokens, uint32_t groups, int nibbles, uint32_t *flags,
+                                                             uint32_t n_flags) {
+    __shared__ uint32_t top_s;
+    const uint32_t t = blockIdx.x, padded = gridDim.x, tid = threadIdx.x;
+    if (tid == 0) {
+        top_s = 0;
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    for (uint32_t i = blockIdx.x * 256u + tid; i < n_flags; i += gridDim.x * 256u) {
+        flags[i] = 0;
+    }
+    // (Whatever this stream did before is complete now: the head kernel may read weights.)
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    constexpr uint32_t HOLD = CHUNK_K / 8u / 256u;
+    uint4 v[HOLD];
+    uint32_t top = 0;  // the largest magnitude's bits
+#pragma unroll
+    for (uint32_t j = 0; j < HOLD; ++j) {
+        const uint32_t i = tid + j * 256u;
+        v[j] = t < tokens && i < groups * 8u ? __ldg(reinterpret_cast<const uint4 *>(hidden + (uint64_t)t * ld) + i)
+                                             : make_uint4(0, 0, 0, 0);
+        const uint32_t w[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            top = max(top, max((w[e] << 16) & 0x7FFF0000u, w[e] & 0x7FFF0000u));
+        }
+    }
+    __syncthreads();
+    top = __reduce_max_sync(0xFFFFFFFFu, top);
+    if ((tid & 31u) == 0u) {
+        atomicMax(&top_s, top);
+    }
+    __syncthreads();
+    // The token's largest magnitude goes to [2^15, 2^16).
+    const int exponent = (int)(top_s >> 23);
+    const int shift = top_s == 0u ? 0 : min(142 - exponent, 126);
+    const float scale = __uint_as_float((uint32_t)(shift + 127) << 23);
+    // (A token of extreme size stays as it is: a scaled sum might overflow where its own does not.)
+    uint32_t lost = shift < -40 || shift > 40 ? 1u : 0u;
+#pragma unroll
+    for (uint32_t j = 0; j < HOLD; ++j) {
+        const uint32_t i = tid + j * 256u, g = i >> 3, chunk = i & 7u;
+        if (g >= groups) {
+            continue;  // (whole warps: groups come in eights)
+        }
+        const uint32_t w[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+        uint32_t h[4];
+        float sum = 0.0f;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float lo = __uint_as_float(w[e] << 16), hi = __uint_as_float(w[e] & 0xFFFF0000u);
+            sum += lo;
+            sum += hi;
+            const __half a = __float2half_rn(__fmul_rn(lo, scale)), b = __float2half_rn(__fmul_rn(hi, scale));
+            lost |= __half2float(a) == __fmul_rn(lo, scale) && __half2float(b) == __fmul_rn(hi, scale) ? 0u : 1u;
+            h[e] = (uint32_t)__half_as_ushort(a) | ((uint32_t)__half_as_ushort(b) << 16);
+        }
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) {
+            sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+        }
+        const size_t at = ((size_t)g * padded + t) * 8u + (chunk ^ (t & 7u));
+        auto ordered = [&](const uint32_t (&x)[4]) -> uint4 {
+            return nibbles ? make_uint4(__byte_perm(x[0], x[2], 0x5410), __byte_perm(x[0], x[2], 0x7632),
+                                        __byte_perm(x[1], x[3], 0x5410), __byte_perm(x[1], x[3], 0x7632))
+                           : make_uint4(__byte_perm(x[0], x[1], 0x5410), __byte_perm(x[0], x[1], 0x7632),
+                                        __byte_perm(x[2], x[3], 0x5410), __byte_perm(x[2], x[3], 0x7632));
+        };
+        p.image[0][at] = ordered(h);
+        p.image[1][at] = ordered(w);
+        if (chunk == 0u) {
+            p.sums[0][g * padded + t] = __fmul_rn(sum, scale);
+            p.sums[1][g * padded + t] = sum;
+        }
+    }
+    const int any = __syncthreads_or((int)lost);
+    if (tid == 0) {
+        p.unscale[t] = __uint_as_float((uint32_t)(127 - shift) << 23);
+        p.inexact[t] = any ? 1u : 0u;
+    }
+}
+
+template <uint32_t N, int FMT>
+__global__ void __launch_bounds__(Shape<N, FMT>::THREADS, 1) lmhead_kernel(const __grid_constant__ Args a) {
+    using S = Shape<N, FMT>;
+    constexpr bool AFFINE = FMT != FMT_S8;
+    constexpr uint32_t RG = FMT == FMT_U4 ? 4u : 2u;  // groups per stage
+    constexpr unsigned FULL = 0xFFFFFFFFu;
     extern __shared__ uint8_t smem_unaligned[];
     const uint32_t base = (smem_u32(smem_unaligned) + 1023u) & ~1023u;
     uint8_t *base_ptr = smem_unaligned + (base - smem_u32(smem_unaligned));
-    volatile uint32_t *abort_word = reinterpret_cast<volatile uint32_t *>(base_ptr + Smem::ABORT);
-    volatile uint32_t *tmem_word = reinterpret_cast<volatile uint32_t *>(base_ptr + Smem::TMEM_ADDR);
-
-    const uint32_t tid = threadIdx.x;
-    const uint32_t warp = tid >> 5;
-    const uint32_t lane = tid & 31u;
-
-    const uint32_t groups = a.k / GROUP_K;
-    const uint32_t n_tiles = (a.rows + TILE_ROWS - 1) / TILE_ROWS;
-    const uint32_t my_tiles = blockIdx.x < n_tiles ? (n_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0u;
-    const uint32_t total_groups = my_tiles * groups;
+    volatile uint32_t *abort_word = reinterpret_cast<volatile uint32_t *>(base_ptr + S::ABORT);
+    volatile uint32_t *tmem_word = reinterpret_cast<volatile uint32_t *>(base_ptr + S::TMEM_ADDR);
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
     const uint64_t wait_ns = a.wait_ns;
 
+    // This block's work, in units of BLOCK_GROUPS groups, numbered through all tiles: an
+    // even share of them, [lo, hi), cut where it ends. A tile that two blocks work on is
+    // one chain of sums all the same (a row's logit must not depend on how many rows the
+    // head has): its second block goes on from the first one's sums. So the beginning of
+    // a tile at the share's end comes first, then whole tiles, and the rest of the tile
+    // that the block before began comes last, when that block has long left its sums.
+    // With fewer tiles than blocks a block would wait for all of its predecessor's work:
+    // every block takes one whole tile (units of `grain`).
+    const uint32_t per_tile = a.groups / BLOCK_GROUPS;
+    const uint32_t n_tiles = (a.rows + TILE_ROWS - 1u) / TILE_ROWS;
+    const uint32_t grain = a.whole_tiles || n_tiles <= gridDim.x ? per_tile : 1u, shares = n_tiles * per_tile / grain;
+    auto share_begin = [&](uint32_t b) { return (uint32_t)((uint64_t)b * shares / gridDim.x) * grain; };
+    const uint32_t lo = share_begin(blockIdx.x), hi = share_begin(blockIdx.x + 1u), n_blocks = hi - lo;
+    const uint32_t begun = hi % per_tile;                                  // units of the tile it begins
+    const uint32_t rest = (per_tile - lo % per_tile) % per_tile;           // units of the tile it ends
+    auto unit_at = [&](uint32_t n) -> uint32_t {                           // its n-th unit
+        return n < begun ? hi - begun + n : n < n_blocks - rest ? lo + rest + (n - begun) : lo + (n - (n_blocks - rest));
+    };
+    constexpr uint32_t STAGES_PER_BLOCK = BLOCK_GROUPS / RG;
+    const uint32_t n_stages = n_blocks * STAGES_PER_BLOCK, total_groups = n_blocks * BLOCK_GROUPS;
+    // (Wait's results: true means that the block has given up.)
+    auto wait = [&](uint32_t bar, uint32_t phase) -> bool { return mbar_wait(base + bar, phase & 1u, abort_word, wait_ns); };
+
     if (tid == 0) {
-        for (int s = 0; s < RAW_STAGES; ++s) {
-            mbar_init(base + Smem::RAW_FULL + 8 * s, 1);
-            mbar_init(base + Smem::RAW_EMPTY + 8 * s, N_CONV_WARPS);
+        for (uint32_t s = 0; s < S::RAW_STAGES; ++s) {
+            mbar_init(base + S::RAW_FULL + 8 * s, 1);
+            mbar_init(base + S::RAW_EMPTY + 8 * s, S::CONV_WARPS);
         }
-        for (int s = 0; s < A_SLOTS; ++s) {
-            mbar_init(base + Smem::A_FULL + 8 * s, N_CONV_WARPS);
+        for (uint32_t s = 0; s < H_SLOTS / 2u; ++s) {
+            mbar_init(base + S::H_FULL + 8 * s, 1);
         }
-        for (int s = 0; s < H_SLOTS; ++s) {
-            mbar_init(base + Smem::H_FULL + 8 * s, 1);
+        for (uint32_t s = 0; s < 2u * S::A_SLOTS; ++s) {
+            mbar_init(base + S::A_FULL + 8 * s, 4);
         }
-        for (int s = 0; s < DONE_SLOTS; ++s) {
-            mbar_init(base + Smem::DONE + 8 * s, 2);
+        for (uint32_t s = 0; s < 2u * DONE_SLOTS; ++s) {
+            mbar_init(base + S::DONE + 8 * s, 1);
         }
-        for (int b = 0; b < ACC_BUFS; ++b) {
-            mbar_init(base + Smem::ACC_EMPTY + 8 * b, N_EPI_WARPS);
+        for (uint32_t b = 0; b < 2u * S::ACC_BUFS; ++b) {
+            mbar_init(base + S::ACC_EMPTY + 8 * b, 4);
         }
-        mbar_init(base + Smem::FINAL, 1);
-        mbar_init(base + Smem::FINAL + 8, 1);
+        for (int w = 0; w < MMA_WARPS; ++w) {
+            mbar_init(base + S::FINAL + 8 * w, 1);
+        }
         *abort_word = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == WARP_MMA) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                         base + Smem::TMEM_ADDR),
+    if (warp == 0u) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(base + S::TMEM_ADDR),
                      "r"(TMEM_COLS)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -400,304 +520,388 @@ __global__ void __launch_bounds__(THREADS, 1) lmhead_int8_kernel(const __grid_co
     tc_fence_after();
     const uint32_t tmem = *tmem_word;
 
-    if (warp == WARP_MMA || warp == WARP_MMA1) {
-        // ---- two issuing threads, one per 128 rows of the tile (issuing a
-        // multiply costs its thread some 60 clocks: one thread cannot keep up)
-        if (lane == 0) {
-            const uint32_t half = warp == WARP_MMA ? 0u : 1u;
-            long long tw_h = 0, tw_acc = 0, tw_a = 0, t_issue = 0, t_commit = 0;
-            LM_T0();
-            for (uint32_t q = 0; q < total_groups; ++q) {
-                const uint32_t as = q % A_SLOTS, hs = q % H_SLOTS, b = q % ACC_BUFS;
-                if (mbar_wait(base + Smem::H_FULL + 8 * hs, (q / H_SLOTS) & 1u, abort_word, wait_ns)) {
-                    break;
-                }
-                LM_ACC(tw_h);
-                if (mbar_wait(base + Smem::ACC_EMPTY + 8 * b, ((q / ACC_BUFS) & 1u) ^ 1u, abort_word, wait_ns)) {
-                    break;
-                }
-                LM_ACC(tw_acc);
-                if (mbar_wait(base + Smem::A_FULL + 8 * as, (q / A_SLOTS) & 1u, abort_word, wait_ns)) {
-                    break;
-                }
-                LM_ACC(tw_a);
-                tc_fence_after();
-                const uint32_t h_addr = base + Smem::HID + hs * H_BYTES;
-#pragma unroll
-                for (uint32_t k4 = 0; k4 < 4; ++k4) {
-                    mma_bf16_ts(tmem + b * ACC_COLS + half * TOK,
-                                tmem + A_COL0 + as * A_COLS + half * (A_COLS / 2) + k4 * 8u,
-                                operand_desc(h_addr + k4 * 32u), k4);
-                }
-                LM_ACC(t_issue);
-                mma_commit(base + Smem::DONE + 8 * (q % DONE_SLOTS));
-                LM_ACC(t_commit);
-            }
-            // The multiplies this thread has issued must have run before the tensor
-            // memory they use is freed. On the normal way out the epilogue has seen
-            // to that already and this wait finds its phase complete; it matters
-            // when the block has given up.
-            mma_commit(base + Smem::FINAL + 8 * half);
-            mbar_drain(base + Smem::FINAL + 8 * half, 0u, wait_ns);
+    // The weights do not come from the launch before this one, and what came before
+    // that has completed (see prepare_hidden_kernel): their loads start at once.
+    bool bf16 = false;
+    if (warp != WARP_LOAD_W) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        uint32_t inexact = 0;
+        for (uint32_t t = lane; t < N; t += 32u) {
+            inexact |= __ldcg(a.prep.inexact + t);
         }
-        __syncwarp();
-    } else if (warp == WARP_LOAD) {
-        // ---- one thread asks the copy engine for every stage of weights and
-        // every group's slice of the hidden states, as far ahead as slots are free
-        if (lane == 0) {
-            const uint32_t stages_per_tile = groups / RG;
-            const uint32_t n_stages = my_tiles * stages_per_tile;
-            long long tw_re = 0, tw_he = 0;
-            // The copies asked for last, per slot (bit s: slot s has one; its phase's
-            // parity beside it): what the way out has to wait for if the block gives up.
-            uint32_t raw_asked = 0, raw_parity = 0, h_asked = 0, h_parity = 0;
-            bool gave_up = false;
-            LM_T0();
-            for (uint32_t i = 0; i < n_stages && !gave_up; ++i) {
-                const uint32_t st = i % RAW_STAGES;
-                const uint32_t tile = blockIdx.x + (i / stages_per_tile) * gridDim.x;
-                const uint32_t kb = (i % stages_per_tile) * (GROUP_K * RG);  // first column of the stage
-                if (mbar_wait(base + Smem::RAW_EMPTY + 8 * st, ((i / RAW_STAGES) & 1u) ^ 1u, abort_word, wait_ns)) {
+        bf16 = __any_sync(FULL, inexact != 0u);
+    }
+
+    if (warp < (uint32_t)WARP_CONV0) {
+        set_registers<S::REGS_CTRL, false>();
+        if (warp < MMA_WARPS) {
+            // ---- four issuing warps: one per 128 rows of the tile and parity of the group (a
+            // group's waits, multiplies and commit take one warp longer than the group's
+            // weights take to arrive). The whole warp goes through
+            // the loop and one elected lane issues: everything the instruction takes is then
+            // the same in all lanes and lives in uniform registers. (Issued from a branch of
+            // lane 0 alone a multiply cost that thread 110 clocks, whatever its size.)
+            const uint32_t mw = __shfl_sync(FULL, warp, 0), half = mw & 1u;
+            const bool leader = elect_one();
+            const uint32_t idesc = instr_desc<N>(bf16);
+            const uint32_t acc0 = tmem + half * 256u, a0 = acc0 + S::A_COL0;
+            for (uint32_t q = mw >> 1; q < total_groups; q += MMA_WARPS / 2) {
+                const uint32_t as = q % S::A_SLOTS, hs = q % H_SLOTS, b = q % S::ACC_BUFS;
+                bool gave_up = wait(S::H_FULL + 8 * (hs / 2u), q / H_SLOTS);
+                gave_up |= wait(S::ACC_EMPTY + 8 * (half * S::ACC_BUFS + b), (q / S::ACC_BUFS) ^ 1u);
+                gave_up |= wait(S::A_FULL + 8 * (half * S::A_SLOTS + as), q / S::A_SLOTS);
+                if (__any_sync(FULL, gave_up)) {
                     break;
                 }
-                LM_ACC(tw_re);
-                if (i == a.lost_stage && blockIdx.x == 0) {
-                    // test hook: nothing is asked for, the stage never fills
-                } else if (!(VARIANT & 16)) {
-                    raw_asked |= 1u << st;
-                    raw_parity = (raw_parity & ~(1u << st)) | (((i / RAW_STAGES) & 1u) << st);
-                    mbar_expect_tx(base + Smem::RAW_FULL + 8 * st, RAW_STAGE_BYTES);
-                    tma_load_2d(base + Smem::RAW + st * RAW_STAGE_BYTES, &a.w_map, base + Smem::RAW_FULL + 8 * st,
-                                (int32_t)(Q4 ? kb / 2u : kb), (int32_t)(tile * TILE_ROWS));  // (a byte offset)
-                } else {
-                    mbar_arrive(base + Smem::RAW_FULL + 8 * st);
-                }
+                tc_fence_after();
+                const uint64_t bdesc = operand_desc(base + S::HID + hs * S::H_BYTES);
+                if (leader) {
 #pragma unroll
-                for (uint32_t gg = 0; gg < RG; ++gg) {
-                    const uint32_t q = i * RG + gg;
-                    const uint32_t hs = q % H_SLOTS;
-                    if (q >= (uint32_t)H_SLOTS) {  // the slot's previous group has been multiplied
-                        if (mbar_wait(base + Smem::DONE + 8 * hs, ((q / H_SLOTS) & 1u) ^ 1u, abort_word, wait_ns)) {
-                            gave_up = true;
-                            break;
+                    for (uint32_t k4 = 0; k4 < 4; ++k4) {
+                        mma_ts(acc0 + b * N, a0 + as * 32u + k4 * 8u, bdesc + k4 * 2u, idesc, k4);
+                    }
+                    mma_commit(base + S::DONE + 8 * (half * DONE_SLOTS + q % DONE_SLOTS));
+                }
+                __syncwarp();
+            }
+            // The multiplies that were issued must have run before the tensor memory they
+            // use is freed. On the normal way out the epilogue has seen to that already and
+            // this wait finds its phase complete; it matters when the block has given up.
+            if (leader) {
+                mma_commit(base + S::FINAL + 8 * mw);
+                mbar_drain(base + S::FINAL + 8 * mw, 0u, wait_ns);
+            }
+            __syncwarp();
+        } else if (warp == WARP_LOAD_W) {
+            // ---- one thread asks for every stage of weights, as far ahead as slots are free
+            if (lane == 0) {
+                // The copies asked for last, per slot (bit s: slot s has one; its phase's
+                // parity beside it): what the way out has to wait for if the block gives up.
+                uint32_t asked = 0, parity = 0;
+                uint32_t tile = 0, stage = 0;
+                for (uint32_t i = 0; i < n_stages; ++i) {
+                    if (i % STAGES_PER_BLOCK == 0u) {
+                        const uint32_t unit = unit_at(i / STAGES_PER_BLOCK);
+                        tile = unit / per_tile;
+                        stage = unit % per_tile * STAGES_PER_BLOCK;
+                    }
+                    const uint32_t st = i % S::RAW_STAGES, use = i / S::RAW_STAGES;
+                    if (wait(S::RAW_EMPTY + 8 * st, use ^ 1u)) {
+                        break;
+                    }
+                    if (!(i == a.lost_stage && blockIdx.x == 0)) {  // (test hook: the stage never fills)
+                        asked |= 1u << st;
+                        parity = (parity & ~(1u << st)) | ((use & 1u) << st);
+                        mbar_expect_tx(base + S::RAW_FULL + 8 * st, RAW_STAGE_BYTES);
+                        tma_load_2d(base + S::RAW + st * RAW_STAGE_BYTES, &a.w_map, base + S::RAW_FULL + 8 * st,
+                                    (int32_t)(a.byte0 + stage * 128u), (int32_t)(tile * TILE_ROWS));
+                    }
+                    ++stage;
+                }
+                asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+                if (*abort_word) {
+                    // The block has given up: the copies asked for land in this block's
+                    // shared memory, so it stays until they have.
+                    for (uint32_t s2 = 0; s2 < S::RAW_STAGES; ++s2) {
+                        if ((asked >> s2) & 1u) {
+                            mbar_drain(base + S::RAW_FULL + 8 * s2, (parity >> s2) & 1u, wait_ns);
                         }
                     }
-                    LM_ACC(tw_he);
-                    if (!(VARIANT & 8)) {
-                        h_asked |= 1u << hs;
-                        h_parity = (h_parity & ~(1u << hs)) | (((q / H_SLOTS) & 1u) << hs);
-                        mbar_expect_tx(base + Smem::H_FULL + 8 * hs, H_BYTES);
-                        tma_load_2d(base + Smem::HID + hs * H_BYTES, &a.h_map, base + Smem::H_FULL + 8 * hs,
-                                    (int32_t)(kb + gg * GROUP_K), 0);
-                    } else {
-                        mbar_arrive(base + Smem::H_FULL + 8 * hs);
+                }
+            }
+            __syncwarp();
+        } else if (warp == WARP_LOAD_H) {
+            // ---- another warp asks for the hidden states' images (and their sums), two
+            // groups per copy. (One group at a time, two waits and two copies by one thread
+            // took longer than a group of 4-bit codes.)
+            uint32_t asked = 0, parity = 0;
+            const uint8_t *image = reinterpret_cast<const uint8_t *>(a.prep.image[bf16 ? 1 : 0]);
+            const float *sums = a.prep.sums[bf16 ? 1 : 0];
+            uint32_t g = 0;
+            static_assert(H_SLOTS == DONE_SLOTS, "the hidden ring and the done ring share their indexing");
+            for (uint32_t q = 0; q < total_groups; q += 2u) {
+                if (q % BLOCK_GROUPS == 0u) {
+                    g = unit_at(q / BLOCK_GROUPS) % per_tile * BLOCK_GROUPS;
+                }
+                const uint32_t pair = (q / 2u) % (H_SLOTS / 2u), use = q / H_SLOTS;
+                bool gave_up = false;
+                if (q >= H_SLOTS && lane < 4u) {  // the slot's previous two groups have been multiplied, by both halves
+                    gave_up = wait(S::DONE + 8 * ((lane & 1u) * DONE_SLOTS + (q + (lane >> 1)) % DONE_SLOTS), use ^ 1u);
+                }
+                if (__any_sync(FULL, gave_up)) {
+                    break;
+                }
+                asked |= 1u << pair;
+                parity = (parity & ~(1u << pair)) | ((use & 1u) << pair);
+                if (lane == 0) {
+                    const uint32_t bar = base + S::H_FULL + 8 * pair;
+                    mbar_expect_tx(bar, 2u * S::H_BYTES + (AFFINE ? 2u * N * 4u : 0u));
+                    bulk_load(base + S::HID + 2u * pair * S::H_BYTES, image + (size_t)g * S::H_BYTES, 2u * S::H_BYTES, bar);
+                    if (AFFINE) {
+                        bulk_load(base + S::SUMS + (q % SUM_SLOTS) * N * 4u, sums + (size_t)g * N, 2u * N * 4u, bar);
+                    }
+                }
+                g += 2u;
+            }
+            if (lane == 0 && *abort_word) {
+                for (uint32_t s2 = 0; s2 < H_SLOTS / 2u; ++s2) {
+                    if ((asked >> s2) & 1u) {
+                        mbar_drain(base + S::H_FULL + 8 * s2, (parity >> s2) & 1u, wait_ns);
                     }
                 }
             }
-            if (*abort_word) {
-                // The block has given up: the copies asked for land in this block's
-                // shared memory, so it stays until they have.
-#pragma unroll
-                for (uint32_t s2 = 0; s2 < (uint32_t)RAW_STAGES; ++s2) {
-                    if ((raw_asked >> s2) & 1u) {
-                        mbar_drain(base + Smem::RAW_FULL + 8 * s2, (raw_parity >> s2) & 1u, wait_ns);
-                    }
-                }
-#pragma unroll
-                for (uint32_t s2 = 0; s2 < (uint32_t)H_SLOTS; ++s2) {
-                    if ((h_asked >> s2) & 1u) {
-                        mbar_drain(base + Smem::H_FULL + 8 * s2, (h_parity >> s2) & 1u, wait_ns);
-                    }
-                }
-            }
-        }
-        __syncwarp();
-    } else if (warp < WARP_EPI0) {
-        // ---- int8 bytes in; one thread per tile row widens them into tensor memory
-        const uint32_t ct = tid - 32u * WARP_CONV0;
-        const uint32_t quad = warp & 3u;                    // the TMEM lanes this warp may write
-        const uint32_t half = (warp - WARP_CONV0) >> 2;     // which 128 rows of the tile
+            __syncwarp();
+        }  // (two idle warps fill up their warpgroup)
+    } else if (warp < (uint32_t)S::WARP_EPI0) {
+        set_registers<S::REGS_CONV, false>();
+        // ---- bytes in; one thread per tile row widens them into tensor memory. With two
+        // teams of eight warps the groups alternate between them.
+        const uint32_t cw = warp - WARP_CONV0, team = cw >> 3;
+        const uint32_t quad = warp & 3u;            // the TMEM lanes this warp may write
+        const uint32_t half = (cw >> 2) & 1u;       // which 128 rows of the tile
         const uint32_t trow = half * 128u + quad * 32u + lane;
-        const uint32_t t_lane = (quad * 32u) << 16;
-        const uint32_t stages_per_tile = groups / RG;
-        const uint32_t n_stages = my_tiles * stages_per_tile;
-        long long tw_raw = 0, tw_ae = 0, t_conv = 0, t_st = 0;
-        bool conv_gave_up = false;
-        LM_T0();
-        for (uint32_t i = 0; i < n_stages; ++i) {
-            const uint32_t st = i % RAW_STAGES;
-            // (the vote takes the place of a __syncwarp: the lanes leave together)
-            if (__any_sync(0xFFFFFFFFu, mbar_wait(base + Smem::RAW_FULL + 8 * st, (i / RAW_STAGES) & 1u, abort_word,
-                                                  wait_ns))) {
-                break;
-            }
-            LM_ACC(tw_raw);
-            const uint32_t raw_row = base + Smem::RAW + st * RAW_STAGE_BYTES + trow * 128u;
+        const uint32_t a_base = tmem + ((quad * 32u) << 16) + half * 256u + S::A_COL0;
+        auto convert = [&](auto wide_exponent) {
+            constexpr bool BF16 = decltype(wide_exponent)::value;
+            for (uint32_t i = 0; i < n_stages; ++i) {
+                const uint32_t st = i % S::RAW_STAGES;
+                // (the vote takes the place of a __syncwarp: the lanes leave together)
+                if (__any_sync(FULL, wait(S::RAW_FULL + 8 * st, i / S::RAW_STAGES))) {
+                    return;
+                }
+                const uint32_t raw_row = base + S::RAW + st * RAW_STAGE_BYTES + trow * 128u;
 #pragma unroll 1
-            for (uint32_t gg = 0; gg < RG; ++gg) {
-                const uint32_t q = i * RG + gg;
-                const uint32_t as = q % A_SLOTS;
-                // Widen first (it needs no slot), then wait for the slot: the
-                // conversion overlaps the multiplies still reading the slot.
-                uint32_t o[2][16];
-#pragma unroll
-                for (uint32_t part = 0; part < 2; ++part) {
-                    if (Q4) {
-                        // 16 bytes = 32 codes of the group's 64.
-                        uint32_t x[4];
+                for (uint32_t gg = team; gg < RG; gg += S::TEAMS) {
+                    const uint32_t q = i * RG + gg, as = q % S::A_SLOTS;
+                    constexpr uint32_t CHUNKS = FMT == FMT_U4 ? 2u : 4u;  // of 16 bytes
+                    constexpr uint32_t CW = 32u / CHUNKS;                 // words of a chunk
+                    auto load_chunk = [&](uint32_t c, uint32_t (&x)[4]) {
                         asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
                                      : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3])
-                                     : "r"(raw_row + (((gg * 2u + part) ^ (trow & 7u)) << 4)));
+                                     : "r"(raw_row + (((gg * CHUNKS + c) ^ (trow & 7u)) << 4)));
+                    };
+                    auto widen_chunk = [&](const uint32_t (&x)[4], uint32_t *o) {
 #pragma unroll
                         for (uint32_t w = 0; w < 4; ++w) {
-                            const uint32_t lo = x[w] & 0x0F0F0F0Fu, hi = (x[w] >> 4) & 0x0F0F0F0Fu;
-                            const uint32_t c0123 = __byte_perm(lo, hi, 0x5140);  // codes 0..3 of the word, a byte each
-                            const uint32_t c4567 = __byte_perm(lo, hi, 0x7362);
-                            widen4_small(c0123, o[part][4 * w + 0], o[part][4 * w + 1]);
-                            widen4_small(c4567, o[part][4 * w + 2], o[part][4 * w + 3]);
-                        }
-                    } else if (!(VARIANT & 2)) {
-#pragma unroll
-                        for (uint32_t c = 0; c < 2; ++c) {
-                            uint32_t x0, x1, x2, x3;
-                            asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-                                         : "=r"(x0), "=r"(x1), "=r"(x2), "=r"(x3)
-                                         : "r"(raw_row + (((gg * 4u + part * 2u + c) ^ (trow & 7u)) << 4)));
-                            widen4<AFFINE>(x0, o[part][8 * c + 0], o[part][8 * c + 1]);
-                            widen4<AFFINE>(x1, o[part][8 * c + 2], o[part][8 * c + 3]);
-                            widen4<AFFINE>(x2, o[part][8 * c + 4], o[part][8 * c + 5]);
-                            widen4<AFFINE>(x3, o[part][8 * c + 6], o[part][8 * c + 7]);
-                        }
-                    } else {
-#pragma unroll
-                        for (uint32_t c = 0; c < 16; ++c) {
-                            o[part][c] = 0x3F803F80u;
-                        }
-                    }
-                }
-                LM_ACC(t_conv);
-                bool gave_up = false;
-                if (q >= (uint32_t)A_SLOTS) {  // group q - 2, the slot's last user, has been multiplied
-                    gave_up = mbar_wait(base + Smem::DONE + 8 * ((q - A_SLOTS) % DONE_SLOTS),
-                                        ((q - A_SLOTS) / DONE_SLOTS) & 1u, abort_word, wait_ns);
-                }
-                LM_ACC(tw_ae);
-                if (__any_sync(0xFFFFFFFFu, gave_up)) {
-                    conv_gave_up = true;
-                    break;
-                }
-                tc_fence_after();
-                const uint32_t a_addr = tmem + t_lane + A_COL0 + as * A_COLS + half * (A_COLS / 2);
-                tmem_st16(a_addr, o[0]);
-                tmem_st16(a_addr + 16u, o[1]);
-                tmem_st_wait();
-                tc_fence_before();
-                // One arrival per warp: arrivals on one barrier are serialised.
-                __syncwarp();
-                if (lane == 0) {
-                    mbar_arrive(base + Smem::A_FULL + 8 * as);
-                }
-                LM_ACC(t_st);
-            }
-            if (conv_gave_up) {
-                break;
-            }
-            // The stage's bytes are in registers or tensor memory: the slot may be refilled.
-            __syncwarp();
-            if (lane == 0) {
-                mbar_arrive(base + Smem::RAW_EMPTY + 8 * st);
-            }
-        }
-    } else {
-        // ---- scale each group's sums and add them up; write the tile
-        const uint32_t e = warp - WARP_EPI0;
-        const uint32_t quad = warp & 3u;   // the TMEM lanes this warp may read
-        const uint32_t half = (e >> 2) & 1u;  // which 128 rows of the tile
-        const uint32_t tok0 = (e >> 3) * (TOK / 2);  // which 32 tokens of the row
-        const uint32_t t_lane = (quad * 32u) << 16;
-        uint32_t q = 0;
-        long long tw_af = 0, t_math = 0, t_store = 0;
-        LM_T0();
-        for (uint32_t ti = 0; ti < my_tiles; ++ti) {
-            const uint32_t tile = blockIdx.x + ti * gridDim.x;
-            const uint32_t row = tile * TILE_ROWS + half * 128u + quad * 32u + lane;
-            const uint32_t rowc = min(row, a.rows - 1u);
-            const uint4 *srow = reinterpret_cast<const uint4 *>(a.scales + (uint64_t)rowc * groups);
-            uint64_t acc[TOK / 4];  // 32 tokens, two per register
-#pragma unroll
-            for (int m = 0; m < TOK / 4; ++m) {
-                acc[m] = 0ull;
-            }
-            if (AFFINE && row < a.rows) {
-                // The sums start from the term the bias kernel left in `out`; the
-                // loads complete while the first groups are multiplied.
-#pragma unroll
-                for (int m = 0; m < TOK / 4; ++m) {
-                    uint32_t lo = 0u, hi = 0u;
-                    if (tok0 + 2u * m < a.tokens) {
-                        lo = __float_as_uint(__ldcg(a.out + (uint64_t)(tok0 + 2 * m) * a.ldo + row));
-                    }
-                    if (tok0 + 2u * m + 1u < a.tokens) {
-                        hi = __float_as_uint(__ldcg(a.out + (uint64_t)(tok0 + 2 * m + 1) * a.ldo + row));
-                    }
-                    acc[m] = pack2(lo, hi);
-                }
-            }
-            uint4 sc_next = __ldg(srow);
-            for (uint32_t g8 = 0; g8 < groups; g8 += 8) {
-                const uint4 sc = sc_next;
-                if (g8 + 8u < groups) {
-                    sc_next = __ldg(srow + (g8 >> 3) + 1u);
-                }
-                const uint32_t sw[4] = {sc.x, sc.y, sc.z, sc.w};
-#pragma unroll
-                for (uint32_t gi = 0; gi < 8; ++gi, ++q) {
-                    const uint32_t b = q % ACC_BUFS;
-                    const float s = __uint_as_float((gi & 1u) ? (sw[gi >> 1] & 0xFFFF0000u) : (sw[gi >> 1] << 16));
-                    const uint64_t s2 = pack2(__float_as_uint(s), __float_as_uint(s));
-                    if (__any_sync(0xFFFFFFFFu, mbar_wait(base + Smem::DONE + 8 * (q % DONE_SLOTS),
-                                                          (q / DONE_SLOTS) & 1u, abort_word, wait_ns))) {
-                        goto epilogue_out;  // the block has given up: nothing more is read or written
-                    }
-                    LM_ACC(tw_af);
-                    tc_fence_after();
-                    const uint32_t taddr = tmem + t_lane + b * ACC_COLS + half * TOK + tok0;
-                    if (!(VARIANT & 1)) {
-#pragma unroll
-                        for (int c = 0; c < TOK / 32; ++c) {
-                            uint32_t v[16];
-                            tmem_ld16(taddr + 16u * c, v);
-                            tmem_ld_wait();
-#pragma unroll
-                            for (int m = 0; m < 8; ++m) {
-                                fma2(acc[8 * c + m], s2, pack2(v[2 * m], v[2 * m + 1]));
+                            if (FMT == FMT_U4) {
+                                widen_nibbles<BF16>(x[w], o[4u * w], o[4u * w + 1u], o[4u * w + 2u], o[4u * w + 3u]);
+                            } else {
+                                widen_bytes<FMT, BF16>(x[w], o[2u * w], o[2u * w + 1u]);
                             }
                         }
+                    };
+                    auto bytes_read = [&]() {  // the stage's bytes are in registers: the slot may be refilled
+                        if (gg + S::TEAMS >= RG) {
+                            __syncwarp();
+                            if (lane == 0) {
+                                mbar_arrive(base + S::RAW_EMPTY + 8 * st);
+                            }
+                        }
+                    };
+                    auto slot_free = [&]() -> bool {  // the slot's last user has been multiplied
+                        bool gave_up = false;
+                        if (q >= S::A_SLOTS) {
+                            const uint32_t before = q - S::A_SLOTS;
+                            gave_up = wait(S::DONE + 8 * (half * DONE_SLOTS + before % DONE_SLOTS), before / DONE_SLOTS);
+                        }
+                        return !__any_sync(FULL, gave_up);
+                    };
+                    const uint32_t to = a_base + as * 32u;
+                    if (!S::LEAN) {
+                        // Widen first (it needs no slot), then wait for the slot: the
+                        // conversion overlaps the multiplies still reading the slot.
+                        uint32_t x[CHUNKS][4], o[32];
+#pragma unroll
+                        for (uint32_t c = 0; c < CHUNKS; ++c) {
+                            load_chunk(c, x[c]);
+                        }
+#pragma unroll
+                        for (uint32_t c = 0; c < CHUNKS; ++c) {
+                            widen_chunk(x[c], o + CW * c);
+                        }
+                        bytes_read();
+                        if (!slot_free()) {
+                            return;
+                        }
+                        tc_fence_after();
+                        tmem_st32(to, o);
                     } else {
-                        acc[gi] += (uint64_t)__float_as_uint(s) + taddr;
+                        // Few registers: the slot first, then half a group at a time.
+                        uint32_t x[CHUNKS][4];
+#pragma unroll
+                        for (uint32_t c = 0; c < CHUNKS; ++c) {
+                            load_chunk(c, x[c]);
+                        }
+                        if (!slot_free()) {
+                            return;
+                        }
+                        tc_fence_after();
+#pragma unroll
+                        for (uint32_t h = 0; h < 2u; ++h) {
+                            uint32_t o[16];
+#pragma unroll
+                            for (uint32_t c = 0; c < CHUNKS / 2u; ++c) {
+                                widen_chunk(x[h * (CHUNKS / 2u) + c], o + CW * c);
+                            }
+                            tmem_st16(to + 16u * h, o);
+                        }
+                        bytes_read();
                     }
+                    tmem_st_wait();
                     tc_fence_before();
+                    // One arrival per warp: arrivals on one barrier are serialised.
                     __syncwarp();
                     if (lane == 0) {
-                        mbar_arrive(base + Smem::ACC_EMPTY + 8 * b);
+                        mbar_arrive(base + S::A_FULL + 8 * (half * S::A_SLOTS + as));
                     }
-                    LM_ACC(t_math);
                 }
             }
+        };
+        if (bf16) {
+            convert(std::true_type());
+        } else {
+            convert(std::false_type());
+        }
+    } else {
+        set_registers<S::REGS_EPI, true>();
+        // ---- scale each group's sums and add them up; write the tile
+        const uint32_t e = warp - S::WARP_EPI0;
+        const uint32_t quad = warp & 3u;      // the TMEM lanes this warp may read
+        const uint32_t half = (e >> 2) & 1u;  // which 128 rows of the tile
+        const uint32_t trow = half * 128u + quad * 32u + lane;
+        const uint32_t acc_base = tmem + ((quad * 32u) << 16) + half * 256u;
+        constexpr uint32_t P = N / 2u;  // tokens come in pairs
+        constexpr float OFFSET = FMT == FMT_U8 ? 128.0f : 0.0f;  // (8-bit codes are widened less 128)
+        float *unscale = reinterpret_cast<float *>(base_ptr + S::UNSCALE);
+        const uint32_t et = tid - 32u * (uint32_t)S::WARP_EPI0, epi_threads = 32u * S::EPI_WARPS;
+        auto epi_sync = [&]() { asm volatile("bar.sync 1, %0;" ::"n"(32 * (int)S::EPI_WARPS) : "memory"); };
+        for (uint32_t t = et; t < N; t += epi_threads) {
+            unscale[t] = bf16 ? 1.0f : __ldcg(a.prep.unscale + t);
+        }
+        epi_sync();
+        uint64_t acc[P];
+#pragma unroll
+        for (uint32_t m = 0; m < P; ++m) {
+            acc[m] = 0ull;
+        }
+        auto write_out = [&](uint32_t row) {
             if (row < a.rows) {
 #pragma unroll
-                for (int m = 0; m < TOK / 4; ++m) {
-                    float lo, hi;
-                    unpack2(acc[m], lo, hi);
-                    if (tok0 + 2u * m < a.tokens) {
-                        a.out[(uint64_t)(tok0 + 2 * m) * a.ldo + row] = lo;
-                    }
-                    if (tok0 + 2u * m + 1u < a.tokens) {
-                        a.out[(uint64_t)(tok0 + 2 * m + 1) * a.ldo + row] = hi;
+                for (uint32_t m = 0; m < P; ++m) {
+                    float v[2];
+                    unpack2(acc[m], v[0], v[1]);
+#pragma unroll
+                    for (uint32_t h = 0; h < 2u; ++h) {
+                        const uint32_t t = 2u * m + h;
+                        if (t < a.tokens) {
+                            float *to = a.out + (uint64_t)t * a.ldo + row;
+                            const float x = __fmul_rn(v[h], unscale[t]);
+                            *to = a.accumulate ? __fadd_rn(*to, x) : x;
+                        }
                     }
                 }
             }
-            LM_ACC(t_store);
+        };
+        // The sums of a tile's beginning, left for the next thread block's warp of the same rows.
+        auto part_of = [&](uint32_t block) { return a.part + (size_t)block * N * TILE_ROWS + trow; };
+        auto flag_of = [&](uint32_t block) { return a.flags + block * S::EPI_WARPS + e; };
+        uint32_t tile = unit_at(0) / per_tile, blk = unit_at(0) % per_tile, q = 0;
+        for (uint32_t n = 0; n < n_blocks; ++n) {
+            const uint32_t row = tile * TILE_ROWS + trow;
+            const uint32_t rowc = min(row, a.rows - 1u);
+            const uint4 sc = __ldg(reinterpret_cast<const uint4 *>(a.scales + (uint64_t)rowc * a.scale_ld) + blk);
+            const uint32_t sw[4] = {sc.x, sc.y, sc.z, sc.w};
+            uint32_t bw[4] = {0, 0, 0, 0};
+            if (AFFINE) {
+                const uint4 bi = __ldg(reinterpret_cast<const uint4 *>(a.biases + (uint64_t)rowc * a.scale_ld) + blk);
+                bw[0] = bi.x;
+                bw[1] = bi.y;
+                bw[2] = bi.z;
+                bw[3] = bi.w;
+            }
+            if (n == n_blocks - rest) {  // (rest = 0: never) on from where the block before stopped
+                const uint64_t t0 = global_ns();
+                for (uint32_t there = 0; !there;) {
+                    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(there) : "l"(flag_of(blockIdx.x - 1u)) : "memory");
+                    if (__any_sync(FULL, !there && (*abort_word != 0u || global_ns() - t0 > wait_ns))) {
+                        *abort_word = 1u;
+                        goto epilogue_out;
+                    }
+                    there = __all_sync(FULL, there);
+                }
+                const float *theirs = part_of(blockIdx.x - 1u);
+#pragma unroll
+                for (uint32_t m = 0; m < P; ++m) {
+                    acc[m] = pack2(__float_as_uint(__ldcg(theirs + (2u * m) * TILE_ROWS)),
+                                   __float_as_uint(__ldcg(theirs + (2u * m + 1u) * TILE_ROWS)));
+                }
+            }
+#pragma unroll
+            for (uint32_t gi = 0; gi < BLOCK_GROUPS; ++gi, ++q) {
+                const uint32_t b = q % S::ACC_BUFS;
+                const float s = __uint_as_float((gi & 1u) ? (sw[gi >> 1] & 0xFFFF0000u) : (sw[gi >> 1] << 16));
+                const uint64_t s2 = pack2(__float_as_uint(s), __float_as_uint(s));
+                if (__any_sync(FULL, wait(S::DONE + 8 * (half * DONE_SLOTS + q % DONE_SLOTS), q / DONE_SLOTS))) {
+                    goto epilogue_out;  // the block has given up: nothing more is read or written
+                }
+                tc_fence_after();
+                const uint32_t taddr = acc_base + b * N;
+#pragma unroll
+                for (uint32_t c = 0; c < N / 16u; ++c) {
+                    uint32_t v[16];
+                    tmem_ld16(taddr + 16u * c, v);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (uint32_t m = 0; m < 8u; ++m) {
+                        fma2(acc[8u * c + m], s2, pack2(v[2u * m], v[2u * m + 1u]));
+                    }
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(base + S::ACC_EMPTY + 8 * (half * S::ACC_BUFS + b));
+                }
+                if (AFFINE) {
+                    const float bias = __uint_as_float((gi & 1u) ? (bw[gi >> 1] & 0xFFFF0000u) : (bw[gi >> 1] << 16));
+                    const float add = __fmaf_rn(OFFSET, s, bias);
+                    const uint64_t add2 = pack2(__float_as_uint(add), __float_as_uint(add));
+                    const ulonglong2 *hs = reinterpret_cast<const ulonglong2 *>(
+                        base_ptr + S::SUMS + (q % SUM_SLOTS) * N * 4u);
+#pragma unroll
+                    for (uint32_t m = 0; m < P / 2u; ++m) {
+                        const ulonglong2 h = hs[m];
+                        fma2(acc[2u * m], add2, h.x);
+                        fma2(acc[2u * m + 1u], add2, h.y);
+                    }
+                }
+            }
+            ++blk;
+            if (blk != per_tile && n + 1u != begun) {
+                continue;
+            }
+            if (blk == per_tile) {
+                write_out(row);
+            } else {
+                float *mine = part_of(blockIdx.x);
+#pragma unroll
+                for (uint32_t m = 0; m < P; ++m) {
+                    float v0, v1;
+                    unpack2(acc[m], v0, v1);
+                    __stcg(mine + (2u * m) * TILE_ROWS, v0);
+                    __stcg(mine + (2u * m + 1u) * TILE_ROWS, v1);
+                }
+                __syncwarp();
+                if (lane == 0) {
+                    __threadfence();
+                    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(flag_of(blockIdx.x)), "r"(1u) : "memory");
+                }
+            }
+#pragma unroll
+            for (uint32_t m = 0; m < P; ++m) {
+                acc[m] = 0ull;
+            }
+            tile = unit_at(n + 1u) / per_tile;
+            blk = unit_at(n + 1u) % per_tile;
         }
     epilogue_out:;
     }
@@ -705,149 +909,11 @@ __global__ void __launch_bounds__(THREADS, 1) lmhead_int8_kernel(const __grid_co
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (warp == WARP_MMA) {
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS)
-                     : "memory");
+    if (warp == 0u) {
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
     }
     if (tid == 0 && *abort_word) {
         atomicOr(a.status_word, 1u << STATUS_TIMEOUT_BIT);
-    }
-}
-
-// Affine storage, the term the multiplier does not see: with the converters
-// widening q - 128,
-//   sum_c (scale * q + bias) * h = scale * sum_c (q - 128) * h + (128 * scale + bias) * sum_c h
-// per group, and this kernel writes out[t, n] = sum_g (128 * scale[n, g] +
-// bias[n, g]) * hsum[g, t]; the head kernel then adds its own sums to it.
-// A thread owns 4 vocabulary rows x 16 tokens, their partial results in registers;
-// the group sums of the hidden states (binary32, index order; [group][token],
-// tokens past the last: 0) come from hidden_group_sums_kernel, which runs
-// before it, one block per group and one thread per token.
-__global__ void __launch_bounds__(TOK) hidden_group_sums_kernel(const __nv_bfloat16 *hidden, uint64_t ld,
-                                                                uint32_t tokens, float *out) {
-    const uint32_t g = blockIdx.x, t = threadIdx.x;
-    float sum = 0.0f;
-    if (t < tokens) {
-        const uint4 *src = reinterpret_cast<const uint4 *>(hidden + (uint64_t)t * ld + (uint64_t)g * GROUP_K);
-#pragma unroll
-        for (int i = 0; i < GROUP_K / 8; ++i) {
-            const uint4 v = __ldg(src + i);
-            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                sum += __uint_as_float(w[j] << 16);
-                sum += __uint_as_float(w[j] & 0xFFFF0000u);
-            }
-        }
-    }
-    out[(uint64_t)g * TOK + t] = sum;
-}
-
-constexpr int BIAS_THREADS = 128;
-constexpr uint32_t BIAS_ROWS = BIAS_THREADS * 4 / 4;  // a warp covers 32 rows x 64 tokens
-constexpr uint32_t BIAS_MAX_GROUPS = 128;             // hidden <= 8192
-
-// Dynamic shared memory: the group sums, then the block's scales and biases,
-// each row padded by 16 bytes so that rows four apart fall into different banks.
-__host__ __device__ constexpr uint32_t bias_row_bytes(uint32_t groups) { return groups * 2u + 16u; }
-__host__ __device__ constexpr uint32_t bias_smem_bytes(uint32_t groups) {
-    return groups * TOK * 4u + 2u * BIAS_ROWS * bias_row_bytes(groups);
-}
-
-__global__ void __launch_bounds__(BIAS_THREADS) affine_bias_term_kernel(
-    const float *group_sums, uint32_t tokens, const __nv_bfloat16 *scales, const __nv_bfloat16 *biases,
-    uint32_t groups, uint32_t rows, float *out, uint64_t ldo, float code_offset) {
-    extern __shared__ __align__(16) uint8_t bias_smem[];
-    float *hsum = reinterpret_cast<float *>(bias_smem);  // [group][token]
-    uint8_t *sc_s = bias_smem + groups * TOK * 4u;
-    const uint32_t row_bytes = bias_row_bytes(groups);
-    uint8_t *bi_s = sc_s + BIAS_ROWS * row_bytes;
-    const uint32_t block_row0 = blockIdx.x * BIAS_ROWS;
-    for (uint32_t i = threadIdx.x; i < groups * TOK / 4u; i += BIAS_THREADS) {
-        reinterpret_cast<float4 *>(hsum)[i] = __ldg(reinterpret_cast<const float4 *>(group_sums) + i);
-    }
-    {
-        const uint32_t per_row = groups / 8u;  // 16-byte pieces of a row
-        for (uint32_t i = threadIdx.x; i < BIAS_ROWS * per_row; i += BIAS_THREADS) {
-            const uint32_t r = i / per_row, piece = i % per_row;
-            const uint32_t rowc = min(block_row0 + r, rows - 1u);
-            const uint4 sv = __ldg(reinterpret_cast<const uint4 *>(scales + (uint64_t)rowc * groups) + piece);
-            const uint4 bv = __ldg(reinterpret_cast<const uint4 *>(biases + (uint64_t)rowc * groups) + piece);
-            *reinterpret_cast<uint4 *>(sc_s + r * row_bytes + piece * 16u) = sv;
-            *reinterpret_cast<uint4 *>(bi_s + r * row_bytes + piece * 16u) = bv;
-        }
-    }
-    __syncthreads();
-    // A thread owns 4 rows x 16 tokens: a group's 16 sums are read once from
-    // shared memory for 64 multiply-adds.
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    // Its rows are 8 apart, so that the eight threads that read scales at
-    // once read consecutive (padded) rows: no bank conflicts, and the stores
-    // of one token fill whole sectors.
-    const uint32_t lrow0 = warp * 32u + (lane >> 2);
-    const uint32_t row0 = block_row0 + lrow0;
-    const uint32_t tok0 = (lane & 3u) * 16u;
-    const uint4 *srow[4], *brow[4];
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        srow[r] = reinterpret_cast<const uint4 *>(sc_s + (lrow0 + 8u * r) * row_bytes);
-        brow[r] = reinterpret_cast<const uint4 *>(bi_s + (lrow0 + 8u * r) * row_bytes);
-    }
-    uint64_t acc[4][8];
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-#pragma unroll
-        for (int m = 0; m < 8; ++m) {
-            acc[r][m] = 0ull;
-        }
-    }
-    for (uint32_t g8 = 0; g8 < groups; g8 += 8) {
-        uint32_t sw[4][4], bw[4][4];
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const uint4 sc = srow[r][g8 >> 3];
-            const uint4 bi = brow[r][g8 >> 3];
-            sw[r][0] = sc.x, sw[r][1] = sc.y, sw[r][2] = sc.z, sw[r][3] = sc.w;
-            bw[r][0] = bi.x, bw[r][1] = bi.y, bw[r][2] = bi.z, bw[r][3] = bi.w;
-        }
-#pragma unroll
-        for (uint32_t gi = 0; gi < 8; ++gi) {
-            const ulonglong2 *hs = reinterpret_cast<const ulonglong2 *>(hsum + (g8 + gi) * TOK + tok0);
-            ulonglong2 h2[4];
-#pragma unroll
-            for (int m = 0; m < 4; ++m) {
-                h2[m] = hs[m];
-            }
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const float s = __uint_as_float((gi & 1u) ? (sw[r][gi >> 1] & 0xFFFF0000u) : (sw[r][gi >> 1] << 16));
-                const float b = __uint_as_float((gi & 1u) ? (bw[r][gi >> 1] & 0xFFFF0000u) : (bw[r][gi >> 1] << 16));
-                const float shift = fmaf(code_offset, s, b);  // (8-bit codes are widened less 128, 4-bit ones as they are)
-                const uint64_t shift2 = pack2(__float_as_uint(shift), __float_as_uint(shift));
-#pragma unroll
-                for (int m = 0; m < 4; ++m) {
-                    fma2(acc[r][2 * m], shift2, h2[m].x);
-                    fma2(acc[r][2 * m + 1], shift2, h2[m].y);
-                }
-            }
-        }
-    }
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        const uint32_t row = row0 + 8u * r;
-        if (row < rows) {
-#pragma unroll
-            for (int m = 0; m < 8; ++m) {
-                float lo, hi;
-                unpack2(acc[r][m], lo, hi);
-                if (tok0 + 2u * m < tokens) {
-                    out[(uint64_t)(tok0 + 2 * m) * ldo + row] = lo;
-                }
-                if (tok0 + 2u * m + 1u < tokens) {
-                    out[(uint64_t)(tok0 + 2 * m + 1) * ldo + row] = hi;
-                }
-            }
-        }
     }
 }
 
