@@ -86,7 +86,6 @@ struct lily_sampler {
     float *lm_part = nullptr;
     uint32_t *lm_flags = nullptr;
     uint32_t lm_tokens = 0;
-    bool merge_attr = false;
 };
 
 namespace {
@@ -274,13 +273,14 @@ struct SplitPlan {
 
 using lily::INLINE_ROWS;
 using lily::INLINE_ROWS_MAX;
+using lily::INLINE_ROWS_MID;
 
 // `lists`: rows may bring a list of ids (history, bias, ban, or ids drawn earlier
 // in the step); `counts`: a history list with a frequency penalty.
 SplitPlan split_plan(const lily_sampler *h, const lily::KArgs &a, uint32_t rows, uint32_t dtype, bool lists,
                      bool counts) {
     SplitPlan p;
-    if (a.cand_out != nullptr || a.merge_in != nullptr) {
+    if (a.merge_in != nullptr || (a.cand_out != nullptr && a.shard_k > lily::SPL_SMALL_K)) {
         return p;
     }
     const uint32_t per = dtype == LILY_F32 ? lily::Piece<float>::PER : lily::Piece<__nv_bfloat16>::PER;
@@ -290,12 +290,14 @@ SplitPlan split_plan(const lily_sampler *h, const lily::KArgs &a, uint32_t rows,
     }
     const uint32_t pieces = lily::split_pieces(a.vocab, per - 1u, per);
     const size_t general = smem_bytes(a.vocab, 1);  // the first block may run the general row code
-    const uint32_t slots = (uint32_t)h->sm_count;
+    // As many blocks per row as still run all rows at once (with a second wave of clusters
+    // 16 rows took 15.6 us, with clusters of half the size 9.9).
     uint32_t lb = 3;
-    while (lb > 0u && ((rows << lb) > slots || (a.vocab / logits) >> lb < lily::SPL_MIN_TILES)) {
+    while (lb > 0u && ((a.vocab / logits) >> lb < lily::SPL_MIN_TILES ||
+                       rows > lily::split_rows_at_once(h->device, h->sm_count, h->max_smem, lb))) {
         --lb;
     }
-    p.sole = (rows << lb) <= (uint32_t)h->sm_count;
+    p.sole = rows <= lily::split_rows_at_once(h->device, h->sm_count, h->max_smem, lb);
     const uint32_t here = (pieces + (1u << lb) - 1u) >> lb, entries = here * logits;
     const size_t fixed = sizeof(lily::SmemFixed) + sizeof(lily::SplitSmem) +
                          (size_t)lily::split_buckets(here, lily::split_u(p.sole ? 1 : 2)) * lily::SPL_NT * 4u;
@@ -355,6 +357,16 @@ int32_t launch_split_inline(lily_sampler *h, cudaStream_t stream, const lily::KA
         std::memcpy(sa.slots, slots, sizeof(uint32_t) * rows);
     }
     return launch_split(h, stream, sa, p, grid_rows ? grid_rows : rows, dtype);
+}
+
+// The argument block that holds the rows' parameters.
+int32_t launch_rows_inline(lily_sampler *h, cudaStream_t stream, const lily::KArgs &a, const SplitPlan &p, uint32_t rows,
+                           uint32_t dtype, const lily_sampling_params_t *params, const uint32_t *steps,
+                           const uint32_t *slots) {
+    return rows <= INLINE_ROWS ? launch_split_inline<INLINE_ROWS>(h, stream, a, p, rows, dtype, params, steps, slots)
+           : rows <= INLINE_ROWS_MID
+               ? launch_split_inline<INLINE_ROWS_MID>(h, stream, a, p, rows, dtype, params, steps, slots)
+               : launch_split_inline<INLINE_ROWS_MAX>(h, stream, a, p, rows, dtype, params, steps, slots);
 }
 
 int32_t launch(lily_sampler *h, cudaStream_t stream, const lily::KArgs &a, uint32_t rows,
@@ -921,11 +933,7 @@ int32_t lily_sample_batch(lily_sampler_t *h, void *stream_, const lily_sample_ar
     a.kept_ld = g.kept_ld;
     a.n_slices = choose_slices(h, g.rows);
     if (in_args) {
-        return g.rows <= INLINE_ROWS
-                   ? launch_split_inline<INLINE_ROWS>(h, stream, a, plan, g.rows, g.logits_dtype, g.params, g.steps,
-                                                      g.count_slots)
-                   : launch_split_inline<INLINE_ROWS_MAX>(h, stream, a, plan, g.rows, g.logits_dtype, g.params,
-                                                          g.steps, g.count_slots);
+        return launch_rows_inline(h, stream, a, plan, g.rows, g.logits_dtype, g.params, g.steps, g.count_slots);
     }
     st = launch(h, stream, a, g.rows, g.logits_dtype, raises_few);
     if (slot >= 0) {
@@ -1121,10 +1129,8 @@ int32_t lmhead_launch(lily_sampler *h, cudaStream_t stream, const lily_lmhead_t 
     return LILY_OK;
 }
 
-// Host parameters of a sharded call: checked, then staged to the device.
-int32_t stage_shard_params(lily_sampler *h, cudaStream_t stream, const lily_sample_args_t &g,
-                           const lily_sampling_params_t **d_params, const uint32_t **d_steps,
-                           int *slot_out) {
+// The host parameters of a sharded call, checked.
+int32_t check_shard_params(lily_sampler *h, const lily_sample_args_t &g) {
     if (g.rows == 0u || g.rows > h->max_rows) {
         return fail(h, LILY_ERR_CAPACITY, "rows outside 1..max_rows");
     }
@@ -1147,6 +1153,13 @@ int32_t stage_shard_params(lily_sampler *h, cudaStream_t stream, const lily_samp
             return fail(h, LILY_ERR_ARG, "sharded sampling needs 1 <= top_k <= 64");
         }
     }
+    return LILY_OK;
+}
+
+// Stages them to the device, for a call of more rows than a launch's own arguments take.
+int32_t stage_shard_params(lily_sampler *h, cudaStream_t stream, const lily_sample_args_t &g,
+                           const lily_sampling_params_t **d_params, const uint32_t **d_steps,
+                           int *slot_out) {
     // What would be staged: [rows][has steps][params][steps].
     const size_t pb = sizeof(lily_sampling_params_t) * g.rows, sb = g.steps ? sizeof(uint32_t) * g.rows : 0;
     std::vector<char> want(8 + pb + sb);
@@ -1177,8 +1190,7 @@ int32_t stage_shard_params(lily_sampler *h, cudaStream_t stream, const lily_samp
     // (A reused slot is read by one more launch: the caller records the slot's
     // event after it, so the ring does not overwrite the slot under that launch.)
     *d_params = reinterpret_cast<const lily_sampling_params_t *>(h->d_stage[slot] + h->layout.params);
-    *d_steps = g.steps != nullptr ? reinterpret_cast<const uint32_t *>(h->d_stage[slot] + h->layout.steps)
-                                  : nullptr;
+    *d_steps = g.steps != nullptr ? reinterpret_cast<const uint32_t *>(h->d_stage[slot] + h->layout.steps) : nullptr;
     *slot_out = slot;
     return LILY_OK;
 }
@@ -1191,10 +1203,7 @@ int32_t shard_candidates(lily_sampler *h, cudaStream_t stream, const lily_sample
     if ((uint64_t)first_id + h->vocab > 0xFFFFFFFFull) {
         return fail(h, LILY_ERR_ARG, "first_id + vocab overflows an id");
     }
-    const lily_sampling_params_t *d_params = nullptr;
-    const uint32_t *d_steps = nullptr;
-    int slot = -1;
-    int32_t st = stage_shard_params(h, stream, g, &d_params, &d_steps, &slot);
+    int32_t st = check_shard_params(h, g);
     if (st != LILY_OK) {
         return st;
     }
@@ -1203,15 +1212,27 @@ int32_t shard_candidates(lily_sampler *h, cudaStream_t stream, const lily_sample
     a.logits = g.logits;
     a.logits_ld = g.logits_ld;
     a.rows = g.rows;
-    a.params = d_params;
-    a.steps = d_steps;
     a.out_ids = nullptr;
     a.shard_k = LILY_SHARD_CANDIDATES;
     a.id_offset = first_id;
     a.cand_out = static_cast<lily::ShardRecord *>(records);
+    const SplitPlan plan = split_plan(h, a, g.rows, g.logits_dtype, false, false);
+    if (plan.take) {  // (the row kernel sums the exponentials in the same launch)
+        a.shard_sums = want_sums ? 1u : 0u;
+    }
+    if (plan.take && g.rows <= INLINE_ROWS_MAX) {
+        return launch_rows_inline(h, stream, a, plan, g.rows, g.logits_dtype, g.params, nullptr, nullptr);
+    }
+    const uint32_t *d_steps = nullptr;
+    int slot = -1;
+    st = stage_shard_params(h, stream, g, &a.params, &d_steps, &slot);
+    if (st != LILY_OK) {
+        return st;
+    }
+    const lily_sampling_params_t *d_params = a.params;
     a.n_slices = choose_slices(h, g.rows);
     // (The kernel of one block per row sums the exponentials in the same pass.)
-    a.shard_sums = want_sums && stream_route(a, g.rows, g.logits_dtype) ? 1u : 0u;
+    a.shard_sums = want_sums && (plan.take || stream_route(a, g.rows, g.logits_dtype)) ? 1u : 0u;
     st = launch(h, stream, a, g.rows, g.logits_dtype);
     if (st == LILY_OK && want_sums && a.shard_sums == 0u) {
         // The candidate launch has left the slice counters and the tickets (all
@@ -1335,19 +1356,23 @@ int32_t merge_draw(lily_sampler_t *h, void *stream_, const void *gathered, uint3
     }
     DeviceGuard guard(h->device);
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-    const lily_sampling_params_t *d_params = nullptr;
-    const uint32_t *d_steps = nullptr;
-    int slot = -1;
-    st = stage_shard_params(h, stream, g, &d_params, &d_steps, &slot);
+    st = check_shard_params(h, g);
     if (st != LILY_OK) {
         return st;
     }
-    if (!h->merge_attr) {
-        CU(h, cudaFuncSetAttribute(lily::merge_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)sizeof(lily::SmemFixed)));
-        h->merge_attr = true;
+    lily::MergeArgs ma;
+    const bool in_args = g.rows <= lily::INLINE_ROWS_MID;
+    int slot = -1;
+    const lily_sampling_params_t *d_params = nullptr;
+    const uint32_t *d_steps = nullptr;
+    if (in_args) {
+        for (uint32_t r = 0; r < g.rows; ++r) {
+            ma.in[r] = lily::row_in(g.params[r], g.steps != nullptr ? g.steps[r] : 0u);
+        }
+    } else if ((st = stage_shard_params(h, stream, g, &d_params, &d_steps, &slot)) != LILY_OK) {
+        return st;
     }
-    lily::KArgs a;
+    lily::KArgs &a = ma.a;
     base_args(h, &a);
     a.vocab = 0xFFFFFFFFu;  // ids are global here
     a.rows = g.rows;
@@ -1367,9 +1392,10 @@ int32_t merge_draw(lily_sampler_t *h, void *stream_, const void *gathered, uint3
     if (peer != nullptr) {
         a.peer = *peer;
     }
-    lily::merge_rows_kernel<<<g.rows, lily::NT, sizeof(lily::SmemFixed), stream>>>(a);
-    CU(h, cudaGetLastError());
-    CU(h, cudaEventRecord(h->ev[slot], stream));
+    CU(h, lily::merge_launch(ma, g.rows, &h->attr_mask, stream));
+    if (!in_args) {
+        CU(h, cudaEventRecord(h->ev[slot], stream));
+    }
     return LILY_OK;
 }
 

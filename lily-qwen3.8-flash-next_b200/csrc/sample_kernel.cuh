@@ -2757,120 +2757,6 @@ static __device__ __noinline__ void sample_whole_row(const KArgs &a, uint32_t ro
     sample_row<T, VEC>(a, row, 0u);
 }
 
-// The draw of a vocabulary-sharded row: the shards' records hold every
-// candidate the row's top-k can contain (each shard kept its own best
-// shard_k >= k), so selecting, cutting and drawing over their union gives
-// what one pass over the whole vocabulary gives. One block per row.
-__device__ __forceinline__ void peer_exchange_row(const KArgs &a, uint32_t row);
-
-static __global__ void __launch_bounds__(NT, 2) merge_rows_kernel(const __grid_constant__ KArgs a) {
-    extern __shared__ uint4 smem_raw[];
-    SmemFixed *sm = reinterpret_cast<SmemFixed *>(smem_raw);
-    const uint32_t tid = threadIdx.x;
-    const uint32_t row = a.row0 + blockIdx.x;
-    if (a.peer.n != 0u) {
-        peer_exchange_row(a, row);  // the row's records of all ranks are in the own buffer after this
-    }
-    const lily_sampling_params_t P = a.params[row];
-    const bool greedy = P.temperature <= 0.0f || P.top_k == 1u;
-    if (tid == 0) {
-        RowCtx c;
-        c.T = greedy ? 1.0f : P.temperature;
-        c.k = greedy ? 1u : (P.top_k == 0u ? KCAP : min(P.top_k, KCAP));
-        c.rep = 1.0f;
-        c.presence = c.frequency = 0.0f;
-        c.top_p = P.top_p;
-        c.min_p = P.min_p;
-        c.use_pen = c.need_counts = c.has_special = false;
-        c.monotone = true;
-        c.argmax_mode = greedy;
-        c.lo = 0;
-        c.hi = a.vocab;
-        c.seen = nullptr;
-        c.counts = nullptr;
-        c.bias_ids = c.ban_ids = nullptr;
-        c.bias_vals = nullptr;
-        c.bias_len = c.ban_len = 0;
-        c.sp_in_smem = true;
-        c.count_draw = false;
-        c.slot = 0;
-        sm->ctx = c;
-        sm->n = 0;
-        sm->err = 0;
-        sm->u_draw = a.uniforms ? a.uniforms[row] : uniform_for(P.seed, a.steps ? a.steps[row] : 0u);
-        sm->step_draw = 0;
-        sm->ckey = sm->key;
-        sm->cid = sm->id;
-        sm->ccap = CAP;
-    }
-    __syncthreads();
-    const uint32_t slots = a.merge_shards * LILY_SHARD_CANDIDATES;
-    for (uint32_t i = tid; i < slots; i += NT) {
-        const ShardRecord *rec = a.merge_in + (uint64_t)(i / LILY_SHARD_CANDIDATES) * a.merge_stride + row;
-        const uint2 e = rec->cand[i % LILY_SHARD_CANDIDATES];
-        if (e.y != 0xFFFFFFFFu) {
-            const uint32_t at = atomicAdd(&sm->n, 1u);
-            sm->key[at] = e.x;
-            sm->id[at] = e.y;
-        }
-    }
-    if (a.out_lse && tid == 0) {
-        // Shards in order: the largest maximum, then the sums rescaled to it.
-        float top = neg_inf();
-        for (uint32_t s = 0; s < a.merge_shards; ++s) {
-            top = fmaxf(top, a.merge_in[(uint64_t)s * a.merge_stride + row].max_adj);
-        }
-        float sum = 0.0f;
-        for (uint32_t s = 0; s < a.merge_shards; ++s) {
-            const ShardRecord *rec = a.merge_in + (uint64_t)s * a.merge_stride + row;
-            sum += rec->sum_exp * expf(rec->max_adj - top);
-        }
-        a.out_lse[row] = top + logf(sum);
-    }
-    __syncthreads();
-    uint32_t n = sm->n;
-    const uint32_t k = sm->ctx.k;
-    if (n == 0u) {
-        if (tid == 0) {
-            a.out_ids[row] = 0xFFFFFFFFu;
-            if (a.out_status) {
-                a.out_status[row] = ROW_INTERNAL;
-            }
-            if (a.kept_n) {
-                a.kept_n[row] = 0;
-            }
-            atomicOr(a.status_word, 1u << ROW_INTERNAL);
-        }
-        return;
-    }
-    if (tid == 0) {
-        sm->n_adj = n;
-    }
-    __syncthreads();
-    bool sorted = false;
-    if (n <= RANKSORT_MAX) {
-        rank_sort(sm, n, k);
-        n = min(n, k);
-        sorted = true;
-    } else if (n > k) {
-        select_topk(sm, n, k);
-        n = k;
-    }
-    if (n <= 64u) {
-        if (tid < 32u) {
-            if (!sorted) {
-                sort_candidates<true>(sm, n);
-            }
-            finalize_warp(sm, a, row, n, P.seed);
-        }
-    } else {
-        if (!sorted) {
-            sort_candidates<false>(sm, n);
-        }
-        finalize<false>(sm, a, row, n, P.seed);
-    }
-}
-
 // Sum over a shard row of exp(adjusted - the shard's maximum), for records
 // made without penalties or lists: adjusted = l / T (l for a greedy row). A
 // row is cut into gridDim.x pieces; every add happens in a fixed order (a

@@ -1,5 +1,7 @@
-// The row kernel's translation unit: its instantiations and their launch.
-#include "split_kernel.cuh"
+// The row kernel's and the merge kernel's translation unit: instantiations and launches.
+#include <atomic>
+
+#include "merge_kernel.cuh"
 
 namespace lily {
 
@@ -9,7 +11,7 @@ template <typename T, uint32_t MAXR>
 cudaError_t launch_one(const SplitArgs<MAXR> &a, uint32_t rows, size_t smem, int max_smem, uint32_t *attr_mask,
                        cudaStream_t stream) {
     auto kernel = split_rows_kernel<T, MAXR, 1>;
-    const uint32_t bit = 1u << ((sizeof(T) == 4 ? 16 : 17) + (MAXR == INLINE_ROWS ? 0 : 2));
+    const uint32_t bit = 1u << ((sizeof(T) == 4 ? 16 : 17) + (MAXR == INLINE_ROWS ? 0 : MAXR == INLINE_ROWS_MID ? 2 : 4));
     if (!(*attr_mask & bit)) {
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
         if (e != cudaSuccess) {
@@ -45,7 +47,68 @@ cudaError_t split_launch(const SplitArgs<MAXR> &a, uint32_t rows, uint32_t dtype
 
 template cudaError_t split_launch<INLINE_ROWS>(const SplitArgs<INLINE_ROWS> &, uint32_t, uint32_t, size_t, int, uint32_t *,
                                                cudaStream_t);
+template cudaError_t split_launch<INLINE_ROWS_MID>(const SplitArgs<INLINE_ROWS_MID> &, uint32_t, uint32_t, size_t, int,
+                                                   uint32_t *, cudaStream_t);
 template cudaError_t split_launch<INLINE_ROWS_MAX>(const SplitArgs<INLINE_ROWS_MAX> &, uint32_t, uint32_t, size_t, int,
                                                    uint32_t *, cudaStream_t);
+
+uint32_t split_rows_at_once(int device, int sm_count, int max_smem, uint32_t log_blocks) {
+    if (log_blocks == 0u) {
+        return (uint32_t)sm_count;
+    }
+    // Asked for once per device; 0: not yet, else 1 + the answer.
+    constexpr int DEVICES = 64;
+    static std::atomic<uint32_t> known[DEVICES][4];
+    std::atomic<uint32_t> *at = device >= 0 && device < DEVICES ? &known[device][log_blocks] : nullptr;
+    uint32_t n = at ? at->load(std::memory_order_relaxed) : 0u;
+    if (n == 0u) {
+        auto kernel = split_rows_kernel<float, INLINE_ROWS, 1>;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(1u << log_blocks, 1, 1);
+        cfg.blockDim = dim3(NT, 1, 1);
+        cfg.dynamicSmemBytes = (size_t)max_smem;  // (one block per SM)
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 1u << log_blocks;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int clusters = 0;
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess || clusters < 0) {
+            clusters = 0;
+            cudaGetLastError();
+        }
+        n = 1u + (uint32_t)clusters;
+        if (at) {
+            at->store(n, std::memory_order_relaxed);
+        }
+    }
+    return n - 1u;
+}
+
+cudaError_t merge_launch(const MergeArgs &a, uint32_t rows, uint32_t *attr_mask, cudaStream_t stream) {
+    constexpr uint32_t bit = 1u << 22;
+    if (!(*attr_mask & bit)) {
+        const cudaError_t e =
+            cudaFuncSetAttribute(merge_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemFixed));
+        if (e != cudaSuccess) {
+            return e;
+        }
+        *attr_mask |= bit;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(rows, 1, 1);
+    cfg.blockDim = dim3(NT, 1, 1);
+    cfg.dynamicSmemBytes = sizeof(SmemFixed);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, merge_rows_kernel, a);
+}
 
 }  // namespace lily

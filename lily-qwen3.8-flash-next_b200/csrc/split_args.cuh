@@ -75,7 +75,9 @@ struct alignas(16) SplitSmem {
     unsigned long long mbar_pool;    // every block's keys have arrived
     unsigned long long mbar_cand;    // first block: every block's candidates have arrived
     unsigned long long mbar_list;    // wide rows: the sorted lists of all blocks have arrived
+    unsigned long long mbar_sums;    // first block: every block's sums of exponentials have arrived
     uint4 head[SPL_MAX_BLOCKS];      // first block: a block's number of candidates, flag, bound
+    uint2 sums[SPL_MAX_BLOCKS * SPL_WARPS];  // first block, a shard's record: (reference, sum) of every warp
     union {
         alignas(16) uint32_t pool[SPL_POOL];     // the best keys of every warp of the cluster
         uint32_t tmax[SPL_MAX_BLOCKS * SPL_NT];  // wide rows: the keys of all its threads
@@ -91,6 +93,7 @@ struct alignas(16) SplitSmem {
     uint32_t bin;
     uint32_t verdict[2];             // what the waiting warps of the first block learn
     uint32_t bound_key;
+    uint32_t record_key;             // a shard's largest adjusted logit
     uint32_t n_slots;                // candidates whose ids are counted in the history
 };
 static_assert(sizeof(SplitSmem) % 16u == 0u, "the arrays behind it are 16-byte aligned");
@@ -134,12 +137,27 @@ __host__ __device__ inline uint32_t split_buckets(uint32_t pieces_of_block, uint
 
 // Launches the kernel for a.a.rows rows from row0 on: logits of `dtype`, `smem` bytes of
 // dynamic shared memory (at most max_smem). `attr_mask`: bits of the kernels whose
-// limit has been raised, the caller's to keep per device. Instantiated for INLINE_ROWS
-// and INLINE_ROWS_MAX rows in split.cu.
+// limit has been raised, the caller's to keep per device. Instantiated for INLINE_ROWS,
+// INLINE_ROWS_MID and INLINE_ROWS_MAX rows in split.cu.
 template <uint32_t MAXR>
 cudaError_t split_launch(const SplitArgs<MAXR> &a, uint32_t rows, uint32_t dtype, size_t smem, int max_smem,
                          uint32_t *attr_mask, cudaStream_t stream);
 
-constexpr uint32_t INLINE_ROWS = 8, INLINE_ROWS_MAX = 64;  // rows whose parameters travel in the kernel's arguments
+// Rows whose parameters travel in the kernel's arguments: sizes of the argument block (a
+// larger one takes longer to launch), the last one as many rows as the chip has SMs.
+constexpr uint32_t INLINE_ROWS = 8, INLINE_ROWS_MID = 64, INLINE_ROWS_MAX = 148;
+
+// The most rows that clusters of 1 << log_blocks blocks run at once, one block per SM. Less
+// than the SMs would hold (15 clusters of eight on 148 SMs, 33 of four): a cluster lies in
+// one group of SMs, and those do not divide evenly.
+uint32_t split_rows_at_once(int device, int sm_count, int max_smem, uint32_t log_blocks);
+
+// The merge of the shards' records (merge_kernel.cuh). a.params set: the rows' parameters
+// and steps are there, else in `in`.
+struct MergeArgs {
+    KArgs a;
+    RowIn in[INLINE_ROWS_MID];
+};
+cudaError_t merge_launch(const MergeArgs &a, uint32_t rows, uint32_t *attr_mask, cudaStream_t stream);
 
 }  // namespace lily

@@ -464,6 +464,8 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(cand_bar), "r"(blocks) : "memory");
             const uint32_t list_bar = (uint32_t)__cvta_generic_to_shared(&ss->mbar_list);
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(list_bar), "r"(blocks) : "memory");
+            const uint32_t sums_bar = (uint32_t)__cvta_generic_to_shared(&ss->mbar_sums);
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sums_bar) : "memory");
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
     }
@@ -522,6 +524,13 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         } else {
             sample_whole_row<T, false>(whole, row);
         }
+        if (a.cand_out) {
+            __syncthreads();
+            if (tid == SPL_NT) {
+                ss->record_key = key_of(__ldcg(&a.cand_out[row].max_adj));
+            }
+            __syncthreads();
+        }
     };
     // What the first block's waiting warps are told, at barrier 2: the row is done, it
     // is drawn alone, or (only to the warps that work) more hands are needed; in the
@@ -545,6 +554,21 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
             draw_alone();
         } else {
             asm volatile("bar.arrive 2, %0;" ::"n"(NT) : "memory");
+        }
+    };
+    // A shard's record of n candidates in key[] / id[], by one warp.
+    auto write_record = [&](uint32_t n) {
+        ShardRecord *rec = a.cand_out + row;
+#pragma unroll
+        for (uint32_t i = lane; i < LILY_SHARD_CANDIDATES; i += 32u) {
+            rec->cand[i] = i < n ? make_uint2(sm->key[i], sm->id[i] + a.id_offset) : make_uint2(0u, 0xFFFFFFFFu);
+        }
+        if (lane == 0) {
+            rec->max_adj = float_of_key(sm->key[0]);
+            if (!a.shard_sums) {
+                rec->sum_exp = 0.0f;
+            }
+            ss->record_key = sm->key[0];
         }
     };
     // The upper half of the block marks the row's history while the lower half reads
@@ -649,7 +673,10 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         hist_len = 0;
     }
     const uint32_t extra_len = list_mode ? a.extra_len : 0u;
-    const uint32_t k = in.k;
+    // A vocabulary shard's launch ends in the row's record, not in a draw: the best shard_k
+    // logits (a greedy row's best one) and, if asked for, the sum of exponentials.
+    const bool shard = a.cand_out != nullptr;
+    const uint32_t k = shard && !(in.flags & ROW_GREEDY) ? a.shard_k : in.k;
     const bool wide = k > SPL_SMALL_K;
     const uint32_t mark_mode = ca.mark_mode;
     // Decided alike by every block of the cluster: rows that end here.
@@ -683,7 +710,6 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
     ahead.draft = draws && row < a.spec.n_spec ? __ldg(a.spec.draft_ids + row) : 0u;
     const float u_row = !draws ? 0.0f : a.uniforms ? __ldg(a.uniforms + row) : in.u;
 
-    LILY_STAMP(14);
     // ---- 1. the stream: maxima and marks
     // Which block an id belongs to, and its place in that block's marks.
     auto place_of = [&](uint32_t id, uint32_t &at) -> uint32_t {
@@ -695,6 +721,109 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
     uint16_t *mark16 = reinterpret_cast<uint16_t *>(marks);
     const bool marked = hist_len + extra_len != 0u;
     const bool counted = marked && need_counts;  // (a list whose multiplicities matter)
+    if (marker && shard && a.shard_sums) {
+        // A shard has no history: this half reads the share a second time (it comes from L2,
+        // just behind the other half) and adds up the exponentials, in the base-2 domain and
+        // relative to each thread's running maximum.
+        const float scale = 1.4426950408889634f / in.temp;
+        float ref = -1e30f, part[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        constexpr uint32_t SU = 4u;
+        for (uint32_t j = warp - SPL_WARPS; j < pieces_here; j += SPL_WARPS * SU) {
+            float m = neg_inf();
+#pragma unroll
+            for (uint32_t i = 0; i < SU; ++i) {
+                q[i] = load_piece(j + SPL_WARPS * i);
+            }
+#pragma unroll
+            for (uint32_t i = 0; i < SU; ++i) {
+                m = fmaxf(m, vec_max<T>(q[i]));
+            }
+            const float y = m * scale;
+            if (y > ref) {
+                const float f = exp2f(ref - y);
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    part[c] *= f;
+                }
+                ref = y;
+            }
+#pragma unroll
+            for (uint32_t i = 0; i < SU; ++i) {
+#pragma unroll
+                for (uint32_t e = 0; e < PER; ++e) {
+                    part[e & 3u] += exp2f(fmaf(vec_get<T>(q[i], e), scale, -ref));  // (a masked -inf adds 0)
+                }
+            }
+        }
+        float sum = (part[0] + part[1]) + (part[2] + part[3]);
+        float top = ref;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            top = fmaxf(top, __shfl_xor_sync(FULL, top, o));
+        }
+        sum *= exp2f(ref - top);
+        sum = sum == sum ? sum : 0.0f;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            sum += __shfl_xor_sync(FULL, sum, o);
+        }
+        uint2 *place = &ss->sums[rank * SPL_WARPS + warp - SPL_WARPS];
+        if (blocks > 1u) {
+            asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+            if (lane == 0) {
+                put_2u32(peer_smem(place, 0), __float_as_uint(top), __float_as_uint(sum), peer_smem(&ss->mbar_sums, 0));
+            }
+        } else if (lane == 0) {
+            *place = make_uint2(__float_as_uint(top), __float_as_uint(sum));
+        }
+        if (rank != 0u) {
+            return;
+        }
+        if (blocks == 1u) {
+            asm volatile("bar.sync 6, %0;" ::"n"(SPL_NT) : "memory");
+        }
+        float total = 0.0f;
+        top = neg_inf();
+        bool late = false;
+        if (warp == SPL_WARPS) {
+            // (Collected before the verdict: the general code uses this memory for its own.)
+            if (blocks > 1u) {
+                if (lane == 0) {
+                    arrive_expect(peer_smem(&ss->mbar_sums, 0), blocks * SPL_WARPS * 8u);
+                }
+                late = !__all_sync(FULL, wait_first_phase(&ss->mbar_sums));
+            }
+            constexpr uint32_t EACH = SPL_MAX_BLOCKS * SPL_WARPS / 32u;
+            uint2 v[EACH];
+#pragma unroll
+            for (uint32_t c = 0; c < EACH; ++c) {
+                const uint32_t at = lane + 32u * c;
+                v[c] = at < blocks * SPL_WARPS ? ss->sums[at] : make_uint2(0xFF800000u, 0u);
+                top = fmaxf(top, __uint_as_float(v[c].x));
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                top = fmaxf(top, __shfl_xor_sync(FULL, top, o));
+            }
+#pragma unroll
+            for (uint32_t c = 0; c < EACH; ++c) {  // (in a fixed order: a lane's two, then the lanes' tree)
+                total += __uint_as_float(v[c].y) * exp2f(__uint_as_float(v[c].x) - top);
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                total += __shfl_xor_sync(FULL, total, o);
+            }
+        }
+        marker_ends();
+        if (tid == SPL_NT) {  // (the record's largest logit is there: written before the verdict)
+            total *= exp2f(top - float_of_key(ss->record_key) * 1.4426950408889634f);
+            a.cand_out[row].sum_exp = total == total ? total : 0.0f;
+            if (late) {
+                atomicOr(a.status_word, 1u << ROW_INTERNAL);
+            }
+        }
+        return;
+    }
     if (marker) {
         // Every block looks at the whole list for the ids of its share. (Sharing the list
         // out and marking in the owner's memory was measured slower from 2000 ids on:
@@ -928,7 +1057,14 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
             verdict(0u, ALONE);
             return;
         }
-        if (lane == 0) {
+        if (shard) {
+            if (lane == 0) {
+                sm->key[0] = win;
+                sm->id[0] = win_id;
+            }
+            __syncwarp();
+            write_record(1u);
+        } else if (lane == 0) {
             a.out_ids[row] = win_id;
             if (a.out_status) {
                 a.out_status[row] = LILY_ROW_OK;
@@ -943,7 +1079,6 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         LILY_STAMP(PH_END);
         return;
     }
-    LILY_STAMP(15);
     if (marked || n_sp != 0u) {
         asm volatile("bar.sync 3, %0;" ::"n"(NT) : "memory");
     }
@@ -1453,8 +1588,12 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
 
     // ---- 4. ranks and the draw
     auto draw = [&](uint32_t n) {  // (n candidates sorted in key[] / id[]; the warp that draws)
-        split_finalize(sm, a, row, n, in.top_p, in.min_p, u_row, a.uniforms ? 0u : in.step, in.seed, counts_draw, slot,
-                       ahead);
+        if (shard) {
+            write_record(n);
+        } else {
+            split_finalize(sm, a, row, n, in.top_p, in.min_p, u_row, a.uniforms ? 0u : in.step, in.seed, counts_draw, slot,
+                           ahead);
+        }
     };
     if (blocks == 1u) {
         spl_sync();  // (head[0] and the candidates are this block's own)
@@ -1574,6 +1713,9 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         }
     }
     spl_sync();
+    if (shard && tid == 0) {
+        ss->record_key = sm->key[0];
+    }
     verdict(1u, DONE);
     LILY_STAMP(PH_SORT);
     if (draws) {
