@@ -262,6 +262,60 @@ int32_t launch_one(lily_sampler *h, cudaStream_t stream_, const lily::KArgs &a, 
     return launch_serialised(h, stream_, kernel, dim3(a.n_slices, rows, 1), smem, a);
 }
 
+// Parameters of more rows than a launch's own arguments take go to the device in the
+// arguments of a launch of their own: stored first, then the stream's previous work is
+// waited for, so that the launch behind it may trust its own wait. (A copy from pinned
+// memory between two kernels cost some 10 us of the stream's time: 256 rows x 32768 took
+// 25.9 us with it.)
+template <uint32_t BYTES>
+struct PutArgs {
+    uint4 *to;
+    uint32_t n;  // 16-byte words
+    uint4 data[BYTES / 16u];
+};
+
+constexpr uint32_t PUT_THREADS = 64;
+
+template <uint32_t BYTES>
+__global__ void __launch_bounds__(PUT_THREADS) put_kernel(const __grid_constant__ PutArgs<BYTES> p) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const uint32_t i = blockIdx.x * PUT_THREADS + threadIdx.x;
+    if (i < p.n) {
+        p.to[i] = p.data[i];
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <uint32_t BYTES>
+cudaError_t put(void *to, const void *from, size_t bytes, cudaStream_t stream) {
+    PutArgs<BYTES> p;
+    p.to = static_cast<uint4 *>(to);
+    p.n = (uint32_t)(bytes / 16u);
+    std::memcpy(p.data, from, bytes);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((p.n + PUT_THREADS - 1u) / PUT_THREADS, 1, 1);
+    cfg.blockDim = dim3(PUT_THREADS, 1, 1);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, put_kernel<BYTES>, p);
+}
+
+// The first `bytes` (a multiple of 256) of a staging slot to the device. (A launch takes
+// somewhat less than 32 KB of arguments.)
+int32_t upload(lily_sampler *h, int slot, size_t bytes, cudaStream_t stream) {
+    void *to = h->d_stage[slot];
+    const void *from = h->h_stage[slot];
+    CU(h, bytes <= 4096u    ? put<4096>(to, from, bytes, stream)
+          : bytes <= 16384u ? put<16384>(to, from, bytes, stream)
+          : bytes <= 32000u ? put<32000>(to, from, bytes, stream)
+                            : cudaMemcpyAsync(to, from, bytes, cudaMemcpyHostToDevice, stream));
+    return LILY_OK;
+}
+
 // How the row kernel is launched: the blocks a row is split over, and how each
 // keeps the history ids of its share.
 struct SplitPlan {
@@ -317,7 +371,10 @@ SplitPlan split_plan(const lily_sampler *h, const lily::KArgs &a, uint32_t rows,
     }
     p.smem = fixed + (size_t)p.mark_words * 4u;
     p.smem = p.smem > general ? p.smem : general;
-    p.take = p.smem <= (size_t)h->max_smem && p.sole;
+    // More rows than SMs: two blocks to an SM, unless the kernel of one block per row takes the
+    // call (aligned logits), which reads further ahead. 256 rows x 151936 bf16: 30.6 us here,
+    // 27.6 there; x 151937, which only the general kernel took: 106.7 -> 31.9.
+    p.take = p.smem <= (size_t)h->max_smem && (p.sole || !stream_route(a, rows, dtype));
     return p;
 }
 
@@ -325,6 +382,7 @@ template <uint32_t MAXR>
 int32_t launch_split(lily_sampler *h, cudaStream_t stream, lily::SplitArgs<MAXR> &sa, const SplitPlan &p,
                      uint32_t rows, uint32_t dtype) {
     sa.log_blocks = p.log_blocks;
+    sa.two_per_sm = p.sole ? 0u : 1u;
     sa.mark_mode = p.mark_mode;
     sa.mark_words = p.mark_words;
     sa.spill_params = reinterpret_cast<lily_sampling_params_t *>(h->spill);
@@ -869,6 +927,7 @@ int32_t lily_sample_batch(lily_sampler_t *h, void *stream_, const lily_sample_ar
         raises_few = raises && g.rows <= 16u;
         plan.take = plan.take && !raises_few;
     }
+    const StageLayout layout = stage_layout(g.rows);
     const bool in_args = plan.take;
     if (!in_args && (!g.params_on_device || g.count_slots != nullptr)) {
         st = next_stage(h, &slot);
@@ -894,21 +953,22 @@ int32_t lily_sample_batch(lily_sampler_t *h, void *stream_, const lily_sample_ar
     }
     if (!g.params_on_device && !in_args) {
         char *hs = h->h_stage[slot];
-        std::memcpy(hs + h->layout.params, g.params, sizeof(lily_sampling_params_t) * g.rows);
+        std::memcpy(hs + layout.params, g.params, sizeof(lily_sampling_params_t) * g.rows);
         d_params = reinterpret_cast<const lily_sampling_params_t *>(h->d_stage[slot] +
-                                                                    h->layout.params);
+                                                                    layout.params);
         if (g.steps != nullptr) {
-            std::memcpy(hs + h->layout.steps, g.steps, sizeof(uint32_t) * g.rows);
-            d_steps = reinterpret_cast<const uint32_t *>(h->d_stage[slot] + h->layout.steps);
+            std::memcpy(hs + layout.steps, g.steps, sizeof(uint32_t) * g.rows);
+            d_steps = reinterpret_cast<const uint32_t *>(h->d_stage[slot] + layout.steps);
         }
     }
     if (g.count_slots != nullptr && !in_args) {
-        std::memcpy(h->h_stage[slot] + h->layout.slots, g.count_slots, sizeof(uint32_t) * g.rows);
-        d_slots = reinterpret_cast<const uint32_t *>(h->d_stage[slot] + h->layout.slots);
+        std::memcpy(h->h_stage[slot] + layout.slots, g.count_slots, sizeof(uint32_t) * g.rows);
+        d_slots = reinterpret_cast<const uint32_t *>(h->d_stage[slot] + layout.slots);
     }
     if (slot >= 0) {
-        CU(h, cudaMemcpyAsync(h->d_stage[slot], h->h_stage[slot], h->layout.total,
-                              cudaMemcpyHostToDevice, stream));
+        if ((st = upload(h, slot, layout.total, stream)) != LILY_OK) {
+            return st;
+        }
     }
     a.params = d_params;
     a.uniforms = g.uniforms;
@@ -983,13 +1043,16 @@ int32_t lily_sample_one(lily_sampler_t *h, void *stream_, const void *logits, ui
         return st;
     }
     char *hs = h->h_stage[slot], *ds = h->d_stage[slot];
-    std::memcpy(hs + h->layout.params, params, sizeof(*params));
-    std::memcpy(hs + h->layout.steps, &step, 4);
-    std::memcpy(hs + h->layout.hist_len, &history_len, 4);
-    CU(h, cudaMemcpyAsync(ds, hs, h->layout.total, cudaMemcpyHostToDevice, stream));
-    a.params = reinterpret_cast<const lily_sampling_params_t *>(ds + h->layout.params);
-    a.steps = reinterpret_cast<const uint32_t *>(ds + h->layout.steps);
-    a.history_len = history_ids ? reinterpret_cast<const uint32_t *>(ds + h->layout.hist_len) : nullptr;
+    const StageLayout layout = stage_layout(1u);
+    std::memcpy(hs + layout.params, params, sizeof(*params));
+    std::memcpy(hs + layout.steps, &step, 4);
+    std::memcpy(hs + layout.hist_len, &history_len, 4);
+    if ((st = upload(h, slot, layout.total, stream)) != LILY_OK) {
+        return st;
+    }
+    a.params = reinterpret_cast<const lily_sampling_params_t *>(ds + layout.params);
+    a.steps = reinterpret_cast<const uint32_t *>(ds + layout.steps);
+    a.history_len = history_ids ? reinterpret_cast<const uint32_t *>(ds + layout.hist_len) : nullptr;
     st = launch(h, stream, a, 1u, logits_dtype, true);
     CU(h, cudaEventRecord(h->ev[slot], stream));
     return st;
@@ -1160,6 +1223,7 @@ int32_t check_shard_params(lily_sampler *h, const lily_sample_args_t &g) {
 int32_t stage_shard_params(lily_sampler *h, cudaStream_t stream, const lily_sample_args_t &g,
                            const lily_sampling_params_t **d_params, const uint32_t **d_steps,
                            int *slot_out) {
+    const StageLayout layout = stage_layout(g.rows);
     // What would be staged: [rows][has steps][params][steps].
     const size_t pb = sizeof(lily_sampling_params_t) * g.rows, sb = g.steps ? sizeof(uint32_t) * g.rows : 0;
     std::vector<char> want(8 + pb + sb);
@@ -1177,20 +1241,21 @@ int32_t stage_shard_params(lily_sampler *h, cudaStream_t stream, const lily_samp
             return st;
         }
         char *hs = h->h_stage[slot];
-        std::memcpy(hs + h->layout.params, g.params, pb);
+        std::memcpy(hs + layout.params, g.params, pb);
         if (sb) {
-            std::memcpy(hs + h->layout.steps, g.steps, sb);
+            std::memcpy(hs + layout.steps, g.steps, sb);
         }
-        CU(h, cudaMemcpyAsync(h->d_stage[slot], h->h_stage[slot], h->layout.total, cudaMemcpyHostToDevice,
-                              stream));
+        if ((st = upload(h, slot, layout.total, stream)) != LILY_OK) {
+            return st;
+        }
         h->shard_slot = slot;
         h->shard_serial = h->slot_serial[slot];
         h->shard_bytes.swap(want);
     }
     // (A reused slot is read by one more launch: the caller records the slot's
     // event after it, so the ring does not overwrite the slot under that launch.)
-    *d_params = reinterpret_cast<const lily_sampling_params_t *>(h->d_stage[slot] + h->layout.params);
-    *d_steps = g.steps != nullptr ? reinterpret_cast<const uint32_t *>(h->d_stage[slot] + h->layout.steps) : nullptr;
+    *d_params = reinterpret_cast<const lily_sampling_params_t *>(h->d_stage[slot] + layout.params);
+    *d_steps = g.steps != nullptr ? reinterpret_cast<const uint32_t *>(h->d_stage[slot] + layout.steps) : nullptr;
     *slot_out = slot;
     return LILY_OK;
 }
@@ -1627,18 +1692,21 @@ int32_t lily_spec_verify(lily_sampler_t *h, void *stream_, const lily_spec_args_
             return st;
         }
         char *hs = h->h_stage[slot], *ds = h->d_stage[slot];
-        auto *sh = reinterpret_cast<uint32_t *>(hs + h->layout.hist_len);
-        std::memcpy(hs + h->layout.params, params, sizeof(params[0]) * g.m);
-        std::memcpy(hs + h->layout.steps, steps, 4u * g.m);
-        std::memcpy(hs + h->layout.slots, slots, 4u * g.m);
+        const StageLayout layout = stage_layout(g.m);
+        auto *sh = reinterpret_cast<uint32_t *>(hs + layout.hist_len);
+        std::memcpy(hs + layout.params, params, sizeof(params[0]) * g.m);
+        std::memcpy(hs + layout.steps, steps, 4u * g.m);
+        std::memcpy(hs + layout.slots, slots, 4u * g.m);
         for (uint32_t j = 0; j < g.m; ++j) {
             sh[j] = g.history_len;
         }
-        CU(h, cudaMemcpyAsync(ds, hs, h->layout.total, cudaMemcpyHostToDevice, stream));
-        a.params = reinterpret_cast<const lily_sampling_params_t *>(ds + h->layout.params);
-        a.steps = reinterpret_cast<const uint32_t *>(ds + h->layout.steps);
-        a.history_len = g.history_ids ? reinterpret_cast<const uint32_t *>(ds + h->layout.hist_len) : nullptr;
-        a.count_slots = g.count_slot ? reinterpret_cast<const uint32_t *>(ds + h->layout.slots) : nullptr;
+        if ((st = upload(h, slot, layout.total, stream)) != LILY_OK) {
+            return st;
+        }
+        a.params = reinterpret_cast<const lily_sampling_params_t *>(ds + layout.params);
+        a.steps = reinterpret_cast<const uint32_t *>(ds + layout.steps);
+        a.history_len = g.history_ids ? reinterpret_cast<const uint32_t *>(ds + layout.hist_len) : nullptr;
+        a.count_slots = g.count_slot ? reinterpret_cast<const uint32_t *>(ds + layout.slots) : nullptr;
     }
     for (uint32_t j = 0; j < launches && st == LILY_OK; ++j) {
         a.row0 = j;

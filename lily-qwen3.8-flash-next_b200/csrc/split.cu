@@ -7,11 +7,11 @@ namespace lily {
 
 namespace {
 
-template <typename T, uint32_t MAXR>
+template <typename T, uint32_t MAXR, int BPS>
 cudaError_t launch_one(const SplitArgs<MAXR> &a, uint32_t rows, size_t smem, int max_smem, uint32_t *attr_mask,
                        cudaStream_t stream) {
-    auto kernel = split_rows_kernel<T, MAXR, 1>;
-    const uint32_t bit = 1u << ((sizeof(T) == 4 ? 16 : 17) + (MAXR == INLINE_ROWS ? 0 : MAXR == INLINE_ROWS_MID ? 2 : 4));
+    auto kernel = split_rows_kernel<T, MAXR, BPS>;
+    const uint32_t bit = 1u << ((sizeof(T) == 4 ? 16 : 17) + (MAXR == INLINE_ROWS ? 0 : MAXR == INLINE_ROWS_MID ? 2 : 4) + (BPS == 1 ? 0 : 7));
     if (!(*attr_mask & bit)) {
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
         if (e != cudaSuccess) {
@@ -41,8 +41,14 @@ cudaError_t launch_one(const SplitArgs<MAXR> &a, uint32_t rows, size_t smem, int
 template <uint32_t MAXR>
 cudaError_t split_launch(const SplitArgs<MAXR> &a, uint32_t rows, uint32_t dtype, size_t smem, int max_smem,
                          uint32_t *attr_mask, cudaStream_t stream) {
-    return dtype == LILY_F32 ? launch_one<float, MAXR>(a, rows, smem, max_smem, attr_mask, stream)
-                             : launch_one<__nv_bfloat16, MAXR>(a, rows, smem, max_smem, attr_mask, stream);
+    if constexpr (MAXR == INLINE_ROWS) {
+        if (a.two_per_sm) {
+            return dtype == LILY_F32 ? launch_one<float, MAXR, 2>(a, rows, smem, max_smem, attr_mask, stream)
+                                     : launch_one<__nv_bfloat16, MAXR, 2>(a, rows, smem, max_smem, attr_mask, stream);
+        }
+    }
+    return dtype == LILY_F32 ? launch_one<float, MAXR, 1>(a, rows, smem, max_smem, attr_mask, stream)
+                             : launch_one<__nv_bfloat16, MAXR, 1>(a, rows, smem, max_smem, attr_mask, stream);
 }
 
 template cudaError_t split_launch<INLINE_ROWS>(const SplitArgs<INLINE_ROWS> &, uint32_t, uint32_t, size_t, int, uint32_t *,

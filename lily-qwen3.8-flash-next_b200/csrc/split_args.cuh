@@ -104,6 +104,7 @@ template <uint32_t MAXR>
 struct SplitArgs {
     KArgs a;
     uint32_t log_blocks;      // log2 of the blocks per row
+    uint32_t two_per_sm;      // more rows than SMs: the instantiation of which two blocks fit
     uint32_t mark_mode;
     uint32_t mark_words;      // 32-bit words of the marks, a multiple of four
     uint32_t inline_params;   // `in` below is valid (else a.params / a.steps)

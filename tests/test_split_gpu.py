@@ -47,3 +47,16 @@ def test_ties_fill_the_candidates(cuda, lily, W):
     for quantise in (16, 4, 1, 0.25):
         b = make_batch(W, rng, 2, 30_000, 50, True, kind="uniform", quantise=quantise, history=50, rep=1.1)
         check(cuda, lily, W, b, 30_000, f"steps of 1/{quantise}")
+
+
+@pytest.mark.parametrize("rows", [16, 34, 65, 297, 315, 316, 620])
+def test_rows_around_the_waves_and_the_argument_blocks(cuda, lily, W, rows):
+    # 16 and 34: more clusters of eight or four than run at once; 65: the largest argument
+    # block; from 149 on two blocks to an SM, the parameters stored by a launch of their own
+    # (of 16 KB up to 315 rows, of 32 KB up to 615, then by a copy).
+    vocab = 9_001
+    rng = np.random.default_rng(rows)
+    for bf16, k, kw in ((True, 64, dict(history=900, rep=1.2, n_bias=3, n_ban=2)), (False, 0, dict(presence=0.3, history=40)),
+                        (False, 1, {}), (True, 30, dict(history=200, frequency=0.2))):
+        b = make_batch(W, rng, rows, vocab, k, bf16, kind="zipf", **kw)
+        check(cuda, lily, W, b, vocab, f"B={rows} bf16={bf16} k={k}")
