@@ -87,11 +87,13 @@ cudaError_t launch_for(const Args &a, Format format, uint32_t sms, cudaStream_t 
 // their scaling all go with it. Measured per call, both launches, back to back (before:
 // 64 always, one pipeline for both halves of a tile, bf16 only, the affine term in a kernel
 // of its own, whole tiles only):
-//   262144 x 4096, symmetric:     64 tokens 325 -> 248 us, 32 tokens 200, 16 tokens 181
-//   248320 x 4096, affine 8 bits: 64 tokens 430 -> 303 us,  4 tokens 435 -> 176
-//   151936 x 2048, affine 4 bits: 64 tokens 102 us, 32 tokens 160 -> 80, 4 tokens 63
-// At 16 tokens the weights' stream bounds it (5.9 TB/s of 6.6 measured for a copy); at 64
-// the integer and FMA pipes do: widening a weight, and one FMA per logit and group.
+//   262144 x 4096, symmetric:     64 tokens 325 -> 245 us, 32 tokens 194, 16 tokens 180
+//   248320 x 4096, affine 8 bits: 64 tokens 430 -> 285 us,  4 tokens 435 -> 172
+//   151936 x 2048, affine 4 bits: 64 tokens 90 us, 32 tokens 160 -> 61, 4 tokens 50
+// (4 bits, 32 tokens, step by step: 80; two groups per hand-over and fewer stages 70; codes
+// as subnormals 61.) At 16 tokens the weights' stream bounds bytes (5.9 TB/s of 6.6
+// measured for a copy); the rest is bound by issue slots (67 % busy before the last step):
+// widening a weight, and one FMA per logit and group.
 cudaError_t launch_head(const Args &a, Format format, uint32_t sms, cudaStream_t stream) {
     switch (padded_tokens(a.tokens)) {
         case 16: return launch_for<16>(a, format, sms, stream);

@@ -17,7 +17,7 @@
 //   * converter warps own one tile row per thread: they widen a group's 64 weights
 //     exactly to 16 bits and store them with tcgen05.st into TENSOR MEMORY, where the
 //     multiplier reads its A operand (lane = row, two values per column);
-//   * two threads, one per 128 rows, issue 4 tcgen05.mma each per group (M = 128, N =
+//   * four warps, two per 128 rows, issue 4 tcgen05.mma each per group (M = 128, N =
 //     tokens, K = 16) into an accumulator that starts from zero: products of two
 //     8-bit significands are exact in binary32;
 //   * epilogue warps read each group's sums back with tcgen05.ld, multiply by the
@@ -29,9 +29,11 @@
 //
 // Binary16 or bf16. Widening a byte to binary16 costs two or three integer
 // instructions per four weights, to bf16 (whose significand does not hold 128 + 255)
-// six; the integer pipe was the busiest one. A bf16 hidden value times a power of two
-// per token fits binary16 exactly if it lies within 2^32 of the token's largest, which
-// hidden states do; a call in which one does not is multiplied in bf16, same results.
+// six; the integer pipe was the busiest one. A 4-bit code takes a mask: alone in 16
+// bits it is a subnormal binary16, which the multiplier takes exactly. A bf16 hidden
+// value times a power of two per token fits binary16 exactly if it lies within 2^32
+// (4-bit codes: 2^28) of the token's largest, which hidden states do; a call in which one
+// does not is multiplied in bf16, same results.
 //
 // Measured at 262144 x 4096, 64 tokens (before: bf16 only, one pipeline for both
 // halves, N = 64 always, the affine term in a kernel of its own): see the figures at
@@ -57,14 +59,12 @@ constexpr int WARP_LOAD_H = 5;
 constexpr int WARP_CONV0 = 8;
 
 constexpr uint32_t RAW_STAGE_BYTES = TILE_ROWS * 128u;  // 32 KB
-constexpr uint32_t H_SLOTS = 8;    // hidden slices in shared memory
-constexpr uint32_t SUM_SLOTS = 16; // their sums: read by the epilogue, at most that far behind
-constexpr uint32_t DONE_SLOTS = 8; // ring of "group q has been multiplied" barriers
 constexpr uint32_t TMEM_COLS = 512;
 
 // What depends on the (padded) number of tokens and the format. Tensor memory per half:
-// ACC_BUFS accumulators of N columns, A_SLOTS operand tiles of 32. The converters are one
-// codes is two weights to widen: two teams of converter warps.
+// ACC_BUFS times PG accumulators of N columns, A_SLOTS times PG operand tiles of 32. The
+// converters are two teams of eight warps, which share the groups; one team where the
+// epilogue of 64 tokens needs the registers.
 template <uint32_t N, int FMT>
 struct Shape {
     static constexpr uint32_t TEAMS = N == 64u && FMT != FMT_S8 ? 1u : 2u;
@@ -79,12 +79,20 @@ struct Shape {
     static constexpr uint32_t REGS_CONV = TEAMS == 1u ? 64u : N == 64u ? 48u : 56u;
     static constexpr uint32_t REGS_EPI = TEAMS == 1u ? 136u : N == 64u ? 120u : 104u;
     static_assert(32u * (8u * REGS_CTRL + CONV_WARPS * REGS_CONV + EPI_WARPS * REGS_EPI) <= THREADS * REGS, "register shares");
-    static constexpr uint32_t ACC_BUFS = N == 64u ? 2u : 4u;
-    static constexpr uint32_t A_SLOTS = 4u;
-    static constexpr uint32_t RAW_STAGES = N == 64u ? 4u : N == 32u ? 5u : 6u;
+    // Groups per hand-over (of operands, of accumulators): a hand-over costs each of its two
+    // sides some 200 to 300 clocks, whatever goes through it.
+    static constexpr uint32_t PG = N == 64u ? 1u : 2u;
+    static constexpr uint32_t ACC_BUFS = 2u;                              // of PG groups
+    static constexpr uint32_t A_SLOTS = N == 64u ? 4u : N == 32u ? 2u : 3u;  // of PG groups
+    // (No more stages than the latency of memory needs: what shared memory leaves of the L1
+    // cache holds the scales' lines, each of which is read eight times.)
+    static constexpr uint32_t RAW_STAGES = N == 64u ? 3u : N == 32u ? 4u : 5u;
+    static constexpr uint32_t H_SLOTS = 8u;                             // hidden slices in shared memory
+    static constexpr uint32_t DONE_SLOTS = H_SLOTS / PG;                // ring of "has been multiplied" barriers
+    static constexpr uint32_t SUM_SLOTS = 2u * H_SLOTS;                 // the slices' sums: the epilogue may be that far behind
     static constexpr uint32_t H_BYTES = N * 128u;
-    static constexpr uint32_t A_COL0 = ACC_BUFS * N;                    // within a half's 256 columns
-    static_assert(A_COL0 + A_SLOTS * 32u <= TMEM_COLS / 2u, "tensor memory columns of a half");
+    static constexpr uint32_t A_COL0 = ACC_BUFS * PG * N;                    // within a half's 256 columns
+    static_assert(A_COL0 + A_SLOTS * PG * 32u <= TMEM_COLS / 2u, "tensor memory columns of a half");
     static_assert(ACC_BUFS <= DONE_SLOTS && A_SLOTS <= DONE_SLOTS, "the rings' phases");
     static constexpr int WARP_EPI0 = WARP_CONV0 + (int)CONV_WARPS;
 
@@ -98,7 +106,7 @@ struct Shape {
     static constexpr uint32_t RAW_EMPTY = RAW_FULL + 8 * RAW_STAGES;
     static constexpr uint32_t H_FULL = RAW_EMPTY + 8 * RAW_STAGES;      // [H_SLOTS / 2]
     static constexpr uint32_t A_FULL = H_FULL + 8 * H_SLOTS;            // [2][A_SLOTS]
-    // DONE[half][q % 8]: a half of group q has been multiplied. One commit tells the
+    // DONE[half][..]: a half of PG groups has been multiplied. One commit tells the
     // converters (slot free), the hidden loader and the epilogue (sums ready).
     static constexpr uint32_t DONE = A_FULL + 2 * 8 * A_SLOTS;          // [2][DONE_SLOTS]
     static constexpr uint32_t ACC_EMPTY = DONE + 2 * 8 * DONE_SLOTS;    // [2][ACC_BUFS]
@@ -351,12 +359,13 @@ __device__ __forceinline__ void widen_bytes(uint32_t x, uint32_t &even, uint32_t
 template <bool BF16>
 __device__ __forceinline__ void widen_nibbles(uint32_t x, uint32_t &a, uint32_t &b, uint32_t &c, uint32_t &d) {
     if (!BF16) {
-        // (A nibble in the upper half of a byte stands for 16 times its value.)
+        // A code alone in 16 bits is a subnormal binary16: 2^-24 times its value, or 2^-20
+        // where it is the upper half of a byte (the hidden image makes up for both).
         const uint32_t y = x >> 8;
-        asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(a) : "r"((x & 0x000F000Fu) | 0x64006400u), "r"(0x64006400u));
-        asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(b) : "r"((x & 0x00F000F0u) | 0x64006400u), "r"(0x2C002C00u), "r"(0xD400D400u));
-        asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(c) : "r"((y & 0x000F000Fu) | 0x64006400u), "r"(0x64006400u));
-        asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"((y & 0x00F000F0u) | 0x64006400u), "r"(0x2C002C00u), "r"(0xD400D400u));
+        a = x & 0x000F000Fu;
+        b = x & 0x00F000F0u;
+        c = y & 0x000F000Fu;
+        d = y & 0x00F000F0u;
     } else {
         asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(a) : "r"((x & 0x000F000Fu) | 0x43004300u), "r"(0x43004300u));
         asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(b) : "r"(((x >> 4) & 0x000F000Fu) | 0x43004300u), "r"(0x43004300u));
@@ -404,6 +413,9 @@ __global__ void __launch_bounds__(256) prepare_hidden_kernel(const Prepared p, c
     const int exponent = (int)(top_s >> 23);
     const int shift = top_s == 0u ? 0 : min(142 - exponent, 126);
     const float scale = __uint_as_float((uint32_t)(shift + 127) << 23);
+    // (4-bit codes: the odd columns' stand for 16 times their value, all for 2^-24 times.)
+    const float scale_odd = nibbles ? __fmul_rn(scale, 0.0625f) : scale;
+    const int codes = nibbles ? 24 : 0;
     // (A token of extreme size stays as it is: a scaled sum might overflow where its own does not.)
     uint32_t lost = shift < -40 || shift > 40 ? 1u : 0u;
 #pragma unroll
@@ -420,8 +432,8 @@ __global__ void __launch_bounds__(256) prepare_hidden_kernel(const Prepared p, c
             const float lo = __uint_as_float(w[e] << 16), hi = __uint_as_float(w[e] & 0xFFFF0000u);
             sum += lo;
             sum += hi;
-            const __half a = __float2half_rn(__fmul_rn(lo, scale)), b = __float2half_rn(__fmul_rn(hi, scale));
-            lost |= __half2float(a) == __fmul_rn(lo, scale) && __half2float(b) == __fmul_rn(hi, scale) ? 0u : 1u;
+            const __half a = __float2half_rn(__fmul_rn(lo, scale)), b = __float2half_rn(__fmul_rn(hi, scale_odd));
+            lost |= __half2float(a) == __fmul_rn(lo, scale) && __half2float(b) == __fmul_rn(hi, scale_odd) ? 0u : 1u;
             h[e] = (uint32_t)__half_as_ushort(a) | ((uint32_t)__half_as_ushort(b) << 16);
         }
 #pragma unroll
@@ -438,13 +450,13 @@ __global__ void __launch_bounds__(256) prepare_hidden_kernel(const Prepared p, c
         p.image[0][at] = ordered(h);
         p.image[1][at] = ordered(w);
         if (chunk == 0u) {
-            p.sums[0][g * padded + t] = __fmul_rn(sum, scale);
+            p.sums[0][g * padded + t] = __fmul_rn(sum, __uint_as_float((uint32_t)(shift - codes + 127) << 23));
             p.sums[1][g * padded + t] = sum;
         }
     }
     const int any = __syncthreads_or((int)lost);
     if (tid == 0) {
-        p.unscale[t] = __uint_as_float((uint32_t)(127 - shift) << 23);
+        p.unscale[t] = __uint_as_float((uint32_t)(127 - shift + codes) << 23);
         p.inexact[t] = any ? 1u : 0u;
     }
 }
@@ -491,13 +503,13 @@ __global__ void __launch_bounds__(Shape<N, FMT>::THREADS, 1) lmhead_kernel(const
             mbar_init(base + S::RAW_FULL + 8 * s, 1);
             mbar_init(base + S::RAW_EMPTY + 8 * s, S::CONV_WARPS);
         }
-        for (uint32_t s = 0; s < H_SLOTS / 2u; ++s) {
+        for (uint32_t s = 0; s < S::H_SLOTS / 2u; ++s) {
             mbar_init(base + S::H_FULL + 8 * s, 1);
         }
         for (uint32_t s = 0; s < 2u * S::A_SLOTS; ++s) {
-            mbar_init(base + S::A_FULL + 8 * s, 4);
+            mbar_init(base + S::A_FULL + 8 * s, 4 * S::PG);
         }
-        for (uint32_t s = 0; s < 2u * DONE_SLOTS; ++s) {
+        for (uint32_t s = 0; s < 2u * S::DONE_SLOTS; ++s) {
             mbar_init(base + S::DONE + 8 * s, 1);
         }
         for (uint32_t b = 0; b < 2u * S::ACC_BUFS; ++b) {
@@ -545,22 +557,25 @@ __global__ void __launch_bounds__(Shape<N, FMT>::THREADS, 1) lmhead_kernel(const
             const bool leader = elect_one();
             const uint32_t idesc = instr_desc<N>(bf16);
             const uint32_t acc0 = tmem + half * 256u, a0 = acc0 + S::A_COL0;
-            for (uint32_t q = mw >> 1; q < total_groups; q += MMA_WARPS / 2) {
-                const uint32_t as = q % S::A_SLOTS, hs = q % H_SLOTS, b = q % S::ACC_BUFS;
-                bool gave_up = wait(S::H_FULL + 8 * (hs / 2u), q / H_SLOTS);
+            for (uint32_t q = mw >> 1; q < total_groups / S::PG; q += MMA_WARPS / 2) {
+                const uint32_t as = q % S::A_SLOTS, hs = q * S::PG % S::H_SLOTS, b = q % S::ACC_BUFS;
+                bool gave_up = wait(S::H_FULL + 8 * (hs / 2u), q * S::PG / S::H_SLOTS);
                 gave_up |= wait(S::ACC_EMPTY + 8 * (half * S::ACC_BUFS + b), (q / S::ACC_BUFS) ^ 1u);
                 gave_up |= wait(S::A_FULL + 8 * (half * S::A_SLOTS + as), q / S::A_SLOTS);
                 if (__any_sync(FULL, gave_up)) {
                     break;
                 }
                 tc_fence_after();
-                const uint64_t bdesc = operand_desc(base + S::HID + hs * S::H_BYTES);
                 if (leader) {
 #pragma unroll
-                    for (uint32_t k4 = 0; k4 < 4; ++k4) {
-                        mma_ts(acc0 + b * N, a0 + as * 32u + k4 * 8u, bdesc + k4 * 2u, idesc, k4);
+                    for (uint32_t g = 0; g < S::PG; ++g) {
+                        const uint64_t bdesc = operand_desc(base + S::HID + (hs + g) * S::H_BYTES);
+#pragma unroll
+                        for (uint32_t k4 = 0; k4 < 4; ++k4) {
+                            mma_ts(acc0 + (b * S::PG + g) * N, a0 + (as * S::PG + g) * 32u + k4 * 8u, bdesc + k4 * 2u, idesc, k4);
+                        }
                     }
-                    mma_commit(base + S::DONE + 8 * (half * DONE_SLOTS + q % DONE_SLOTS));
+                    mma_commit(base + S::DONE + 8 * (half * S::DONE_SLOTS + q % S::DONE_SLOTS));
                 }
                 __syncwarp();
             }
@@ -618,15 +633,15 @@ __global__ void __launch_bounds__(Shape<N, FMT>::THREADS, 1) lmhead_kernel(const
             const uint8_t *image = reinterpret_cast<const uint8_t *>(a.prep.image[bf16 ? 1 : 0]);
             const float *sums = a.prep.sums[bf16 ? 1 : 0];
             uint32_t g = 0;
-            static_assert(H_SLOTS == DONE_SLOTS, "the hidden ring and the done ring share their indexing");
+            static_assert(S::H_SLOTS == S::DONE_SLOTS * S::PG, "the hidden ring and the done ring share their indexing");
             for (uint32_t q = 0; q < total_groups; q += 2u) {
                 if (q % BLOCK_GROUPS == 0u) {
                     g = unit_at(q / BLOCK_GROUPS) % per_tile * BLOCK_GROUPS;
                 }
-                const uint32_t pair = (q / 2u) % (H_SLOTS / 2u), use = q / H_SLOTS;
+                const uint32_t pair = (q / 2u) % (S::H_SLOTS / 2u), use = q / S::H_SLOTS;
                 bool gave_up = false;
-                if (q >= H_SLOTS && lane < 4u) {  // the slot's previous two groups have been multiplied, by both halves
-                    gave_up = wait(S::DONE + 8 * ((lane & 1u) * DONE_SLOTS + (q + (lane >> 1)) % DONE_SLOTS), use ^ 1u);
+                if (q >= S::H_SLOTS && lane < 4u / S::PG) {  // the slot's previous two groups have been multiplied, by both halves
+                    gave_up = wait(S::DONE + 8 * ((lane & 1u) * S::DONE_SLOTS + (q / S::PG + (lane >> 1)) % S::DONE_SLOTS), use ^ 1u);
                 }
                 if (__any_sync(FULL, gave_up)) {
                     break;
@@ -638,13 +653,13 @@ __global__ void __launch_bounds__(Shape<N, FMT>::THREADS, 1) lmhead_kernel(const
                     mbar_expect_tx(bar, 2u * S::H_BYTES + (AFFINE ? 2u * N * 4u : 0u));
                     bulk_load(base + S::HID + 2u * pair * S::H_BYTES, image + (size_t)g * S::H_BYTES, 2u * S::H_BYTES, bar);
                     if (AFFINE) {
-                        bulk_load(base + S::SUMS + (q % SUM_SLOTS) * N * 4u, sums + (size_t)g * N, 2u * N * 4u, bar);
+                        bulk_load(base + S::SUMS + (q % S::SUM_SLOTS) * N * 4u, sums + (size_t)g * N, 2u * N * 4u, bar);
                     }
                 }
                 g += 2u;
             }
             if (lane == 0 && *abort_word) {
-                for (uint32_t s2 = 0; s2 < H_SLOTS / 2u; ++s2) {
+                for (uint32_t s2 = 0; s2 < S::H_SLOTS / 2u; ++s2) {
                     if ((asked >> s2) & 1u) {
                         mbar_drain(base + S::H_FULL + 8 * s2, (parity >> s2) & 1u, wait_ns);
                     }
@@ -672,7 +687,8 @@ __global__ void __launch_bounds__(Shape<N, FMT>::THREADS, 1) lmhead_kernel(const
                 const uint32_t raw_row = base + S::RAW + st * RAW_STAGE_BYTES + trow * 128u;
 #pragma unroll 1
                 for (uint32_t gg = team; gg < RG; gg += S::TEAMS) {
-                    const uint32_t q = i * RG + gg, as = q % S::A_SLOTS;
+                    const uint32_t q = (i * RG + gg) / S::PG, as = q % S::A_SLOTS;
+                    static_assert(S::PG == 1u || S::TEAMS == 2u, "each team converts one group of a hand-over");
                     constexpr uint32_t CHUNKS = FMT == FMT_U4 ? 2u : 4u;  // of 16 bytes
                     constexpr uint32_t CW = 32u / CHUNKS;                 // words of a chunk
                     auto load_chunk = [&](uint32_t c, uint32_t (&x)[4]) {
@@ -702,11 +718,11 @@ __global__ void __launch_bounds__(Shape<N, FMT>::THREADS, 1) lmhead_kernel(const
                         bool gave_up = false;
                         if (q >= S::A_SLOTS) {
                             const uint32_t before = q - S::A_SLOTS;
-                            gave_up = wait(S::DONE + 8 * (half * DONE_SLOTS + before % DONE_SLOTS), before / DONE_SLOTS);
+                            gave_up = wait(S::DONE + 8 * (half * S::DONE_SLOTS + before % S::DONE_SLOTS), before / S::DONE_SLOTS);
                         }
                         return !__any_sync(FULL, gave_up);
                     };
-                    const uint32_t to = a_base + as * 32u;
+                    const uint32_t to = a_base + (as * S::PG + (S::PG == 2u ? team : 0u)) * 32u;
                     if (!S::LEAN) {
                         // Widen first (it needs no slot), then wait for the slot: the
                         // conversion overlaps the multiplies still reading the slot.
@@ -838,14 +854,16 @@ __global__ void __launch_bounds__(Shape<N, FMT>::THREADS, 1) lmhead_kernel(const
             }
 #pragma unroll
             for (uint32_t gi = 0; gi < BLOCK_GROUPS; ++gi, ++q) {
-                const uint32_t b = q % S::ACC_BUFS;
+                const uint32_t p = q / S::PG, b = p % S::ACC_BUFS;
                 const float s = __uint_as_float((gi & 1u) ? (sw[gi >> 1] & 0xFFFF0000u) : (sw[gi >> 1] << 16));
                 const uint64_t s2 = pack2(__float_as_uint(s), __float_as_uint(s));
-                if (__any_sync(FULL, wait(S::DONE + 8 * (half * DONE_SLOTS + q % DONE_SLOTS), q / DONE_SLOTS))) {
-                    goto epilogue_out;  // the block has given up: nothing more is read or written
+                if (gi % S::PG == 0u) {
+                    if (__any_sync(FULL, wait(S::DONE + 8 * (half * S::DONE_SLOTS + p % S::DONE_SLOTS), p / S::DONE_SLOTS))) {
+                        goto epilogue_out;  // the block has given up: nothing more is read or written
+                    }
+                    tc_fence_after();
                 }
-                tc_fence_after();
-                const uint32_t taddr = acc_base + b * N;
+                const uint32_t taddr = acc_base + (b * S::PG + gi % S::PG) * N;
 #pragma unroll
                 for (uint32_t c = 0; c < N / 16u; ++c) {
                     uint32_t v[16];
@@ -856,17 +874,19 @@ __global__ void __launch_bounds__(Shape<N, FMT>::THREADS, 1) lmhead_kernel(const
                         fma2(acc[8u * c + m], s2, pack2(v[2u * m], v[2u * m + 1u]));
                     }
                 }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) {
-                    mbar_arrive(base + S::ACC_EMPTY + 8 * (half * S::ACC_BUFS + b));
+                if (gi % S::PG == S::PG - 1u) {
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) {
+                        mbar_arrive(base + S::ACC_EMPTY + 8 * (half * S::ACC_BUFS + b));
+                    }
                 }
                 if (AFFINE) {
                     const float bias = __uint_as_float((gi & 1u) ? (bw[gi >> 1] & 0xFFFF0000u) : (bw[gi >> 1] << 16));
                     const float add = __fmaf_rn(OFFSET, s, bias);
                     const uint64_t add2 = pack2(__float_as_uint(add), __float_as_uint(add));
                     const ulonglong2 *hs = reinterpret_cast<const ulonglong2 *>(
-                        base_ptr + S::SUMS + (q % SUM_SLOTS) * N * 4u);
+                        base_ptr + S::SUMS + (q % S::SUM_SLOTS) * N * 4u);
 #pragma unroll
                     for (uint32_t m = 0; m < P / 2u; ++m) {
                         const ulonglong2 h = hs[m];
