@@ -391,8 +391,8 @@ def main():
     kernel_ms = total_ms / args.steps  # average launch duration over the timed region (one launch per step)
     peak, peak_kind = peaks()
     achieved = alg_bytes / (kernel_ms * 1e-3) / 1e9
-    kernel_name = ("stream_rows_kernel<bf16> (one block per row)" if n_here * 8 > 148
-                   else "cluster_rows_kernel<bf16> (a cluster of eight blocks per row)")
+    kernel_name = ("stream_rows_kernel<bf16> (one block per row)" if n_here > 148
+                   else "split_rows_kernel<bf16> (a cluster of one to eight blocks per row)")
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "traffic": ncu_traffic() if world == 1 else None,
                 "peak_kind": peak_kind, "kernel": kernel_name, "kernel_ms": kernel_ms,
@@ -566,7 +566,7 @@ def lmhead_sharded(torch, dist, lily, dev, stream, world, rank, steps):
             "rows_per_s": tokens / (step_ms * 1e-3), "steps": steps,
             "head_kernel_us": head_ms * 1e3, "head_bytes_per_gpu": head_bytes,
             "head_gbs_per_gpu": gbs, "head_frac_of_hbm": gbs / peak, "peak_kind": peak_kind,
-            "head_traffic_1gpu": ncu_traffic("lmhead_int8_kernel_dram_bytes_per_launch"),
+            "head_traffic_1gpu": ncu_traffic("lmhead_kernel_dram_bytes_per_launch"),
             "affine_head_us": affine_ms * 1e3,
             "affine_head_frac_of_hbm": (head_bytes + per * (hidden // 64) * 2) / (affine_ms * 1e-3) / 1e9 / peak,
             "affine4_head_us": None if q4_ms is None else q4_ms * 1e3,

@@ -20,7 +20,6 @@ constexpr uint32_t SPL_HITS = 512;       // vectors of a block that may reach th
 constexpr uint32_t SPL_FLAGGED = 2048;   // buckets that may reach the bound
 constexpr uint32_t SPL_SORTED = 2048;    // candidates of a wide row
 constexpr uint32_t SPL_MIN_TILES = SPL_WARPS / 2u;  // pieces of a block, at least
-constexpr uint32_t SPL_COUNT_MAX = 32767;      // of an id in a history list (a mark's top bit says "on a list")
 constexpr uint32_t SPL_NAN_KEY = 0xFFFFFFFFu;  // a candidate that came out a NaN
 
 // How a block keeps the history ids of its share.

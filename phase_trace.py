@@ -23,13 +23,11 @@ NAMES = ["start", "bitmaps", "lists", "pass 2 / stream", "adjust + select", "mer
          "first threshold", "pass 1", "pass 1 met", "maxima", "search", "threshold set",
          "threshold taken", "collected", "entry"]
 ENTRY = 16
-# The small-batch kernel (a cluster of eight blocks per row) leaves its own stamps;
+# The row kernel (a cluster of up to eight blocks per row) leaves its own stamps;
 # block r of a row's cluster is listed as "slice" r.
-CLUSTER_NAMES = {0: "slice loaded, cluster running", 1: "history counted", 2: "lists, penalties, block maximum",
-                 3: "cluster maximum", 9: "histogram", 4: "cluster barrier", 5: "histograms summed, k-th bin",
-                 10: "candidates placed in every block", 6: "cluster barrier", 11: "ranked within bins",
-                 8: "cluster barrier", 7: "draw written"}
-CLUSTER_ORDER = [16, 0, 1, 2, 3, 9, 4, 5, 10, 6, 11, 8, 7]
+CLUSTER_NAMES = {9: "share read", 8: "bound known", 2: "vectors found", 4: "candidates sent", 5: "all there",
+                 6: "ranked", 7: "draw written"}
+CLUSTER_ORDER = [16, 9, 8, 2, 4, 5, 6, 7]
 # The order in which a block of the two-pass route reaches its stamps.
 ORDER = [16, 0, 1, 14, 15, 9, 10, 11, 12, 13, 8, 2, 3, 4, 5, 6, 7]
 
@@ -95,7 +93,7 @@ def main(argv) -> None:
                     if c[ENTRY] == 0:
                         continue
                     last = max(int(v) for v in c)
-                    # (The 4-row batch goes to the small-batch kernel: eight blocks per row.)
+                    # (The 4-row batch goes to the row kernel: eight blocks per row.)
                     cluster = clk.shape[0] <= 8 and c[13] == 0 and c[12] == 0
                     print(f"  row {r} block {sl}: enters {(c[ENTRY] - t0) / 1e3:5.1f}, leaves "
                           f"{(last - t0) / 1e3:5.1f} us after the launch's first block | " +
