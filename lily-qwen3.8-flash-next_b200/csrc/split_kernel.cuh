@@ -603,7 +603,8 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
     };
     // The row's first history ids go first. (Their number is not known yet; the row
     // has room for history_ld of them.)
-    constexpr uint32_t HU = 8u;
+    constexpr uint32_t HU = SPL_U < 8u ? SPL_U : 8u;  // (16-byte words of ids in flight a thread: they lie in q)
+    static_assert(HU <= SPL_U, "the history's words in flight");
     const uint32_t *hist = a.history_ids + (uint64_t)row * a.history_ld;
     const uint32_t lead = (4u - ((uint32_t)(reinterpret_cast<uintptr_t>(hist) >> 2) & 3u)) & 3u;  // ids before the first 16-byte boundary
     const uint4 *h4 = reinterpret_cast<const uint4 *>(hist + lead);
@@ -737,6 +738,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         const float scale = 1.4426950408889634f / in.temp;
         float ref = -1e30f, part[4] = {0.0f, 0.0f, 0.0f, 0.0f};
         constexpr uint32_t SU = 4u;
+        static_assert(SU <= SPL_U, "the vectors in flight");
         for (uint32_t j = warp - SPL_WARPS; j < pieces_here; j += SPL_WARPS * SU) {
             float m = neg_inf();
 #pragma unroll

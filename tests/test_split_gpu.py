@@ -60,3 +60,30 @@ def test_rows_around_the_waves_and_the_argument_blocks(cuda, lily, W, rows):
                         (False, 1, {}), (True, 30, dict(history=200, frequency=0.2))):
         b = make_batch(W, rng, rows, vocab, k, bf16, kind="zipf", **kw)
         check(cuda, lily, W, b, vocab, f"B={rows} bf16={bf16} k={k}")
+
+
+def long_lists(W, rng, rows, vocab, k, bf16, length, **kw):
+    """Rows of unequal lists up to `length` ids; the ids that a lost part of the list would change
+    (each row's best logits, some of them several times) stand in the list's last quarter."""
+    b = make_batch(W, rng, rows, vocab, k, bf16, kind="zipf", history=length, **kw)
+    b.history_len = rng.integers(length - length // 8, length + 1, rows).astype(np.uint32)
+    b.history_len[0] = length
+    lf = b.logits_f32()
+    for r in range(rows):
+        n = int(b.history_len[r])
+        best = np.argpartition(lf[r], vocab - 40)[vocab - 40:].astype(np.uint32)
+        at = n - n // 4 + rng.choice(n // 4, 60, replace=False)
+        b.history[r, at] = np.concatenate([best, best[:20]])
+    return b
+
+
+@pytest.mark.parametrize("rows,length,vocab,bf16", [
+    (149, 6143, 20_011, True), (149, 6144, 20_480, False), (149, 6145, 50_304, True), (200, 8192, 20_011, False),
+    (296, 8193, 20_011, True), (256, 20_000, 50_304, True), (160, 32_768, 20_011, False)])
+def test_long_lists_with_two_blocks_per_sm(cuda, lily, W, rows, length, vocab, bf16):
+    # More rows than SMs, not aligned (20011) or aligned but short: 6144 ids are what the
+    # block's marking half has in flight at a time.
+    rng = np.random.default_rng([rows, length, vocab])
+    for k, kw in ((30, dict(rep=1.3)), (50, dict(presence=0.7)), (20, dict(frequency=0.4, rep=1.1)), (1, dict(presence=1.5))):
+        b = long_lists(W, rng, rows, vocab, k, bf16, length, **kw)
+        check(cuda, lily, W, b, vocab, f"B={rows} V={vocab} n={length} {kw}", params_on_device=k == 50)
