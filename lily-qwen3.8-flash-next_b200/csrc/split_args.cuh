@@ -70,11 +70,18 @@ __host__ __device__ inline RowIn row_in(const lily_sampling_params_t &P, uint32_
     return r;
 }
 
+// The barriers at which the blocks of a row meet.
+enum {
+    MEET_POOL = 0,    // every block's keys have arrived
+    MEET_CANDIDATES,  // first block: every block's candidates have arrived
+    MEET_LISTS,       // wide rows: the sorted lists of all blocks have arrived
+    MEET_SUMS,        // first block: every block's sums of exponentials have arrived
+    MEET_GONE,        // wide rows: this block's list has arrived in every block
+    MEETS
+};
+
 struct alignas(16) SplitSmem {
-    unsigned long long mbar_pool;    // every block's keys have arrived
-    unsigned long long mbar_cand;    // first block: every block's candidates have arrived
-    unsigned long long mbar_list;    // wide rows: the sorted lists of all blocks have arrived
-    unsigned long long mbar_sums;    // first block: every block's sums of exponentials have arrived
+    unsigned long long mbar[MEETS];
     uint4 head[SPL_MAX_BLOCKS];      // first block: a block's number of candidates, flag, bound
     uint2 sums[SPL_MAX_BLOCKS * SPL_WARPS];  // first block, a shard's record: (reference, sum) of every warp
     union {

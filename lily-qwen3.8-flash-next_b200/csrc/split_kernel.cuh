@@ -70,6 +70,9 @@ __device__ __forceinline__ void put_4u32(uint32_t at, uint32_t x, uint32_t y, ui
                  "r"(x), "r"(y), "r"(z), "r"(w), "r"(bar)
                  : "memory");
 }
+__device__ __forceinline__ void arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
 __device__ __forceinline__ void arrive_expect(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.release.cluster.shared::cluster.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
                  : "memory");
@@ -239,6 +242,116 @@ static __device__ __noinline__ void split_finalize_wide(SmemFixed *sm, SplitSmem
             atomicOr(a.seen_table + (uint64_t)slot * a.seen_words + (id >> 5), 1u << (id & 31u));
         }
     }
+}
+
+// Every block sorts its list and sends it to all blocks; then each knows its
+// entries' ranks in the row (their places in the eight lists, by bisection) and
+// sends them to the first block, to where they belong. (Merged by the first block
+// alone, 1300 entries took 6 to 9 us: gathers from one SM's shared memory.)
+// All SPL_NT threads. The number of candidates, merged behind *ss in the first block; 0: there
+// is no such list (the first block draws the row alone), and in the other blocks.
+static __device__ __noinline__ uint32_t merge_lists(SmemFixed *sm, SplitSmem *ss, uint32_t log_blocks, uint32_t sent,
+                                                   uint32_t hard) {
+    constexpr unsigned FULL = 0xFFFFFFFFu;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, rank = blockIdx.x, blocks = 1u << log_blocks;
+    const uint32_t cap = CAP >> log_blocks, cand_bar = blocks > 1u ? peer_smem(&ss->mbar[MEET_CANDIDATES], 0) : 0u;
+    constexpr uint32_t OWN = SPL_MAX_BLOCKS * SPL_NT / 2u;
+    unsigned long long *own = reinterpret_cast<unsigned long long *>(ss->tmax);
+    unsigned long long *lists = reinterpret_cast<unsigned long long *>(sm->key);  // over key and id: CAP
+    unsigned long long *best_of = reinterpret_cast<unsigned long long *>(ss + 1);  // SPL_SORTED (the marks have served)
+    if (tid == 0 && sent < OWN) {
+        own[sent] = 0ull;  // (they are counted in pairs)
+    }
+    spl_sync();
+    const ulonglong2 *pairs = reinterpret_cast<const ulonglong2 *>(own);
+    for (uint32_t i = tid; i < sent; i += SPL_NT) {
+        const unsigned long long mine = own[i];
+        uint32_t place = 0;
+#pragma unroll 8
+        for (uint32_t j = 0; j < (sent + 1u) / 2u; ++j) {
+            const ulonglong2 o = pairs[j];
+            place += (o.x > mine ? 1u : 0u) + (o.y > mine ? 1u : 0u);
+        }
+        (blocks > 1u ? lists + rank * cap : best_of)[place] = mine;
+    }
+    uint32_t total = sent;
+    bool lost = hard != 0u;
+    if (blocks > 1u) {
+        // (One copy per block: stores of a thread each cost the SM some 4 clocks a piece.)
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        spl_sync();
+        if (tid < blocks) {
+            const uint32_t list_bar = peer_smem(&ss->mbar[MEET_LISTS], tid);
+            const uint32_t bytes = tid != rank ? (sent * 8u + 15u) & ~15u : 0u;
+            put_4u32(peer_smem(&ss->head[rank], tid), sent, hard, 0u, 0u, list_bar);
+            if (bytes != 0u) {
+                asm volatile(
+                    "cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                        peer_smem(lists + rank * cap, tid)),
+                    "r"((uint32_t)__cvta_generic_to_shared(lists + rank * cap)), "r"(bytes), "r"(list_bar)
+                    : "memory");
+            }
+            arrive_expect(list_bar, bytes + 16u);
+        }
+        lost = !wait_first_phase(&ss->mbar[MEET_LISTS]);
+        // A copy completes in its receiver, but its source is the sender's shared memory: no
+        // block leaves or draws alone in that memory before every receiver has said so.
+        if (tid < blocks && !lost) {
+            arrive(peer_smem(&ss->mbar[MEET_GONE], tid));
+        }
+        const uint4 head = lane < blocks ? ss->head[lane] : make_uint4(0, 0, 0, 0);
+        total = __reduce_add_sync(FULL, head.x);
+        lost = __any_sync(FULL, lost || head.y != 0u);
+    }
+    if (lost || total == 0u || total > SPL_SORTED) {  // (every block decides alike)
+        if (blocks > 1u) {
+            wait_first_phase(&ss->mbar[MEET_GONE]);
+        }
+        return 0u;
+    }
+    if (blocks > 1u) {
+        uint32_t n_of[SPL_MAX_BLOCKS], longest = 1;  // (its own list counts for nothing)
+#pragma unroll
+        for (uint32_t r = 0; r < SPL_MAX_BLOCKS; ++r) {
+            n_of[r] = r < blocks && r != rank ? ss->head[r].x : 0u;
+            longest = max(longest, n_of[r]);
+        }
+        for (uint32_t i = tid; i < sent; i += SPL_NT) {
+            const unsigned long long x = lists[rank * cap + i];
+            uint32_t low[SPL_MAX_BLOCKS], place = i;
+#pragma unroll
+            for (uint32_t r = 0; r < SPL_MAX_BLOCKS; ++r) {
+                low[r] = 0;
+            }
+            // (Steps of falling powers of two: low counts the entries known to be larger.
+            // Eight independent chains of loads, no branches: that is what makes it fast.)
+            for (uint32_t step = 1u << (31 - __clz(longest)); step != 0u; step >>= 1) {
+#pragma unroll
+                for (uint32_t r = 0; r < SPL_MAX_BLOCKS; ++r) {
+                    const uint32_t to = low[r] + step;
+                    const unsigned long long at = lists[(r * cap + min(to, cap) - 1u) & (CAP - 1u)];
+                    low[r] = (uint32_t)(to <= n_of[r]) & (uint32_t)(at > x) ? to : low[r];
+                }
+            }
+#pragma unroll
+            for (uint32_t r = 0; r < SPL_MAX_BLOCKS; ++r) {
+                place += low[r];
+            }
+            put_2u32(peer_smem(best_of + place, 0), (uint32_t)x, (uint32_t)(x >> 32), cand_bar);
+        }
+        if (tid == 0) {
+            arrive_expect(cand_bar, sent * 8u);
+        }
+        if (rank != 0u) {
+            wait_first_phase(&ss->mbar[MEET_GONE]);
+            return 0u;
+        }
+        if (!wait_first_phase(&ss->mbar[MEET_CANDIDATES]) || !wait_first_phase(&ss->mbar[MEET_GONE])) {
+            ss->hard = 2;
+        }
+    }
+    spl_sync();
+    return ss->hard != 0u ? 0u : total;
 }
 
 // What a speculative row needs of its proposal, asked for while the row is still
@@ -457,7 +570,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
     LILY_STAMP(PH_ENTRY);
 
     // What needs no input comes first (see sample_row on the launch attribute).
-    if (tid == 0) {
+    if (tid == 32u) {  // (two warps share the stores: they stand before the block's first barrier)
         ss->n_flagged = 0;
         ss->n_hits = 0;
         ss->n_listed = 0;
@@ -466,17 +579,13 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         ss->n_live = 0;
         ss->hard = 0;
         ss->bound_key = 0;
-        if (blocks > 1u) {
-            const uint32_t pool_bar = (uint32_t)__cvta_generic_to_shared(&ss->mbar_pool);
-            const uint32_t cand_bar = (uint32_t)__cvta_generic_to_shared(&ss->mbar_cand);
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(pool_bar) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(cand_bar), "r"(blocks) : "memory");
-            const uint32_t list_bar = (uint32_t)__cvta_generic_to_shared(&ss->mbar_list);
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(list_bar), "r"(blocks) : "memory");
-            const uint32_t sums_bar = (uint32_t)__cvta_generic_to_shared(&ss->mbar_sums);
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sums_bar) : "memory");
-            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        }
+    }
+    if (blocks > 1u && tid < MEETS) {
+        const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&ss->mbar[tid]);
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar),
+                     "r"(tid == MEET_POOL || tid == MEET_SUMS ? 1u : blocks)
+                     : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     for (uint32_t w = tid; w < ca.mark_words / 4u; w += NT) {
         reinterpret_cast<uint4 *>(marks)[w] = make_uint4(0, 0, 0, 0);
@@ -782,7 +891,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         if (blocks > 1u) {
             asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
             if (lane == 0) {
-                put_2u32(peer_smem(place, 0), __float_as_uint(top), __float_as_uint(sum), peer_smem(&ss->mbar_sums, 0));
+                put_2u32(peer_smem(place, 0), __float_as_uint(top), __float_as_uint(sum), peer_smem(&ss->mbar[MEET_SUMS], 0));
             }
         } else if (lane == 0) {
             *place = make_uint2(__float_as_uint(top), __float_as_uint(sum));
@@ -800,9 +909,9 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
             // (Collected before the verdict: the general code uses this memory for its own.)
             if (blocks > 1u) {
                 if (lane == 0) {
-                    arrive_expect(peer_smem(&ss->mbar_sums, 0), blocks * SPL_WARPS * 8u);
+                    arrive_expect(peer_smem(&ss->mbar[MEET_SUMS], 0), blocks * SPL_WARPS * 8u);
                 }
-                late = !__all_sync(FULL, wait_first_phase(&ss->mbar_sums));
+                late = !__all_sync(FULL, wait_first_phase(&ss->mbar[MEET_SUMS]));
             }
             constexpr uint32_t EACH = SPL_MAX_BLOCKS * SPL_WARPS / 32u;
             uint2 v[EACH];
@@ -1031,7 +1140,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         if (blocks > 1u) {
             asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
             if (lane == 0) {
-                put_2u32(peer_smem(&ss->pool[2u * (rank * SPL_WARPS + warp)], 0), m, mi, peer_smem(&ss->mbar_pool, 0));
+                put_2u32(peer_smem(&ss->pool[2u * (rank * SPL_WARPS + warp)], 0), m, mi, peer_smem(&ss->mbar[MEET_POOL], 0));
             }
         } else {
             if (lane == 0) {
@@ -1045,9 +1154,9 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         bool ok = true;
         if (blocks > 1u) {
             if (tid == 0) {
-                arrive_expect(peer_smem(&ss->mbar_pool, 0), blocks * SPL_WARPS * 8u);
+                arrive_expect(peer_smem(&ss->mbar[MEET_POOL], 0), blocks * SPL_WARPS * 8u);
             }
-            ok = warp != 0u || wait_first_phase(&ss->mbar_pool);
+            ok = warp != 0u || wait_first_phase(&ss->mbar[MEET_POOL]);
         } else {
             spl_sync();
         }
@@ -1180,7 +1289,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
             const uint32_t to = (rank * SPL_WARPS + warp) * rounds + r, placed = (m & ~255u) | to;
             if (blocks > 1u) {
                 if (lane < blocks) {
-                    put_u32(peer_smem(&ss->pool[to], lane), placed, peer_smem(&ss->mbar_pool, lane));
+                    put_u32(peer_smem(&ss->pool[to], lane), placed, peer_smem(&ss->mbar[MEET_POOL], lane));
                 }
             } else if (lane == 0) {
                 ss->pool[to] = placed;
@@ -1188,9 +1297,9 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         }
         if (blocks > 1u) {
             if (tid == 0) {
-                arrive_expect(peer_smem(&ss->mbar_pool, rank), n * 4u);
+                arrive_expect(peer_smem(&ss->mbar[MEET_POOL], rank), n * 4u);
             }
-            if (!wait_first_phase(&ss->mbar_pool)) {
+            if (!wait_first_phase(&ss->mbar[MEET_POOL])) {
                 ss->hard = 1;
             }
         } else {
@@ -1232,10 +1341,10 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         // The maxima of the whole cluster, 32 bins per unit under the largest.
         if (blocks > 1u) {
             if (tid == 0) {
-                arrive_expect(peer_smem(&ss->mbar_pool, rank), blocks * SPL_NT * 4u);
+                arrive_expect(peer_smem(&ss->mbar[MEET_POOL], rank), blocks * SPL_NT * 4u);
             }
             for (uint32_t r = 0; r < blocks; ++r) {
-                put_u32(peer_smem(&ss->tmax[rank * SPL_NT + tid], r), key, peer_smem(&ss->mbar_pool, r));
+                put_u32(peer_smem(&ss->tmax[rank * SPL_NT + tid], r), key, peer_smem(&ss->mbar[MEET_POOL], r));
             }
         } else {
             ss->tmax[tid] = key;
@@ -1246,7 +1355,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         if (tid == 0) {
             ss->bin = NONE;
         }
-        if (blocks > 1u && !wait_first_phase(&ss->mbar_pool)) {
+        if (blocks > 1u && !wait_first_phase(&ss->mbar[MEET_POOL])) {
             ss->hard = 1;
         }
         spl_sync();
@@ -1394,7 +1503,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
     const uint32_t cap = CAP >> log_blocks;
     const uint32_t n_hits = ss->n_hits;
     uint2 *cand = reinterpret_cast<uint2 *>(sm->key);  // over key and id: CAP of them, a region per block
-    const uint32_t bar = blocks > 1u ? peer_smem(&ss->mbar_cand, 0) : 0u;
+    const uint32_t bar = blocks > 1u ? peer_smem(&ss->mbar[MEET_CANDIDATES], 0) : 0u;
     const uint32_t cand_at = blocks > 1u ? peer_smem(cand + rank * cap, 0) : 0u;
     // (Wide rows: first here, over the pool, which has served.)
     constexpr uint32_t OWN = SPL_MAX_BLOCKS * SPL_NT / 2u;
@@ -1481,107 +1590,19 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
     const uint32_t hard = (ss->hard != 0u || n_hits > SPL_HITS || ss->n_sent > most || n_slots > TH_BINS) ? 1u : 0u;
     const bool counts_draw = use_pen && table_mode;
     if (wide) {
-        // Every block sorts its list and sends it to all blocks; then each knows its
-        // entries' ranks in the row (their places in the eight lists, by bisection) and
-        // sends them to the first block, to where they belong. (Merged by the first block
-        // alone, 1300 entries took 6 to 9 us: gathers from one SM's shared memory.)
-        unsigned long long *lists = reinterpret_cast<unsigned long long *>(sm->key);  // over key and id: CAP
-        unsigned long long *best_of = reinterpret_cast<unsigned long long *>(ss + 1);  // SPL_SORTED (the marks have served)
-        if (tid == 0 && sent < OWN) {
-            own[sent] = 0ull;  // (they are counted in pairs)
-        }
-        spl_sync();
-        const ulonglong2 *pairs = reinterpret_cast<const ulonglong2 *>(own);
-        for (uint32_t i = tid; i < sent; i += SPL_NT) {
-            const unsigned long long mine = own[i];
-            uint32_t place = 0;
-#pragma unroll 8
-            for (uint32_t j = 0; j < (sent + 1u) / 2u; ++j) {
-                const ulonglong2 o = pairs[j];
-                place += (o.x > mine ? 1u : 0u) + (o.y > mine ? 1u : 0u);
-            }
-            (blocks > 1u ? lists + rank * cap : best_of)[place] = mine;
-        }
-        uint32_t total = sent;
-        bool lost = hard != 0u;
-        if (blocks > 1u) {
-            // (One copy per block: stores of a thread each cost the SM some 4 clocks a piece.)
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            spl_sync();
-            if (tid < blocks) {
-                const uint32_t list_bar = peer_smem(&ss->mbar_list, tid);
-                const uint32_t bytes = tid != rank ? (sent * 8u + 15u) & ~15u : 0u;
-                put_4u32(peer_smem(&ss->head[rank], tid), sent, hard, 0u, 0u, list_bar);
-                if (bytes != 0u) {
-                    asm volatile(
-                        "cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                            peer_smem(lists + rank * cap, tid)),
-                        "r"((uint32_t)__cvta_generic_to_shared(lists + rank * cap)), "r"(bytes), "r"(list_bar)
-                        : "memory");
-                }
-                arrive_expect(list_bar, bytes + 16u);
-            }
-            lost = !wait_first_phase(&ss->mbar_list);
-            const uint4 head = lane < blocks ? ss->head[lane] : make_uint4(0, 0, 0, 0);
-            total = __reduce_add_sync(FULL, head.x);
-            lost = __any_sync(FULL, lost || head.y != 0u);
-        }
         LILY_STAMP(PH_LOCAL_SELECT);
-        if (lost || total == 0u || total > SPL_SORTED) {  // (every block decides alike)
-            if (rank == 0u) {
-                verdict(0u, ALONE);
-            }
+        const uint32_t total = merge_lists(sm, ss, log_blocks, sent, hard);
+        if (rank != 0u) {
             return;
         }
-        if (blocks > 1u) {
-            uint32_t n_of[SPL_MAX_BLOCKS], longest = 1;  // (its own list counts for nothing)
-#pragma unroll
-            for (uint32_t r = 0; r < SPL_MAX_BLOCKS; ++r) {
-                n_of[r] = r < blocks && r != rank ? ss->head[r].x : 0u;
-                longest = max(longest, n_of[r]);
-            }
-            for (uint32_t i = tid; i < sent; i += SPL_NT) {
-                const unsigned long long x = lists[rank * cap + i];
-                uint32_t low[SPL_MAX_BLOCKS], place = i;
-#pragma unroll
-                for (uint32_t r = 0; r < SPL_MAX_BLOCKS; ++r) {
-                    low[r] = 0;
-                }
-                // (Steps of falling powers of two: low counts the entries known to be larger.
-                // Eight independent chains of loads, no branches: that is what makes it fast.)
-                for (uint32_t step = 1u << (31 - __clz(longest)); step != 0u; step >>= 1) {
-#pragma unroll
-                    for (uint32_t r = 0; r < SPL_MAX_BLOCKS; ++r) {
-                        const uint32_t to = low[r] + step;
-                        const unsigned long long at = lists[(r * cap + min(to, cap) - 1u) & (CAP - 1u)];
-                        low[r] = (uint32_t)(to <= n_of[r]) & (uint32_t)(at > x) ? to : low[r];
-                    }
-                }
-#pragma unroll
-                for (uint32_t r = 0; r < SPL_MAX_BLOCKS; ++r) {
-                    place += low[r];
-                }
-                put_2u32(peer_smem(best_of + place, 0), (uint32_t)x, (uint32_t)(x >> 32), bar);
-            }
-            if (tid == 0) {
-                arrive_expect(bar, sent * 8u);
-            }
-            if (rank != 0u) {
-                return;
-            }
-            LILY_STAMP(PH_MERGE);
-            if (!wait_first_phase(&ss->mbar_cand)) {
-                ss->hard = 2;
-            }
-        }
-        spl_sync();
-        if (ss->hard != 0u) {
+        LILY_STAMP(PH_MERGE);
+        if (total == 0u) {
             verdict(0u, ALONE);
             return;
         }
         verdict(0u, DONE);
         LILY_STAMP(PH_SORT);
-        split_finalize_wide(sm, ss, best_of, a, row, min(total, k), in.top_p, in.min_p,
+        split_finalize_wide(sm, ss, reinterpret_cast<const unsigned long long *>(ss + 1), a, row, min(total, k), in.top_p, in.min_p,
                             a.uniforms ? __ldg(a.uniforms + row) : in.u, counts_draw, slot);
         LILY_STAMP(PH_END);
         return;
@@ -1617,7 +1638,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
             return;
         }
     } else {
-        const bool late = blocks > 1u && !wait_first_phase(&ss->mbar_cand);
+        const bool late = blocks > 1u && !wait_first_phase(&ss->mbar[MEET_CANDIDATES]);
         LILY_STAMP(PH_MERGE);
         const uint4 head = lane < blocks ? ss->head[lane] : make_uint4(0, 0, 0, 0);
         const uint32_t n = __reduce_add_sync(FULL, head.x);
@@ -1674,7 +1695,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         }
         verdict(0u, HANDS);
     }
-    if (blocks > 1u && !wait_first_phase(&ss->mbar_cand)) {
+    if (blocks > 1u && !wait_first_phase(&ss->mbar[MEET_CANDIDATES])) {
         ss->hard = 2;
     }
     LILY_STAMP(PH_MERGE);

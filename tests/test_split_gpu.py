@@ -5,6 +5,7 @@ and every way of keeping the history. Ids and kept sets are exact, as everywhere
 import numpy as np
 import pytest
 
+from gpu_util import assert_parity, make_params, np_u32, oracle_rows, run_batch, t_f32, t_logits
 from test_sampler_gpu import check, make_batch
 
 pytestmark = pytest.mark.gpu
@@ -87,3 +88,31 @@ def test_long_lists_with_two_blocks_per_sm(cuda, lily, W, rows, length, vocab, b
     for k, kw in ((30, dict(rep=1.3)), (50, dict(presence=0.7)), (20, dict(frequency=0.4, rep=1.1)), (1, dict(presence=1.5))):
         b = long_lists(W, rng, rows, vocab, k, bf16, length, **kw)
         check(cuda, lily, W, b, vocab, f"B={rows} V={vocab} n={length} {kw}", params_on_device=k == 50)
+
+
+@pytest.mark.parametrize("vocab,bf16,owner", [(65_536, False, 0), (65_536, True, 3), (40_009, False, 7)])
+def test_wide_rows_whose_candidates_are_one_blocks(cuda, lily, W, vocab, bf16, owner):
+    # The blocks of a cluster send each other their sorted lists. Here one block has (nearly)
+    # all candidates: the others have nothing to rank and are the first to be done, while
+    # theirs and its lists are still on their way. Launch after launch, so that the next
+    # one's blocks take their places.
+    rng = np.random.default_rng([7, vocab, owner])
+    rows, piece = 6, 256 if bf16 else 128
+    x = rng.uniform(-8, -7, (rows, vocab)).astype(np.float32)
+    mine = (np.arange(vocab) // piece) % 8 == owner
+    x[:, mine] = rng.uniform(0, 8, (rows, int(mine.sum())))
+    params = [dict(temperature=1.2, top_k=[0, 300, 1000][r % 3], top_p=0.98, min_p=0.0, seed=r) for r in range(rows)]
+    b = W.Batch(W.to_bf16_bits(x) if bf16 else x, bf16, params, rng.random(rows, dtype=np.float32))
+    want = oracle_rows(b)
+    s = lily.SamplerScratch(vocab, max_rows=rows)
+    logits, out = t_logits(cuda, b), cuda.zeros((40, rows), dtype=cuda.int32, device="cuda")
+    prepared = [s.prepare_sample_batch(logits, make_params(lily, b), out[i], uniforms=t_f32(cuda, b.uniforms))
+                for i in range(len(out))]
+    for p in prepared:
+        s.sample_prepared(p)
+    cuda.cuda.synchronize()
+    assert s.status() == lily.OK
+    got = np_u32(out)
+    assert all(list(row) == [d.token for d in want] for row in got)
+    assert_parity(b, run_batch(cuda, lily, s, b), want, label=f"V={vocab} owner {owner}")
+    s.close()
