@@ -147,22 +147,28 @@ int32_t lily_sampler_status(lily_sampler_t *h, void *stream);
 /*
  * src/metal.rs:856-861 wait_fence and :1276-1279 Fence::wait_until(value,
  * timeout_ms): the reference bounds its waits on the GPU on the host side. Here
- * the only waits are inside the LM-head kernel (one role of a block waiting for
- * another's copies, conversions or multiplies), and each is bounded on the
- * device: after `nanoseconds` (default and 0: one second) the block gives up,
- * lets the copies and multiplies it still has in flight land, frees its tensor
- * memory and returns. The launch completes like any other; the logits it was to
- * write are not valid, and the next lily_sampler_status returns
- * LILY_ERR_TIMEOUT (once: the status is cleared by reading it). The handle stays
- * usable. The sampler's own kernels wait on nothing another block produces.
+ * the waits are inside the LM-head kernel (one role of a block waiting for
+ * another's copies, conversions or multiplies, a block for the sums of the one
+ * before it), inside the row kernel (a row's blocks waiting for one another) and
+ * in lily_merge_draw_peer, and each is bounded on the device: after `nanoseconds`
+ * (default and 0: one second) the block gives up, lets what it still has in flight
+ * (copies, multiplies, the other blocks' stores) land, frees its tensor memory and
+ * returns. The launch completes like any other; the logits it was to write are not
+ * valid, a row it was to draw gets id 0xFFFFFFFF, and the next lily_sampler_status
+ * returns LILY_ERR_TIMEOUT (once: the status is cleared by reading it). The handle
+ * stays usable.
  *
  * inject_lost_copy is the device-side sibling of inject_fault, for tests: the
  * next LM-head launch on this handle (and only that one) leaves out the copy of
  * weight stage `stage` of its first block, so that the wait of the stage's
- * consumers runs out. No reference counterpart.
+ * consumers runs out. inject_lost_arrival likewise for the next draw: in each of its
+ * clusters, block `block` waits for one arrival too many at one of its barriers (1 the
+ * pool of keys, 2 the candidates, 3 the lists of a row that keeps many, 4 a shard's sums,
+ * 5 the sent lists' receipt). No reference counterpart.
  */
 int32_t lily_sampler_set_wait_limit(lily_sampler_t *h, uint64_t nanoseconds);
 void lily_sampler_inject_lost_copy(lily_sampler_t *h, uint32_t stage);
+void lily_sampler_inject_lost_arrival(lily_sampler_t *h, uint32_t barrier, uint32_t block);
 
 /*
  * src/kernels/sample.rs:145-174 reset_counts / uncount / copy_counts_from on

@@ -174,6 +174,8 @@ def lib():
         L.lily_sampler_set_wait_limit.restype = C.c_int32
         L.lily_sampler_inject_lost_copy.argtypes = [C.c_void_p, C.c_uint32]
         L.lily_sampler_inject_lost_copy.restype = None
+        L.lily_sampler_inject_lost_arrival.argtypes = [C.c_void_p, C.c_uint32, C.c_uint32]
+        L.lily_sampler_inject_lost_arrival.restype = None
         L.lily_sampler_clear_fault.argtypes = [C.c_void_p]
         L.lily_sampler_clear_fault.restype = None
         L.lily_sampler_status.argtypes = [C.c_void_p, C.c_void_p]
@@ -361,13 +363,17 @@ class SamplerScratch:
     def status(self, stream=None) -> int:
         return int(lib().lily_sampler_status(self._h, _stream_ptr(stream)))
 
-    # -- bounded waits of the LM-head kernel (src/metal.rs:856-861, 1276-1279)
+    # -- bounded waits of the kernels (src/metal.rs:856-861, 1276-1279)
     def set_wait_limit(self, nanoseconds: int):
         self._check(lib().lily_sampler_set_wait_limit(self._h, nanoseconds))
 
     def inject_lost_copy(self, stage: int):
         """Test hook: the next LM-head launch leaves out one weight copy of its first block."""
         lib().lily_sampler_inject_lost_copy(self._h, stage)
+
+    def inject_lost_arrival(self, barrier: int, block: int):
+        """Test hook: a wait of block `block` of the next draw's clusters runs out."""
+        lib().lily_sampler_inject_lost_arrival(self._h, barrier, block)
 
     # -- histogram slots (src/kernels/sample.rs:145-174)
     def reset_counts(self, slot: int = 0, stream=None):

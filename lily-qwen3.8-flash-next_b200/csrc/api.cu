@@ -50,7 +50,8 @@ struct lily_sampler {
     uint32_t vocab = 0, max_rows = 0, max_history = 0, max_list = 0, flags = 0;
     std::string last_error;
     int32_t fault = 0;
-    uint64_t wait_ns = 1000000000ull;     // bound of the waits inside the LM-head kernel
+    uint64_t wait_ns = 1000000000ull;     // bound of the waits inside the kernels
+    uint32_t lost_arrival = 0;            // test hook: what SplitArgs::lost of the next row-kernel launch is
     uint32_t lost_stage = 0xFFFFFFFFu;    // test hook: a weight copy the next head launch leaves out
     int sm_count = 0;
     int max_smem = 0;
@@ -387,6 +388,9 @@ int32_t launch_split(lily_sampler *h, cudaStream_t stream, lily::SplitArgs<MAXR>
     sa.two_per_sm = p.sole ? 0u : 1u;
     sa.mark_mode = p.mark_mode;
     sa.mark_words = p.mark_words;
+    sa.wait_ns = h->wait_ns;
+    sa.lost = h->lost_arrival;
+    h->lost_arrival = 0;  // one launch only
     sa.spill_params = reinterpret_cast<lily_sampling_params_t *>(h->spill);
     sa.spill_steps = reinterpret_cast<uint32_t *>(h->spill + INLINE_ROWS_MAX * sizeof(lily_sampling_params_t));
     sa.spill_slots = sa.spill_steps + INLINE_ROWS_MAX;
@@ -704,6 +708,12 @@ void lily_sampler_inject_lost_copy(lily_sampler_t *h, uint32_t stage) {
     }
 }
 
+void lily_sampler_inject_lost_arrival(lily_sampler_t *h, uint32_t barrier, uint32_t block) {
+    if (h) {
+        h->lost_arrival = barrier ? (block << 8) | (barrier & 255u) : 0u;
+    }
+}
+
 int32_t lily_sampler_status(lily_sampler_t *h, void *stream_) {
     if (h == nullptr) {
         return LILY_ERR_ARG;
@@ -718,7 +728,7 @@ int32_t lily_sampler_status(lily_sampler_t *h, void *stream_) {
     CU(h, cudaStreamSynchronize(stream));
     if (*h->h_status & (1u << lily_head::STATUS_TIMEOUT_BIT)) {
         return fail(h, LILY_ERR_TIMEOUT,
-                    "a bounded wait ran out (inside the LM-head kernel, or for a peer's records): the results are not valid");
+                    "a bounded wait ran out (inside a kernel, or for a peer's records): the results are not valid");
     }
     if (*h->h_status != 0u) {
         char buf[96];

@@ -62,6 +62,7 @@ struct Geo {
 
 // Row status bits OR-ed into the handle's status word.
 constexpr uint32_t ROW_INTERNAL = 8;  // candidate buffer overflow: a bug, never expected
+constexpr uint32_t STATUS_TIMEOUT_BIT = 30;  // not a row's: a bounded wait ran out
 
 // What one vocabulary shard tells the others about a row: its best candidates
 // in order (monotone key of the adjusted logit, vocabulary id; unused entries
@@ -2920,7 +2921,7 @@ __device__ __forceinline__ void peer_exchange_row(const KArgs &a, uint32_t row) 
             }
         }
         if (__any_sync(0xFFFFFFFFu, late) && tid == 0) {
-            atomicOr(a.status_word, 1u << 30);
+            atomicOr(a.status_word, 1u << STATUS_TIMEOUT_BIT);
         }
     }
     __syncthreads();

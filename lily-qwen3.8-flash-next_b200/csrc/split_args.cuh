@@ -101,6 +101,7 @@ struct alignas(16) SplitSmem {
     uint32_t bound_key;
     uint32_t record_key;             // a shard's largest adjusted logit
     uint32_t n_slots;                // candidates whose ids are counted in the history
+    uint32_t late;                   // a wait of this block ran out: others may still store into it
 };
 static_assert(sizeof(SplitSmem) % 16u == 0u, "the arrays behind it are 16-byte aligned");
 
@@ -116,6 +117,10 @@ struct SplitArgs {
     uint32_t inline_params;   // `in` below is valid (else a.params / a.steps)
     uint32_t inline_slots;
     uint32_t inline_history;  // 1 + the history length of every row (0: a.history_len)
+    // Test hook: block lost >> 8 of every cluster waits for one arrival too many at its
+    // barrier (lost & 255) - 1, so that the wait runs out (0: none).
+    uint32_t lost;
+    uint64_t wait_ns;         // the bound of every wait of a block for the others
     // Device words of the handle: where the first block puts what travelled here
     // when it hands a row to the general code.
     lily_sampling_params_t *spill_params;

@@ -78,11 +78,14 @@ __device__ __forceinline__ void arrive_expect(uint32_t bar, uint32_t bytes) {
                  : "memory");
 }
 
-// Waits for the first phase of a barrier in this block, some milliseconds at most
-// (the other blocks of the cluster are running: they only have to get there).
-__device__ __forceinline__ bool wait_first_phase(const unsigned long long *bar) {
+// Waits for the first phase of a barrier in this block, for at most `limit_ns`; true
+// if it is complete. (The other blocks of the cluster are running and only have to get
+// there: the limit is met only where something is wrong. The clock is looked at after
+// 16 polls.)
+__device__ __forceinline__ bool wait_first_phase(const unsigned long long *bar, uint64_t limit_ns) {
     const uint32_t at = (uint32_t)__cvta_generic_to_shared(bar);
-    for (uint32_t i = 0; i < (1u << 18); ++i) {
+    uint64_t t0 = 0;
+    for (uint32_t i = 0;; ++i) {
         uint32_t done;
         asm volatile(
             "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n"
@@ -93,8 +96,38 @@ __device__ __forceinline__ bool wait_first_phase(const unsigned long long *bar) 
         if (done) {
             return true;
         }
+        if ((i & 15u) == 15u) {
+            const uint64_t now = (uint64_t)global_ns();
+            if (t0 == 0u) {
+                t0 = now;
+            } else if (now - t0 > limit_ns) {
+                return false;
+            }
+        }
     }
-    return false;
+}
+
+// All threads of the cluster that have not returned yet meet here, for a thread that has
+// met the others at most once before (`met`: at the start). A block whose wait ran out goes
+// through it before it returns or uses its shared memory for anything else: the others'
+// waits are bounded too, so each of them comes here or returns, and until then it may
+// store into this block.
+__device__ __forceinline__ void meet_cluster(bool met) {
+    if (!met) {
+        asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    }
+    asm volatile("barrier.cluster.arrive.release;\n barrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// Every thread of the block's working half learns whether one of them says so.
+__device__ __forceinline__ bool spl_any(bool mine) {
+    uint32_t any;
+    asm volatile(
+        "{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n barrier.cta.red.or.pred q, 1, %2, p;\n selp.u32 %0, 1, 0, q;\n}"
+        : "=r"(any)
+        : "r"(mine ? 1u : 0u), "n"(SPL_NT)
+        : "memory");
+    return any != 0u;
 }
 
 // The largest of a vector's logits; NaN if one is.
@@ -251,7 +284,7 @@ static __device__ __noinline__ void split_finalize_wide(SmemFixed *sm, SplitSmem
 // All SPL_NT threads. The number of candidates, merged behind *ss in the first block; 0: there
 // is no such list (the first block draws the row alone), and in the other blocks.
 static __device__ __noinline__ uint32_t merge_lists(SmemFixed *sm, SplitSmem *ss, uint32_t log_blocks, uint32_t sent,
-                                                   uint32_t hard) {
+                                                   uint32_t hard, uint64_t wait_ns) {
     constexpr unsigned FULL = 0xFFFFFFFFu;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, rank = blockIdx.x, blocks = 1u << log_blocks;
     const uint32_t cap = CAP >> log_blocks, cand_bar = blocks > 1u ? peer_smem(&ss->mbar[MEET_CANDIDATES], 0) : 0u;
@@ -293,7 +326,10 @@ static __device__ __noinline__ uint32_t merge_lists(SmemFixed *sm, SplitSmem *ss
             }
             arrive_expect(list_bar, bytes + 16u);
         }
-        lost = !wait_first_phase(&ss->mbar[MEET_LISTS]);
+        lost = spl_any(!wait_first_phase(&ss->mbar[MEET_LISTS], wait_ns));
+        if (lost) {
+            ss->late = 1;
+        }
         // A copy completes in its receiver, but its source is the sender's shared memory: no
         // block leaves or draws alone in that memory before every receiver has said so.
         if (tid < blocks && !lost) {
@@ -304,8 +340,8 @@ static __device__ __noinline__ uint32_t merge_lists(SmemFixed *sm, SplitSmem *ss
         lost = __any_sync(FULL, lost || head.y != 0u);
     }
     if (lost || total == 0u || total > SPL_SORTED) {  // (every block decides alike)
-        if (blocks > 1u) {
-            wait_first_phase(&ss->mbar[MEET_GONE]);
+        if (blocks > 1u && !wait_first_phase(&ss->mbar[MEET_GONE], wait_ns)) {
+            ss->late = 1;
         }
         return 0u;
     }
@@ -343,11 +379,14 @@ static __device__ __noinline__ uint32_t merge_lists(SmemFixed *sm, SplitSmem *ss
             arrive_expect(cand_bar, sent * 8u);
         }
         if (rank != 0u) {
-            wait_first_phase(&ss->mbar[MEET_GONE]);
+            if (!wait_first_phase(&ss->mbar[MEET_GONE], wait_ns)) {
+                ss->late = 1;
+            }
             return 0u;
         }
-        if (!wait_first_phase(&ss->mbar[MEET_CANDIDATES]) || !wait_first_phase(&ss->mbar[MEET_GONE])) {
+        if (!wait_first_phase(&ss->mbar[MEET_CANDIDATES], wait_ns) || !wait_first_phase(&ss->mbar[MEET_GONE], wait_ns)) {
             ss->hard = 2;
+            ss->late = 1;
         }
     }
     spl_sync();
@@ -579,11 +618,12 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         ss->n_live = 0;
         ss->hard = 0;
         ss->bound_key = 0;
+        ss->late = 0;
     }
     if (blocks > 1u && tid < MEETS) {
         const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&ss->mbar[tid]);
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar),
-                     "r"(tid == MEET_POOL || tid == MEET_SUMS ? 1u : blocks)
+                     "r"((tid == MEET_POOL || tid == MEET_SUMS ? 1u : blocks) + (ca.lost == (rank << 8 | (tid + 1u)) ? 1u : 0u))
                      : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -600,8 +640,35 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
 
     const T *row_ptr = reinterpret_cast<const T *>(a.logits) + (uint64_t)row * a.logits_ld;
     const uint32_t skip = (uint32_t)(reinterpret_cast<uintptr_t>(row_ptr) & 15u) / (uint32_t)sizeof(T);
+    // The row's wait ran out (all NT threads of the first block): the row has no result, and the
+    // status word says so.
+    auto give_up = [&]() {
+        if (tid == 0) {
+            if (a.cand_out) {
+                a.cand_out[row].max_adj = neg_inf();
+                a.cand_out[row].sum_exp = 0.0f;
+            } else {
+                a.out_ids[row] = 0xFFFFFFFFu;
+                if (a.out_status) {
+                    a.out_status[row] = ROW_INTERNAL;
+                }
+                if (a.kept_n) {
+                    a.kept_n[row] = 0;
+                }
+            }
+            atomicOr(a.status_word, 1u << STATUS_TIMEOUT_BIT);
+        }
+        if (a.cand_out && tid < LILY_SHARD_CANDIDATES) {
+            a.cand_out[row].cand[tid] = make_uint2(0u, 0xFFFFFFFFu);
+        }
+        meet_cluster(tid < SPL_NT || a.shard_sums != 0u);
+    };
     // The first block draws the row alone with the general row code, all NT threads.
     auto draw_alone = [&]() {
+        if (ss->late != 0u) {
+            give_up();
+            return;
+        }
         KArgs whole = a;
         whole.n_slices = 1;
         if (ca.inline_params) {
@@ -646,6 +713,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
             __syncthreads();
             if (tid == SPL_NT) {
                 ss->record_key = key_of(__ldcg(&a.cand_out[row].max_adj));
+                ss->late = 0;  // (the general code's memory, meanwhile)
             }
             __syncthreads();
         }
@@ -911,7 +979,10 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
                 if (lane == 0) {
                     arrive_expect(peer_smem(&ss->mbar[MEET_SUMS], 0), blocks * SPL_WARPS * 8u);
                 }
-                late = !__all_sync(FULL, wait_first_phase(&ss->mbar[MEET_SUMS]));
+                late = !__all_sync(FULL, wait_first_phase(&ss->mbar[MEET_SUMS], ca.wait_ns));
+                if (late) {
+                    ss->late = 1;  // (before the verdict)
+                }
             }
             constexpr uint32_t EACH = SPL_MAX_BLOCKS * SPL_WARPS / 32u;
             uint2 v[EACH];
@@ -938,9 +1009,13 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         if (tid == SPL_NT) {  // (the record's largest logit is there: written before the verdict)
             total *= exp2f(top - float_of_key(ss->record_key) * 1.4426950408889634f);
             a.cand_out[row].sum_exp = total == total ? total : 0.0f;
-            if (late) {
-                atomicOr(a.status_word, 1u << ROW_INTERNAL);
+            if (ss->late != 0u) {
+                a.cand_out[row].sum_exp = 0.0f;
+                atomicOr(a.status_word, 1u << STATUS_TIMEOUT_BIT);
             }
+        }
+        if (late) {
+            meet_cluster(true);
         }
         return;
     }
@@ -1156,7 +1231,10 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
             if (tid == 0) {
                 arrive_expect(peer_smem(&ss->mbar[MEET_POOL], 0), blocks * SPL_WARPS * 8u);
             }
-            ok = warp != 0u || wait_first_phase(&ss->mbar[MEET_POOL]);
+            ok = warp != 0u || wait_first_phase(&ss->mbar[MEET_POOL], ca.wait_ns);
+            if (!ok) {
+                ss->late = 1;
+            }
         } else {
             spl_sync();
         }
@@ -1299,8 +1377,8 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
             if (tid == 0) {
                 arrive_expect(peer_smem(&ss->mbar[MEET_POOL], rank), n * 4u);
             }
-            if (!wait_first_phase(&ss->mbar[MEET_POOL])) {
-                ss->hard = 1;
+            if (!wait_first_phase(&ss->mbar[MEET_POOL], ca.wait_ns)) {
+                ss->hard = ss->late = 1;
             }
         } else {
             spl_sync();
@@ -1355,8 +1433,8 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         if (tid == 0) {
             ss->bin = NONE;
         }
-        if (blocks > 1u && !wait_first_phase(&ss->mbar[MEET_POOL])) {
-            ss->hard = 1;
+        if (blocks > 1u && !wait_first_phase(&ss->mbar[MEET_POOL], ca.wait_ns)) {
+            ss->hard = ss->late = 1;
         }
         spl_sync();
         uint32_t keys[SPL_MAX_BLOCKS], m = 0;
@@ -1591,8 +1669,11 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
     const bool counts_draw = use_pen && table_mode;
     if (wide) {
         LILY_STAMP(PH_LOCAL_SELECT);
-        const uint32_t total = merge_lists(sm, ss, log_blocks, sent, hard);
+        const uint32_t total = merge_lists(sm, ss, log_blocks, sent, hard, ca.wait_ns);
         if (rank != 0u) {
+            if (ss->late != 0u) {
+                meet_cluster(true);
+            }
             return;
         }
         LILY_STAMP(PH_MERGE);
@@ -1617,6 +1698,9 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
     }
     LILY_STAMP(PH_LOCAL_SELECT);
     if (rank != 0u) {
+        if (ss->late != 0u) {
+            meet_cluster(true);
+        }
         return;
     }
 
@@ -1638,7 +1722,10 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
             return;
         }
     } else {
-        const bool late = blocks > 1u && !wait_first_phase(&ss->mbar[MEET_CANDIDATES]);
+        const bool late = blocks > 1u && !wait_first_phase(&ss->mbar[MEET_CANDIDATES], ca.wait_ns);
+        if (late) {
+            ss->late = 1;
+        }
         LILY_STAMP(PH_MERGE);
         const uint4 head = lane < blocks ? ss->head[lane] : make_uint4(0, 0, 0, 0);
         const uint32_t n = __reduce_add_sync(FULL, head.x);
@@ -1695,8 +1782,9 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         }
         verdict(0u, HANDS);
     }
-    if (blocks > 1u && !wait_first_phase(&ss->mbar[MEET_CANDIDATES])) {
+    if (blocks > 1u && !wait_first_phase(&ss->mbar[MEET_CANDIDATES], ca.wait_ns)) {
         ss->hard = 2;
+        ss->late = 1;
     }
     LILY_STAMP(PH_MERGE);
     const uint4 head = lane < blocks ? ss->head[lane] : make_uint4(0, 0, 0, 0);

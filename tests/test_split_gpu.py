@@ -116,3 +116,71 @@ def test_wide_rows_whose_candidates_are_one_blocks(cuda, lily, W, vocab, bf16, o
     assert all(list(row) == [d.token for d in want] for row in got)
     assert_parity(b, run_batch(cuda, lily, s, b), want, label=f"V={vocab} owner {owner}")
     s.close()
+
+
+@pytest.mark.parametrize("barrier,block,lost", [(1, 0, True), (1, 1, False), (2, 0, True), (2, 1, False)])
+def test_a_wait_of_a_narrow_row_that_runs_out(cuda, lily, W, barrier, block, lost):
+    """A block that waits for the others of its row gives up after the handle's limit: the
+    launch completes and its shared memory stays until nobody stores into it. Without the first
+    block's own arrivals the row has no result, and the status says so once; with another
+    block's missing the first one draws the row alone. The next launch is as ever."""
+    vocab, rows = 60_001, 3
+    b = make_batch(W, np.random.default_rng([barrier, block]), rows, vocab, 40, False, kind="zipf", history=300, rep=1.1)
+    s = lily.SamplerScratch(vocab, max_rows=rows)
+    s.set_wait_limit(2_000_000)
+    s.inject_lost_arrival(barrier, block)
+    res = run_batch(cuda, lily, s, b)
+    want = oracle_rows(b)
+    if lost:
+        assert list(res.ids) == [0xFFFFFFFF] * rows and (res.status == 8).all() and not res.kept_n.any()
+        assert s.status() == lily.ERR_TIMEOUT
+    else:
+        assert_parity(b, res, want)
+    assert s.status() == lily.OK
+    s.set_wait_limit(0)
+    assert_parity(b, run_batch(cuda, lily, s, b), want)
+    assert s.status() == lily.OK
+    s.close()
+
+
+@pytest.mark.parametrize("barrier,block,lost", [(1, 0, True), (3, 0, True), (3, 2, True), (5, 0, True), (5, 2, False)])
+def test_a_wait_of_a_wide_row_that_runs_out(cuda, lily, W, barrier, block, lost):
+    vocab, rows = 60_001, 2
+    b = make_batch(W, np.random.default_rng([barrier, block, 1]), rows, vocab, 0, False, kind="zipf")
+    s = lily.SamplerScratch(vocab, max_rows=rows)
+    s.set_wait_limit(2_000_000)
+    s.inject_lost_arrival(barrier, block)
+    res = run_batch(cuda, lily, s, b)
+    want = oracle_rows(b)
+    if lost:
+        assert list(res.ids) == [0xFFFFFFFF] * rows and (res.status == 8).all()
+        assert s.status() == lily.ERR_TIMEOUT
+    else:
+        assert_parity(b, res, want)
+    assert s.status() == lily.OK
+    s.set_wait_limit(0)
+    assert_parity(b, run_batch(cuda, lily, s, b), want)
+    s.close()
+
+
+def test_a_wait_for_an_argmax_and_for_a_shards_sums_that_runs_out(cuda, lily, W):
+    vocab, rows = 60_001, 2
+    b = make_batch(W, np.random.default_rng(3), rows, vocab, 40, False, kind="zipf")
+    logits, out = t_logits(cuda, b), cuda.zeros(rows, dtype=cuda.int32, device="cuda")
+    s = lily.SamplerScratch(vocab, max_rows=rows)
+    s.set_wait_limit(2_000_000)
+    s.inject_lost_arrival(1, 0)
+    s.argmax_batch(logits, out)
+    assert s.status() == lily.ERR_TIMEOUT and list(np_u32(out)) == [0xFFFFFFFF] * rows
+    s.argmax_batch(logits, out)
+    assert s.status() == lily.OK and list(np_u32(out)) == list(b.logits.argmax(1))
+    # (the candidates are there, their sum is not)
+    records = [cuda.zeros((rows, lily.SHARD_RECORD_BYTES), dtype=cuda.uint8, device="cuda") for _ in range(2)]
+    s.shard_candidates(logits, make_params(lily, b), records[0], want_sums=True)
+    assert s.status() == lily.OK
+    s.inject_lost_arrival(4, 0)
+    s.shard_candidates(logits, make_params(lily, b), records[1], want_sums=True)
+    assert s.status() == lily.ERR_TIMEOUT
+    good, bad = (r.cpu().numpy() for r in records)
+    assert np.array_equal(good[:, :516], bad[:, :516]) and not bad[:, 516:].any() and good[:, 516:].any()
+    s.close()
