@@ -60,7 +60,6 @@ struct lily_sampler {
     uint32_t *tickets = nullptr;
     uint32_t *status_word = nullptr;
     char *arena = nullptr;  // the device workspaces below are places in it, the staging ring's host side lies behind h_status
-    char *spill = nullptr;  // inline parameters of rows the row kernel hands to the general code
     uint32_t *counts_scratch = nullptr;
     uint32_t *counts_table = nullptr;
     uint32_t *seen_table = nullptr;
@@ -391,10 +390,6 @@ int32_t launch_split(lily_sampler *h, cudaStream_t stream, lily::SplitArgs<MAXR>
     sa.wait_ns = h->wait_ns;
     sa.lost = h->lost_arrival;
     h->lost_arrival = 0;  // one launch only
-    sa.spill_params = reinterpret_cast<lily_sampling_params_t *>(h->spill);
-    sa.spill_steps = reinterpret_cast<uint32_t *>(h->spill + INLINE_ROWS_MAX * sizeof(lily_sampling_params_t));
-    sa.spill_slots = sa.spill_steps + INLINE_ROWS_MAX;
-    sa.spill_history = sa.spill_slots + INLINE_ROWS_MAX;
     CU(h, lily::split_launch<MAXR>(sa, rows, dtype, p.smem, h->max_smem, &h->attr_mask, stream));
     return LILY_OK;
 }
@@ -629,7 +624,6 @@ int32_t lily_sampler_create(int32_t device, uint32_t vocab, uint32_t max_rows,
         cleared = at;
         place(h->part, (size_t)max_rows * lily::CAP * sizeof(uint2));
         place(h->part_n, (size_t)max_rows * lily::MAX_SLICES * 4);
-        place(h->spill, INLINE_ROWS_MAX * (sizeof(lily_sampling_params_t) + 12));
         // (Here, and not by the first head call: that took 1.2 to 2.3 ms longer for it.)
         place(h->lm_prepared, lily_head::prepared_bytes());
         place(h->lm_part, lily_head::part_bytes(h->lm_tokens, (uint32_t)h->sm_count));

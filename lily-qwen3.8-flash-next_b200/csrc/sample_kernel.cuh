@@ -1624,9 +1624,19 @@ enum { PH_START = 0, PH_BITMAPS, PH_LISTS, PH_STREAM, PH_LOCAL_SELECT, PH_MERGE,
         }                                                                                  \
     } while (0)
 
-// One slice (thread block) of one row. `row` indexes every per-row array.
+// What a row's kernel knows of the row from its own arguments, where the arrays of the
+// arguments would otherwise be read.
+struct RowGiven {
+    lily_sampling_params_t params;
+    uint32_t step, slot, history_len;
+    bool has_slot, has_history;
+};
+
+// One slice (thread block) of one row, cut into at most `cut` of them. `row` indexes every
+// per-row array; given: null, or in the thread's own memory.
 template <typename T, bool VEC>
-__device__ __forceinline__ void sample_row(const KArgs &a, const uint32_t row, const uint32_t slice) {
+__device__ __forceinline__ void sample_row(const KArgs &a, const uint32_t row, const uint32_t slice, const uint32_t cut,
+                                           const RowGiven *given) {
     extern __shared__ uint4 smem_raw[];
     SmemFixed *sm = reinterpret_cast<SmemFixed *>(smem_raw);
     uint4 *ring = reinterpret_cast<uint4 *>(sm + 1);
@@ -1641,7 +1651,7 @@ __device__ __forceinline__ void sample_row(const KArgs &a, const uint32_t row, c
     // the previous kernel of the stream is still finishing, and wait below for
     // its memory before they read anything. (Without the attribute the two
     // instructions do nothing.)
-    const bool whole_row_seen = a.n_slices == 1u;  // the block's slice is the whole row: the bitmap's size is known
+    const bool whole_row_seen = cut == 1u;  // the block's slice is the whole row: the bitmap's size is known
     if (tid < BLOOM_WORDS) {
         sm->bloom[tid] = 0;
     }
@@ -1660,13 +1670,14 @@ __device__ __forceinline__ void sample_row(const KArgs &a, const uint32_t row, c
     // Everything the block has to know about its row is asked for first, in
     // one go: these few loads would otherwise queue behind the first rounds of
     // logits that every block of the launch asks for below.
-    const uint32_t hist_len_row = (a.history_ids && a.history_len) ? __ldg(a.history_len + row) : 0u;
+    const uint32_t hist_len_row = given && given->has_history ? given->history_len
+                                  : (a.history_ids && a.history_len) ? __ldg(a.history_len + row) : 0u;
     const int32_t forced = a.forced_ids ? __ldg(a.forced_ids + row) : -1;
     const uint32_t bias_len_row = (a.bias_ids && a.bias_len) ? __ldg(a.bias_len + row) : 0u;
     const uint32_t ban_len_row = (a.ban_ids && a.ban_len) ? __ldg(a.ban_len + row) : 0u;
-    const uint32_t slot_row = a.count_slots ? __ldg(a.count_slots + row) : 0u;
+    const uint32_t slot_row = given && given->has_slot ? given->slot : a.count_slots ? __ldg(a.count_slots + row) : 0u;
     const float u_row = a.uniforms ? __ldg(a.uniforms + row) : 0.0f;
-    const uint32_t step_row = (!a.uniforms && a.steps) ? __ldg(a.steps + row) : 0u;
+    const uint32_t step_row = a.uniforms ? 0u : given ? given->step : a.steps ? __ldg(a.steps + row) : 0u;
     lily_sampling_params_t P;
     if (a.force_greedy) {
         P.temperature = 0.0f;
@@ -1677,6 +1688,8 @@ __device__ __forceinline__ void sample_row(const KArgs &a, const uint32_t row, c
         P.frequency_penalty = 0.0f;
         P.repetition_penalty = 1.0f;
         P.seed = 0;
+    } else if (given) {
+        P = given->params;
     } else {
         // 40 bytes, 8-byte aligned: five 8-byte loads.
         const uint2 *pp = reinterpret_cast<const uint2 *>(a.params + row);
@@ -1694,7 +1707,7 @@ __device__ __forceinline__ void sample_row(const KArgs &a, const uint32_t row, c
     // With one slice per row, where the logits are does not depend on the
     // row's parameters: the first three rounds are asked for before the
     // parameters have arrived (into the stages pass 1 reads them from).
-    const bool early = VEC && a.n_slices == 1u && a.vocab >= 3u * Geo<T>::ROUND;
+    const bool early = VEC && cut == 1u && a.vocab >= 3u * Geo<T>::ROUND;
     if (early) {
         const char *src = reinterpret_cast<const char *>(reinterpret_cast<const T *>(a.logits) +
                                                          (uint64_t)row * a.logits_ld + tid * Geo<T>::GROUP);
@@ -1804,7 +1817,7 @@ __device__ __forceinline__ void sample_row(const KArgs &a, const uint32_t row, c
     // the two-pass route: merging slices of a thousand candidates each costs
     // more than one block streaming the whole row.)
     const bool one_block = c.k > 128u && (!c.use_pen || c.monotone) && a.cand_out == nullptr;
-    const uint32_t want = one_block ? 1u : min(a.n_slices, CAP / c.k);
+    const uint32_t want = one_block ? 1u : min(cut, CAP / c.k);
     const uint32_t slice_len = (((a.vocab + want - 1u) / want) + 255u) & ~255u;
     const uint32_t n_slices = (a.vocab + slice_len - 1u) / slice_len;
     if (slice >= n_slices) {
@@ -1813,7 +1826,7 @@ __device__ __forceinline__ void sample_row(const KArgs &a, const uint32_t row, c
     c.lo = slice * slice_len;
     c.hi = min(a.vocab, c.lo + slice_len);
     c.seen = seen;
-    const bool table_mode = a.count_slots != nullptr;
+    const bool table_mode = a.count_slots != nullptr || (given && given->has_slot);
     const uint32_t slot = table_mode ? slot_row : 0u;
     c.count_draw = c.use_pen && table_mode;
     c.slot = slot;
@@ -2748,14 +2761,14 @@ __device__ __forceinline__ void sample_row(const KArgs &a, const uint32_t row, c
 // Grid (slices, rows): block (x, y) takes slice x of row row0 + y.
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(NT, 2) sample_rows_kernel(const __grid_constant__ KArgs a) {
-    sample_row<T, VEC>(a, a.row0 + blockIdx.y, blockIdx.x);
+    sample_row<T, VEC>(a, a.row0 + blockIdx.y, blockIdx.x, a.n_slices, nullptr);
 }
 
-// The whole row in one block, out of line: what stream_rows_kernel calls for a
-// row it does not take itself.
+// The whole row in one block, out of line: what the kernels of other routes call for a
+// row they do not take themselves.
 template <typename T, bool VEC = true>
-static __device__ __noinline__ void sample_whole_row(const KArgs &a, uint32_t row) {
-    sample_row<T, VEC>(a, row, 0u);
+static __device__ __noinline__ void sample_whole_row(const KArgs &a, uint32_t row, const RowGiven *given = nullptr) {
+    sample_row<T, VEC>(a, row, 0u, 1u, given);
 }
 
 // Sum over a shard row of exp(adjusted - the shard's maximum), for records

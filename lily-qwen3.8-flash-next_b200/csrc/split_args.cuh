@@ -115,16 +115,12 @@ struct SplitArgs {
     uint32_t mark_mode;
     uint32_t mark_words;      // 32-bit words of the marks, a multiple of four
     uint32_t inline_params;   // `in` below is valid (else a.params / a.steps)
-    uint32_t inline_slots;
+    uint32_t inline_slots;    // `slots` below is (both only with inline_params)
     uint32_t inline_history;  // 1 + the history length of every row (0: a.history_len)
     // Test hook: block lost >> 8 of every cluster waits for one arrival too many at its
     // barrier (lost & 255) - 1, so that the wait runs out (0: none).
     uint32_t lost;
     uint64_t wait_ns;         // the bound of every wait of a block for the others
-    // Device words of the handle: where the first block puts what travelled here
-    // when it hands a row to the general code.
-    lily_sampling_params_t *spill_params;
-    uint32_t *spill_steps, *spill_slots, *spill_history;
     RowIn in[MAXR];
     // Keys that a warp gives to the pool of a row that keeps k: so much above its share
     // that all but some three of the best k are in the pool. (What is missing there

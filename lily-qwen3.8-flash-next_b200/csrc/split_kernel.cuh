@@ -669,45 +669,30 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
             give_up();
             return;
         }
-        KArgs whole = a;
-        whole.n_slices = 1;
+        RowGiven given;
         if (ca.inline_params) {
-            if (tid == 0) {
-                const RowIn &in = ca.in[row];
-                lily_sampling_params_t P;
-                P.temperature = (in.flags & ROW_GREEDY) ? 0.0f : in.temp;
-                P.top_k = in.k;
-                P.top_p = in.top_p;
-                P.min_p = in.min_p;
-                P.presence_penalty = in.presence;
-                P.frequency_penalty = in.frequency;
-                P.repetition_penalty = in.rep;
-                P.reserved = 0;
-                P.seed = in.seed;
-                ca.spill_params[row] = P;
-                ca.spill_steps[row] = in.step;
-            }
-            whole.params = ca.spill_params;
-            whole.steps = ca.spill_steps;
+            const RowIn &in = ca.in[row];
+            given.params.temperature = (in.flags & ROW_GREEDY) ? 0.0f : in.temp;
+            given.params.top_k = in.k;
+            given.params.top_p = in.top_p;
+            given.params.min_p = in.min_p;
+            given.params.presence_penalty = in.presence;
+            given.params.frequency_penalty = in.frequency;
+            given.params.repetition_penalty = in.rep;
+            given.params.reserved = 0;
+            given.params.seed = in.seed;
+            given.step = in.step;
+            given.has_slot = ca.inline_slots != 0u;
+            given.slot = ca.inline_slots ? ca.slots[row] : 0u;
+            given.has_history = ca.inline_history != 0u;
+            given.history_len = ca.inline_history ? ca.inline_history - 1u : 0u;
         }
-        if (ca.inline_slots) {
-            if (tid == 0) {
-                ca.spill_slots[row] = ca.slots[row];
-            }
-            whole.count_slots = ca.spill_slots;
-        }
-        if (ca.inline_history) {
-            if (tid == 0) {
-                ca.spill_history[row] = ca.inline_history - 1u;
-            }
-            whole.history_len = ca.spill_history;
-        }
-        __threadfence();
+        const RowGiven *in_args = ca.inline_params ? &given : nullptr;
         __syncthreads();
         if (skip == 0u) {
-            sample_whole_row<T, true>(whole, row);
+            sample_whole_row<T, true>(a, row, in_args);
         } else {
-            sample_whole_row<T, false>(whole, row);
+            sample_whole_row<T, false>(a, row, in_args);
         }
         if (a.cand_out) {
             __syncthreads();
