@@ -429,7 +429,7 @@ int32_t launch_rows_inline(lily_sampler *h, cudaStream_t stream, const lily::KAr
 }
 
 int32_t launch(lily_sampler *h, cudaStream_t stream, const lily::KArgs &a, uint32_t rows,
-               uint32_t dtype, bool slices = false) {
+               uint32_t dtype) {
     const size_t smem = smem_bytes(a.vocab, a.n_slices);
     if (smem > (size_t)h->max_smem) {
         return fail(h, LILY_ERR_CAPACITY, "vocabulary too large for the shared-memory bitmap");
@@ -439,7 +439,7 @@ int32_t launch(lily_sampler *h, cudaStream_t stream, const lily::KArgs &a, uint3
                                       (a.history_ids != nullptr && a.count_slots == nullptr) || a.extra_len != 0u ||
                                           a.bias_ids != nullptr || a.ban_ids != nullptr,
                                       !a.force_greedy);
-    if (plan.take && !slices) {
+    if (plan.take) {
         lily::SplitArgs<INLINE_ROWS> sa;
         sa.a = a;
         sa.inline_params = sa.inline_slots = sa.inline_history = 0;
@@ -918,21 +918,14 @@ int32_t lily_sample_batch(lily_sampler_t *h, void *stream_, const lily_sample_ar
     // Host parameters (and slots) of up to INLINE_ROWS_MAX rows travel in the
     // kernel's own arguments: nothing is staged, no copy sits in front of the launch.
     SplitPlan plan;
-    bool raises_few = false;
     if (!g.params_on_device && g.rows <= INLINE_ROWS_MAX) {
         const bool history = g.history_ids != nullptr && g.count_slots == nullptr;
-        bool counts = false, raises = false;
+        bool counts = false;
         for (uint32_t r = 0; r < g.rows; ++r) {
-            const lily_sampling_params_t &p = g.params[r];
-            counts = counts || p.frequency_penalty != 0.0f;
-            raises = raises || p.repetition_penalty < 1.0f || p.presence_penalty < 0.0f || p.frequency_penalty < 0.0f;
+            counts = counts || g.params[r].frequency_penalty != 0.0f;
         }
         plan = split_plan(h, a, g.rows, g.logits_dtype, history || g.bias_ids != nullptr || g.ban_ids != nullptr,
                           history && counts);
-        // (A few rows whose penalties can raise a logit, which the row kernel leaves to one
-        // block: the general kernel cuts them into slices.)
-        raises_few = raises && g.rows <= 16u;
-        plan.take = plan.take && !raises_few;
     }
     const StageLayout layout = stage_layout(g.rows);
     const bool in_args = plan.take;
@@ -1002,7 +995,7 @@ int32_t lily_sample_batch(lily_sampler_t *h, void *stream_, const lily_sample_ar
     if (in_args) {
         return launch_rows_inline(h, stream, a, plan, g.rows, g.logits_dtype, g.params, g.steps, g.count_slots);
     }
-    st = launch(h, stream, a, g.rows, g.logits_dtype, raises_few);
+    st = launch(h, stream, a, g.rows, g.logits_dtype);
     if (slot >= 0) {
         CU(h, cudaEventRecord(h->ev[slot], stream));
     }
@@ -1037,10 +1030,8 @@ int32_t lily_sample_one(lily_sampler_t *h, void *stream_, const void *logits, ui
     a.history_ld = history_len;
     a.out_ids = out_id;
     a.n_slices = choose_slices(h, 1u);
-    const bool raises = params->repetition_penalty < 1.0f || params->presence_penalty < 0.0f ||
-                        params->frequency_penalty < 0.0f;
     const SplitPlan plan = split_plan(h, a, 1u, logits_dtype, history_ids != nullptr, params->frequency_penalty != 0.0f);
-    if (plan.take && !raises) {
+    if (plan.take) {
         return launch_split_inline<INLINE_ROWS>(h, stream, a, plan, 1u, logits_dtype, params, &step, nullptr,
                                                 1u + history_len);
     }
@@ -1060,7 +1051,7 @@ int32_t lily_sample_one(lily_sampler_t *h, void *stream_, const void *logits, ui
     a.params = reinterpret_cast<const lily_sampling_params_t *>(ds + layout.params);
     a.steps = reinterpret_cast<const uint32_t *>(ds + layout.steps);
     a.history_len = history_ids ? reinterpret_cast<const uint32_t *>(ds + layout.hist_len) : nullptr;
-    st = launch(h, stream, a, 1u, logits_dtype, true);
+    st = launch(h, stream, a, 1u, logits_dtype);
     CU(h, cudaEventRecord(h->ev[slot], stream));
     return st;
 }
@@ -1682,9 +1673,8 @@ int32_t lily_spec_verify(lily_sampler_t *h, void *stream_, const lily_spec_args_
     const uint32_t launches = pen ? g.m : 1u, rows = pen ? 1u : g.m;
     a.n_slices = choose_slices(h, rows);
     const bool listed = g.count_slot == nullptr && pen;
-    const bool raises = p.repetition_penalty < 1.0f || p.presence_penalty < 0.0f || p.frequency_penalty < 0.0f;
     const SplitPlan plan = split_plan(h, a, rows, g.logits_dtype, listed, p.frequency_penalty != 0.0f);
-    const bool in_args = plan.take && !raises;
+    const bool in_args = plan.take;
     lily_sampling_params_t params[8];
     uint32_t steps[8], slots[8];
     for (uint32_t j = 0; j < g.m; ++j) {
@@ -1723,7 +1713,7 @@ int32_t lily_spec_verify(lily_sampler_t *h, void *stream_, const lily_spec_args_
         }
         st = in_args ? launch_split_inline<INLINE_ROWS>(h, stream, a, plan, pen ? j + 1u : g.m, g.logits_dtype, params,
                                                         steps, g.count_slot ? slots : nullptr, 1u + g.history_len, rows)
-                     : launch(h, stream, a, rows, g.logits_dtype, true);
+                     : launch(h, stream, a, rows, g.logits_dtype);
     }
     if (st == LILY_OK) {
         if (g.m > 1u) {

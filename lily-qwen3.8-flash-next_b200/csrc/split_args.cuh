@@ -24,6 +24,10 @@ constexpr uint32_t SPL_NAN_KEY = 0xFFFFFFFFu;  // a candidate that came out a Na
 
 // How a block keeps the history ids of its share.
 enum { MARK_BITS = 0, MARK_BYTES = 1, MARK_COUNTS = 2 };
+// Flags of a mark: the id is on the bias or ban list; it has been looked at already (a row
+// whose penalties can raise a logit). MARK_MAX: the largest count beside them.
+constexpr uint32_t BYTE_LISTED = 0x80u, BYTE_CLAIMED = 0x40u, BYTE_MAX = 0x3Fu;
+constexpr uint32_t HALF_LISTED = 0x8000u, HALF_CLAIMED = 0x4000u, MARK_MAX = 0x3FFFu;
 
 template <typename T>
 struct Piece {
@@ -101,6 +105,7 @@ struct alignas(16) SplitSmem {
     uint32_t bound_key;
     uint32_t record_key;             // a shard's largest adjusted logit
     uint32_t n_slots;                // candidates whose ids are counted in the history
+    float least;                     // what an adjusted logit has to reach
     uint32_t late;                   // a wait of this block ran out: others may still store into it
 };
 static_assert(sizeof(SplitSmem) % 16u == 0u, "the arrays behind it are 16-byte aligned");

@@ -27,10 +27,12 @@
 // slices through global memory, or a cluster that kept the row in shared memory).
 //
 // A row that keeps more than 64 candidates takes its bound from the maxima of all
-// threads of the cluster, and all blocks rank its candidates. Rows this kernel does not
-// take (penalties that can raise a logit, a NaN, more ties than the buffers hold, ...)
-// are drawn by the first block alone with the general row code: the results do
-// not depend on the way.
+// threads of the cluster, and all blocks rank its candidates. Where penalties can raise a
+// logit, an emitted id may be among the best whatever its logit: once the bound is known
+// the block's other half looks at these ids, and what may reach it is a candidate of its
+// own, as the ids on the bias list are. Rows this kernel does not take (a NaN, more ties
+// than the buffers hold, ...) are drawn by the first block alone with the general row
+// code: the results do not depend on the way.
 //
 // Every warp reads 512 consecutive bytes at a time, and the pieces go round the
 // blocks and warps in turn: neighbouring ids, which often have similar logits, end
@@ -588,6 +590,131 @@ static __device__ __noinline__ void split_finalize(SmemFixed *sm, const KArgs &a
     }
 }
 
+// The logit, as it was before the division by the temperature, with the penalties for an
+// id that was emitted `count` times.
+__device__ __forceinline__ float penalise(float x, uint32_t count, float rep, float presence, float frequency) {
+    if (count != 0u) {
+        x = x > 0.0f ? __fdiv_rn(x, rep) : __fmul_rn(x, rep);
+        x = __fsub_rn(x, __fadd_rn(presence, __fmul_rn(frequency, (float)count)));
+    }
+    return x;
+}
+
+// Penalties that can raise a logit: the block's emitted ids whose adjusted logits may reach
+// ss->least (a NaN does) join the ids of the bias list in tkey[] / tid[]; those on the bias
+// or ban list themselves are left out. The marking half of the block, while the other half
+// reads again what reaches the bound. A look costs no division: the logit is adjusted
+// exactly where all candidates are. Measured, presence penalty -0.3, 4096 ids: 4 rows x
+// 151936 bf16 17.5 us (the row left to one block: 95; in slices: 34), 148 x 50257 f32 21 (82).
+// A step of eight ids a thread costs 1.6 us (32000 ids, 4 rows: 41 us), latency all. No loop over an id's bits: lanes that went round one a
+// different number of times took 0.5 us a round (148 rows x 50257: 50 of 98 us).
+struct Emitted {
+    const uint32_t *hist;  // the row's list ...
+    uint32_t hist_len, extra_len, slot;
+    float rep, presence, frequency;
+    bool table, need_counts, has_lists;  // table: ... or histogram slot `slot`
+};
+
+__device__ __forceinline__ void take_emitted(SmemFixed *sm, SplitSmem *ss, const Emitted &in, float inv, float least,
+                                             uint32_t id, float l, uint32_t count) {
+    const float y = l > 0.0f ? l * inv : l * in.rep, pen = in.presence + in.frequency * (float)count;
+    // (Away from the adjusted logit by a few roundings of 2^-24 of these three at most.)
+    if (!(y - pen < least - (1e-6f * (fabsf(y) + fabsf(pen) + fabsf(least)) + 1e-37f))) {
+        const uint32_t to = atomicAdd(&ss->n_listed, 1u);
+        if (to < KCAP) {
+            sm->tkey[to] = __float_as_uint(l);
+            sm->tid[to] = id;
+        } else {
+            ss->hard = 1;
+        }
+    }
+}
+
+template <typename T>
+static __device__ __noinline__ void emitted_candidates(SmemFixed *sm, SplitSmem *ss, const KArgs &a, const T *row_ptr,
+                                                      uint32_t log_blocks, uint32_t *marks, uint32_t mark_mode,
+                                                      const Emitted &in) {
+    constexpr uint32_t PER = Piece<T>::PER, SHIFT = Piece<T>::SHIFT, NONE = 0xFFFFFFFFu;
+    const uint32_t t = threadIdx.x - SPL_NT, rank = blockIdx.x, blocks = 1u << log_blocks, vocab = a.vocab;
+    const uint32_t skip = (uint32_t)(reinterpret_cast<uintptr_t>(row_ptr) & 15u) / (uint32_t)sizeof(T);
+    const float inv = __fdiv_rn(1.0f, in.rep), least = ss->least;
+    const bool bytes = mark_mode == MARK_BYTES;
+    if (!in.table) {
+        // The list once more: the first of an id's entries to get there claims its mark.
+        constexpr uint32_t U = 8u;  // ids of a thread on their way
+        const uint32_t total = in.hist_len + in.extra_len, listed_or_claimed = bytes ? BYTE_LISTED | BYTE_CLAIMED
+                                                                                     : HALF_LISTED | HALF_CLAIMED;
+        for (uint32_t i0 = 0; i0 < total; i0 += U * SPL_NT) {
+            uint32_t id[U], was[U], shift[U];
+            T l[U];  // (nothing is done with what is asked for before all of it has been)
+#pragma unroll
+            for (uint32_t u = 0; u < U; ++u) {
+                const uint32_t i = i0 + u * SPL_NT + t;
+                id[u] = i < in.hist_len ? __ldg(in.hist + i) : i < total ? __ldcg(a.extra_ids + (i - in.hist_len)) : NONE;
+            }
+#pragma unroll
+            for (uint32_t u = 0; u < U; ++u) {
+                const uint32_t place = id[u] + skip, piece = place >> SHIFT;
+                const uint32_t at = ((piece >> log_blocks) << SHIFT) | (place & (Piece<T>::LOGITS - 1u));
+                shift[u] = bytes ? (at & 3u) * 8u : (at & 1u) * 16u;
+                was[u] = 0u;
+                l[u] = T(0.0f);
+                if (id[u] < vocab && (piece & (blocks - 1u)) == rank) {
+                    l[u] = row_ptr[id[u]];
+                    was[u] = atomicOr(marks + (at >> (bytes ? 2u : 1u)), (bytes ? BYTE_CLAIMED : HALF_CLAIMED) << shift[u]);
+                }
+            }
+#pragma unroll
+            for (uint32_t u = 0; u < U; ++u) {
+                const uint32_t mark = was[u] >> shift[u], count = mark & (bytes ? BYTE_MAX : MARK_MAX);
+                if (count != 0u && (mark & listed_or_claimed) == 0u) {
+                    take_emitted(sm, ss, in, inv, least, id[u], widen(l[u]), count);
+                }
+            }
+        }
+        return;
+    }
+    // The slot's bits over the block's pieces: a warp per piece, a lane per vector.
+    constexpr uint32_t U = 2u;
+    const uint32_t lane = t & 31u, pieces = split_pieces(vocab, skip, PER);
+    const uint32_t *seen = a.seen_table + (uint64_t)in.slot * a.seen_words;
+    const uint32_t *counts = a.counts_table + (uint64_t)in.slot * vocab;
+    for (uint32_t j0 = t >> 5; (j0 << log_blocks) < pieces; j0 += U * SPL_WARPS) {
+        uint32_t bits[U];
+        float l[U][PER];
+#pragma unroll
+        for (uint32_t u = 0; u < U; ++u) {
+            const uint32_t j = j0 + u * SPL_WARPS, first_id = (((j << log_blocks) | rank) * 32u + lane) * PER - skip;
+            bits[u] = 0u;
+#pragma unroll
+            for (uint32_t e = 0; e < PER; ++e) {
+                const uint32_t id = first_id + e;
+                bits[u] |= id < vocab && ((__ldcg(seen + (id >> 5)) >> (id & 31u)) & 1u) ? 1u << e : 0u;
+            }
+#pragma unroll
+            for (uint32_t e = 0; e < PER; ++e) {
+                l[u][e] = (bits[u] >> e) & 1u ? widen(row_ptr[first_id + e]) : 0.0f;
+            }
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < U; ++u) {
+            const uint32_t j = j0 + u * SPL_WARPS, first_id = (((j << log_blocks) | rank) * 32u + lane) * PER - skip;
+#pragma unroll
+            for (uint32_t e = 0; e < PER; ++e) {
+                // (first_id may lie in front of the row, mod 2^32: ids are added up in 32 bits, then used.)
+                const uint32_t at = (j << SHIFT) | (lane * PER + e), id = first_id + e;
+                if ((bits[u] >> e) & 1u) {
+                    const bool listed = in.has_lists && (bytes ? reinterpret_cast<const uint8_t *>(marks)[at] & BYTE_LISTED
+                                                               : reinterpret_cast<const uint16_t *>(marks)[at] & HALF_LISTED);
+                    if (!listed) {
+                        take_emitted(sm, ss, in, inv, least, id, l[u][e], in.need_counts ? __ldcg(counts + id) : 1u);
+                    }
+                }
+            }
+        }
+    }
+}
+
 // Grid (blocks per row, rows), clusters of (blocks per row), NT threads, of which
 // SPL_NT do the work. BPS: blocks per SM the registers are cut for; with one, a
 // block whose share fits one bucket keeps it in registers.
@@ -851,8 +978,14 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
     const uint32_t k = shard && !(in.flags & ROW_GREEDY) ? a.shard_k : in.k;
     const bool wide = k > SPL_SMALL_K;
     const uint32_t mark_mode = ca.mark_mode;
+    const bool marked = hist_len + extra_len != 0u;
+    const bool counted = marked && need_counts;  // (a list whose multiplicities matter)
+    const bool raises = (in.flags & ROW_RAISES) != 0u;
+    const bool count_later = counted && !raises;  // (... but only the candidates')
+    const bool emitted = raises && (table_mode || marked);
     // Decided alike by every block of the cluster: rows that end here.
-    const bool general = (in.flags & ROW_RAISES) || n_sp > SP_SMEM ||
+    const bool general = n_sp > SP_SMEM || (raises && marked && mark_mode == MARK_BITS) ||
+                         (raises && counted && hist_len + extra_len > MARK_MAX) ||
                          (n_sp != 0u && mark_mode == MARK_BITS) ||
                          (list_mode && need_counts && mark_mode != MARK_COUNTS) ||
                          (wide && (row < a.spec.n_spec || min(vocab / PER, blocks * SPL_NT) * 8u < 9u * k));
@@ -891,8 +1024,6 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
     };
     uint8_t *mark8 = reinterpret_cast<uint8_t *>(marks);
     uint16_t *mark16 = reinterpret_cast<uint16_t *>(marks);
-    const bool marked = hist_len + extra_len != 0u;
-    const bool counted = marked && need_counts;  // (a list whose multiplicities matter)
     if (marker && shard && a.shard_sums) {
         // A shard has no history: this half reads the share a second time (it comes from L2,
         // just behind the other half) and adds up the exponentials, in the base-2 domain and
@@ -1070,6 +1201,9 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         if (!marked) {
         } else if (mark_mode == MARK_BYTES) {
             mark_all([&](uint32_t at) { mark8[at] = 1; });
+        } else if (mark_mode == MARK_COUNTS && counted && raises) {
+            // (At most MARK_MAX ids: no count reaches into the flags or its neighbour.)
+            mark_all([&](uint32_t at) { atomicAdd(marks + (at >> 1), 1u << ((at & 1u) * 16u)); });
         } else if (mark_mode == MARK_COUNTS) {
             mark_all([&](uint32_t at) { mark16[at] = 1; });
         } else {
@@ -1109,9 +1243,9 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
                 }
                 if (first) {
                     if (mark_mode == MARK_BYTES) {
-                        mark8[at] |= 0x80u;
+                        mark8[at] |= BYTE_LISTED;
                     } else {
-                        mark16[at] |= 0x8000u;
+                        mark16[at] |= HALF_LISTED;
                     }
                     if (!banned) {
                         const uint32_t to = atomicAdd(&ss->n_listed, 1u);
@@ -1124,16 +1258,23 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         if (marked || n_sp != 0u) {
             asm volatile("bar.arrive 3, %0;" ::"n"(NT) : "memory");
         }
-        if (counted) {
+        if (emitted) {
+            const Emitted r = {hist, hist_len, extra_len, slot, in.rep, in.presence, in.frequency, table_mode, need_counts,
+                               n_sp != 0u};
+            asm volatile("bar.sync 4, %0;" ::"n"(NT) : "memory");
+            emitted_candidates<T>(sm, ss, a, row_ptr, log_blocks, marks, mark_mode, r);
+            asm volatile("bar.arrive 5, %0;" ::"n"(NT) : "memory");
+        }
+        if (count_later) {
             asm volatile("bar.sync 4, %0;" ::"n"(NT) : "memory");
             if (ss->n_slots != 0u) {
                 // The candidates' marks name their counters.
                 each_four([&](const uint4 &x) {
                     uint32_t at, m[4] = {0, 0, 0, 0};
-                    m[0] = place_of(x.x, at) == rank ? mark16[at] & 0x7FFFu : 0u;
-                    m[1] = place_of(x.y, at) == rank ? mark16[at] & 0x7FFFu : 0u;
-                    m[2] = place_of(x.z, at) == rank ? mark16[at] & 0x7FFFu : 0u;
-                    m[3] = place_of(x.w, at) == rank ? mark16[at] & 0x7FFFu : 0u;
+                    m[0] = place_of(x.x, at) == rank ? mark16[at] & MARK_MAX : 0u;
+                    m[1] = place_of(x.y, at) == rank ? mark16[at] & MARK_MAX : 0u;
+                    m[2] = place_of(x.z, at) == rank ? mark16[at] & MARK_MAX : 0u;
+                    m[3] = place_of(x.w, at) == rank ? mark16[at] & MARK_MAX : 0u;
                     // (Adding equal ids of a warp up first, with a match instruction, was slower: one
                     // greedy row with 16000 ids, a good part of them the same, 18.4 -> 20.2 us.)
                     if (max(max(m[0], m[1]), max(m[2], m[3])) >= 2u) {
@@ -1272,14 +1413,8 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
     }
     LILY_STAMP(PH_PASS1);
 
-    // The logit, as it was before the division by the temperature, with the
-    // penalties for an id that was emitted `count` times.
     auto penalised = [&](float x, uint32_t count) -> float {
-        if (count != 0u) {
-            x = x > 0.0f ? __fdiv_rn(x, in.rep) : __fmul_rn(x, in.rep);
-            x = __fsub_rn(x, __fadd_rn(in.presence, __fmul_rn(in.frequency, (float)count)));
-        }
-        return x;
+        return penalise(x, count, in.rep, in.presence, in.frequency);
     };
     // The mark of an id of this block's share: how often it was emitted (without a
     // frequency penalty any number but 0 will do), and LISTED if it is on a bias or
@@ -1292,10 +1427,10 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
             place_of(id, at);
             if (mark_mode == MARK_BYTES) {
                 const uint32_t x = mark8[at];
-                m = (x & 0x7Fu) | (x >> 7 << 31);
+                m = (x & BYTE_MAX) | ((x & BYTE_LISTED) ? LISTED : 0u);
             } else if (mark_mode == MARK_COUNTS) {
                 const uint32_t x = mark16[at];
-                m = (x & 0x7FFFu) | (x >> 15 << 31);
+                m = (x & MARK_MAX) | ((x & HALF_LISTED) ? LISTED : 0u);
             } else {
                 m = (marks[at >> 5] >> (at & 31u)) & 1u;
             }
@@ -1325,7 +1460,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
             }
             const uint32_t m = mark_of(id_at(warp + SPL_WARPS * best_j, e));
             // (Not yet counted: left out, which can only lower the bound.)
-            x = (m & LISTED) || (counted && m != 0u) ? neg_inf() : penalised(x, m);
+            x = (m & LISTED) || (count_later && m != 0u) ? neg_inf() : penalised(x, m);
         }
         key = key_of(__fadd_rn(x, 0.0f));
     }
@@ -1502,6 +1637,12 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
             ss->hit_at[to] = first_id;
         }
     };
+    if (emitted) {
+        if (tid == 0) {
+            ss->least = hopeless ? -neg_inf() : least;
+        }
+        asm volatile("bar.arrive 4, %0;" ::"n"(NT) : "memory");
+    }
     if (hopeless) {
         ss->hard = 1;
     } else if (BPS == 1 && buckets == 1u) {
@@ -1559,7 +1700,11 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
             }
         }
     }
-    spl_sync();
+    if (emitted) {
+        asm volatile("bar.sync 5, %0;" ::"n"(NT) : "memory");
+    } else {
+        spl_sync();
+    }
     LILY_STAMP(PH_LISTS);
     // ... and their logits, a thread each: what reaches the bound is adjusted, divided
     // and sent to the first block, and so are the ids of the bias list.
@@ -1575,7 +1720,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
     // f(id, logit, whether it comes from the bias list) for every one that may be among
     // the best: a thread per vector, mostly with one such logit.
     const uint32_t n_vecs = n_hits <= SPL_HITS && ss->hard == 0u ? n_hits : 0u;
-    const uint32_t n_all = n_vecs + (ss->hard == 0u ? ss->n_listed : 0u);
+    const uint32_t n_all = n_vecs + (ss->hard == 0u ? ss->n_listed : 0u);  // (more of these than there is room for: hard)
     auto each_logit = [&](auto f) {
         for (uint32_t i = tid; i < n_all; i += SPL_NT) {
             if (i < n_vecs) {
@@ -1598,7 +1743,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         }
     };
     uint32_t n_slots = 0;
-    if (counted) {
+    if (count_later) {
         // The markers count the candidates' ids in the history: a counter each.
         each_logit([&](uint32_t id, float, bool listed) {
             const uint32_t m = mark_of(id);
@@ -1608,7 +1753,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
                     uint32_t at;
                     place_of(id, at);
                     sm->thist[to] = 0;
-                    mark16[at] = (uint16_t)((mark16[at] & 0x8000u) | (to + 2u));
+                    mark16[at] = (uint16_t)((mark16[at] & HALF_LISTED) | (to + 2u));
                 }
             }
         });
@@ -1625,7 +1770,10 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
                 return;  // (its own entry stands for it)
             }
             m &= ~LISTED;
-            if (counted && m != 0u) {
+            if (raises && m != 0u && !listed) {
+                return;  // (likewise)
+            }
+            if (count_later && m != 0u) {
                 m = m >= 2u ? sm->thist[m - 2u] : 0u;
             }
             x = penalised(x, m);

@@ -184,3 +184,59 @@ def test_a_wait_for_an_argmax_and_for_a_shards_sums_that_runs_out(cuda, lily, W)
     good, bad = (r.cpu().numpy() for r in records)
     assert np.array_equal(good[:, :516], bad[:, :516]) and not bad[:, 516:].any() and good[:, 516:].any()
     s.close()
+
+
+RAISING = [dict(history=700, presence=-0.6), dict(history=3000, rep=0.7), dict(history=2000, frequency=-0.2, rep=1.1),
+           dict(history=900, frequency=0.1, presence=-1.0, n_bias=9, n_ban=3), dict(history=5, presence=-40.0)]
+
+
+@pytest.mark.parametrize("rows,vocab,bf16", [(1, 1024, False), (3, 2048, True), (4, 60_001, True), (20, 9_001, False),
+                                             (70, 9_001, True), (149, 9_001, False)])
+def test_penalties_that_raise_a_logit(cuda, lily, W, rows, vocab, bf16):
+    # An emitted id may be among the best whatever its logit: with lists in every way of
+    # keeping them, narrow, wide and greedy rows, parameters on either side.
+    rng = np.random.default_rng([rows, vocab])
+    for i, kw in enumerate(RAISING):
+        b = make_batch(W, rng, rows, vocab, [40, 1, 0, 20, 64][i], bf16, kind="zipf", **kw)
+        for r in range(0, rows, 3):  # the row's worst ids are on its list
+            b.history[r, :4] = np.argpartition(b.logits_f32()[r], 4)[:4].astype(np.uint32)
+        for dev in (False, True):
+            check(cuda, lily, W, b, vocab, f"B={rows} V={vocab} {kw}", params_on_device=dev)
+        b = make_batch(W, rng, rows, vocab, [0, 40, 64, 1, 2][i], bf16, kind="uniform", **kw)
+        check(cuda, lily, W, b, vocab, f"B={rows} V={vocab} {kw} uniform")
+
+
+def test_more_ids_than_a_raising_count_holds(cuda, lily, W):
+    # Lists of mostly one id, around the most that a half word counts: the longer one is the
+    # general code's.
+    rng = np.random.default_rng(8)
+    b = make_batch(W, rng, 3, 9_001, 40, True, kind="zipf", history=40_000, frequency=-0.001)
+    b.history[:, :16_300] = 17
+    b.history_len[:] = [40_000, 16_383, 16_384]
+    check(cuda, lily, W, b, 9_001, "long list")
+
+
+@pytest.mark.parametrize("lists", [{}, dict(n_bias=7, n_ban=4)])
+@pytest.mark.parametrize("pen", [dict(presence_penalty=-0.7), dict(frequency_penalty=-0.1, repetition_penalty=1.2)])
+def test_penalties_that_raise_a_logit_of_a_slot(cuda, lily, W, pen, lists):
+    rng = np.random.default_rng(12)
+    rows, vocab = 5, 60_001
+    b = make_batch(W, rng, rows, vocab, 40, False, kind="zipf", **lists)
+    for p in b.params:
+        p.update(pen)
+    counts = np.zeros((rows, vocab), dtype=np.uint32)
+    s = lily.SamplerScratch(vocab, max_rows=rows, max_history=0, counts_table=True)
+    for r in range(rows):
+        ids = rng.integers(0, vocab, 3000)
+        ids[:4] = np.argpartition(b.logits[r], 4)[:4]
+        if lists:
+            ids[4:8] = b.bias_ids[r, :4]
+        np.add.at(counts[r], ids, 1)
+        s.write_counts(counts[r], slot=r)
+    for dev in (False, True):
+        res = run_batch(cuda, lily, s, b, count_slots=list(range(rows)), params_on_device=dev)
+        assert_parity(b, res, oracle_rows(b, counts=counts))
+        for r in range(rows):
+            counts[r, res.ids[r]] += 1
+            assert np.array_equal(s.read_counts(slot=r), counts[r])
+    s.close()
