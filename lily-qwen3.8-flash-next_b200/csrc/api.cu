@@ -321,7 +321,7 @@ int32_t upload(lily_sampler *h, int slot, size_t bytes, cudaStream_t stream) {
 struct SplitPlan {
     bool take = false;
     bool sole = false;   // at most one block per SM
-    uint32_t log_blocks = 0, mark_mode = lily::MARK_BITS, mark_words = 0;
+    uint32_t log_blocks = 0, log_live = 0, mark_mode = lily::MARK_BITS, mark_words = 0;
     size_t smem = 0;
 };
 
@@ -356,6 +356,7 @@ SplitPlan split_plan(const lily_sampler *h, const lily::KArgs &a, uint32_t rows,
     const size_t fixed = sizeof(lily::SmemFixed) + sizeof(lily::SplitSmem) +
                          (size_t)lily::split_buckets(here, lily::split_u(p.sole ? 1 : 2)) * lily::SPL_NT * 4u;
     p.log_blocks = lb;
+    p.log_live = (a.vocab / logits) >> lb < lily::SPL_WARPS ? 2u : 3u;
     if (lists) {
         const size_t limit = p.sole ? (size_t)h->max_smem : 113u * 1024u;
         if (counts && fixed + (size_t)entries * 2u <= limit) {
@@ -384,6 +385,7 @@ template <uint32_t MAXR>
 int32_t launch_split(lily_sampler *h, cudaStream_t stream, lily::SplitArgs<MAXR> &sa, const SplitPlan &p,
                      uint32_t rows, uint32_t dtype) {
     sa.log_blocks = p.log_blocks;
+    sa.log_live = p.log_live;
     sa.two_per_sm = p.sole ? 0u : 1u;
     sa.mark_mode = p.mark_mode;
     sa.mark_words = p.mark_words;

@@ -10,6 +10,8 @@ namespace lily {
 
 constexpr uint32_t SPL_NT = 256;         // threads at work; the other half of the block waits for a row of the general code
 constexpr uint32_t SPL_WARPS = SPL_NT / 32;
+constexpr uint32_t SPL_LOG_NT = 8;
+static_assert(1u << SPL_LOG_NT == SPL_NT, "");
 // Vectors of a bucket: a thread's loads in flight (with two blocks per SM as many
 // as 64 registers a thread hold).
 __host__ __device__ constexpr uint32_t split_u(int bps) { return bps == 1 ? 10u : 6u; }
@@ -19,7 +21,9 @@ constexpr uint32_t SPL_POOL = 256;       // keys in the pool a narrow row's boun
 constexpr uint32_t SPL_HITS = 512;       // vectors of a block that may reach the bound
 constexpr uint32_t SPL_FLAGGED = 2048;   // buckets that may reach the bound
 constexpr uint32_t SPL_SORTED = 2048;    // candidates of a wide row
-constexpr uint32_t SPL_MIN_TILES = SPL_WARPS / 2u;  // pieces of a block, at least
+// Pieces of a block, at least: half of its warps have one. (With a piece for every warp, and
+// so fewer blocks, 4096 bf16 that keep 64 took 14.2 us instead of 12.9.)
+constexpr uint32_t SPL_MIN_TILES = SPL_WARPS / 2u;
 constexpr uint32_t SPL_NAN_KEY = 0xFFFFFFFFu;  // a candidate that came out a NaN
 
 // How a block keeps the history ids of its share.
@@ -116,6 +120,7 @@ template <uint32_t MAXR>
 struct SplitArgs {
     KArgs a;
     uint32_t log_blocks;      // log2 of the blocks per row
+    uint32_t log_live;        // log2 of the warps of a block that have pieces, at least (2 or 3)
     uint32_t two_per_sm;      // more rows than SMs: the instantiation of which two blocks fit
     uint32_t mark_mode;
     uint32_t mark_words;      // 32-bit words of the marks, a multiple of four
@@ -129,10 +134,11 @@ struct SplitArgs {
     RowIn in[MAXR];
     // Keys that a warp gives to the pool of a row that keeps k: so much above its share
     // that all but some three of the best k are in the pool. (What is missing there
-    // lowers the bound by as many places.)
+    // lowers the bound by as many places. Shares of all warps where half of them have nothing
+    // left the pool with fewer than k keys, and the row to the general code: 1 x 520, 20 kept, 25 us.)
     __device__ __forceinline__ uint32_t rounds_of(uint32_t k) const {
-        const uint32_t share10 = (k * 10u) >> (3u + log_blocks);  // tenths
-        static_assert(SPL_WARPS == 8u, "");
+        const uint32_t share10 = (k * 10u) >> (log_live + log_blocks);  // tenths
+        static_assert(SPL_WARPS == 8u && SPL_MIN_TILES == 4u, "");
         return min((share10 * 13u + 170u) / 100u, SPL_POOL / (SPL_WARPS << log_blocks));
     }
     uint32_t slots[MAXR];

@@ -279,6 +279,13 @@ static __device__ __noinline__ void split_finalize_wide(SmemFixed *sm, SplitSmem
     }
 }
 
+// A block's candidates of a wide row: over the pool, which has served, or over key and id.
+constexpr uint32_t WIDE_OWN = SPL_MAX_BLOCKS * SPL_NT / 2u;
+__device__ __forceinline__ unsigned long long *wide_own(SmemFixed *sm, SplitSmem *ss, uint32_t blocks) {
+    static_assert(SPL_SORTED < CAP, "one block's candidates and the pair's other half");
+    return reinterpret_cast<unsigned long long *>(blocks > 1u ? ss->tmax : sm->key);
+}
+
 // Every block sorts its list and sends it to all blocks; then each knows its
 // entries' ranks in the row (their places in the eight lists, by bisection) and
 // sends them to the first block, to where they belong. (Merged by the first block
@@ -290,11 +297,10 @@ static __device__ __noinline__ uint32_t merge_lists(SmemFixed *sm, SplitSmem *ss
     constexpr unsigned FULL = 0xFFFFFFFFu;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, rank = blockIdx.x, blocks = 1u << log_blocks;
     const uint32_t cap = CAP >> log_blocks, cand_bar = blocks > 1u ? peer_smem(&ss->mbar[MEET_CANDIDATES], 0) : 0u;
-    constexpr uint32_t OWN = SPL_MAX_BLOCKS * SPL_NT / 2u;
-    unsigned long long *own = reinterpret_cast<unsigned long long *>(ss->tmax);
+    unsigned long long *own = wide_own(sm, ss, blocks);
     unsigned long long *lists = reinterpret_cast<unsigned long long *>(sm->key);  // over key and id: CAP
     unsigned long long *best_of = reinterpret_cast<unsigned long long *>(ss + 1);  // SPL_SORTED (the marks have served)
-    if (tid == 0 && sent < OWN) {
+    if (tid == 0 && (blocks == 1u || sent < WIDE_OWN)) {
         own[sent] = 0ull;  // (they are counted in pairs)
     }
     spl_sync();
@@ -983,12 +989,24 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
     const bool raises = (in.flags & ROW_RAISES) != 0u;
     const bool count_later = counted && !raises;  // (... but only the candidates')
     const bool emitted = raises && (table_mode || marked);
+    // A row that keeps many takes its bound from at most SPL_MAX_BLOCKS * SPL_NT maxima: one of
+    // every thread, or, of a short row over four or eight blocks, those of `groups` parts of a
+    // thread's logits. (One maximum a thread, 3 x 8192 bf16, 1024 kept: not enough of them, the
+    // general code's 42 us. With fewer blocks their ranking takes longer than that code: 55.)
+    const uint32_t most_pieces = (pieces + blocks - 1u) >> log_blocks;
+    // (Of the threads that take part: half of them where the other half has nothing, or, of
+    // eight blocks, one warp of it a piece: without its logits the bound is somewhat lower.)
+    const uint32_t log_live = most_pieces <= (log_blocks == 3u ? 5u : SPL_MIN_TILES) ? SPL_LOG_NT - 1u : SPL_LOG_NT;
+    const uint32_t groups = BPS == 1 && log_blocks >= 2u && most_pieces <= SPL_WARPS * SPL_U
+                                ? SPL_MAX_BLOCKS * SPL_NT >> (log_live + log_blocks) : 1u;
+    const bool wide_fits = min(vocab / PER, blocks << log_live) * min(groups, PER) * 8u >= 9u * k &&
+                           (groups == 1u || most_pieces * 32u <= SPL_HITS || k * 5u <= blocks * SPL_HITS * 3u);
     // Decided alike by every block of the cluster: rows that end here.
     const bool general = n_sp > SP_SMEM || (raises && marked && mark_mode == MARK_BITS) ||
                          (raises && counted && hist_len + extra_len > MARK_MAX) ||
                          (n_sp != 0u && mark_mode == MARK_BITS) ||
                          (list_mode && need_counts && mark_mode != MARK_COUNTS) ||
-                         (wide && (row < a.spec.n_spec || min(vocab / PER, blocks * SPL_NT) * 8u < 9u * k));
+                         (wide && (row < a.spec.n_spec || !wide_fits));
     if (status != LILY_ROW_OK || general) {
         if (status != LILY_ROW_OK && rank == 0u && tid == 0) {
             a.out_ids[row] = status == LILY_ROW_FORCED ? (uint32_t)forced : 0xFFFFFFFFu;
@@ -1449,20 +1467,24 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         return ((((j << log_blocks) | rank) * 32u + lane) * PER + e) - skip;
     };
     // This thread's best logit, adjusted but for the temperature (which keeps the order).
+    auto adjusted = [&](float x, uint32_t j, uint32_t e) -> uint32_t {  // (of piece j of the block)
+        if (use_pen || n_sp != 0u) {
+            const uint32_t m = mark_of(id_at(j, e));
+            // (Not yet counted: left out, which can only lower the bound.)
+            x = (m & LISTED) || (count_later && m != 0u) ? neg_inf() : penalised(x, m);
+        }
+        return key_of(__fadd_rn(x, 0.0f));
+    };
     uint32_t key = 0u;
     if (best_j != NONE) {
-        float x = best;
+        uint32_t e = 0;
         if (use_pen || n_sp != 0u) {
-            uint32_t e = 0;
 #pragma unroll
             for (int i = (int)PER - 1; i >= 0; --i) {
                 e = vec_get<T>(best_v, (uint32_t)i) == best ? (uint32_t)i : e;
             }
-            const uint32_t m = mark_of(id_at(warp + SPL_WARPS * best_j, e));
-            // (Not yet counted: left out, which can only lower the bound.)
-            x = (m & LISTED) || (count_later && m != 0u) ? neg_inf() : penalised(x, m);
         }
-        key = key_of(__fadd_rn(x, 0.0f));
+        key = adjusted(best, warp + SPL_WARPS * best_j, e);
     }
     if (bad) {
         ss->hard = 1;  // (read after the next barrier)
@@ -1539,13 +1561,31 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         // The maxima of the whole cluster, 32 bins per unit under the largest.
         if (blocks > 1u) {
             if (tid == 0) {
-                arrive_expect(peer_smem(&ss->mbar[MEET_POOL], rank), blocks * SPL_NT * 4u);
+                arrive_expect(peer_smem(&ss->mbar[MEET_POOL], rank), (blocks * groups << log_live) * 4u);
             }
-            for (uint32_t r = 0; r < blocks; ++r) {
-                put_u32(peer_smem(&ss->tmax[rank * SPL_NT + tid], r), key, peer_smem(&ss->mbar[MEET_POOL], r));
+        }
+        for (uint32_t g = 0; g < groups && tid >> log_live == 0u; ++g) {
+            if (BPS == 1 && groups > 1u) {  // (all of the thread's vectors are in q)
+                float m = neg_inf();
+                uint32_t m_at = NONE;
+#pragma unroll
+                for (uint32_t i = 0; i < SPL_U * PER; ++i) {
+                    const float x = vec_get<T>(q[i / PER], i % PER);
+                    if ((i & (groups - 1u)) == g && x > m) {
+                        m = x;
+                        m_at = i;
+                    }
+                }
+                key = m_at == NONE ? 0u : adjusted(m, warp + SPL_WARPS * (m_at / PER), m_at % PER);
             }
-        } else {
-            ss->tmax[tid] = key;
+            const uint32_t to = ((rank * groups + g) << log_live) + tid;
+            if (blocks > 1u) {
+                for (uint32_t r = 0; r < blocks; ++r) {
+                    put_u32(peer_smem(&ss->tmax[to], r), key, peer_smem(&ss->mbar[MEET_POOL], r));
+                }
+            } else {
+                ss->tmax[to] = key;
+            }
         }
         for (uint32_t b = tid; b < TH_BINS; b += SPL_NT) {
             sm->thist[b] = 0;
@@ -1560,7 +1600,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         uint32_t keys[SPL_MAX_BLOCKS], m = 0;
 #pragma unroll
         for (uint32_t r = 0; r < SPL_MAX_BLOCKS; ++r) {
-            keys[r] = r < blocks ? ss->tmax[r * SPL_NT + tid] : 0u;
+            keys[r] = r * SPL_NT + tid < blocks * groups << log_live ? ss->tmax[r * SPL_NT + tid] : 0u;
             m = max(m, keys[r]);
         }
         m = __reduce_max_sync(FULL, m);
@@ -1714,9 +1754,9 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
     const uint32_t bar = blocks > 1u ? peer_smem(&ss->mbar[MEET_CANDIDATES], 0) : 0u;
     const uint32_t cand_at = blocks > 1u ? peer_smem(cand + rank * cap, 0) : 0u;
     // (Wide rows: first here, over the pool, which has served.)
-    constexpr uint32_t OWN = SPL_MAX_BLOCKS * SPL_NT / 2u;
-    unsigned long long *own = reinterpret_cast<unsigned long long *>(ss->tmax);
-    const uint32_t most = wide ? min(cap, OWN) : cap;
+    // (A block alone: where the others' lists would be.)
+    unsigned long long *own = wide_own(sm, ss, blocks);
+    const uint32_t most = wide ? (blocks > 1u ? min(cap, WIDE_OWN) : SPL_SORTED) : cap;
     // f(id, logit, whether it comes from the bias list) for every one that may be among
     // the best: a thread per vector, mostly with one such logit.
     const uint32_t n_vecs = n_hits <= SPL_HITS && ss->hard == 0u ? n_hits : 0u;

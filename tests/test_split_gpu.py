@@ -17,7 +17,7 @@ def W(lily):
     return w
 
 
-# 8 pieces per block at least (2048 bf16, 1024 f32 logits); a bucket is 80 pieces.
+# 4 pieces per block at least (1024 bf16, 512 f32 logits); a bucket is 80 pieces.
 EDGES = [2047, 2048, 2049, 16383, 16384, 16385, 20480 * 2 - 1, 20480 * 2 + 8, 60001]
 
 
@@ -240,3 +240,19 @@ def test_penalties_that_raise_a_logit_of_a_slot(cuda, lily, W, pen, lists):
             counts[r, res.ids[r]] += 1
             assert np.array_equal(s.read_counts(slot=r), counts[r])
     s.close()
+
+
+@pytest.mark.parametrize("bf16", [False, True])
+@pytest.mark.parametrize("vocab", [511, 512, 1023, 1024, 1025, 2047, 2048, 2049, 4095, 4096, 4097, 6000, 7300, 8192,
+                                   9000, 10_001])
+def test_short_rows(cuda, lily, W, vocab, bf16):
+    # Around the least that the kernel takes (four pieces: 512 f32, 1024 bf16 logits), where
+    # half of a block's warps have nothing, few blocks share a row and a wide row's bound comes
+    # from parts of a thread's logits; with tens of rows few blocks share any row.
+    rng = np.random.default_rng([vocab, bf16])
+    for rows, k, kw in ((1, 20, dict(history=300, rep=1.1)), (2, 64, dict(history=9, presence=0.4, n_bias=5, n_ban=2)),
+                        (3, 0, dict(history=400, rep=1.3, frequency=0.1)), (2, 910, {}), (1, 300, dict(n_ban=4)),
+                        (40, 0, dict(history=200, presence=-0.5)), (80, 500, dict(history=200, presence=0.5)),
+                        (3, 1023, dict(kind="uniform")), (150, 700, {})):
+        b = make_batch(W, rng, rows, vocab, k, bf16, **{"kind": "zipf", **kw})
+        check(cuda, lily, W, b, vocab, f"V={vocab} k={k} B={rows}", params_on_device=rows == 2)
