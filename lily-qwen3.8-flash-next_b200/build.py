@@ -62,7 +62,8 @@ def _run(cmd, verbose=False):
 
 
 def _calls_command():
-    """g++ for the extension module: torch's headers and libraries, the library beside it."""
+    """g++ for the extension module: torch's headers and libraries, the library beside it (by its
+    soname, so that a package that was moved or copied finds its own)."""
     import sysconfig
 
     import torch
@@ -73,8 +74,8 @@ def _calls_command():
     return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={abi}",
             "-I", os.path.join(root, "include"), "-I", os.path.join(root, "include", "torch", "csrc", "api", "include"),
             "-I", os.path.join(cuda, "include"), "-I", sysconfig.get_paths()["include"], CALLS_SOURCE,
-            "-L", os.path.join(root, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda", LIB,
-            "-Wl,-rpath,$ORIGIN", "-o", CALLS]
+            "-L", os.path.join(root, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda",
+            "-L", HERE, "-l:" + os.path.basename(LIB), "-Wl,-rpath,$ORIGIN", "-o", CALLS]
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -94,7 +95,8 @@ def build(force: bool = False, verbose: bool = False) -> str:
             jobs.append([nvcc, *NVCC_FLAGS, *extra, "-I", INCLUDE, "-c", "-o", obj, src])
     with ThreadPoolExecutor(max_workers=max(1, len(jobs))) as pool:
         list(pool.map(lambda cmd: _run(cmd, verbose), jobs))
-    _run([nvcc, *ARCH_FLAGS, "-shared", "-Xcompiler", "-fPIC", "-o", LIB, *objects])
+    _run([nvcc, *ARCH_FLAGS, "-shared", "-Xcompiler", "-fPIC", "-Xlinker", "-soname=" + os.path.basename(LIB), "-o", LIB,
+          *objects])
     if force or _older(CALLS, max(headers, os.path.getmtime(CALLS_SOURCE))):
         _run(_calls_command())
     else:

@@ -109,3 +109,31 @@ def test_no_product_file_touches_the_oracle():
             if f.endswith((".py", ".cu", ".cuh", ".cpp", ".h")):
                 text = open(os.path.join(dirpath, f)).read()
                 assert "oracle" not in text.lower(), f
+
+
+def test_a_copied_package_is_on_its_own(lily, tmp_path):
+    """The extension module finds the library beside it, wherever the package lies; without
+    the module the calls go through ctypes, with a warning."""
+    import shutil
+    import subprocess
+    import sys
+
+    lily.lib()
+    package = os.path.dirname(os.path.abspath(lily.LIB_PATH))
+    copy = tmp_path / os.path.basename(package)
+    shutil.copytree(package, copy, ignore=shutil.ignore_patterns("build", "csrc", "__pycache__"))
+    shutil.copy(os.path.join(ROOT, "lily_b200.py"), tmp_path)
+    code = ("import lily_b200 as lily\n"
+            "m = lily.calls()\n"
+            "print(sorted({l.split()[-1] for l in open('/proc/self/maps') if 'liblily_sampler' in l or '_lily_calls' in l}))\n"
+            "print(m.sample_prepared(1, 2, 3) is None)\n")
+
+    def run():
+        return subprocess.run([sys.executable, "-c", code], cwd=tmp_path, capture_output=True, text=True, check=True)
+
+    maps, none = run().stdout.splitlines()
+    assert eval(maps) == [str(copy / "_lily_calls.so"), str(copy / "liblily_sampler.so")] and none == "True"
+    (copy / "_lily_calls.so").unlink()
+    alone = run()
+    assert eval(alone.stdout.splitlines()[0]) == [str(copy / "liblily_sampler.so")]
+    assert alone.stdout.splitlines()[1] == "True" and "RuntimeWarning" in alone.stderr
