@@ -10,6 +10,7 @@ source file, side by side; a file is compiled again when it or a header is newer
 from __future__ import annotations
 
 import os
+import re
 import subprocess
 import sys
 from concurrent.futures import ThreadPoolExecutor
@@ -21,6 +22,7 @@ OBJ = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "liblily_sampler.so")
 CALLS = os.path.join(HERE, "_lily_calls.so")
 CALLS_SOURCE = os.path.join(CSRC, "python_ext.cpp")
+HEAD_SOURCE = os.path.join(CSRC, "lmhead.cu")
 
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = [*ARCH_FLAGS, "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC"]
@@ -59,6 +61,22 @@ def _run(cmd, verbose=False):
         raise RuntimeError(" ".join(cmd[:1]) + " failed:\n" + proc.stdout + proc.stderr)
     if verbose:
         sys.stderr.write(proc.stderr)
+    return proc.stderr
+
+
+def check_head_registers(report: str) -> None:
+    """Refuses a head kernel that the compiler did not give the registers its warps share out
+    (Shape::REGS in lmhead_kernel.cuh): it would wait for registers it does not have, and
+    the library would refuse to launch it. `report`: what ptxas -v said."""
+    found = re.findall(r"Compiling entry function '\w*lmhead_kernelILj(\d+)ELi(\d)E\w*'.*?Used (\d+) registers", report,
+                       re.S)
+    if len(found) != 9:
+        raise RuntimeError(f"the compiler reported {len(found)} of the LM head's 9 kernels")
+    for tokens, fmt, used in found:
+        want = 80 if tokens == "64" and fmt != "0" else 64
+        if int(used) != want:
+            raise RuntimeError(f"lmhead_kernel<{tokens}, {fmt}> was compiled for {used} registers a thread instead of {want} "
+                               "(another compiler, or flags in LILY_NVCC_EXTRA?): its shares have to be cut anew")
 
 
 def _calls_command():
@@ -92,9 +110,16 @@ def build(force: bool = False, verbose: bool = False) -> str:
         obj = os.path.join(OBJ, os.path.basename(src) + ".o")
         objects.append(obj)
         if force or _older(obj, max(headers, os.path.getmtime(src))):
-            jobs.append([nvcc, *NVCC_FLAGS, *extra, "-I", INCLUDE, "-c", "-o", obj, src])
+            report = ["-Xptxas", "-v"] if src == HEAD_SOURCE and not verbose else []
+            jobs.append([nvcc, *NVCC_FLAGS, *extra, *report, "-I", INCLUDE, "-c", "-o", obj, src])
     with ThreadPoolExecutor(max_workers=max(1, len(jobs))) as pool:
-        list(pool.map(lambda cmd: _run(cmd, verbose), jobs))
+        for cmd, said in zip(jobs, pool.map(lambda cmd: _run(cmd, verbose), jobs)):
+            if cmd[-1] == HEAD_SOURCE:
+                try:
+                    check_head_registers(said)
+                except RuntimeError:
+                    os.unlink(cmd[-2])
+                    raise
     _run([nvcc, *ARCH_FLAGS, "-shared", "-Xcompiler", "-fPIC", "-Xlinker", "-soname=" + os.path.basename(LIB), "-o", LIB,
           *objects])
     if force or _older(CALLS, max(headers, os.path.getmtime(CALLS_SOURCE))):

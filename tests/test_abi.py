@@ -137,3 +137,27 @@ def test_a_copied_package_is_on_its_own(lily, tmp_path):
     alone = run()
     assert eval(alone.stdout.splitlines()[0]) == [str(copy / "liblily_sampler.so")]
     assert alone.stdout.splitlines()[1] == "True" and "RuntimeWarning" in alone.stderr
+
+
+def test_the_build_refuses_a_head_of_other_registers(lily):
+    import importlib
+
+    import pytest
+
+    build = importlib.import_module("lily_b200.build")
+
+    def report(change=None):
+        lines = []
+        for tokens in (16, 32, 64):
+            for fmt in (0, 1, 2):
+                used = 80 if tokens == 64 and fmt else 64
+                lines += [f"ptxas info    : Compiling entry function '_ZN9lily_head13lmhead_kernelILj{tokens}ELi{fmt}EEEvNS_4ArgsE'"
+                          " for 'sm_100a'", "    0 bytes stack frame, 0 bytes spill stores",
+                          f"ptxas info    : Used {change if change and (tokens, fmt) == (64, 0) else used} registers, 3 barriers"]
+        return "\n".join(lines)
+
+    build.check_head_registers(report())
+    with pytest.raises(RuntimeError, match="72 registers"):
+        build.check_head_registers(report(72))
+    with pytest.raises(RuntimeError, match="0 of"):
+        build.check_head_registers("")
