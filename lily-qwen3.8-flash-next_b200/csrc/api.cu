@@ -80,10 +80,10 @@ struct lily_sampler {
     std::vector<char> shard_bytes;
     float *lm_logits = nullptr;  // LILY_FLAG_LMHEAD: F32 [64, lm_ld]
     uint64_t lm_ld = 0;
-    // The LM head's workspaces: the hidden states' images, the sums of tiles that two
-    // blocks work on (for lm_tokens padded tokens) and the flags that say they are there.
-    char *lm_prepared = nullptr;
-    float *lm_part = nullptr;
+    // The LM head's workspaces: the hidden states' images (for lm_tokens padded tokens) and
+    // the flags of sums handed on. lm_more: those of calls of more tokens than max_rows or of
+    // more than CHUNK_K columns, made by the first of them.
+    char *lm_prepared = nullptr, *lm_more = nullptr;
     uint32_t *lm_flags = nullptr;
     uint32_t lm_tokens = 0;
 };
@@ -626,9 +626,8 @@ int32_t lily_sampler_create(int32_t device, uint32_t vocab, uint32_t max_rows,
         cleared = at;
         place(h->part, (size_t)max_rows * lily::CAP * sizeof(uint2));
         place(h->part_n, (size_t)max_rows * lily::MAX_SLICES * 4);
-        // (Here, and not by the first head call: that took 1.2 to 2.3 ms longer for it.)
-        place(h->lm_prepared, lily_head::prepared_bytes());
-        place(h->lm_part, lily_head::part_bytes(h->lm_tokens, (uint32_t)h->sm_count));
+        // (Here, and not by the first head call: an allocation took that 1.2 to 2.3 ms.)
+        place(h->lm_prepared, lily_head::prepared_bytes(h->lm_tokens));
         place(h->lm_flags, lily_head::flag_bytes((uint32_t)h->sm_count));
         if (flags & LILY_FLAG_LMHEAD) {
             place(h->lm_logits, (size_t)lily_head::TOK * h->lm_ld * sizeof(float));
@@ -661,6 +660,7 @@ void lily_sampler_destroy(lily_sampler_t *h) {
     DeviceGuard guard(h->device);
     cudaDeviceSynchronize();
     cudaFree(h->arena);
+    cudaFree(h->lm_more);
     if (h->h_status) {
         cudaFreeHost(h->h_status);
     }
@@ -1168,11 +1168,20 @@ int32_t lmhead_launch(lily_sampler *h, cudaStream_t stream, const lily_lmhead_t 
     a.rows = head->rows;
     a.out = out;
     a.ldo = out_ld;
-    a.prep = lily_head::prepared_at(h->lm_prepared);
-    a.part = h->lm_part;
+    const uint32_t padded = lily_head::padded_tokens(tokens);
+    const size_t prepared = (lily_head::prepared_bytes(lily_head::TOK) + 255u) & ~size_t(255);
+    if ((padded > h->lm_tokens || head->hidden > lily_head::CHUNK_K) && h->lm_more == nullptr) {
+        // (The stream may be under capture: the allocation is no part of the graph.)
+        char *at = nullptr;
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        CU(h, cudaThreadExchangeStreamCaptureMode(&mode));
+        const cudaError_t e = cudaMalloc(&at, prepared + lily_head::part_bytes((uint32_t)h->sm_count));
+        CU(h, cudaThreadExchangeStreamCaptureMode(&mode));
+        CU(h, e);
+        h->lm_more = at;
+    }
+    a.prep = lily_head::prepared_at(padded > h->lm_tokens ? h->lm_more : h->lm_prepared, padded);
     a.flags = h->lm_flags;
-    // (The sums' place is laid out for the handle's rows; a call of more gives every block whole tiles.)
-    a.whole_tiles = lily_head::padded_tokens(tokens) > h->lm_tokens ? 1u : 0u;
     a.status_word = h->status_word;
     a.wait_ns = h->wait_ns;
     a.lost_stage = h->lost_stage;
@@ -1184,6 +1193,7 @@ int32_t lmhead_launch(lily_sampler *h, cudaStream_t stream, const lily_lmhead_t 
         a.scales = static_cast<const __nv_bfloat16 *>(head->scales_bf16) + k0 / lily_head::GROUP_K;
         a.biases = affine ? static_cast<const __nv_bfloat16 *>(head->biases_bf16) + k0 / lily_head::GROUP_K : nullptr;
         a.accumulate = k0 != 0u ? 1u : 0u;
+        a.part = k0 != 0u ? reinterpret_cast<float *>(h->lm_more + prepared) : nullptr;
         CU(h, lily_head::launch_prepare(a.prep, static_cast<const __nv_bfloat16 *>(hidden) + k0, hidden_ld, tokens,
                                         a.groups, format, a.flags, (uint32_t)h->sm_count, stream));
         CU(h, lily_head::launch_head(a, format, (uint32_t)h->sm_count, stream));

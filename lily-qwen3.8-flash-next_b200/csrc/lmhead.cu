@@ -5,16 +5,16 @@
 
 namespace lily_head {
 
-Prepared prepared_at(void *base) {
+Prepared prepared_at(void *base, uint32_t padded) {
     Prepared p;
     uint8_t *at = static_cast<uint8_t *>(base);
     for (int i = 0; i < 2; ++i) {
         p.image[i] = reinterpret_cast<uint4 *>(at);
-        at += (size_t)TOK * CHUNK_K * 2u;
+        at += (size_t)padded * CHUNK_K * 2u;
     }
     for (int i = 0; i < 2; ++i) {
         p.sums[i] = reinterpret_cast<float *>(at);
-        at += (size_t)TOK * (CHUNK_K / GROUP_K) * 4u;
+        at += (size_t)padded * (CHUNK_K / GROUP_K) * 4u;
     }
     p.unscale = reinterpret_cast<float *>(at);
     p.inexact = reinterpret_cast<uint32_t *>(at + TOK * 4u);

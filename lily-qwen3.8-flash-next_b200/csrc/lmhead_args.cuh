@@ -45,12 +45,11 @@ struct Args {
     uint64_t ldo;
     Prepared prep;
     // Every thread block takes an even share of the tiles, cut where it ends. The sums of a
-    // tile that a block begins and the next one ends go through `part` ([grid][padded
-    // tokens][TILE_ROWS]) and are there once `flags` ([grid][EPILOGUE_WARPS], cleared by
-    // launch_prepare) says so. whole_tiles: no tile is cut, neither is used.
+    // tile that a block begins and the next one ends go through `out`, or through `part`
+    // ([grid][padded tokens][TILE_ROWS]; launches that add to `out`), and are there once
+    // `flags` ([grid][EPILOGUE_WARPS], cleared by launch_prepare) says so.
     float *part;
     uint32_t *flags;
-    uint32_t whole_tiles;
     uint32_t *status_word;
     uint64_t wait_ns;           // the bound of every wait inside the kernel
     // Test hook: block 0 does not ask for the weights of this stage (~0: none),
@@ -60,17 +59,15 @@ struct Args {
 
 __host__ __device__ inline uint32_t padded_tokens(uint32_t tokens) { return tokens <= 16u ? 16u : tokens <= 32u ? 32u : 64u; }
 
-// Sizes of the workspaces a handle keeps.
-inline size_t prepared_bytes() {
-    return 2u * (size_t)TOK * CHUNK_K * 2u + 2u * (size_t)TOK * (CHUNK_K / GROUP_K) * 4u + 2u * TOK * 4u;
+// Sizes of the workspaces: the hidden states' images, flags, and `part`.
+inline size_t prepared_bytes(uint32_t padded) {
+    return 2u * (size_t)padded * CHUNK_K * 2u + 2u * (size_t)padded * (CHUNK_K / GROUP_K) * 4u + 2u * TOK * 4u;
 }
-inline size_t part_bytes(uint32_t tokens, uint32_t sms) {
-    return (size_t)sms * padded_tokens(tokens) * TILE_ROWS * sizeof(float);
-}
+inline size_t part_bytes(uint32_t sms) { return (size_t)sms * TOK * TILE_ROWS * sizeof(float); }
 
 inline size_t flag_bytes(uint32_t sms) { return (size_t)sms * EPILOGUE_WARPS * sizeof(uint32_t); }
 
-Prepared prepared_at(void *base);
+Prepared prepared_at(void *base, uint32_t padded);
 
 // The two launches of a head (or of 8192 columns of one): the hidden states' images,
 // then the products. hidden: bf16 [tokens, hidden_ld], from the launch's first column on.

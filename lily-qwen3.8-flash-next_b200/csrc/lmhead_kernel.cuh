@@ -485,7 +485,7 @@ __global__ void __launch_bounds__(Shape<N, FMT>::THREADS, 1) lmhead_kernel(const
     // every block takes one whole tile (units of `grain`).
     const uint32_t per_tile = a.groups / BLOCK_GROUPS;
     const uint32_t n_tiles = (a.rows + TILE_ROWS - 1u) / TILE_ROWS;
-    const uint32_t grain = a.whole_tiles || n_tiles <= gridDim.x ? per_tile : 1u, shares = n_tiles * per_tile / grain;
+    const uint32_t grain = n_tiles <= gridDim.x ? per_tile : 1u, shares = n_tiles * per_tile / grain;
     auto share_begin = [&](uint32_t b) { return (uint32_t)((uint64_t)b * shares / gridDim.x) * grain; };
     const uint32_t lo = share_begin(blockIdx.x), hi = share_begin(blockIdx.x + 1u), n_blocks = hi - lo;
     const uint32_t begun = hi % per_tile;                                  // units of the tile it begins
@@ -818,8 +818,12 @@ __global__ void __launch_bounds__(Shape<N, FMT>::THREADS, 1) lmhead_kernel(const
                 }
             }
         };
-        // The sums of a tile's beginning, left for the next thread block's warp of the same rows.
-        auto part_of = [&](uint32_t block) { return a.part + (size_t)block * N * TILE_ROWS + trow; };
+        // The sums of a tile's beginning, left for the next thread block's warp of the same rows: where
+        // the tile's logits will be, unless something to add to lies there.
+        const uint64_t part_ld = a.part ? (uint64_t)TILE_ROWS : a.ldo;
+        auto part_of = [&](uint32_t block, uint32_t row) {
+            return a.part ? a.part + (size_t)block * N * TILE_ROWS + trow : a.out + row;
+        };
         auto flag_of = [&](uint32_t block) { return a.flags + block * S::EPI_WARPS + e; };
         uint32_t tile = unit_at(0) / per_tile, blk = unit_at(0) % per_tile, q = 0;
         for (uint32_t n = 0; n < n_blocks; ++n) {
@@ -845,11 +849,13 @@ __global__ void __launch_bounds__(Shape<N, FMT>::THREADS, 1) lmhead_kernel(const
                     }
                     there = __all_sync(FULL, there);
                 }
-                const float *theirs = part_of(blockIdx.x - 1u);
+                if (row < a.rows) {
+                    const float *theirs = part_of(blockIdx.x - 1u, row);
 #pragma unroll
-                for (uint32_t m = 0; m < P; ++m) {
-                    acc[m] = pack2(__float_as_uint(__ldcg(theirs + (2u * m) * TILE_ROWS)),
-                                   __float_as_uint(__ldcg(theirs + (2u * m + 1u) * TILE_ROWS)));
+                    for (uint32_t m = 0; m < P; ++m) {
+                        acc[m] = pack2(2u * m < a.tokens ? __float_as_uint(__ldcg(theirs + (2u * m) * part_ld)) : 0u,
+                                       2u * m + 1u < a.tokens ? __float_as_uint(__ldcg(theirs + (2u * m + 1u) * part_ld)) : 0u);
+                    }
                 }
             }
 #pragma unroll
@@ -902,13 +908,19 @@ __global__ void __launch_bounds__(Shape<N, FMT>::THREADS, 1) lmhead_kernel(const
             if (blk == per_tile) {
                 write_out(row);
             } else {
-                float *mine = part_of(blockIdx.x);
+                if (row < a.rows) {
+                    float *mine = part_of(blockIdx.x, row);
 #pragma unroll
-                for (uint32_t m = 0; m < P; ++m) {
-                    float v0, v1;
-                    unpack2(acc[m], v0, v1);
-                    __stcg(mine + (2u * m) * TILE_ROWS, v0);
-                    __stcg(mine + (2u * m + 1u) * TILE_ROWS, v1);
+                    for (uint32_t m = 0; m < P; ++m) {
+                        float v0, v1;
+                        unpack2(acc[m], v0, v1);
+                        if (2u * m < a.tokens) {
+                            __stcg(mine + (2u * m) * part_ld, v0);
+                        }
+                        if (2u * m + 1u < a.tokens) {
+                            __stcg(mine + (2u * m + 1u) * part_ld, v1);
+                        }
+                    }
                 }
                 __syncwarp();
                 if (lane == 0) {

@@ -50,3 +50,13 @@ def test_head_at_the_edges_of_its_shapes(cuda, lily, tokens, hidden, rows, max_r
     assert np.isfinite(got).all()
     assert np.all(np.abs(got - exact) <= bound), float((np.abs(got - exact) / bound).max())
     scratch.close()
+
+
+def test_a_handle_of_few_rows_is_small(cuda, lily):
+    # (The head's workspaces follow max_rows; those of calls of more tokens are made by such calls.)
+    handles = [lily.SamplerScratch(151_936, max_rows=1, max_history=0)]
+    before = cuda.cuda.mem_get_info()[0]
+    handles += [lily.SamplerScratch(151_936, max_rows=1, max_history=0) for _ in range(32)]
+    assert before - cuda.cuda.mem_get_info()[0] <= 32 << 20
+    for h in handles:
+        h.close()
