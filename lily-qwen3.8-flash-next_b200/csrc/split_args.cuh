@@ -108,7 +108,6 @@ struct alignas(16) SplitSmem {
     uint32_t verdict[2];             // what the waiting warps of the first block learn
     uint32_t bound_key;
     uint32_t record_key;             // a shard's largest adjusted logit
-    uint32_t n_slots;                // candidates whose ids are counted in the history
     float least;                     // what an adjusted logit has to reach
     uint32_t late;                   // a wait of this block ran out: others may still store into it
 };

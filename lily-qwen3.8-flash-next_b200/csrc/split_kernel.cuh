@@ -747,7 +747,6 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         ss->n_hits = 0;
         ss->n_listed = 0;
         ss->n_sent = 0;
-        ss->n_slots = 0;
         ss->n_live = 0;
         ss->hard = 0;
         ss->bound_key = 0;
@@ -987,23 +986,26 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
     const bool marked = hist_len + extra_len != 0u;
     const bool counted = marked && need_counts;  // (a list whose multiplicities matter)
     const bool raises = (in.flags & ROW_RAISES) != 0u;
-    const bool count_later = counted && !raises;  // (... but only the candidates')
     const bool emitted = raises && (table_mode || marked);
     // A row that keeps many takes its bound from at most SPL_MAX_BLOCKS * SPL_NT maxima: one of
     // every thread, or, of a short row over four or eight blocks, those of `groups` parts of a
     // thread's logits. (One maximum a thread, 3 x 8192 bf16, 1024 kept: not enough of them, the
     // general code's 42 us. With fewer blocks their ranking takes longer than that code: 55.)
     const uint32_t most_pieces = (pieces + blocks - 1u) >> log_blocks;
-    // (Of the threads that take part: half of them where the other half has nothing, or, of
-    // eight blocks, one warp of it a piece: without its logits the bound is somewhat lower.)
-    const uint32_t log_live = most_pieces <= (log_blocks == 3u ? 5u : SPL_MIN_TILES) ? SPL_LOG_NT - 1u : SPL_LOG_NT;
-    const uint32_t groups = BPS == 1 && log_blocks >= 2u && most_pieces <= SPL_WARPS * SPL_U
-                                ? SPL_MAX_BLOCKS * SPL_NT >> (log_live + log_blocks) : 1u;
-    const bool wide_fits = min(vocab / PER, blocks << log_live) * min(groups, PER) * 8u >= 9u * k &&
-                           (groups == 1u || most_pieces * 32u <= SPL_HITS || k * 5u <= blocks * SPL_HITS * 3u);
+    uint32_t log_live = SPL_LOG_NT, groups = 1u;
+    bool wide_fits = true;
+    if (wide) {
+        // (Of the threads that take part: half of them where the other half has nothing, or, of
+        // eight blocks, one warp of it a piece: without its logits the bound is somewhat lower.)
+        log_live = most_pieces <= (log_blocks == 3u ? 5u : SPL_MIN_TILES) ? SPL_LOG_NT - 1u : SPL_LOG_NT;
+        if (BPS == 1 && log_blocks >= 2u && most_pieces <= SPL_WARPS * SPL_U) {
+            groups = SPL_MAX_BLOCKS * SPL_NT >> (log_live + log_blocks);
+        }
+        wide_fits = min(vocab / PER, blocks << log_live) * min(groups, PER) * 8u >= 9u * k &&
+                    (groups == 1u || most_pieces * 32u <= SPL_HITS || k * 5u <= blocks * SPL_HITS * 3u);
+    }
     // Decided alike by every block of the cluster: rows that end here.
     const bool general = n_sp > SP_SMEM || (raises && marked && mark_mode == MARK_BITS) ||
-                         (raises && counted && hist_len + extra_len > MARK_MAX) ||
                          (n_sp != 0u && mark_mode == MARK_BITS) ||
                          (list_mode && need_counts && mark_mode != MARK_COUNTS) ||
                          (wide && (row < a.spec.n_spec || !wide_fits));
@@ -1196,9 +1198,12 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         if (t < 4u) {
             sm->sp_ids[min(n_sp, SP_SMEM) + t] = NONE;
         }
-        // (Any thread may write the same mark: how often an id occurs is counted later, and
-        // only for the candidates. Counting every id here took 6 us for 8192 ids: real
-        // histories repeat a few ids very often, and all in one block's share.)
+        // Any thread may write the same mark; where a frequency penalty counts, every id is an add
+        // of its own: 1 to 2.6 us for 16000 ids of a skewed history, whose most frequent id is a
+        // fifth of it. (Marks first, and the candidates' ids counted in a second pass over the list:
+        // 6 us, 4 x 151936 bf16 with 15953 ids 18.4 us against 13.9 here; and the bound had to leave out
+        // what was not counted yet, so that rows which had emitted most of a short vocabulary went
+        // to the general code: 6 x 8448 with as many ids, 1024 kept, 76 to 136 us against 26.)
         auto mark_all = [&](auto mark) {
             each_four([&](const uint4 &x) {
                 uint32_t at;
@@ -1219,9 +1224,31 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         if (!marked) {
         } else if (mark_mode == MARK_BYTES) {
             mark_all([&](uint32_t at) { mark8[at] = 1; });
-        } else if (mark_mode == MARK_COUNTS && counted && raises) {
-            // (At most MARK_MAX ids: no count reaches into the flags or its neighbour.)
-            mark_all([&](uint32_t at) { atomicAdd(marks + (at >> 1), 1u << ((at & 1u) * 16u)); });
+        } else if (mark_mode == MARK_COUNTS && counted) {
+            auto add = [&](uint32_t at) { atomicAdd(marks + (at >> 1), 1u << ((at & 1u) * 16u)); };
+            // No count may reach into the flags or its neighbour (one id so often: the general code).
+            if (hist_len + extra_len <= 0xFFFFu) {
+                mark_all(add);
+                if (hist_len + extra_len > MARK_MAX) {
+                    constexpr uint32_t FLAGS = (HALF_LISTED | HALF_CLAIMED) * 0x10001u;
+                    asm volatile("bar.sync 6, %0;" ::"n"(SPL_NT) : "memory");
+                    for (uint32_t w = t; w < ca.mark_words / 4u; w += SPL_NT) {
+                        const uint4 m = reinterpret_cast<const uint4 *>(marks)[w];
+                        if (((m.x | m.y | m.z | m.w) & FLAGS) != 0u) {
+                            ss->hard = 1;
+                        }
+                    }
+                }
+            } else {
+                // (A look first, with room for all threads that looked at the same time.)
+                mark_all([&](uint32_t at) {
+                    if (static_cast<volatile uint16_t *>(mark16)[at] < MARK_MAX - 4u * SPL_NT) {
+                        add(at);
+                    } else {
+                        ss->hard = 1;
+                    }
+                });
+            }
         } else if (mark_mode == MARK_COUNTS) {
             mark_all([&](uint32_t at) { mark16[at] = 1; });
         } else {
@@ -1282,30 +1309,6 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
             asm volatile("bar.sync 4, %0;" ::"n"(NT) : "memory");
             emitted_candidates<T>(sm, ss, a, row_ptr, log_blocks, marks, mark_mode, r);
             asm volatile("bar.arrive 5, %0;" ::"n"(NT) : "memory");
-        }
-        if (count_later) {
-            asm volatile("bar.sync 4, %0;" ::"n"(NT) : "memory");
-            if (ss->n_slots != 0u) {
-                // The candidates' marks name their counters.
-                each_four([&](const uint4 &x) {
-                    uint32_t at, m[4] = {0, 0, 0, 0};
-                    m[0] = place_of(x.x, at) == rank ? mark16[at] & MARK_MAX : 0u;
-                    m[1] = place_of(x.y, at) == rank ? mark16[at] & MARK_MAX : 0u;
-                    m[2] = place_of(x.z, at) == rank ? mark16[at] & MARK_MAX : 0u;
-                    m[3] = place_of(x.w, at) == rank ? mark16[at] & MARK_MAX : 0u;
-                    // (Adding equal ids of a warp up first, with a match instruction, was slower: one
-                    // greedy row with 16000 ids, a good part of them the same, 18.4 -> 20.2 us.)
-                    if (max(max(m[0], m[1]), max(m[2], m[3])) >= 2u) {
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            if (m[e] >= 2u) {
-                                atomicAdd(&sm->thist[m[e] - 2u], 1u);
-                            }
-                        }
-                    }
-                });
-                asm volatile("bar.arrive 5, %0;" ::"n"(NT) : "memory");
-            }
         }
         marker_ends();
         return;
@@ -1470,8 +1473,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
     auto adjusted = [&](float x, uint32_t j, uint32_t e) -> uint32_t {  // (of piece j of the block)
         if (use_pen || n_sp != 0u) {
             const uint32_t m = mark_of(id_at(j, e));
-            // (Not yet counted: left out, which can only lower the bound.)
-            x = (m & LISTED) || (count_later && m != 0u) ? neg_inf() : penalised(x, m);
+            x = (m & LISTED) ? neg_inf() : penalised(x, m);  // (a listed id: left out, which can only lower the bound)
         }
         return key_of(__fadd_rn(x, 0.0f));
     };
@@ -1782,27 +1784,6 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
             }
         }
     };
-    uint32_t n_slots = 0;
-    if (count_later) {
-        // The markers count the candidates' ids in the history: a counter each.
-        each_logit([&](uint32_t id, float, bool listed) {
-            const uint32_t m = mark_of(id);
-            if ((m & ~LISTED) != 0u && (listed || !(m & LISTED))) {
-                const uint32_t to = atomicAdd(&ss->n_slots, 1u);
-                if (to < TH_BINS) {
-                    uint32_t at;
-                    place_of(id, at);
-                    sm->thist[to] = 0;
-                    mark16[at] = (uint16_t)((mark16[at] & HALF_LISTED) | (to + 2u));
-                }
-            }
-        });
-        asm volatile("bar.sync 1, %0;\n bar.arrive 4, %1;" ::"n"(SPL_NT), "n"(NT) : "memory");
-        n_slots = ss->n_slots;
-        if (n_slots != 0u) {
-            asm volatile("bar.sync 5, %0;" ::"n"(NT) : "memory");
-        }
-    }
     each_logit([&](uint32_t id, float x, bool listed) {
         if (use_pen || n_sp != 0u) {
             uint32_t m = mark_of(id);
@@ -1812,9 +1793,6 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
             m &= ~LISTED;
             if (raises && m != 0u && !listed) {
                 return;  // (likewise)
-            }
-            if (count_later && m != 0u) {
-                m = m >= 2u ? sm->thist[m - 2u] : 0u;
             }
             x = penalised(x, m);
         }
@@ -1838,7 +1816,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
     });
     spl_sync();
     const uint32_t sent = min(ss->n_sent, most);
-    const uint32_t hard = (ss->hard != 0u || n_hits > SPL_HITS || ss->n_sent > most || n_slots > TH_BINS) ? 1u : 0u;
+    const uint32_t hard = (ss->hard != 0u || n_hits > SPL_HITS || ss->n_sent > most) ? 1u : 0u;
     const bool counts_draw = use_pen && table_mode;
     if (wide) {
         LILY_STAMP(PH_LOCAL_SELECT);

@@ -206,6 +206,37 @@ def test_penalties_that_raise_a_logit(cuda, lily, W, rows, vocab, bf16):
         check(cuda, lily, W, b, vocab, f"B={rows} V={vocab} {kw} uniform")
 
 
+@pytest.mark.parametrize("rows,vocab,bf16", [(1, 1024, True), (6, 8448, True), (5, 16_001, False), (40, 8200, False)])
+def test_lists_that_cover_the_vocabulary(cuda, lily, W, rows, vocab, bf16):
+    # Most ids have been emitted, some of them often: their multiplicities decide the bound.
+    rng = np.random.default_rng([rows, vocab])
+    for k, kw in ((20, dict(frequency=0.2, presence=0.5)), (0, dict(frequency=0.2)), (1, dict(frequency=0.7)),
+                  (500, dict(frequency=0.05, n_bias=6, n_ban=2))):
+        for n in (vocab // 7, 15_953, 32_000):
+            b = make_batch(W, rng, rows, vocab, k, bf16, kind="zipf", history=n, **kw)
+            b.history[::2] = rng.integers(0, vocab, b.history[::2].shape)  # (the other rows': mostly a few ids)
+            b.history_len[:] = n
+            check(cuda, lily, W, b, vocab, f"B={rows} V={vocab} k={k} n={n}")
+
+
+@pytest.mark.parametrize("same,length", [(16_383, 17_000), (16_384, 17_000), (33_000, 65_535), (65_535, 65_535),
+                                         (15_358, 70_000), (15_359, 70_000), (66_000, 70_000)])
+def test_one_id_as_often_as_a_mark_counts(cuda, lily, W, same, length):
+    # (A half word less two flags; lists beyond 65535 ids are looked at one by one.)
+    rng = np.random.default_rng([same, length])
+    for frequency in (0.0001, -0.0001):
+        b = make_batch(W, rng, 2, 9_001, 40, True, kind="zipf", history=length, frequency=frequency)
+        top = b.logits_f32().argmax(1)
+        for r in range(2):
+            b.history[r] = rng.integers(0, 9_000, length)
+            b.history[r] += b.history[r] >= top[r]  # (any id but the row's best)
+            b.history[r, rng.choice(length, same, replace=False)] = top[r]
+        b.history_len[:] = length
+        s = lily.SamplerScratch(9_001, max_rows=2, max_history=70_000)
+        assert_parity(b, run_batch(cuda, lily, s, b), oracle_rows(b), label=f"{same} times one id of {length}")
+        s.close()
+
+
 def test_more_ids_than_a_raising_count_holds(cuda, lily, W):
     # Lists of mostly one id, around the most that a half word counts: the longer one is the
     # general code's.
