@@ -216,14 +216,12 @@ bool stream_route(const lily::KArgs &a, uint32_t rows, uint32_t dtype) {
 template <typename T, bool VEC>
 int32_t launch_one(lily_sampler *h, cudaStream_t stream_, const lily::KArgs &a, uint32_t rows,
                    size_t smem) {
-    // More rows than the row kernel takes at once (and at least 16: fewer rows with
-    // lists or wide cuts are better off cut into slices), aligned logits, long rows
-    // and nothing special about the call: the kernel of one block per row (which runs
-    // the general code itself, on the whole row, for the rows it does not take).
-    // Below a block slot's worth of rows a block streams alone, and gets a deeper
-    // ring. A vocabulary shard's candidate launch goes the same way and ends in the
-    // rows' records. (Short rows, unaligned logits, speculative calls and the merge
-    // of shards: the general kernel, rows cut into slices.)
+    // What the row kernel leaves (split_plan): aligned long rows, more of them than SMs, go to
+    // the kernel of one block per row, which runs the general code itself, on the whole row,
+    // for the rows it does not take; a vocabulary shard's candidate launch goes the same way
+    // and ends in the rows' records. (16 rows and more of vocabularies whose marks do not fit a
+    // block of the row kernel, beyond 700000, too.) Everything else, rows shorter than the row
+    // kernel's least and the merge of shards among it: the general kernel, rows cut into slices.
     const bool stream = VEC && stream_route(a, rows, sizeof(T) == 4 ? LILY_F32 : LILY_BF16);
     if (stream) {
         lily::KArgs whole = a;
@@ -236,16 +234,6 @@ int32_t launch_one(lily_sampler *h, cudaStream_t stream_, const lily::KArgs &a, 
                 return st;
             }
             return launch_serialised(h, stream_, kernel, dim3(rows, 1, 1), smem1, whole);
-        }
-        // A block per SM at most: the deep ring, if the SM's shared memory holds it.
-        const size_t deep = ((smem1 + 15u) & ~size_t(15)) + lily::StreamDepth<7>::EXTRA_BYTES;
-        if (deep <= (size_t)h->max_smem) {
-            auto kernel = lily::stream_rows_kernel<T, 7>;
-            const int32_t st = raise_smem_limit(h, kernel, 1u << (sizeof(T) == 4 ? 10 : 11));
-            if (st != LILY_OK) {
-                return st;
-            }
-            return launch_serialised(h, stream_, kernel, dim3(rows, 1, 1), deep, whole);
         }
         auto kernel = lily::stream_rows_kernel<T, 3>;
         const int32_t st = raise_smem_limit(h, kernel, 1u << (sizeof(T) == 4 ? 6 : 7));

@@ -32,24 +32,14 @@
 
 namespace lily {
 
-constexpr uint32_t STREAM_MIN_ROUNDS = 8;  // launches with shorter rows use sample_rows_kernel
+constexpr uint32_t STREAM_MIN_ROUNDS = 8;  // shorter rows go to the row kernel, or in slices
 constexpr uint32_t STREAM_K_MAX = 64;      // finalize_warp holds two candidates per lane
 // AHEAD (template argument of the kernel): rounds of the ring in flight beyond the
 // one being read. With a block slot's worth of rows two measured faster than
 // three (33.4 against 34.0 us per 256-row launch; asking L2 for further rounds
-// ahead of the ring was slower still: the stream is not short of requests). With
-// fewer rows than SMs a block streams alone against the latency of its own
-// requests: it has the SM's shared memory to itself, and takes a ring of eight
-// stages with seven rounds in flight (112 KB per block) and four 16-byte loads of
-// history ids per thread and round instead of two.
-template <uint32_t AHEAD>
-struct StreamDepth {
-    static_assert(AHEAD == 2u || AHEAD == 3u || AHEAD == 7u, "a ring of four stages, or of eight");
-    static constexpr uint32_t STAGES = AHEAD <= 3u ? 4u : 8u;     // of the ring
-    static constexpr uint32_t HQ = AHEAD <= 3u ? 2u : 4u;         // 16-byte history loads per thread and round
-    static constexpr uint32_t BLOCKS = AHEAD <= 3u ? 2u : 1u;     // per SM
-    static constexpr uint32_t EXTRA_BYTES = (STAGES - 4u) * NT * FRAG_BYTES;  // stages beyond the four shared ones
-};
+// ahead of the ring was slower still: the stream is not short of requests).
+constexpr uint32_t STREAM_STAGES = 4;      // of the ring
+constexpr uint32_t STREAM_HQ = 2;          // 16-byte loads of history ids per thread and round
 
 __device__ __forceinline__ void mbar_init(unsigned long long *bar, uint32_t count) {
     const uint32_t at = (uint32_t)__cvta_generic_to_shared(bar);
@@ -257,8 +247,9 @@ __device__ __forceinline__ uint32_t small_select(SmemFixed *sm, uint32_t n, uint
 }
 
 template <typename T, uint32_t AHEAD>
-__global__ void __launch_bounds__(NT, StreamDepth<AHEAD>::BLOCKS) stream_rows_kernel(const __grid_constant__ KArgs a) {
-    constexpr uint32_t NS = StreamDepth<AHEAD>::STAGES, HQ = StreamDepth<AHEAD>::HQ;
+__global__ void __launch_bounds__(NT, 2) stream_rows_kernel(const __grid_constant__ KArgs a) {
+    static_assert(AHEAD < STREAM_STAGES, "rounds in flight");
+    constexpr uint32_t NS = STREAM_STAGES, HQ = STREAM_HQ;
     extern __shared__ uint4 smem_raw[];
     SmemFixed *sm = reinterpret_cast<SmemFixed *>(smem_raw);
     uint4 *ring = reinterpret_cast<uint4 *>(sm + 1);
@@ -324,18 +315,10 @@ __global__ void __launch_bounds__(NT, StreamDepth<AHEAD>::BLOCKS) stream_rows_ke
     // The ring: stages 0 and 1 behind the fixed block, stages 2 and 3 in the
     // (here unused) candidate arrays key and id, one round each.
     static_assert(CAP * 4u == NT * FRAG_BYTES && STAGES == 2, "key[] and id[] are one round each");
-    // (Stages 4 to 7 of the deep ring lie behind the seen bits, where the general
-    // row code, should the row go to it, has nothing.)
+    static_assert(NS == 4u, "");
     const uint32_t slot_a = (uint32_t)__cvta_generic_to_shared(ring) + tid * FRAG_BYTES;
     const uint32_t slot_b = (uint32_t)__cvta_generic_to_shared(sm->key) + tid * FRAG_BYTES;
-    const uint32_t slot_c = (uint32_t)__cvta_generic_to_shared(seen) +
-                            ((((a.vocab + 255u) & ~255u) + 31u) / 32u + 8u) * 4u + tid * FRAG_BYTES;
-    auto stage_at = [&](uint32_t st) -> uint32_t {
-        if (NS == 4u) {
-            return ((st & 2u) ? slot_b : slot_a) + (st & 1u) * ROUND_BYTES;
-        }
-        return (st < 2u ? slot_a : st < 4u ? slot_b - 2u * ROUND_BYTES : slot_c - 4u * ROUND_BYTES) + st * ROUND_BYTES;
-    };
+    auto stage_at = [&](uint32_t st) -> uint32_t { return ((st & 2u) ? slot_b : slot_a) + (st & 1u) * ROUND_BYTES; };
 #pragma unroll
     for (uint32_t j = 0; j < AHEAD; ++j) {
         lean_copy_round(stage_at(j), src0 + j * ROUND_BYTES);
