@@ -8,7 +8,7 @@
 
 namespace lily {
 
-constexpr uint32_t SPL_NT = 256;         // threads at work; the other half of the block waits for a row of the general code
+constexpr uint32_t SPL_NT = 256;         // threads that read the logits; the block's other half marks the row's history
 constexpr uint32_t SPL_WARPS = SPL_NT / 32;
 constexpr uint32_t SPL_LOG_NT = 8;
 static_assert(1u << SPL_LOG_NT == SPL_NT, "");
@@ -16,7 +16,7 @@ static_assert(1u << SPL_LOG_NT == SPL_NT, "");
 // as 64 registers a thread hold).
 __host__ __device__ constexpr uint32_t split_u(int bps) { return bps == 1 ? 10u : 6u; }
 constexpr uint32_t SPL_MAX_BLOCKS = 8;   // blocks of a cluster (the portable size)
-constexpr uint32_t SPL_SMALL_K = 64;     // up to here a block's bound is its own; finalize_warp's limit
+constexpr uint32_t SPL_SMALL_K = 64;     // up to here a row's bound comes from the pool and one warp draws (split_finalize)
 constexpr uint32_t SPL_POOL = 256;       // keys in the pool a narrow row's bound is taken from
 constexpr uint32_t SPL_HITS = 512;       // vectors of a block that may reach the bound
 constexpr uint32_t SPL_FLAGGED = 2048;   // buckets that may reach the bound
