@@ -566,7 +566,6 @@ def lmhead_sharded(torch, dist, lily, dev, stream, world, rank, steps):
             "rows_per_s": tokens / (step_ms * 1e-3), "steps": steps,
             "head_kernel_us": head_ms * 1e3, "head_bytes_per_gpu": head_bytes,
             "head_gbs_per_gpu": gbs, "head_frac_of_hbm": gbs / peak, "peak_kind": peak_kind,
-            "head_traffic_1gpu": ncu_traffic("lmhead_kernel_dram_bytes_per_launch"),
             "affine_head_us": affine_ms * 1e3,
             "affine_head_frac_of_hbm": (head_bytes + per * (hidden // 64) * 2) / (affine_ms * 1e-3) / 1e9 / peak,
             "affine4_head_us": None if q4_ms is None else q4_ms * 1e3,
