@@ -92,7 +92,7 @@ cudaError_t launch_for(const Args &a, Format format, uint32_t sms, cudaStream_t 
 //   151936 x 2048, affine 4 bits: 64 tokens 90 us, 32 tokens 160 -> 61, 4 tokens 50
 // (4 bits, 32 tokens, step by step: 80; two groups per hand-over and fewer stages 70; codes
 // as subnormals 61; sums of shared tiles handed on through the logits' place instead of a
-// workspace: + 0.6 at 4 bits and 32 tokens, nothing elsewhere.) At 16 tokens the weights' stream bounds bytes (5.9 TB/s of 6.6
+// workspace: + 0.6 to 1.2 at 4 bits, nothing elsewhere.) At 16 tokens the weights' stream bounds bytes (5.9 TB/s of 6.6
 // measured for a copy); the rest is bound by issue slots (67 % busy before the last step):
 // widening a weight, and one FMA per logit and group.
 cudaError_t launch_head(const Args &a, Format format, uint32_t sms, cudaStream_t stream) {
