@@ -180,8 +180,8 @@ static __device__ __noinline__ uint4 edge_vec(const T *row_ptr, uint32_t vocab, 
 // The draw of a row that keeps more than 64 candidates, sorted in `best`: the
 // softmax weights, the prefix sums in rank order with one rounding per add
 // (tests/unit/kernels/sample.rs:37-46), the cut, the draw. All SPL_NT threads.
-static __device__ __noinline__ void split_finalize_wide(SmemFixed *sm, SplitSmem *ss, const unsigned long long *best,
-                                                       const KArgs &a, uint32_t row, uint32_t n,
+__device__ __forceinline__ void split_finalize_wide(SmemFixed *sm, SplitSmem *ss, const unsigned long long *best,
+                                                    const KArgs &a, uint32_t row, uint32_t n,
                                                  float top_p, float min_p, float u, bool counts_draw, uint32_t slot) {
     const uint32_t tid = threadIdx.x;
     float *p = reinterpret_cast<float *>(sm->tkey), *cum = reinterpret_cast<float *>(sm->tid);
@@ -461,8 +461,8 @@ __device__ __forceinline__ void rank_sums(const float *w, uint32_t n, float &c0,
 // softmax weights, the prefix sums in rank order (tests/unit/kernels/sample.rs:37-46),
 // the cut, the draw (speculative: tests/unit/kernels/sample.rs:264-283, src/kernels/
 // metal/sample.metal:597-658), the outputs. lane i holds ranks i and i + 32.
-static __device__ __noinline__ void split_finalize(SmemFixed *sm, const KArgs &a, uint32_t row, uint32_t n, float top_p, float min_p,
-                                            float u, uint32_t step, uint64_t seed, bool counts_draw, uint32_t slot,
+__device__ __forceinline__ void split_finalize(SmemFixed *sm, const KArgs &a, uint32_t row, uint32_t n, float top_p, float min_p,
+                                               float u, uint32_t step, uint64_t seed, bool counts_draw, uint32_t slot,
                                             const SpecAhead &ahead) {
     constexpr unsigned FULL = 0xFFFFFFFFu;
     const uint32_t lane = threadIdx.x & 31u;
@@ -1857,18 +1857,11 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
     }
 
     // ---- 4. ranks and the draw
-    auto draw = [&](uint32_t n) {  // (n candidates sorted in key[] / id[]; the warp that draws)
-        if (shard) {
-            write_record(n);
-        } else {
-            split_finalize(sm, a, row, n, in.top_p, in.min_p, u_row, a.uniforms ? 0u : in.step, in.seed, counts_draw, slot,
-                           ahead);
-        }
-    };
     if (blocks == 1u) {
         spl_sync();  // (head[0] and the candidates are this block's own)
     }
     // Hardly more candidates than the row keeps: one warp does the rest.
+    uint32_t n_ranked = 0;  // candidates sorted in key[] / id[]
     if (warp != 0u) {
         if (!wait_verdict(0u)) {
             return;
@@ -1926,76 +1919,81 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
                 sm->id[p1] = c1.y;
             }
             __syncwarp();
-            LILY_STAMP(PH_SORT);
-            draw(min(n, k));
-            LILY_STAMP(PH_END);
-            verdict(0u, DONE);
-            return;
+            n_ranked = min(n, k);
+        } else {
+            verdict(0u, HANDS);
         }
-        verdict(0u, HANDS);
     }
-    if (blocks > 1u && !wait_first_phase(&ss->mbar[MEET_CANDIDATES], ca.wait_ns)) {
-        ss->hard = 2;
-        ss->late = 1;
-    }
-    LILY_STAMP(PH_MERGE);
-    const uint4 head = lane < blocks ? ss->head[lane] : make_uint4(0, 0, 0, 0);
-    // Every block's bound holds for the row: what does not reach the largest is out.
-    const uint32_t least_key = __reduce_max_sync(FULL, lane < blocks ? key_of(__uint_as_float(head.z)) : 0u);
-    const uint32_t kmin = key_of(__fdiv_rn(float_of_key(least_key), in.temp));
-    if (__any_sync(FULL, head.y != 0u)) {
-        ss->hard = 2;
-    }
-    unsigned long long *packed = reinterpret_cast<unsigned long long *>(sm->tkey);  // (key, ~id), over tkey and tid
-    {
-        // A region to each of as many teams of whole warps: the live ones.
-        const uint32_t team = SPL_NT >> log_blocks, first = tid & (team - 1u);
-        const uint32_t region = tid / team, n_region = __shfl_sync(FULL, head.x, (int)region);
-        const uint2 *mine = cand + region * cap;
-        for (uint32_t i = first; i - lane < n_region; i += team) {
-            const uint2 e = i < n_region ? mine[i] : make_uint2(0u, 0u);
-            const bool live = e.x >= kmin && i < n_region;
-            const unsigned who = __ballot_sync(FULL, live);
-            if (who != 0u) {
-                uint32_t at = 0;
-                if (lane == 0) {
-                    at = atomicAdd(&ss->n_live, (uint32_t)__popc(who));
-                }
-                at = __shfl_sync(FULL, at, 0) + __popc(who & ((1u << lane) - 1u));
-                if (live && at < KCAP) {
-                    packed[at] = ((unsigned long long)e.x << 32) | (uint32_t)~e.y;
+    const bool alone = n_ranked != 0u;  // (the warp that has ranked them)
+    if (!alone) {
+        if (blocks > 1u && !wait_first_phase(&ss->mbar[MEET_CANDIDATES], ca.wait_ns)) {
+            ss->hard = 2;
+            ss->late = 1;
+        }
+        LILY_STAMP(PH_MERGE);
+        const uint4 head = lane < blocks ? ss->head[lane] : make_uint4(0, 0, 0, 0);
+        // Every block's bound holds for the row: what does not reach the largest is out.
+        const uint32_t least_key = __reduce_max_sync(FULL, lane < blocks ? key_of(__uint_as_float(head.z)) : 0u);
+        const uint32_t kmin = key_of(__fdiv_rn(float_of_key(least_key), in.temp));
+        if (__any_sync(FULL, head.y != 0u)) {
+            ss->hard = 2;
+        }
+        unsigned long long *packed = reinterpret_cast<unsigned long long *>(sm->tkey);  // (key, ~id), over tkey and tid
+        {
+            // A region to each of as many teams of whole warps: the live ones.
+            const uint32_t team = SPL_NT >> log_blocks, first = tid & (team - 1u);
+            const uint32_t region = tid / team, n_region = __shfl_sync(FULL, head.x, (int)region);
+            const uint2 *mine = cand + region * cap;
+            for (uint32_t i = first; i - lane < n_region; i += team) {
+                const uint2 e = i < n_region ? mine[i] : make_uint2(0u, 0u);
+                const bool live = e.x >= kmin && i < n_region;
+                const unsigned who = __ballot_sync(FULL, live);
+                if (who != 0u) {
+                    uint32_t at = 0;
+                    if (lane == 0) {
+                        at = atomicAdd(&ss->n_live, (uint32_t)__popc(who));
+                    }
+                    at = __shfl_sync(FULL, at, 0) + __popc(who & ((1u << lane) - 1u));
+                    if (live && at < KCAP) {
+                        packed[at] = ((unsigned long long)e.x << 32) | (uint32_t)~e.y;
+                    }
                 }
             }
         }
-    }
-    spl_sync();
-    const uint32_t n_live = ss->n_live;
-    if (ss->hard != 0u || n_live == 0u || n_live > KCAP) {
-        verdict(1u, ALONE);
-        return;
-    }
-    for (uint32_t c = tid; c < n_live; c += SPL_NT) {
-        const unsigned long long mine = packed[c];
-        uint32_t before = 0;
-#pragma unroll 8
-        for (uint32_t j = 0; j < n_live; ++j) {
-            before += packed[j] > mine ? 1u : 0u;
+        spl_sync();
+        const uint32_t n_live = ss->n_live;
+        if (ss->hard != 0u || n_live == 0u || n_live > KCAP) {
+            verdict(1u, ALONE);
+            return;
         }
-        if (before < k) {
-            sm->key[before] = (uint32_t)(mine >> 32);
-            sm->id[before] = ~(uint32_t)mine;
+        for (uint32_t c = tid; c < n_live; c += SPL_NT) {
+            const unsigned long long mine = packed[c];
+            uint32_t before = 0;
+    #pragma unroll 8
+            for (uint32_t j = 0; j < n_live; ++j) {
+                before += packed[j] > mine ? 1u : 0u;
+            }
+            if (before < k) {
+                sm->key[before] = (uint32_t)(mine >> 32);
+                sm->id[before] = ~(uint32_t)mine;
+            }
         }
+        spl_sync();
+        n_ranked = min(n_live, k);
     }
-    spl_sync();
-    if (shard && tid == 0) {
-        ss->record_key = sm->key[0];
-    }
-    verdict(1u, DONE);
     LILY_STAMP(PH_SORT);
+    // (One place for the draw, part of the kernel's body: called as a function it took the launch's
+    // arguments by their address, and every one of them was a load from memory.)
     if (draws) {
-        draw(min(n_live, k));
+        if (shard) {
+            write_record(n_ranked);
+        } else {
+            split_finalize(sm, a, row, n_ranked, in.top_p, in.min_p, u_row, a.uniforms ? 0u : in.step, in.seed, counts_draw,
+                           slot, ahead);
+        }
     }
     LILY_STAMP(PH_END);
+    verdict(alone ? 0u : 1u, DONE);  // (a shard's record is written by then)
 }
 
 }  // namespace lily
