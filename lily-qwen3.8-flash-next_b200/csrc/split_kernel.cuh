@@ -207,42 +207,62 @@ __device__ __forceinline__ void split_finalize_wide(SmemFixed *sm, SplitSmem *ss
         ss->bin = n;      // the first rank whose prefix sum exceeds the target
     }
     spl_sync();
+    float *ends = reinterpret_cast<float *>(ss->tmax);  // sums up to every fourth rank (the maxima have served)
+    static_assert(KCAP / 4u == SPL_NT, "four ranks a thread");
     if (tid == 0) {
-        // A chain of n dependent adds (4 clocks each); the loads run 32 ranks ahead of it.
-        // (Ranks past n weigh 0, and s + 0 is s.)
+        // A chain of n dependent adds; all that stands beside it is a load of four weights and the
+        // store of every fourth sum. (Ranks past n weigh 0, and s + 0 is s.)
         const float4 *p4 = reinterpret_cast<const float4 *>(p);
-        float4 *c4 = reinterpret_cast<float4 *>(cum);
+        float4 *e4 = reinterpret_cast<float4 *>(ends);
         constexpr uint32_t A = 8;
         float s = 0.0f;
-        float4 v[A], w[A];
+        float4 v[2][A];
 #pragma unroll
         for (uint32_t h = 0; h < A; ++h) {
-            v[h] = p4[h];
+            v[0][h] = p4[h];
         }
-        for (uint32_t i = 0; i < n; i += 4u * A) {
-            const uint32_t next = min(i / 4u + A, KCAP / 4u - A);
+        for (uint32_t i = 0; i < n; i += 8u * A) {
 #pragma unroll
-            for (uint32_t h = 0; h < A; ++h) {
-                w[h] = p4[next + h];
-            }
+            for (uint32_t side = 0; side < 2u; ++side) {
+                const uint32_t at = i / 4u + side * A, next = min(at + A, KCAP / 4u - A);
 #pragma unroll
-            for (uint32_t h = 0; h < A; ++h) {
-                float4 o;
-                o.x = s = __fadd_rn(s, v[h].x);
-                o.y = s = __fadd_rn(s, v[h].y);
-                o.z = s = __fadd_rn(s, v[h].z);
-                o.w = s = __fadd_rn(s, v[h].w);
-                c4[i / 4u + h] = o;
-                v[h] = w[h];
+                for (uint32_t h = 0; h < A; ++h) {
+                    v[side ^ 1u][h] = p4[next + h];
+                }
+                float o[4];
+#pragma unroll
+                for (uint32_t h = 0; h < A; ++h) {
+                    const float4 x = v[side][h];
+                    s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, x.x), x.y), x.z), x.w);
+                    o[h & 3u] = s;
+                    if ((h & 3u) == 3u) {
+                        e4[(at + h) >> 2] = make_float4(o[0], o[1], o[2], o[3]);
+                    }
+                }
             }
         }
+        ss->least = s;  // (what it held has served)
     }
     spl_sync();
-    const float limit = __fmul_rn(top_p, cum[n - 1u]);
-    for (uint32_t i = tid + 1u; i < n; i += SPL_NT) {
-        if (!(cum[i - 1u] < limit && p[i] >= min_p)) {
-            atomicMin(&ss->n_live, i);
-            break;  // (this thread's later ranks are larger)
+    // Every thread its four ranks' sums, the same adds once more, and the cut.
+    const float limit = __fmul_rn(top_p, ss->least);
+    if (4u * tid < n) {
+        float before = tid != 0u ? ends[tid - 1u] : 0.0f;
+        const float4 x = reinterpret_cast<const float4 *>(p)[tid];
+        const float w[4] = {x.x, x.y, x.z, x.w};
+        float c[4];
+        uint32_t stop = n;
+#pragma unroll
+        for (uint32_t e = 0; e < 4u; ++e) {
+            const uint32_t i = 4u * tid + e;
+            if (stop == n && i != 0u && i < n && !(before < limit && w[e] >= min_p)) {
+                stop = i;
+            }
+            c[e] = before = __fadd_rn(before, w[e]);
+        }
+        reinterpret_cast<float4 *>(cum)[tid] = make_float4(c[0], c[1], c[2], c[3]);
+        if (stop < n) {
+            atomicMin(&ss->n_live, stop);
         }
     }
     spl_sync();
