@@ -303,7 +303,7 @@ __device__ __forceinline__ void split_finalize_wide(SmemFixed *sm, SplitSmem *ss
 // A block's candidates of a wide row: over the pool, which has served, or over key and id.
 constexpr uint32_t WIDE_OWN = SPL_MAX_BLOCKS * SPL_NT / 2u;
 __device__ __forceinline__ unsigned long long *wide_own(SmemFixed *sm, SplitSmem *ss, uint32_t blocks) {
-    static_assert(SPL_SORTED < CAP, "one block's candidates and the pair's other half");
+    static_assert(2u * SPL_SORTED <= CAP, "one block's candidates, and their runs in order");
     return reinterpret_cast<unsigned long long *>(blocks > 1u ? ss->tmax : sm->key);
 }
 
@@ -321,18 +321,46 @@ static __device__ __noinline__ uint32_t merge_lists(SmemFixed *sm, SplitSmem *ss
     unsigned long long *own = wide_own(sm, ss, blocks);
     unsigned long long *lists = reinterpret_cast<unsigned long long *>(sm->key);  // over key and id: CAP
     unsigned long long *best_of = reinterpret_cast<unsigned long long *>(ss + 1);  // SPL_SORTED (the marks have served)
-    if (tid == 0 && (blocks == 1u || sent < WIDE_OWN)) {
-        own[sent] = 0ull;  // (they are counted in pairs)
+    // Every warp puts its runs of 32 in order; then an entry's place is the number of larger ones in
+    // each run, by bisection, eight runs at a time.
+    const uint32_t runs = (sent + 31u) / 32u;
+    unsigned long long *run_of = blocks > 1u ? best_of : own + SPL_SORTED;
+    for (uint32_t c = tid >> 5; c < runs; c += SPL_WARPS) {
+        unsigned long long x = c * 32u + lane < sent ? own[c * 32u + lane] : 0ull;
+#pragma unroll
+        for (uint32_t size = 2u; size <= 32u; size <<= 1) {
+#pragma unroll
+            for (uint32_t stride = size >> 1; stride > 0u; stride >>= 1) {
+                const unsigned long long other = __shfl_xor_sync(FULL, x, stride);
+                const bool larger = ((lane & size) == 0u) == ((lane & stride) == 0u);
+                x = (other > x) == larger ? other : x;
+            }
+        }
+        run_of[c * 32u + lane] = x;
     }
     spl_sync();
-    const ulonglong2 *pairs = reinterpret_cast<const ulonglong2 *>(own);
     for (uint32_t i = tid; i < sent; i += SPL_NT) {
-        const unsigned long long mine = own[i];
+        const unsigned long long mine = run_of[i];
         uint32_t place = 0;
-#pragma unroll 8
-        for (uint32_t j = 0; j < (sent + 1u) / 2u; ++j) {
-            const ulonglong2 o = pairs[j];
-            place += (o.x > mine ? 1u : 0u) + (o.y > mine ? 1u : 0u);
+        for (uint32_t c0 = 0; c0 < runs; c0 += SPL_WARPS) {
+            uint32_t low[SPL_WARPS];
+#pragma unroll
+            for (uint32_t c = 0; c < SPL_WARPS; ++c) {
+                low[c] = 0;
+            }
+#pragma unroll
+            for (uint32_t step = 32u; step != 0u; step >>= 1) {
+#pragma unroll
+                for (uint32_t c = 0; c < SPL_WARPS; ++c) {
+                    const uint32_t to = low[c] + step;
+                    const unsigned long long at = run_of[min(c0 + c, runs - 1u) * 32u + min(to, 32u) - 1u];
+                    low[c] = to <= 32u && at > mine ? to : low[c];
+                }
+            }
+#pragma unroll
+            for (uint32_t c = 0; c < SPL_WARPS; ++c) {
+                place += c0 + c < runs ? low[c] : 0u;
+            }
         }
         (blocks > 1u ? lists + rank * cap : best_of)[place] = mine;
     }
