@@ -770,6 +770,71 @@ static __device__ __noinline__ void emitted_candidates(SmemFixed *sm, SplitSmem 
     }
 }
 
+// The first block draws the row alone with the general row code, all NT threads; or, where a wait
+// for the row ran out, the row has no result, and the status word says so. (A function of its
+// own: it stands at a dozen places of the kernel, none of them on its way.)
+template <typename T, uint32_t MAXR>
+static __device__ __noinline__ void draw_alone_row(const SplitArgs<MAXR> &ca, SmemFixed *sm, SplitSmem *ss, uint32_t row,
+                                                   uint32_t skip) {
+    const KArgs &a = ca.a;
+    const uint32_t tid = threadIdx.x;
+    if (ss->late != 0u) {
+        if (tid == 0) {
+            if (a.cand_out) {
+                a.cand_out[row].max_adj = neg_inf();
+                a.cand_out[row].sum_exp = 0.0f;
+            } else {
+                a.out_ids[row] = 0xFFFFFFFFu;
+                if (a.out_status) {
+                    a.out_status[row] = ROW_INTERNAL;
+                }
+                if (a.kept_n) {
+                    a.kept_n[row] = 0;
+                }
+            }
+            atomicOr(a.status_word, 1u << STATUS_TIMEOUT_BIT);
+        }
+        if (a.cand_out && tid < LILY_SHARD_CANDIDATES) {
+            a.cand_out[row].cand[tid] = make_uint2(0u, 0xFFFFFFFFu);
+        }
+        meet_cluster(tid < SPL_NT || a.shard_sums != 0u);
+        return;
+    }
+    RowGiven given;
+    if (ca.inline_params) {
+        const RowIn &in = ca.in[row];
+        given.params.temperature = (in.flags & ROW_GREEDY) ? 0.0f : in.temp;
+        given.params.top_k = in.k;
+        given.params.top_p = in.top_p;
+        given.params.min_p = in.min_p;
+        given.params.presence_penalty = in.presence;
+        given.params.frequency_penalty = in.frequency;
+        given.params.repetition_penalty = in.rep;
+        given.params.reserved = 0;
+        given.params.seed = in.seed;
+        given.step = in.step;
+        given.has_slot = ca.inline_slots != 0u;
+        given.slot = ca.inline_slots ? ca.slots[row] : 0u;
+        given.has_history = ca.inline_history != 0u;
+        given.history_len = ca.inline_history ? ca.inline_history - 1u : 0u;
+    }
+    const RowGiven *in_args = ca.inline_params ? &given : nullptr;
+    __syncthreads();
+    if (skip == 0u) {
+        sample_whole_row<T, true>(a, row, in_args);
+    } else {
+        sample_whole_row<T, false>(a, row, in_args);
+    }
+    if (a.cand_out) {
+        __syncthreads();
+        if (tid == SPL_NT) {
+            ss->record_key = key_of(__ldcg(&a.cand_out[row].max_adj));
+            ss->late = 0;  // (the general code's memory, meanwhile)
+        }
+        __syncthreads();
+    }
+}
+
 // Grid (blocks per row, rows), clusters of (blocks per row), NT threads, of which
 // SPL_NT do the work. BPS: blocks per SM the registers are cut for; with one, a
 // block whose share fits one bucket keeps it in registers.
@@ -821,69 +886,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
 
     const T *row_ptr = reinterpret_cast<const T *>(a.logits) + (uint64_t)row * a.logits_ld;
     const uint32_t skip = (uint32_t)(reinterpret_cast<uintptr_t>(row_ptr) & 15u) / (uint32_t)sizeof(T);
-    // The row's wait ran out (all NT threads of the first block): the row has no result, and the
-    // status word says so.
-    auto give_up = [&]() {
-        if (tid == 0) {
-            if (a.cand_out) {
-                a.cand_out[row].max_adj = neg_inf();
-                a.cand_out[row].sum_exp = 0.0f;
-            } else {
-                a.out_ids[row] = 0xFFFFFFFFu;
-                if (a.out_status) {
-                    a.out_status[row] = ROW_INTERNAL;
-                }
-                if (a.kept_n) {
-                    a.kept_n[row] = 0;
-                }
-            }
-            atomicOr(a.status_word, 1u << STATUS_TIMEOUT_BIT);
-        }
-        if (a.cand_out && tid < LILY_SHARD_CANDIDATES) {
-            a.cand_out[row].cand[tid] = make_uint2(0u, 0xFFFFFFFFu);
-        }
-        meet_cluster(tid < SPL_NT || a.shard_sums != 0u);
-    };
-    // The first block draws the row alone with the general row code, all NT threads.
-    auto draw_alone = [&]() {
-        if (ss->late != 0u) {
-            give_up();
-            return;
-        }
-        RowGiven given;
-        if (ca.inline_params) {
-            const RowIn &in = ca.in[row];
-            given.params.temperature = (in.flags & ROW_GREEDY) ? 0.0f : in.temp;
-            given.params.top_k = in.k;
-            given.params.top_p = in.top_p;
-            given.params.min_p = in.min_p;
-            given.params.presence_penalty = in.presence;
-            given.params.frequency_penalty = in.frequency;
-            given.params.repetition_penalty = in.rep;
-            given.params.reserved = 0;
-            given.params.seed = in.seed;
-            given.step = in.step;
-            given.has_slot = ca.inline_slots != 0u;
-            given.slot = ca.inline_slots ? ca.slots[row] : 0u;
-            given.has_history = ca.inline_history != 0u;
-            given.history_len = ca.inline_history ? ca.inline_history - 1u : 0u;
-        }
-        const RowGiven *in_args = ca.inline_params ? &given : nullptr;
-        __syncthreads();
-        if (skip == 0u) {
-            sample_whole_row<T, true>(a, row, in_args);
-        } else {
-            sample_whole_row<T, false>(a, row, in_args);
-        }
-        if (a.cand_out) {
-            __syncthreads();
-            if (tid == SPL_NT) {
-                ss->record_key = key_of(__ldcg(&a.cand_out[row].max_adj));
-                ss->late = 0;  // (the general code's memory, meanwhile)
-            }
-            __syncthreads();
-        }
-    };
+    auto draw_alone = [&]() { draw_alone_row<T, MAXR>(ca, sm, ss, row, skip); };
     // What the first block's waiting warps are told, at barrier 2: the row is done, it
     // is drawn alone, or (only to the warps that work) more hands are needed; in the
     // last case there is a second verdict. Threads that wait return only if they are
