@@ -945,6 +945,10 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         if (t < whole_end && (t != 0u || skip == 0u)) {
             return __ldg(vec0 + t * 32u);
         }
+        if (t >= pieces) {  // (most of a short share's: not worth a call)
+            constexpr uint32_t NO = sizeof(T) == 4 ? 0xFF800000u : 0xFF80FF80u;  // -inf
+            return make_uint4(NO, NO, NO, NO);
+        }
         return edge_vec<T>(row_ptr, vocab, skip, t * 32u + lane);
     };
     // The row's first history ids go first. (Their number is not known yet; the row
