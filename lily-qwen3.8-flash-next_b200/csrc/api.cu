@@ -195,6 +195,21 @@ int32_t launch_serialised(lily_sampler *h, cudaStream_t stream, Kernel kernel, d
     return LILY_OK;
 }
 
+int32_t launch_accept(lily_sampler *h, cudaStream_t stream, const uint32_t *draws, const uint32_t *ids, uint32_t id_offset,
+                      uint32_t m, uint32_t *ctrl, uint32_t pos0, uint32_t ratio, uint32_t chain, uint32_t stride) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(1, 1, 1);
+    cfg.blockDim = dim3(1, 1, 1);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    CU(h, cudaLaunchKernelEx(&cfg, lily::spec_accept_kernel, draws, ids, id_offset, m, ctrl, pos0, ratio, chain, stride));
+    return LILY_OK;
+}
+
 template <typename Kernel>
 int32_t raise_smem_limit(lily_sampler *h, Kernel kernel, uint32_t bit) {
     if (!(h->attr_mask & bit)) {
@@ -1717,8 +1732,7 @@ int32_t lily_spec_verify(lily_sampler_t *h, void *stream_, const lily_spec_args_
     }
     if (st == LILY_OK) {
         if (g.m > 1u) {
-            lily::spec_accept_kernel<<<1, 1, 0, stream>>>(g.out_ids, g.draft_ids, 0u, g.m,
-                                                          g.out_accepted, 0u, 1u, 0u, 0u);
+            st = launch_accept(h, stream, g.out_ids, g.draft_ids, 0u, g.m, g.out_accepted, 0u, 1u, 0u, 0u);
         } else {
             CU(h, cudaMemsetAsync(g.out_accepted, 0, 4, stream));
         }
@@ -1747,10 +1761,7 @@ int32_t lily_spec_accept(lily_sampler_t *h, void *stream_, const uint32_t *draws
         return fail(h, LILY_ERR_ARG, "stride must be nonzero");
     }
     DeviceGuard guard(h->device);
-    lily::spec_accept_kernel<<<1, 1, 0, static_cast<cudaStream_t>(stream_)>>>(
-        draws, ids, 1u, m, ctrl, pos0, ratio, chain, stride);
-    CU(h, cudaGetLastError());
-    return LILY_OK;
+    return launch_accept(h, static_cast<cudaStream_t>(stream_), draws, ids, 1u, m, ctrl, pos0, ratio, chain, stride);
 }
 
 // ------------------------------------------------ allocation-free draw --
