@@ -77,14 +77,17 @@ __device__ __forceinline__ void arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void arrive_expect(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.release.cluster.shared::cluster.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
+    // (Relaxed: what it counts on comes by stores that order themselves with the barrier. A release
+    // waits for every store of the thread before it.)
+    asm volatile("mbarrier.arrive.expect_tx.relaxed.cluster.shared::cluster.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
                  : "memory");
 }
 
 // Waits for the first phase of a barrier in this block, for at most `limit_ns`; true
 // if it is complete. (The other blocks of the cluster are running and only have to get
 // there: the limit is met only where something is wrong. The clock is looked at after
-// 16 polls.)
+// 16 polls. A later meeting has twice the limit of the one before it: a block whose wait there
+// ran out still comes here, and says so.)
 __device__ __forceinline__ bool wait_first_phase(const unsigned long long *bar, uint64_t limit_ns) {
     const uint32_t at = (uint32_t)__cvta_generic_to_shared(bar);
     uint64_t t0 = 0;
@@ -383,7 +386,7 @@ static __device__ __noinline__ uint32_t merge_lists(SmemFixed *sm, SplitSmem *ss
             }
             arrive_expect(list_bar, bytes + 16u);
         }
-        lost = spl_any(!wait_first_phase(&ss->mbar[MEET_LISTS], wait_ns));
+        lost = spl_any(!wait_first_phase(&ss->mbar[MEET_LISTS], 2u * wait_ns));
         if (lost) {
             ss->late = 1;
         }
@@ -397,7 +400,7 @@ static __device__ __noinline__ uint32_t merge_lists(SmemFixed *sm, SplitSmem *ss
         lost = __any_sync(FULL, lost || head.y != 0u);
     }
     if (lost || total == 0u || total > SPL_SORTED) {  // (every block decides alike)
-        if (blocks > 1u && !wait_first_phase(&ss->mbar[MEET_GONE], wait_ns)) {
+        if (blocks > 1u && !wait_first_phase(&ss->mbar[MEET_GONE], 4u * wait_ns)) {
             ss->late = 1;
         }
         return 0u;
@@ -436,12 +439,12 @@ static __device__ __noinline__ uint32_t merge_lists(SmemFixed *sm, SplitSmem *ss
             arrive_expect(cand_bar, sent * 8u);
         }
         if (rank != 0u) {
-            if (!wait_first_phase(&ss->mbar[MEET_GONE], wait_ns)) {
+            if (!wait_first_phase(&ss->mbar[MEET_GONE], 4u * wait_ns)) {
                 ss->late = 1;
             }
             return 0u;
         }
-        if (!wait_first_phase(&ss->mbar[MEET_CANDIDATES], wait_ns) || !wait_first_phase(&ss->mbar[MEET_GONE], wait_ns)) {
+        if (!wait_first_phase(&ss->mbar[MEET_CANDIDATES], 4u * wait_ns) || !wait_first_phase(&ss->mbar[MEET_GONE], 4u * wait_ns)) {
             ss->hard = 2;
             ss->late = 1;
         }
@@ -1922,7 +1925,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
             return;
         }
     } else {
-        const bool late = blocks > 1u && !wait_first_phase(&ss->mbar[MEET_CANDIDATES], ca.wait_ns);
+        const bool late = blocks > 1u && !wait_first_phase(&ss->mbar[MEET_CANDIDATES], 2u * ca.wait_ns);
         if (late) {
             ss->late = 1;
         }
@@ -1981,7 +1984,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
     }
     const bool alone = n_ranked != 0u;  // (the warp that has ranked them)
     if (!alone) {
-        if (blocks > 1u && !wait_first_phase(&ss->mbar[MEET_CANDIDATES], ca.wait_ns)) {
+        if (blocks > 1u && !wait_first_phase(&ss->mbar[MEET_CANDIDATES], 2u * ca.wait_ns)) {
             ss->hard = 2;
             ss->late = 1;
         }
