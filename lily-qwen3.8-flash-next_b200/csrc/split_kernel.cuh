@@ -22,10 +22,13 @@
 // dependent steps, and each of the two meetings of the cluster costs a microsecond. So
 // blocks meet by stores that complete a barrier in the receiver, no warp waits for one
 // that it does not need, and the draw's adds run in two chains of 32 lanes. Measured back
-// to back: 1 row x 151936 f32 with a history of 4096 ids 50 -> 10.8 us, 64 rows x
-// 151936 bf16 with histories 32 -> 15.8, argmax of 1 x 32768 9.2 -> 4.7 (before: cut in
-// slices through global memory, or a cluster that kept the row in shared memory; what a
-// shard's record, penalties that raise a logit and bounded waits need costs these 0.3 to 1 us).
+// to back: 1 row x 151936 f32 with a history of 4096 ids 50 -> 9.5 us, 64 rows x
+// 151936 bf16 with histories 32 -> 14.5, argmax of 1 x 32768 9.2 -> 3.55 (before: cut in
+// slices through global memory, or a cluster that kept the row in shared memory). A warp gets
+// through an instruction in some 2.8 clocks, and what is on the way there counts: functions
+// that take the launch's arguments by address load each of them from memory (1 us), an
+// arrival that releases waits for the thread's stores (0.3 us each), and code that a call never
+// runs still slows it where it stands between what it does run.
 //
 // A row that keeps more than 64 candidates takes its bound from the maxima of all
 // threads of the cluster, and all blocks rank its candidates. Where penalties can raise a
@@ -214,7 +217,9 @@ __device__ __forceinline__ void split_finalize_wide(SmemFixed *sm, SplitSmem *ss
     static_assert(KCAP / 4u == SPL_NT, "four ranks a thread");
     if (tid == 0) {
         // A chain of n dependent adds; all that stands beside it is a load of four weights and the
-        // store of every fourth sum. (Ranks past n weigh 0, and s + 0 is s.)
+        // store of every fourth sum. (Ranks past n weigh 0, and s + 0 is s. With every sum stored,
+        // and the weights loaded ahead moved from register to register, an add took 8 clocks
+        // instead of 4.5: 1024 kept, 8100 -> 4560 clocks.)
         const float4 *p4 = reinterpret_cast<const float4 *>(p);
         float4 *e4 = reinterpret_cast<float4 *>(ends);
         constexpr uint32_t A = 8;
@@ -325,7 +330,8 @@ static __device__ __noinline__ uint32_t merge_lists(SmemFixed *sm, SplitSmem *ss
     unsigned long long *lists = reinterpret_cast<unsigned long long *>(sm->key);  // over key and id: CAP
     unsigned long long *best_of = reinterpret_cast<unsigned long long *>(ss + 1);  // SPL_SORTED (the marks have served)
     // Every warp puts its runs of 32 in order; then an entry's place is the number of larger ones in
-    // each run, by bisection, eight runs at a time.
+    // each run, by bisection, eight runs at a time. (Counted over the whole list, 150 entries a
+    // block took 6900 clocks, so 2200.)
     const uint32_t runs = (sent + 31u) / 32u;
     unsigned long long *run_of = blocks > 1u ? best_of : own + SPL_SORTED;
     for (uint32_t c = tid >> 5; c < runs; c += SPL_WARPS) {

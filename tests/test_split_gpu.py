@@ -287,3 +287,21 @@ def test_short_rows(cuda, lily, W, vocab, bf16):
                         (3, 1023, dict(kind="uniform")), (150, 700, {})):
         b = make_batch(W, rng, rows, vocab, k, bf16, **{"kind": "zipf", **kw})
         check(cuda, lily, W, b, vocab, f"V={vocab} k={k} B={rows}", params_on_device=rows == 2)
+
+
+@pytest.mark.parametrize("rows,vocab,bf16", [(6, 60_001, False), (100, 9_001, True)])
+def test_rows_that_keep_many_at_the_edges_of_their_runs(cuda, lily, W, rows, vocab, bf16):
+    """A wide row's lists are put in order by runs of 32, its weights added up four at a time: kept
+    counts around multiples of both, cut by top-p and min-p and not, a row over eight blocks
+    and in one."""
+    rng = np.random.default_rng([rows, vocab])
+    ks = [65, 66, 67, 68, 95, 96, 97, 127, 128, 129, 191, 193, 255, 256, 257, 511, 513, 1021, 1022, 1023, 1024, 0]
+    for at in range(0, len(ks), rows):
+        x = rng.normal(0.0, 2.0, (rows, vocab)).astype(np.float32)
+        params = [dict(temperature=1.1, top_k=ks[(at + r) % len(ks)], top_p=[1.0, 0.97, 0.6][r % 3],
+                       min_p=[0.0, 0.0, 0.01][(r + at) % 3], seed=r) for r in range(rows)]
+        b = W.Batch(W.to_bf16_bits(x) if bf16 else x, bf16, params, rng.random(rows, dtype=np.float32))
+        s = lily.SamplerScratch(vocab, max_rows=rows)
+        assert_parity(b, run_batch(cuda, lily, s, b), oracle_rows(b), label=f"from {at}")
+        assert s.status() == lily.OK
+        s.close()
