@@ -80,9 +80,16 @@ __device__ __forceinline__ void arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void arrive_expect(uint32_t bar, uint32_t bytes) {
-    // (Relaxed: what it counts on comes by stores that order themselves with the barrier. A release
+    // (Relaxed: what it counts on comes by stores that order themselves with the barrier, and the
+    // receiver writes nothing into this block that it was not free to write before. A release
     // waits for every store of the thread before it.)
     asm volatile("mbarrier.arrive.expect_tx.relaxed.cluster.shared::cluster.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
+                 : "memory");
+}
+// The same where the receiver goes on to write over memory that this block has read: its reads
+// (in order with this arrival by a barrier of the block) come before those writes.
+__device__ __forceinline__ void arrive_expect_release(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.release.cluster.shared::cluster.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
                  : "memory");
 }
 
@@ -333,7 +340,18 @@ static __device__ __noinline__ uint32_t merge_lists(SmemFixed *sm, SplitSmem *ss
     // each run, by bisection, eight runs at a time. (Counted over the whole list, 150 entries a
     // block took 6900 clocks, so 2200.)
     const uint32_t runs = (sent + 31u) / 32u;
-    unsigned long long *run_of = blocks > 1u ? best_of : own + SPL_SORTED;
+    // (Over the vectors that reach the bound, which have served.)
+    static_assert(WIDE_OWN * 8u <= 2u * LCAP * 4u, "");
+    unsigned long long *run_of = blocks > 1u ? reinterpret_cast<unsigned long long *>(sm->lkey) : own + SPL_SORTED;
+    // Behind the lists' meeting the others store into the first block's best_of, where its threads have
+    // read their marks: the arrival releases those reads, which lie before the caller's last barrier.
+    // It counts on a list that is still to be sent, from here and by a warp that mostly has no run to
+    // put in order. (3 x 151936 f32, 1024 kept: 16.8 us without a release, 16.9 so, 17.25 with it where the
+    // list is sent.)
+    auto bytes_for = [&](uint32_t to) -> uint32_t { return to != rank ? (sent * 8u + 15u) & ~15u : 0u; };
+    if (blocks > 1u && tid - (SPL_NT - 32u) < blocks) {
+        arrive_expect_release(peer_smem(&ss->mbar[MEET_LISTS], lane), bytes_for(lane) + 16u);
+    }
     for (uint32_t c = tid >> 5; c < runs; c += SPL_WARPS) {
         unsigned long long x = c * 32u + lane < sent ? own[c * 32u + lane] : 0ull;
 #pragma unroll
@@ -381,7 +399,7 @@ static __device__ __noinline__ uint32_t merge_lists(SmemFixed *sm, SplitSmem *ss
         spl_sync();
         if (tid < blocks) {
             const uint32_t list_bar = peer_smem(&ss->mbar[MEET_LISTS], tid);
-            const uint32_t bytes = tid != rank ? (sent * 8u + 15u) & ~15u : 0u;
+            const uint32_t bytes = bytes_for(tid);
             put_4u32(peer_smem(&ss->head[rank], tid), sent, hard, 0u, 0u, list_bar);
             if (bytes != 0u) {
                 asm volatile(
@@ -390,7 +408,6 @@ static __device__ __noinline__ uint32_t merge_lists(SmemFixed *sm, SplitSmem *ss
                     "r"((uint32_t)__cvta_generic_to_shared(lists + rank * cap)), "r"(bytes), "r"(list_bar)
                     : "memory");
             }
-            arrive_expect(list_bar, bytes + 16u);
         }
         lost = spl_any(!wait_first_phase(&ss->mbar[MEET_LISTS], 2u * wait_ns));
         if (lost) {
