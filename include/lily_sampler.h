@@ -156,8 +156,10 @@ int32_t lily_sampler_status(lily_sampler_t *h, void *stream);
  * returns. The launch completes like any other; the logits it was to write are not
  * valid, a row it was to draw gets id 0xFFFFFFFF, and the next lily_sampler_status
  * returns LILY_ERR_TIMEOUT (once: the status is cleared by reading it). The handle
- * stays usable. (Where the blocks of a row meet more than once, the second and third meeting
- * wait twice and four times as long: a block whose earlier wait ran out still comes there.)
+ * stays usable. (Where the blocks of a row meet more than once, the earlier meetings wait a part
+ * of it, so that a block whose wait ran out still comes to the later ones: half and the whole, for
+ * a row that keeps more than 64 candidates a quarter, half and the whole. A wait alone thus
+ * ends within the limit, all of a row's waits together within 1.75 of it.)
  *
  * inject_lost_copy is the device-side sibling of inject_fault, for tests: the
  * next LM-head launch on this handle (and only that one) leaves out the copy of

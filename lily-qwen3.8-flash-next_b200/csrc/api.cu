@@ -392,7 +392,7 @@ int32_t launch_split(lily_sampler *h, cudaStream_t stream, lily::SplitArgs<MAXR>
     sa.two_per_sm = p.sole ? 0u : 1u;
     sa.mark_mode = p.mark_mode;
     sa.mark_words = p.mark_words;
-    sa.wait_ns = h->wait_ns < (1ull << 60) ? h->wait_ns : 1ull << 60;  // (the kernel's later meetings wait two and four times as long)
+    sa.wait_ns = h->wait_ns;
     sa.lost = h->lost_arrival;
     h->lost_arrival = 0;  // one launch only
     CU(h, lily::split_launch<MAXR>(sa, rows, dtype, p.smem, h->max_smem, &h->attr_mask, stream));

@@ -129,7 +129,8 @@ struct SplitArgs {
     // Test hook: block lost >> 8 of every cluster waits for one arrival too many at its
     // barrier (lost & 255) - 1, so that the wait runs out (0: none).
     uint32_t lost;
-    uint64_t wait_ns;         // the bound of every wait of a block for the others
+    uint64_t wait_ns;         // the bound of every wait of a block for the others (wait_first_phase: a row's
+                              // earlier meetings have a part of it)
     RowIn in[MAXR];
     // Keys that a warp gives to the pool of a row that keeps k: so much above its share
     // that all but some three of the best k are in the pool. (What is missing there

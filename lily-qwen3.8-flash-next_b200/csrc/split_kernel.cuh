@@ -93,14 +93,16 @@ __device__ __forceinline__ void arrive_expect_release(uint32_t bar, uint32_t byt
                  : "memory");
 }
 
-// Waits for the first phase of a barrier in this block, for at most `limit_ns`; true
+// Waits for the first phase of a barrier in this block, for at most `limit_ns` since `t0`; true
 // if it is complete. (The other blocks of the cluster are running and only have to get
 // there: the limit is met only where something is wrong. The clock is looked at after
-// 16 polls. A later meeting has twice the limit of the one before it: a block whose wait there
-// ran out still comes here, and says so.)
-__device__ __forceinline__ bool wait_first_phase(const unsigned long long *bar, uint64_t limit_ns) {
+// 16 polls; t0 = 0: since then.)
+// The row's last meeting has the launch's limit, the one before it half of that, the pool of a wide
+// row a quarter: a block whose wait for the keys ran out still comes to the later meetings, in time to
+// say so there. (It does not send on what it has not got: of a wide row that lost its lists the
+// others wait for candidates and receipt in vain.)
+__device__ __forceinline__ bool wait_first_phase(const unsigned long long *bar, uint64_t limit_ns, uint64_t &t0) {
     const uint32_t at = (uint32_t)__cvta_generic_to_shared(bar);
-    uint64_t t0 = 0;
     for (uint32_t i = 0;; ++i) {
         uint32_t done;
         asm volatile(
@@ -121,6 +123,11 @@ __device__ __forceinline__ bool wait_first_phase(const unsigned long long *bar, 
             }
         }
     }
+}
+
+__device__ __forceinline__ bool wait_first_phase(const unsigned long long *bar, uint64_t limit_ns) {
+    uint64_t t0 = 0;
+    return wait_first_phase(bar, limit_ns, t0);
 }
 
 // All threads of the cluster that have not returned yet meet here, for a thread that has
@@ -392,7 +399,7 @@ static __device__ __noinline__ uint32_t merge_lists(SmemFixed *sm, SplitSmem *ss
         (blocks > 1u ? lists + rank * cap : best_of)[place] = mine;
     }
     uint32_t total = sent;
-    bool lost = hard != 0u;
+    bool lost = hard != 0u, gave_up = false;
     if (blocks > 1u) {
         // (One copy per block: stores of a thread each cost the SM some 4 clocks a piece.)
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -409,21 +416,22 @@ static __device__ __noinline__ uint32_t merge_lists(SmemFixed *sm, SplitSmem *ss
                     : "memory");
             }
         }
-        lost = spl_any(!wait_first_phase(&ss->mbar[MEET_LISTS], 2u * wait_ns));
-        if (lost) {
+        gave_up = spl_any(!wait_first_phase(&ss->mbar[MEET_LISTS], wait_ns >> 1));
+        if (gave_up) {
             ss->late = 1;
         }
         // A copy completes in its receiver, but its source is the sender's shared memory: no
         // block leaves or draws alone in that memory before every receiver has said so.
-        if (tid < blocks && !lost) {
+        if (tid < blocks && !gave_up) {
             arrive(peer_smem(&ss->mbar[MEET_GONE], tid));
         }
         const uint4 head = lane < blocks ? ss->head[lane] : make_uint4(0, 0, 0, 0);
         total = __reduce_add_sync(FULL, head.x);
-        lost = __any_sync(FULL, lost || head.y != 0u);
+        lost = __any_sync(FULL, gave_up || head.y != 0u);
     }
     if (lost || total == 0u || total > SPL_SORTED) {  // (every block decides alike)
-        if (blocks > 1u && !wait_first_phase(&ss->mbar[MEET_GONE], 4u * wait_ns)) {
+        // (Whoever gave up meets all of the cluster before it leaves; its own receipt will not come.)
+        if (blocks > 1u && !gave_up && !wait_first_phase(&ss->mbar[MEET_GONE], wait_ns)) {
             ss->late = 1;
         }
         return 0u;
@@ -462,12 +470,13 @@ static __device__ __noinline__ uint32_t merge_lists(SmemFixed *sm, SplitSmem *ss
             arrive_expect(cand_bar, sent * 8u);
         }
         if (rank != 0u) {
-            if (!wait_first_phase(&ss->mbar[MEET_GONE], 4u * wait_ns)) {
+            if (!wait_first_phase(&ss->mbar[MEET_GONE], wait_ns)) {
                 ss->late = 1;
             }
             return 0u;
         }
-        if (!wait_first_phase(&ss->mbar[MEET_CANDIDATES], 4u * wait_ns) || !wait_first_phase(&ss->mbar[MEET_GONE], 4u * wait_ns)) {
+        uint64_t t0 = 0;  // (the two share the limit)
+        if (!wait_first_phase(&ss->mbar[MEET_CANDIDATES], wait_ns, t0) || !wait_first_phase(&ss->mbar[MEET_GONE], wait_ns, t0)) {
             ss->hard = 2;
             ss->late = 1;
         }
@@ -1603,7 +1612,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
             if (tid == 0) {
                 arrive_expect(peer_smem(&ss->mbar[MEET_POOL], rank), n * 4u);
             }
-            if (!wait_first_phase(&ss->mbar[MEET_POOL], ca.wait_ns)) {
+            if (!wait_first_phase(&ss->mbar[MEET_POOL], ca.wait_ns >> 1)) {
                 ss->hard = ss->late = 1;
             }
         } else {
@@ -1677,7 +1686,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         if (tid == 0) {
             ss->bin = NONE;
         }
-        if (blocks > 1u && !wait_first_phase(&ss->mbar[MEET_POOL], ca.wait_ns)) {
+        if (blocks > 1u && !wait_first_phase(&ss->mbar[MEET_POOL], ca.wait_ns >> 2)) {
             ss->hard = ss->late = 1;
         }
         spl_sync();
@@ -1948,7 +1957,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
             return;
         }
     } else {
-        const bool late = blocks > 1u && !wait_first_phase(&ss->mbar[MEET_CANDIDATES], 2u * ca.wait_ns);
+        const bool late = blocks > 1u && !wait_first_phase(&ss->mbar[MEET_CANDIDATES], ca.wait_ns);
         if (late) {
             ss->late = 1;
         }
@@ -2007,7 +2016,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
     }
     const bool alone = n_ranked != 0u;  // (the warp that has ranked them)
     if (!alone) {
-        if (blocks > 1u && !wait_first_phase(&ss->mbar[MEET_CANDIDATES], 2u * ca.wait_ns)) {
+        if (blocks > 1u && !wait_first_phase(&ss->mbar[MEET_CANDIDATES], ca.wait_ns)) {
             ss->hard = 2;
             ss->late = 1;
         }

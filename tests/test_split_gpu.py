@@ -186,6 +186,34 @@ def test_a_wait_for_an_argmax_and_for_a_shards_sums_that_runs_out(cuda, lily, W)
     s.close()
 
 
+@pytest.mark.parametrize("barrier,block,k,share", [
+    (1, 0, 40, 0.5), (2, 0, 40, 1.0), (1, 0, 1, 1.0),
+    (1, 0, 0, 0.25), (3, 0, 0, 1.0), (3, 2, 0, 1.0), (5, 0, 0, 1.0), (5, 2, 0, 1.0)])
+def test_a_lost_arrival_is_given_up_within_the_limit(cuda, lily, W, barrier, block, k, share):
+    """However late in the row the meeting is: the limit bounds the wait, and the row's other waits
+    for a block that gave up end with it. (What is missing costs the share of the limit its meeting has; a
+    block that lost the lists keeps the others, which wait for its receipt, for the whole.)"""
+    vocab, rows, limit = 60_001, 2, 40e6
+    b = make_batch(W, np.random.default_rng([barrier, block, k]), rows, vocab, k, False, kind="zipf")
+    s = lily.SamplerScratch(vocab, max_rows=rows)
+    logits, out = t_logits(cuda, b), cuda.zeros(rows, dtype=cuda.int32, device="cuda")
+    p = s.prepare_sample_batch(logits, make_params(lily, b), out, uniforms=t_f32(cuda, b.uniforms))
+    s.sample_prepared(p)
+    s.set_wait_limit(int(limit))
+    s.inject_lost_arrival(barrier, block)
+    t0, t1 = cuda.cuda.Event(enable_timing=True), cuda.cuda.Event(enable_timing=True)
+    cuda.cuda.synchronize()
+    t0.record()
+    s.sample_prepared(p)
+    t1.record()
+    cuda.cuda.synchronize()
+    took = t0.elapsed_time(t1) * 1e6 / limit
+    # (Beside the waits the launch takes microseconds; a quarter of the limit, 10 ms, is room for a busy host.)
+    assert 0.95 * share < took < share + 0.25, took
+    assert s.status() == (lily.OK if (barrier, block) == (5, 2) else lily.ERR_TIMEOUT)
+    s.close()
+
+
 RAISING = [dict(history=700, presence=-0.6), dict(history=3000, rep=0.7), dict(history=2000, frequency=-0.2, rep=1.1),
            dict(history=900, frequency=0.1, presence=-1.0, n_bias=9, n_ban=3), dict(history=5, presence=-40.0)]
 
