@@ -150,6 +150,49 @@ def test_dense_draft_distribution_and_greedy_match(cuda, lily, W):
     scratch.close()
 
 
+@pytest.mark.parametrize("vocab", [4099, 60_001])
+def test_steps_one_behind_the_other_in_the_same_buffers(cuda, lily, W, vocab):
+    # Nobody waits between the steps: each one's rows are set up under the count of the one before, the
+    # count under its own step's rows, and all steps draw into the same words.
+    scratch = lily.SamplerScratch(vocab, max_rows=3)
+    out = cuda.full((3,), -1, dtype=cuda.int32, device="cuda")
+    calls, want = [], []
+    for step in range(16):
+        greedy = step % 3 == 2
+        x = W.config3_step(step, vocab=vocab, greedy=greedy)
+        if greedy:  # (one or both of the drafts are what the target says)
+            n = 1 + step % 2
+            x.draft_ids[:n] = np.argmax(x.target_f32(), axis=1)[:n]
+        st, ids, acc = oracle.spec_verify(x.target_f32(), oracle.params(**x.params), x.draft_ids, x.u_accept, x.u_resid,
+                                          q_dense=x.q)
+        if greedy:
+            assert np.array_equal(ids, np.argmax(x.target_f32(), axis=1).astype(np.uint32))
+        assert st == 0
+        want.append((ids, acc))
+        calls.append((cuda.from_numpy(x.target.view(np.int16)).view(cuda.bfloat16).cuda(), lily.SamplingParams(**x.params),
+                      t_u32(cuda, x.draft_ids),
+                      dict(mode=lily.SPEC_GREEDY_MATCH if greedy else lily.SPEC_REJECTION, q_dense=t_f32(cuda, x.q),
+                           u_accept=t_f32(cuda, x.u_accept), u_resid=t_f32(cuda, x.u_resid)),
+                      t_u32(cuda, np.concatenate([[0], x.draft_ids]))))
+    assert {acc for _, acc in want} == {0, 1, 2}
+    rounds = 12
+    accepted = cuda.full((rounds, len(calls)), -1, dtype=cuda.int32, device="cuda")
+    ctrl = cuda.zeros((rounds, len(calls), lily.ctrl_words(1, 1)), dtype=cuda.int32, device="cuda")
+    into = [[(accepted[r, i:i + 1], ctrl[r, i]) for i in range(len(calls))] for r in range(rounds)]
+    cuda.cuda.synchronize()
+    for r in range(rounds):
+        for i, (target, params, drafts, kw, ids) in enumerate(calls):
+            scratch.spec_verify(target, params, drafts, out, into[r][i][0], **kw)
+            if r % 2:  # (and the count as a call of its own, of the same draws)
+                scratch.spec_accept(out, ids, into[r][i][1], 7, 1, 1, 1)
+    cuda.cuda.synchronize()
+    counts = [acc for _, acc in want]
+    assert np.array_equal(np_u32(accepted), np.tile(np.array(counts, dtype=np.uint32), (rounds, 1)))
+    assert np.array_equal(np_u32(ctrl)[1::2, :, 0], np.tile(np.array(counts, dtype=np.uint32), (rounds // 2, 1)))
+    assert np.array_equal(np_u32(out), want[-1][0])
+    scratch.close()
+
+
 @pytest.mark.parametrize("table", [False, True])
 def test_rows_of_a_step_share_the_penalty_state(cuda, lily, W, table):
     # src/qwen4exp/model.rs:3008-3012: row j's penalties see the draws of rows < j.

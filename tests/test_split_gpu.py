@@ -317,19 +317,53 @@ def test_short_rows(cuda, lily, W, vocab, bf16):
         check(cuda, lily, W, b, vocab, f"V={vocab} k={k} B={rows}", params_on_device=rows == 2)
 
 
-@pytest.mark.parametrize("rows,vocab,bf16", [(6, 60_001, False), (100, 9_001, True)])
-def test_rows_that_keep_many_at_the_edges_of_their_runs(cuda, lily, W, rows, vocab, bf16):
-    """A wide row's lists are put in order by runs of 32, its weights added up four at a time: kept
-    counts around multiples of both, cut by top-p and min-p and not, a row over eight blocks
-    and in one."""
+def cut_by_min_p(x, temp, cut):
+    """A min-p that ends a row's kept set at rank `cut` or, where the weights there are too close to each
+    other, four ranks or more later; and that rank."""
+    w = np.sort(x.astype(np.float64))[::-1] / temp
+    w = np.exp(w - w[0])
+    while w[cut - 1] < w[cut] * (1.0 + 1e-4):
+        cut += 4
+    return float(np.float32(np.sqrt(w[cut - 1] * w[cut]))), cut
+
+
+@pytest.mark.parametrize("rows,vocab,bf16,most", [(6, 60_001, False, 1024), (30, 30_001, False, 1024),
+                                                  (60, 60_001, False, 455), (100, 9_001, False, 227),
+                                                  (100, 9_001, True, 227)])
+def test_rows_that_keep_many_at_the_edges_of_their_runs(cuda, lily, W, rows, vocab, bf16, most):
+    """A wide row's lists are put in order by runs of 32, its weights added up four at a time, each
+    thread cuts among four of them: kept counts around multiples of both, uncut, ended by top-p, and
+    ended by min-p at every one of a thread's four ranks. A row over eight, four and two blocks and in
+    one, with up to as many kept as the kernel ranks there by itself."""
     rng = np.random.default_rng([rows, vocab])
-    ks = [65, 66, 67, 68, 95, 96, 97, 127, 128, 129, 191, 193, 255, 256, 257, 511, 513, 1021, 1022, 1023, 1024, 0]
-    for at in range(0, len(ks), rows):
+    ks = [65, 66, 67, 68, 95, 96, 97, 127, 128, 129, 191, 193, 225, 226, 227, 255, 256, 257, 453, 454, 455, 511, 513, 1021,
+          1022, 1023, 1024, 0]
+    ways = [(k, way, i) for i, k in enumerate(k for k in ks if (k or 1024) <= most)
+            for way in ("uncut", "top-p", "min-p", "min-p, an odd rank")]
+    ended = {0: 0, 1: 0, 2: 0, 3: 0}
+    for at in range(0, len(ways), rows):
         x = rng.normal(0.0, 2.0, (rows, vocab)).astype(np.float32)
-        params = [dict(temperature=1.1, top_k=ks[(at + r) % len(ks)], top_p=[1.0, 0.97, 0.6][r % 3],
-                       min_p=[0.0, 0.0, 0.01][(r + at) % 3], seed=r) for r in range(rows)]
-        b = W.Batch(W.to_bf16_bits(x) if bf16 else x, bf16, params, rng.random(rows, dtype=np.float32))
+        bits = W.to_bf16_bits(x) if bf16 else x
+        values = W.bf16_bits_to_f32(bits) if bf16 else x
+        params, ends = [], []
+        for r in range(rows):
+            k, way, i = ways[(at + r) % len(ways)]
+            p, end = dict(temperature=1.1, top_k=k, seed=r), k or 1024
+            if way == "top-p":
+                p["top_p"], end = (0.9, 0.6, 0.3)[i % 3], None
+            elif way != "uncut":
+                half = end // 2
+                p["min_p"], end = cut_by_min_p(values[r], 1.1, half - half % 4 + (2 * i + way.endswith("odd rank")) % 4)
+                assert end < (k or 1024)
+                ended[end % 4] += 1
+            params.append(p)
+            ends.append(end)
+        b = W.Batch(bits, bf16, params, rng.random(rows, dtype=np.float32))
+        want = oracle_rows(b)
+        for p, end, d in zip(params, ends, want):  # (what ends the set is what the test means to end it)
+            assert len(d.kept_ids) == end if end else len(d.kept_ids) < (p["top_k"] or 1024)
         s = lily.SamplerScratch(vocab, max_rows=rows)
-        assert_parity(b, run_batch(cuda, lily, s, b), oracle_rows(b), label=f"from {at}")
+        assert_parity(b, run_batch(cuda, lily, s, b), want, label=f"from {at}")
         assert s.status() == lily.OK
         s.close()
+    assert min(ended.values()) > 0, ended
