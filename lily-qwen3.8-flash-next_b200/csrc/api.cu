@@ -377,9 +377,9 @@ SplitPlan split_plan(const lily_sampler *h, const lily::KArgs &a, uint32_t rows,
     p.smem = p.smem > general ? p.smem : general;
     // More rows than SMs: two blocks to an SM, unless the kernel of one block per row takes the
     // call (aligned logits), which reads further ahead. 256 rows x 151936 bf16: 30.6 us here,
-    // 27.6 there. What only the general kernel took, 256 rows: x 151937 bf16 without lists
-    // 117 -> 32.5, with 4096 ids a row 122 -> 34.9, with 32768 128 -> 41.9; x 50257 f32 with
-    // 8192 ids 55.5 -> 26.2.
+    // 27.6 there. What only the general kernel took, 256 rows with ids of a power law: x 151937
+    // bf16 without lists 31.6, with 4096 ids a row 35.0, with 32768 49.5; x 50257 f32 with 8192
+    // ids 28.5 (the general kernel, by its first measurement: 117, 122, 128 and 55.5).
     p.take = p.smem <= (size_t)h->max_smem && (p.sole || !stream_route(a, rows, dtype));
     return p;
 }

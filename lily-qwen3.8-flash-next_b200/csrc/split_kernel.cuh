@@ -1,6 +1,7 @@
 // The row kernel: a row's vocabulary is split over the blocks of a cluster (one,
 // two, four or eight of them, as many as leave every SM something to do), which
-// meet once.
+// meet once (an argmax), twice, or (a row that keeps many) at the pool, at the exchange of their
+// lists and at the first block's candidates and every block's receipt.
 //
 //   1. 256 threads of a block look at its vectors of the row (16 bytes each) and keep the
 //      largest logit they saw; ten vectors (a bucket) share one maximum in shared
@@ -19,13 +20,14 @@
 //      in rank order, the cut and the draw (or writes a shard's record).
 //
 // What bounds it is latency, not memory: a call of a few rows is a chain of some ten
-// dependent steps, and each of the two meetings of the cluster costs a microsecond. So
-// blocks meet by stores that complete a barrier in the receiver, no warp waits for one
-// that it does not need, and the draw's adds run in two chains of 32 lanes. Measured back
-// to back: 1 row x 151936 f32 with a history of 4096 ids 50 -> 9.5 us, 64 rows x
-// 151936 bf16 with histories 32 -> 14.5, argmax of 1 x 32768 9.2 -> 3.55 (before: cut in
-// slices through global memory, or a cluster that kept the row in shared memory). A warp gets
-// through an instruction in some 2.8 clocks, and what is on the way there counts: functions
+// dependent steps: from the share read to the bound known, with the pool's meeting in between, 1.4 to
+// 1.65 us, from the candidates sent to all of them there 0.1 to 0.25. So blocks meet by stores
+// that complete a barrier in the receiver, no warp waits for one that it does not need, and the
+// draw's adds run in two chains of 32 lanes. Measured back to back: 1 row x 151936 f32 with a history of 4096 ids 50 -> 9.35 us, 64 rows x
+// 151936 bf16 with histories 32 -> 14.4, argmax of 1 x 32768 9.2 -> 3.55 (before: cut in
+// slices through global memory, or a cluster that kept the row in shared memory). Code that the
+// warps run once is slow code: of the 21 clocks between two instructions of a warp 6 to 7.5 wait for the
+// instruction itself and 7.5 at barriers. So what stands on the way counts: functions
 // that take the launch's arguments by address load each of them from memory (1 us), an
 // arrival that releases waits for the thread's stores (0.3 us each), and code that a call never
 // runs still slows it where it stands between what it does run.
@@ -818,7 +820,7 @@ static __device__ __noinline__ void draw_alone_row(const SplitArgs<MAXR> &ca) {
     const KArgs &a = ca.a;
     const uint32_t tid = threadIdx.x, row = a.row0 + blockIdx.y;
     const T *row_ptr = reinterpret_cast<const T *>(a.logits) + (uint64_t)row * a.logits_ld;
-    const uint32_t skip = (uint32_t)(reinterpret_cast<uintptr_t>(row_ptr) & 15u);
+    const bool aligned = (reinterpret_cast<uintptr_t>(row_ptr) & 15u) == 0u;
     if (ss->late != 0u) {
         if (tid == 0) {
             if (a.cand_out) {
@@ -861,7 +863,7 @@ static __device__ __noinline__ void draw_alone_row(const SplitArgs<MAXR> &ca) {
     }
     const RowGiven *in_args = ca.inline_params ? &given : nullptr;
     __syncthreads();
-    if (skip == 0u) {
+    if (aligned) {
         sample_row<T, true>(a, row, 0u, 1u, in_args);
     } else {
         sample_row<T, false>(a, row, 0u, 1u, in_args);
