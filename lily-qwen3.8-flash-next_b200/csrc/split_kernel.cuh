@@ -24,7 +24,7 @@
 // 1.65 us, from the candidates sent to all of them there 0.1 to 0.25. So blocks meet by stores
 // that complete a barrier in the receiver, no warp waits for one that it does not need, and the
 // draw's adds run in two chains of 32 lanes. Measured back to back: 1 row x 151936 f32 with a history of 4096 ids 50 -> 9.35 us, 64 rows x
-// 151936 bf16 with histories 32 -> 14.4, argmax of 1 x 32768 9.2 -> 3.55 (before: cut in
+// 151936 bf16 with histories 32 -> 14.4, argmax of 1 x 32768 9.2 -> 3.25 (before: cut in
 // slices through global memory, or a cluster that kept the row in shared memory). Code that the
 // warps run once is slow code: of the 21 clocks between two instructions of a warp 6 to 7.5 wait for the
 // instruction itself and 7.5 at barriers. So what stands on the way counts: functions
@@ -878,6 +878,23 @@ static __device__ __noinline__ void draw_alone_row(const SplitArgs<MAXR> &ca) {
     }
 }
 
+// What the first block's waiting threads are told: the row is done, it is drawn alone, or more hands
+// are needed.
+enum { DONE = 0, ALONE = 1, HANDS = 2 };
+
+// The end of an argmax row for the first block's threads that look at its logits and then only wait. (A
+// function: as part of the kernel's body it stood on the way of the warp they wait for. 1 x 32768
+// f32 3.5 - 3.8 -> 3.25 us.)
+template <typename T, uint32_t MAXR>
+static __device__ __noinline__ void wait_for_the_end(const SplitArgs<MAXR> &ca) {
+    extern __shared__ uint4 smem_raw[];
+    const SplitSmem *ss = reinterpret_cast<const SplitSmem *>(reinterpret_cast<SmemFixed *>(smem_raw) + 1);
+    asm volatile("bar.sync 2, %0;" ::"n"(NT) : "memory");
+    if (ss->verdict[0] == ALONE) {
+        draw_alone_row<T, MAXR>(ca);
+    }
+}
+
 // Grid (blocks per row, rows), clusters of (blocks per row), NT threads, of which
 // SPL_NT do the work. BPS: blocks per SM the registers are cut for; with one, a
 // block whose share fits one bucket keeps it in registers.
@@ -934,7 +951,6 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
     // is drawn alone, or (only to the warps that work) more hands are needed; in the
     // last case there is a second verdict. Threads that wait return only if they are
     // needed.
-    enum { DONE = 0, ALONE = 1, HANDS = 2 };
     auto wait_verdict = [&](uint32_t at) -> bool {
         asm volatile("bar.sync 2, %0;" ::"n"(NT) : "memory");
         const uint32_t v = ss->verdict[at];
@@ -1485,7 +1501,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
             spl_sync();
         }
         if (warp != 0u) {
-            wait_verdict(0u);
+            wait_for_the_end<T>(ca);
             return;
         }
         uint32_t top = 0u, at = NONE;
