@@ -13,7 +13,8 @@
 //
 //   * one thread asks the copy engine (TMA, 128-byte swizzle) for 256 rows x 128 bytes
 //     of weights per stage, another for each group's slice of the hidden states (a
-//     ready image, see prepare_hidden_kernel);
+//     ready image, see prepare_hidden_kernel); two warps copy the rows' scales and biases,
+//     eight groups of them at a time;
 //   * converter warps own one tile row per thread: they widen a group's 64 weights
 //     exactly to 16 bits and store them with tcgen05.st into TENSOR MEMORY, where the
 //     multiplier reads its A operand (lane = row, two values per column);
@@ -52,10 +53,12 @@
 
 namespace lily_head {
 
-// Warps: four that multiply, two that load (two idle), then converters, then the epilogue.
+// Warps: four that multiply, four that load (weights, hidden states, two for the scales), then
+// converters, then the epilogue.
 constexpr int MMA_WARPS = 4;
 constexpr int WARP_LOAD_W = 4;
 constexpr int WARP_LOAD_H = 5;
+constexpr int WARP_LOAD_S0 = 6;
 constexpr int WARP_CONV0 = 8;
 
 constexpr uint32_t RAW_STAGE_BYTES = TILE_ROWS * 128u;  // 32 KB
@@ -84,12 +87,18 @@ struct Shape {
     static constexpr uint32_t PG = N == 64u ? 1u : 2u;
     static constexpr uint32_t ACC_BUFS = 2u;                              // of PG groups
     static constexpr uint32_t A_SLOTS = N == 64u ? 4u : N == 32u ? 2u : 3u;  // of PG groups
-    // (No more stages than the latency of memory needs: what shared memory leaves of the L1
-    // cache holds the scales' lines, each of which is read eight times.)
     static constexpr uint32_t RAW_STAGES = N == 64u ? 3u : N == 32u ? 4u : 5u;
     static constexpr uint32_t H_SLOTS = 8u;                             // hidden slices in shared memory
     static constexpr uint32_t DONE_SLOTS = H_SLOTS / PG;                // ring of "has been multiplied" barriers
     static constexpr uint32_t SUM_SLOTS = 2u * H_SLOTS;                 // the slices' sums: the epilogue may be that far behind
+    // Units of scales (and biases) in shared memory, so that they are there when the epilogue, which
+    // is the slowest of the roles, comes to them. (Loaded by the epilogue, its warps waited some
+    // 40 to 100 clocks of a group's 700 to 1200 for them: 4 bits, 32 tokens 61.5 -> 58.4 us, affine
+    // bytes, 64 tokens 296 -> 293, 4 tokens 173.6 -> 171.4; sizes at launch_head.)
+    static constexpr uint32_t S_SLOTS = 4u;
+    static_assert(BLOCK_GROUPS * 2u == 16u, "a row's scales of a unit are one copy");
+    static constexpr uint32_t S_ARRAY_BYTES = TILE_ROWS * 16u;          // 16 bytes a row
+    static constexpr uint32_t S_SLOT_BYTES = (FMT != FMT_S8 ? 2u : 1u) * S_ARRAY_BYTES;
     static constexpr uint32_t H_BYTES = N * 128u;
     static constexpr uint32_t A_COL0 = ACC_BUFS * PG * N;                    // within a half's 256 columns
     static_assert(A_COL0 + A_SLOTS * PG * 32u <= TMEM_COLS / 2u, "tensor memory columns of a half");
@@ -100,7 +109,8 @@ struct Shape {
     static constexpr uint32_t HID = 0;
     static constexpr uint32_t RAW = HID + H_SLOTS * H_BYTES;
     static constexpr uint32_t SUMS = RAW + RAW_STAGES * RAW_STAGE_BYTES;
-    static constexpr uint32_t UNSCALE = SUMS + SUM_SLOTS * N * 4u;
+    static constexpr uint32_t SCALES = SUMS + SUM_SLOTS * N * 4u;
+    static constexpr uint32_t UNSCALE = SCALES + S_SLOTS * S_SLOT_BYTES;
     static constexpr uint32_t BARS = UNSCALE + N * 4u;
     static constexpr uint32_t RAW_FULL = BARS;                          // [RAW_STAGES]
     static constexpr uint32_t RAW_EMPTY = RAW_FULL + 8 * RAW_STAGES;
@@ -111,7 +121,9 @@ struct Shape {
     static constexpr uint32_t DONE = A_FULL + 2 * 8 * A_SLOTS;          // [2][DONE_SLOTS]
     static constexpr uint32_t ACC_EMPTY = DONE + 2 * 8 * DONE_SLOTS;    // [2][ACC_BUFS]
     static constexpr uint32_t FINAL = ACC_EMPTY + 2 * 8 * ACC_BUFS;     // [MMA_WARPS] an issuing warp's last commit
-    static constexpr uint32_t TMEM_ADDR = FINAL + 8 * MMA_WARPS;
+    static constexpr uint32_t S_FULL = FINAL + 8 * MMA_WARPS;            // [S_SLOTS]
+    static constexpr uint32_t S_EMPTY = S_FULL + 8 * S_SLOTS;            // [S_SLOTS]
+    static constexpr uint32_t TMEM_ADDR = S_EMPTY + 8 * S_SLOTS;
     static constexpr uint32_t ABORT = TMEM_ADDR + 4;
     static constexpr uint32_t BYTES = ABORT + 4 + 1024;                  // room to align the base
     static_assert(BYTES <= 227u * 1024u, "shared memory of one block");
@@ -230,6 +242,11 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
                  "l"(src), "r"(bytes), "r"(bar)
                  : "memory");
+}
+
+// A thread's copy of 16 bytes into shared memory (the 128 bytes they lie in are asked into L2).
+__device__ __forceinline__ void copy_async16(uint32_t dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global.L2::128B [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 
 // kind::f16: D binary32, A and B both binary16 or both bf16, both K-major, M = 128.
@@ -518,6 +535,10 @@ __global__ void __launch_bounds__(Shape<N, FMT>::THREADS, 1) lmhead_kernel(const
         for (int w = 0; w < MMA_WARPS; ++w) {
             mbar_init(base + S::FINAL + 8 * w, 1);
         }
+        for (uint32_t s = 0; s < S::S_SLOTS; ++s) {
+            mbar_init(base + S::S_FULL + 8 * s, 64);
+            mbar_init(base + S::S_EMPTY + 8 * s, S::EPI_WARPS);
+        }
         *abort_word = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -532,10 +553,10 @@ __global__ void __launch_bounds__(Shape<N, FMT>::THREADS, 1) lmhead_kernel(const
     tc_fence_after();
     const uint32_t tmem = *tmem_word;
 
-    // The weights do not come from the launch before this one, and what came before
+    // The weights and scales do not come from the launch before this one, and what came before
     // that has completed (see prepare_hidden_kernel): their loads start at once.
     bool bf16 = false;
-    if (warp != WARP_LOAD_W) {
+    if (warp != WARP_LOAD_W && (warp & ~1u) != WARP_LOAD_S0) {
         asm volatile("griddepcontrol.wait;" ::: "memory");
         uint32_t inexact = 0;
         for (uint32_t t = lane; t < N; t += 32u) {
@@ -666,7 +687,30 @@ __global__ void __launch_bounds__(Shape<N, FMT>::THREADS, 1) lmhead_kernel(const
                 }
             }
             __syncwarp();
-        }  // (two idle warps fill up their warpgroup)
+        } else {
+            // ---- two warps ask for the scales (and biases) of every unit, a row's 16 bytes a copy
+            const uint32_t r0 = tid - 32u * (uint32_t)WARP_LOAD_S0;
+            for (uint32_t n = 0; n < n_blocks; ++n) {
+                const uint32_t slot = n % S::S_SLOTS, unit = unit_at(n), to = base + S::SCALES + slot * S::S_SLOT_BYTES;
+                if (__any_sync(FULL, wait(S::S_EMPTY + 8 * slot, (n / S::S_SLOTS) ^ 1u))) {
+                    break;
+                }
+                const uint32_t tile = unit / per_tile, first = unit % per_tile * BLOCK_GROUPS;
+#pragma unroll
+                for (uint32_t i = 0; i < TILE_ROWS / 64u; ++i) {
+                    const uint32_t trow = r0 + 64u * i;
+                    const uint64_t at = (uint64_t)min(tile * TILE_ROWS + trow, a.rows - 1u) * a.scale_ld + first;
+                    copy_async16(to + trow * 16u, a.scales + at);
+                    if (AFFINE) {
+                        copy_async16(to + S::S_ARRAY_BYTES + trow * 16u, a.biases + at);
+                    }
+                }
+                // (The barrier counts this thread once its copies are there.)
+                asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(base + S::S_FULL + 8 * slot) : "memory");
+            }
+            // (Whether or not the block has given up: nothing is on its way when it ends.)
+            asm volatile("cp.async.wait_all;" ::: "memory");
+        }
     } else if (warp < (uint32_t)S::WARP_EPI0) {
         set_registers<S::REGS_CONV, false>();
         // ---- bytes in; one thread per tile row widens them into tensor memory. With two
@@ -828,16 +872,29 @@ __global__ void __launch_bounds__(Shape<N, FMT>::THREADS, 1) lmhead_kernel(const
         uint32_t tile = unit_at(0) / per_tile, blk = unit_at(0) % per_tile, q = 0;
         for (uint32_t n = 0; n < n_blocks; ++n) {
             const uint32_t row = tile * TILE_ROWS + trow;
-            const uint32_t rowc = min(row, a.rows - 1u);
-            const uint4 sc = __ldg(reinterpret_cast<const uint4 *>(a.scales + (uint64_t)rowc * a.scale_ld) + blk);
-            const uint32_t sw[4] = {sc.x, sc.y, sc.z, sc.w};
-            uint32_t bw[4] = {0, 0, 0, 0};
-            if (AFFINE) {
-                const uint4 bi = __ldg(reinterpret_cast<const uint4 *>(a.biases + (uint64_t)rowc * a.scale_ld) + blk);
-                bw[0] = bi.x;
-                bw[1] = bi.y;
-                bw[2] = bi.z;
-                bw[3] = bi.w;
+            uint32_t sw[4], bw[4] = {0, 0, 0, 0};
+            {
+                const uint32_t slot = n % S::S_SLOTS;
+                if (__any_sync(FULL, wait(S::S_FULL + 8 * slot, n / S::S_SLOTS))) {
+                    goto epilogue_out;
+                }
+                const uint4 *from = reinterpret_cast<const uint4 *>(base_ptr + S::SCALES + slot * S::S_SLOT_BYTES) + trow;
+                const uint4 sc = from[0];
+                sw[0] = sc.x;
+                sw[1] = sc.y;
+                sw[2] = sc.z;
+                sw[3] = sc.w;
+                if (AFFINE) {
+                    const uint4 bi = from[TILE_ROWS];
+                    bw[0] = bi.x;
+                    bw[1] = bi.y;
+                    bw[2] = bi.z;
+                    bw[3] = bi.w;
+                }
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(base + S::S_EMPTY + 8 * slot);
+                }
             }
             if (n == n_blocks - rest) {  // (rest = 0: never) on from where the block before stopped
                 const uint64_t t0 = global_ns();
