@@ -147,6 +147,19 @@ __device__ __forceinline__ uint64_t global_ns() {
     return t;
 }
 
+// Whether the phase with the given parity is complete; waits for a while if it is not.
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return done != 0u;
+}
+
 // Waits for the phase with the given parity to complete, for at most
 // `limit_ns`; once any wait of the block has run out, none blocks any more.
 // Returns true if it gave up (this wait ran out, or another had): the caller
@@ -157,15 +170,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
                                           uint64_t limit_ns) {
     uint64_t t0 = 0;
     for (uint32_t spin = 0;; ++spin) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(done)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (done) {
+        if (mbar_try(bar, parity)) {
             return false;
         }
         if ((spin & 15u) == 15u) {
@@ -181,6 +186,20 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
             }
         }
     }
+}
+
+// The same for a whole warp, whose lanes go on together: most waits find their phase complete,
+// or complete while the first look waits, and then cost a look, a vote and a branch that no
+// lane takes alone. (The kernel is bound by what its warps issue, and a group has some 36 waits: 12
+// instructions each with the vote behind a loop of each lane's own, 8 so; a group's 2525 became
+// 2383. 64 tokens, symmetric 248 -> 243.5 us, affine bytes 288.5 -> 283, 4 bits, 32 tokens 58.4 -> 57.3;
+// sizes at launch_head.)
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile uint32_t *abort_word,
+                                          uint64_t limit_ns) {
+    if (__all_sync(0xFFFFFFFFu, mbar_try(bar, parity))) {
+        return false;
+    }
+    return __any_sync(0xFFFFFFFFu, mbar_wait(bar, parity, abort_word, limit_ns));
 }
 
 // The same wait for the way out of a block that has given up: it does not look
@@ -514,6 +533,7 @@ __global__ void __launch_bounds__(Shape<N, FMT>::THREADS, 1) lmhead_kernel(const
     const uint32_t n_stages = n_blocks * STAGES_PER_BLOCK, total_groups = n_blocks * BLOCK_GROUPS;
     // (Wait's results: true means that the block has given up.)
     auto wait = [&](uint32_t bar, uint32_t phase) -> bool { return mbar_wait(base + bar, phase & 1u, abort_word, wait_ns); };
+    auto wait_all = [&](uint32_t bar, uint32_t phase) -> bool { return warp_wait(base + bar, phase & 1u, abort_word, wait_ns); };
 
     if (tid == 0) {
         for (uint32_t s = 0; s < S::RAW_STAGES; ++s) {
@@ -580,10 +600,9 @@ __global__ void __launch_bounds__(Shape<N, FMT>::THREADS, 1) lmhead_kernel(const
             const uint32_t acc0 = tmem + half * 256u, a0 = acc0 + S::A_COL0;
             for (uint32_t q = mw >> 1; q < total_groups / S::PG; q += MMA_WARPS / 2) {
                 const uint32_t as = q % S::A_SLOTS, hs = q * S::PG % S::H_SLOTS, b = q % S::ACC_BUFS;
-                bool gave_up = wait(S::H_FULL + 8 * (hs / 2u), q * S::PG / S::H_SLOTS);
-                gave_up |= wait(S::ACC_EMPTY + 8 * (half * S::ACC_BUFS + b), (q / S::ACC_BUFS) ^ 1u);
-                gave_up |= wait(S::A_FULL + 8 * (half * S::A_SLOTS + as), q / S::A_SLOTS);
-                if (__any_sync(FULL, gave_up)) {
+                if (wait_all(S::H_FULL + 8 * (hs / 2u), q * S::PG / S::H_SLOTS) ||
+                    wait_all(S::A_FULL + 8 * (half * S::A_SLOTS + as), q / S::A_SLOTS) ||
+                    wait_all(S::ACC_EMPTY + 8 * (half * S::ACC_BUFS + b), (q / S::ACC_BUFS) ^ 1u)) {
                     break;
                 }
                 tc_fence_after();
@@ -692,7 +711,7 @@ __global__ void __launch_bounds__(Shape<N, FMT>::THREADS, 1) lmhead_kernel(const
             const uint32_t r0 = tid - 32u * (uint32_t)WARP_LOAD_S0;
             for (uint32_t n = 0; n < n_blocks; ++n) {
                 const uint32_t slot = n % S::S_SLOTS, unit = unit_at(n), to = base + S::SCALES + slot * S::S_SLOT_BYTES;
-                if (__any_sync(FULL, wait(S::S_EMPTY + 8 * slot, (n / S::S_SLOTS) ^ 1u))) {
+                if (wait_all(S::S_EMPTY + 8 * slot, (n / S::S_SLOTS) ^ 1u)) {
                     break;
                 }
                 const uint32_t tile = unit / per_tile, first = unit % per_tile * BLOCK_GROUPS;
@@ -724,8 +743,7 @@ __global__ void __launch_bounds__(Shape<N, FMT>::THREADS, 1) lmhead_kernel(const
             constexpr bool BF16 = decltype(wide_exponent)::value;
             for (uint32_t i = 0; i < n_stages; ++i) {
                 const uint32_t st = i % S::RAW_STAGES;
-                // (the vote takes the place of a __syncwarp: the lanes leave together)
-                if (__any_sync(FULL, wait(S::RAW_FULL + 8 * st, i / S::RAW_STAGES))) {
+                if (wait_all(S::RAW_FULL + 8 * st, i / S::RAW_STAGES)) {
                     return;
                 }
                 const uint32_t raw_row = base + S::RAW + st * RAW_STAGE_BYTES + trow * 128u;
@@ -759,12 +777,8 @@ __global__ void __launch_bounds__(Shape<N, FMT>::THREADS, 1) lmhead_kernel(const
                         }
                     };
                     auto slot_free = [&]() -> bool {  // the slot's last user has been multiplied
-                        bool gave_up = false;
-                        if (q >= S::A_SLOTS) {
-                            const uint32_t before = q - S::A_SLOTS;
-                            gave_up = wait(S::DONE + 8 * (half * S::DONE_SLOTS + before % S::DONE_SLOTS), before / S::DONE_SLOTS);
-                        }
-                        return !__any_sync(FULL, gave_up);
+                        const uint32_t before = q - S::A_SLOTS;
+                        return q < S::A_SLOTS || !wait_all(S::DONE + 8 * (half * S::DONE_SLOTS + before % S::DONE_SLOTS), before / S::DONE_SLOTS);
                     };
                     const uint32_t to = a_base + (as * S::PG + (S::PG == 2u ? team : 0u)) * 32u;
                     if (!S::LEAN) {
@@ -844,6 +858,11 @@ __global__ void __launch_bounds__(Shape<N, FMT>::THREADS, 1) lmhead_kernel(const
         for (uint32_t m = 0; m < P; ++m) {
             acc[m] = 0ull;
         }
+        // (At 16 tokens, where the weights' stream is the bound, the look by itself is the faster form here:
+        // affine bytes, 4 tokens, 171.2 us against 174.5.)
+        auto gave_up_on = [&](uint32_t bar, uint32_t phase) -> bool {
+            return N == 16u ? __any_sync(FULL, wait(bar, phase)) != 0 : wait_all(bar, phase);
+        };
         auto write_out = [&](uint32_t row) {
             if (row < a.rows) {
 #pragma unroll
@@ -875,7 +894,7 @@ __global__ void __launch_bounds__(Shape<N, FMT>::THREADS, 1) lmhead_kernel(const
             uint32_t sw[4], bw[4] = {0, 0, 0, 0};
             {
                 const uint32_t slot = n % S::S_SLOTS;
-                if (__any_sync(FULL, wait(S::S_FULL + 8 * slot, n / S::S_SLOTS))) {
+                if (wait_all(S::S_FULL + 8 * slot, n / S::S_SLOTS)) {
                     goto epilogue_out;
                 }
                 const uint4 *from = reinterpret_cast<const uint4 *>(base_ptr + S::SCALES + slot * S::S_SLOT_BYTES) + trow;
@@ -921,7 +940,7 @@ __global__ void __launch_bounds__(Shape<N, FMT>::THREADS, 1) lmhead_kernel(const
                 const float s = __uint_as_float((gi & 1u) ? (sw[gi >> 1] & 0xFFFF0000u) : (sw[gi >> 1] << 16));
                 const uint64_t s2 = pack2(__float_as_uint(s), __float_as_uint(s));
                 if (gi % S::PG == 0u) {
-                    if (__any_sync(FULL, wait(S::DONE + 8 * (half * S::DONE_SLOTS + p % S::DONE_SLOTS), p / S::DONE_SLOTS))) {
+                    if (gave_up_on(S::DONE + 8 * (half * S::DONE_SLOTS + p % S::DONE_SLOTS), p / S::DONE_SLOTS)) {
                         goto epilogue_out;  // the block has given up: nothing more is read or written
                     }
                     tc_fence_after();
