@@ -199,40 +199,15 @@ static __device__ __noinline__ uint4 edge_vec(const T *row_ptr, uint32_t vocab, 
 }
 
 
-// The draw of a row that keeps more than 64 candidates, sorted in `best`: the
-// softmax weights, the prefix sums in rank order with one rounding per add
-// (tests/unit/kernels/sample.rs:37-46), the cut, the draw. All SPL_NT threads.
-__device__ __forceinline__ void split_finalize_wide(SmemFixed *sm, SplitSmem *ss, const unsigned long long *best,
-                                                    const KArgs &a, uint32_t row, uint32_t n, float top_p, float min_p,
-                                                    float u, bool counts_draw, uint32_t slot) {
+// The sum of p[0, 4 * tid), added up in rank order with one rounding per add
+// (tests/unit/kernels/sample.rs:37-46), for each of the SPL_NT threads; the sum of all n of them goes to
+// ss->least. p: KCAP weights, those past n are 0. Here by one thread, a chain of n dependent adds.
+__device__ __forceinline__ float chain_of_sums(SplitSmem *ss, const float *p, uint32_t n) {
     const uint32_t tid = threadIdx.x;
-    float *p = reinterpret_cast<float *>(sm->tkey), *cum = reinterpret_cast<float *>(sm->tid);
-    const float top = float_of_key((uint32_t)(best[0] >> 32));
-    if (top == neg_inf() || top == -neg_inf()) {
-        if (tid == 0) {
-            a.out_ids[row] = 0xFFFFFFFFu;
-            if (a.out_status) {
-                a.out_status[row] = LILY_ROW_NONFINITE;
-            }
-            if (a.kept_n) {
-                a.kept_n[row] = 0;
-            }
-            atomicOr(a.status_word, 1u << LILY_ROW_NONFINITE);
-        }
-        return;
-    }
-    for (uint32_t i = tid; i < KCAP; i += SPL_NT) {
-        p[i] = i < n ? exp_f32(__fsub_rn(float_of_key((uint32_t)(best[i] >> 32)), top)) : 0.0f;
-    }
-    if (tid == 0) {
-        ss->n_live = n;   // the first rank that is not kept
-        ss->bin = n;      // the first rank whose prefix sum exceeds the target
-    }
-    spl_sync();
     float *ends = reinterpret_cast<float *>(ss->tmax);  // sums up to every fourth rank (the maxima have served)
     static_assert(KCAP / 4u == SPL_NT, "four ranks a thread");
     if (tid == 0) {
-        // A chain of n dependent adds; all that stands beside it is a load of four weights and the
+        // All that stands beside the adds is a load of four weights and the
         // store of every fourth sum. (Ranks past n weigh 0, and s + 0 is s. With every sum stored,
         // and the weights loaded ahead moved from register to register, an add took 8 clocks
         // instead of 4.5: 1024 kept, 8100 -> 4560 clocks.)
@@ -268,10 +243,151 @@ __device__ __forceinline__ void split_finalize_wide(SmemFixed *sm, SplitSmem *ss
         ss->least = s;  // (what it held has served)
     }
     spl_sync();
+    return tid != 0u ? ends[tid - 1u] : 0.0f;
+}
+
+// The same sums without the chain. While the sum stays between two powers of two it is a multiple
+// of its last place u, and adding x adds x rounded to a multiple of u, whatever the sum is (but
+// for a tie, which goes by the sum's last bit). So every thread finds from approximate sums, with a
+// margin above what n roundings can do, which power of two its four adds lie at; where that is one and no
+// add ties, it rounds its weights by itself, and these add up exactly, in any order, as integers in
+// units of 2^-23. Some eleven threads are left, those in which the sum passes a power of two: one thread
+// makes their adds one after the other, with what lies between two of them as one more, exact,
+// add. 1024 kept: 4560 clocks of a chain become some 1700. Up to CHAIN_MAX the chain is the shorter
+// (3 x 151936 f32, by the chain and so: 320 kept 12.60 and 12.66 us, 384 12.86 and 12.76, 512 13.58 and
+// 13.16, 1024 16.94 and 15.49).
+constexpr uint32_t CHAIN_MAX = 384;
+__device__ __forceinline__ float sums_in_rank_order(SmemFixed *sm, SplitSmem *ss, const float *p, uint32_t n) {
+    constexpr unsigned FULL = 0xFFFFFFFFu;
+    constexpr uint32_t LIST = 32;       // threads whose adds are made one after the other, at most
+    constexpr float UNIT = 8388608.0f;  // 2^23
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    static_assert(KCAP / 4u == SPL_NT && SPL_WARPS == 8u, "four ranks a thread");
+    // (Over the maxima, which have served.)
+    float *totals = reinterpret_cast<float *>(ss->tmax), *after = totals + 8;
+    uint32_t *whole = ss->tmax + 64, *count = whole + 8, *list_at = whole + 16;
+    float4 *list_x = reinterpret_cast<float4 *>(ss->tmax + 128);
+    const float4 x = reinterpret_cast<const float4 *>(p)[tid];
+    float incl = __fadd_rn(__fadd_rn(x.x, x.y), __fadd_rn(x.z, x.w));
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const float t = __shfl_up_sync(FULL, incl, o);
+        incl = lane >= (uint32_t)o ? __fadd_rn(incl, t) : incl;
+    }
+    if (lane == 31u) {
+        totals[warp] = incl;
+    }
+    const float up = __shfl_up_sync(FULL, incl, 1);
+    spl_sync();
+    float before = 0.0f;
+#pragma unroll
+    for (uint32_t w = 0; w < SPL_WARPS; ++w) {
+        before = w < warp ? __fadd_rn(before, totals[w]) : before;
+    }
+    // (1024 adds are off by less than 2^-14 of the sum, these sums by less than 2^-19.)
+    constexpr float MARGIN = 1.220703125e-4f;  // 2^-13
+    const uint32_t lo = __float_as_uint(__fmul_rn(lane != 0u ? __fadd_rn(before, up) : before, 1.0f - MARGIN));
+    const uint32_t hi = __float_as_uint(__fmul_rn(__fadd_rn(before, incl), 1.0f + MARGIN));
+    const float power = __uint_as_float(lo & 0x7F800000u);
+    auto rounded = [&](float v) -> float { return __fsub_rn(__fadd_rn(v, power), power); };  // (v at most `power`)
+    const float rx = rounded(x.x), ry = rounded(x.y), rz = rounded(x.z), rw = rounded(x.w);
+    const float tie = __fmul_rn(power, 5.9604644775390625e-8f);  // half of the last place
+    const bool ties = fabsf(__fsub_rn(x.x, rx)) == tie || fabsf(__fsub_rn(x.y, ry)) == tie ||
+                      fabsf(__fsub_rn(x.z, rz)) == tie || fabsf(__fsub_rn(x.w, rw)) == tie;
+    // (A thread past the last rank adds nothing. Below 512 a run between two powers fits 32 bits.)
+    const bool dead = 4u * tid >= n;
+    const bool one_by_one = !dead && (((lo ^ hi) >> 23) != 0u || ties || power < 1.0f || power > 512.0f ||
+                                      fmaxf(fmaxf(x.x, x.y), fmaxf(x.z, x.w)) > power);
+    uint32_t units = 0;
+    if (!dead && !one_by_one) {
+        units = __float2uint_rn(__fmul_rn(__fadd_rn(__fadd_rn(rx, ry), __fadd_rn(rz, rw)), UNIT));
+    }
+    uint32_t sum = units;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(FULL, sum, o);
+        sum += lane >= (uint32_t)o ? t : 0u;
+    }
+    const unsigned who = __ballot_sync(FULL, one_by_one);
+    if (lane == 31u) {
+        whole[warp] = sum;
+        count[warp] = __popc(who);
+    }
+    spl_sync();
+    uint32_t at = sum - units, j = __popc(who & ((1u << lane) - 1u)), n_list = 0;
+#pragma unroll
+    for (uint32_t w = 0; w < SPL_WARPS; ++w) {
+        at += w < warp ? whole[w] : 0u;
+        j += w < warp ? count[w] : 0u;
+        n_list += count[w];
+    }
+    if (n_list > LIST) {  // (a tail of hardly anything beside a power of two)
+        spl_sync();
+        return chain_of_sums(ss, p, n);
+    }
+    if (one_by_one) {
+        list_at[j] = at;
+        list_x[j] = x;
+    }
+    if (tid == SPL_NT - 1u) {
+        list_at[n_list] = at + units;
+    }
+    spl_sync();
+    auto exact = [&](uint32_t u) -> float { return __fmul_rn(__uint2float_rn(u), 1.0f / UNIT); };
+    if (tid == 0) {
+        float s = 0.0f;
+        float4 v = list_x[0];  // (rank 0 is always one of them)
+        uint32_t here = list_at[0];
+        for (uint32_t i = 0; i < n_list; ++i) {
+            const float4 next_v = list_x[min(i + 1u, LIST - 1u)];
+            const uint32_t next = list_at[i + 1u];
+            s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, v.x), v.y), v.z), v.w);
+            after[i] = s;
+            s = __fadd_rn(s, exact(next - here));
+            v = next_v;
+            here = next;
+        }
+        ss->least = s;  // (what it held has served)
+    }
+    spl_sync();
+    return j != 0u ? __fadd_rn(after[j - 1u], exact(at - list_at[j - 1u])) : 0.0f;
+}
+
+// The draw of a row that keeps more than 64 candidates, sorted in `best`: the
+// softmax weights, the prefix sums in rank order with one rounding per add
+// (tests/unit/kernels/sample.rs:37-46), the cut, the draw. All SPL_NT threads.
+__device__ __forceinline__ void split_finalize_wide(SmemFixed *sm, SplitSmem *ss, const unsigned long long *best,
+                                                    const KArgs &a, uint32_t row, uint32_t n, float top_p, float min_p,
+                                                    float u, bool counts_draw, uint32_t slot) {
+    const uint32_t tid = threadIdx.x;
+    float *p = reinterpret_cast<float *>(sm->tkey), *cum = reinterpret_cast<float *>(sm->tid);
+    const float top = float_of_key((uint32_t)(best[0] >> 32));
+    if (top == neg_inf() || top == -neg_inf()) {
+        if (tid == 0) {
+            a.out_ids[row] = 0xFFFFFFFFu;
+            if (a.out_status) {
+                a.out_status[row] = LILY_ROW_NONFINITE;
+            }
+            if (a.kept_n) {
+                a.kept_n[row] = 0;
+            }
+            atomicOr(a.status_word, 1u << LILY_ROW_NONFINITE);
+        }
+        return;
+    }
+    for (uint32_t i = tid; i < KCAP; i += SPL_NT) {
+        p[i] = i < n ? exp_f32(__fsub_rn(float_of_key((uint32_t)(best[i] >> 32)), top)) : 0.0f;
+    }
+    if (tid == 0) {
+        ss->n_live = n;   // the first rank that is not kept
+        ss->bin = n;      // the first rank whose prefix sum exceeds the target
+    }
+    spl_sync();
+    const float before_mine = n > CHAIN_MAX ? sums_in_rank_order(sm, ss, p, n) : chain_of_sums(ss, p, n);
     // Every thread its four ranks' sums, the same adds once more, and the cut.
     const float limit = __fmul_rn(top_p, ss->least);
     if (4u * tid < n) {
-        float before = tid != 0u ? ends[tid - 1u] : 0.0f;
+        float before = before_mine;
         const float4 x = reinterpret_cast<const float4 *>(p)[tid];
         const float w[4] = {x.x, x.y, x.z, x.w};
         float c[4];
@@ -522,23 +638,29 @@ __device__ __forceinline__ void spec_ahead(const SpecArgs &s, uint32_t row, uint
 __device__ __forceinline__ void rank_sums(const float *w, uint32_t n, float &c0, float &c1) {
     const uint32_t lane = threadIdx.x & 31u;
     const float4 *w4 = reinterpret_cast<const float4 *>(w);
+    // (Eight loads at a time: one in front of its four adds cost each add 20 clocks instead of 5.)
+    auto half = [&](uint32_t first, float &c) {
+        float4 v[8];
+#pragma unroll
+        for (uint32_t i = 0; i < 8u; ++i) {
+            v[i] = w4[first / 4u + i];
+        }
+#pragma unroll
+        for (uint32_t i = 0; i < 8u; ++i) {
+            const uint32_t at = first + 4u * i, mine = lane + first;
+            if (at < n) {
+                c = mine >= at ? __fadd_rn(c, v[i].x) : c;
+                c = mine >= at + 1u ? __fadd_rn(c, v[i].y) : c;
+                c = mine >= at + 2u ? __fadd_rn(c, v[i].z) : c;
+                c = mine >= at + 3u ? __fadd_rn(c, v[i].w) : c;
+            }
+        }
+    };
     c0 = 0.0f;
-#pragma unroll 2
-    for (uint32_t i = 0; i < 32u && i < n; i += 4u) {
-        const float4 v = w4[i >> 2];
-        c0 = lane >= i ? __fadd_rn(c0, v.x) : c0;
-        c0 = lane >= i + 1u ? __fadd_rn(c0, v.y) : c0;
-        c0 = lane >= i + 2u ? __fadd_rn(c0, v.z) : c0;
-        c0 = lane >= i + 3u ? __fadd_rn(c0, v.w) : c0;
-    }
+    half(0u, c0);
     c1 = __shfl_sync(0xFFFFFFFFu, c0, 31);
-#pragma unroll 2
-    for (uint32_t i = 32u; i < n; i += 4u) {
-        const float4 v = w4[i >> 2];
-        c1 = lane + 32u >= i ? __fadd_rn(c1, v.x) : c1;
-        c1 = lane + 32u >= i + 1u ? __fadd_rn(c1, v.y) : c1;
-        c1 = lane + 32u >= i + 2u ? __fadd_rn(c1, v.z) : c1;
-        c1 = lane + 32u >= i + 3u ? __fadd_rn(c1, v.w) : c1;
+    if (n > 32u) {
+        half(32u, c1);
     }
 }
 
@@ -1812,17 +1934,20 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
             }
         }
     } else {
-        for (uint32_t b = 0; b < buckets; ++b) {
-            const bool over = (buckets == 1u ? bm : bmax[b * SPL_NT + tid]) >= least;
-            const unsigned who = __ballot_sync(FULL, over);
-            if (who != 0u) {
-                uint32_t at = 0;
-                if (lane == 0) {
-                    at = atomicAdd(&ss->n_flagged, (uint32_t)__popc(who));
+        for (uint32_t b0 = 0; b0 < buckets; b0 += 32u) {
+            uint32_t over = buckets == 1u && bm >= least ? 1u : 0u;
+            if (buckets != 1u) {
+                const float *mine = bmax + b0 * SPL_NT + tid;
+                const uint32_t end = min(buckets - b0, 32u);
+#pragma unroll 4
+                for (uint32_t b = 0; b < end; ++b) {
+                    over |= mine[b * SPL_NT] >= least ? 1u << b : 0u;
                 }
-                at = __shfl_sync(FULL, at, 0) + __popc(who & ((1u << lane) - 1u));
-                if (over && at < SPL_FLAGGED) {
-                    ss->flagged[at] = (uint16_t)(b * SPL_NT + tid);
+            }
+            if (over != 0u) {  // (few threads: an add each is sooner there than a vote and an add a bucket)
+                uint32_t at = atomicAdd(&ss->n_flagged, (uint32_t)__popc(over));
+                for (; over != 0u && at < SPL_FLAGGED; over &= over - 1u) {
+                    ss->flagged[at++] = (uint16_t)((b0 + (uint32_t)__ffs(over) - 1u) * SPL_NT + tid);
                 }
             }
         }

@@ -367,3 +367,33 @@ def test_rows_that_keep_many_at_the_edges_of_their_runs(cuda, lily, W, rows, voc
         assert s.status() == lily.OK
         s.close()
     assert min(ended.values()) > 0, ended
+
+
+@pytest.mark.parametrize("kind", ["flat", "coarse", "even", "steep", "beside a power of two"])
+def test_sums_of_many_weights_bit_for_bit(cuda, lily, W, kind):
+    """The prefix sums of a row that keeps more than 384 are not one chain of adds, but have its bits:
+    draws at sums and the values beside them, and the kept probabilities (weight / sum of all) bit for
+    bit. Equal weights; weights that tie when they are rounded to the sum's last place; a tail that
+    leaves the sum at a power of two for hundreds of adds (a chain after all)."""
+    vocab, rows = 40_000, 8
+    i = np.arange(vocab)
+    profile = {"flat": np.maximum(i - 1400, 0) * -0.01, "coarse": i // 100 / -8.0, "even": i * -0.0005, "steep": i * -0.02,
+               "beside a power of two": np.where(i < 256, 0.0, -10.0 - 0.0005 * (i - 256))}[kind].astype(np.float32)
+    rng = np.random.default_rng(len(kind))
+    s = lily.SamplerScratch(vocab, max_rows=rows)
+    for k in (384, 385, 388, 511, 778, 1023, 1024):
+        x = np.stack([rng.permutation(profile) for _ in range(rows)])
+        b = W.Batch(x, False, [dict(temperature=1.0, top_k=k, seed=r) for r in range(rows)], np.zeros(rows, np.float32))
+        for at in (0.999, 0.51, 0.1, 0.003):
+            for r, d in enumerate(oracle_rows(b)):  # u: a prefix sum over the mass, or up to three floats beside it
+                n = len(d.kept_ids)  # (fewer than k where a tail adds nothing any more: the sum before it is all)
+                assert n == k or kind == "steep"
+                u = np.cumsum(d.kept_prob.astype(np.float32), dtype=np.float32)[int(at * n)].view(np.uint32)
+                b.uniforms[r] = min((u + np.uint32(r) - np.uint32(4)).view(np.float32), np.float32(1 - 2.0 ** -24))
+            want, res = oracle_rows(b), run_batch(cuda, lily, s, b)
+            assert_parity(b, res, want, label=f"{kind} k={k} at {at}")
+            for r, d in enumerate(want):
+                bits = d.kept_prob.astype(np.float32).view(np.uint32)
+                assert np.array_equal(res.kept_probs[r, :len(bits)].view(np.uint32), bits), f"{kind} k={k} row {r}"
+    assert s.status() == lily.OK
+    s.close()
