@@ -71,6 +71,7 @@ struct lily_sampler {
     int ring_pos = 0;
     uint32_t *h_status = nullptr;
     uint32_t attr_mask = 0;  // kernel variants whose shared-memory limit is raised
+    uint64_t split_mask = 0;  // likewise, of the row kernel
     long long *phase_clocks = nullptr;
     // The parameters a sharded call staged last: a decode step stages the same
     // rows for its candidate call and its merge call, and usually again next step.
@@ -386,7 +387,7 @@ SplitPlan split_plan(const lily_sampler *h, const lily::KArgs &a, uint32_t rows,
 
 template <uint32_t MAXR>
 int32_t launch_split(lily_sampler *h, cudaStream_t stream, lily::SplitArgs<MAXR> &sa, const SplitPlan &p,
-                     uint32_t rows, uint32_t dtype) {
+                     uint32_t has, uint32_t rows, uint32_t dtype) {
     sa.log_blocks = p.log_blocks;
     sa.log_live = p.log_live;
     sa.two_per_sm = p.sole ? 0u : 1u;
@@ -395,7 +396,7 @@ int32_t launch_split(lily_sampler *h, cudaStream_t stream, lily::SplitArgs<MAXR>
     sa.wait_ns = h->wait_ns;
     sa.lost = h->lost_arrival;
     h->lost_arrival = 0;  // one launch only
-    CU(h, lily::split_launch<MAXR>(sa, rows, dtype, p.smem, h->max_smem, &h->attr_mask, stream));
+    CU(h, lily::split_launch<MAXR>(sa, has, rows, dtype, p.smem, h->max_smem, &h->split_mask, stream));
     return LILY_OK;
 }
 
@@ -414,13 +415,17 @@ int32_t launch_split_inline(lily_sampler *h, cudaStream_t stream, const lily::KA
     sa.inline_params = 1;
     sa.inline_slots = slots != nullptr ? 1u : 0u;
     sa.inline_history = inline_history;
+    uint32_t has = (a.cand_out != nullptr ? lily::HAS_SHARD : 0u) | (a.spec.n_spec != 0u ? lily::HAS_SPEC : 0u) |
+                   (a.bias_ids != nullptr || a.ban_ids != nullptr ? lily::HAS_LISTS : 0u);
     for (uint32_t r = 0; r < rows; ++r) {
         sa.in[r] = lily::row_in(params[r], steps != nullptr ? steps[r] : 0u);
+        has |= (sa.in[r].k > lily::SPL_SMALL_K && a.cand_out == nullptr ? lily::HAS_WIDE : 0u) |
+               (sa.in[r].flags & lily::ROW_RAISES ? lily::HAS_RAISES : 0u);
     }
     if (slots != nullptr) {
         std::memcpy(sa.slots, slots, sizeof(uint32_t) * rows);
     }
-    return launch_split(h, stream, sa, p, grid_rows ? grid_rows : rows, dtype);
+    return launch_split(h, stream, sa, p, has, grid_rows ? grid_rows : rows, dtype);
 }
 
 // The argument block that holds the rows' parameters.
@@ -448,7 +453,9 @@ int32_t launch(lily_sampler *h, cudaStream_t stream, const lily::KArgs &a, uint3
         lily::SplitArgs<INLINE_ROWS> sa;
         sa.a = a;
         sa.inline_params = sa.inline_slots = sa.inline_history = 0;
-        return launch_split(h, stream, sa, plan, rows, dtype);
+        // (Parameters on the device: what their rows keep is not known here.)
+        return launch_split(h, stream, sa, plan, a.force_greedy && a.cand_out == nullptr ? lily::HAS_ARGMAX : lily::HAS_ALL, rows,
+                            dtype);
     }
     const size_t esize = dtype == LILY_F32 ? 4 : 2;
     const bool vec = (reinterpret_cast<uintptr_t>(a.logits) % 16u == 0u) &&

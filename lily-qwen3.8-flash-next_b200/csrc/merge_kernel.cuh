@@ -133,7 +133,7 @@ static __global__ void __launch_bounds__(NT, 2) merge_rows_kernel(const __grid_c
     SpecAhead ahead;
     ahead.draft = ahead.n_q = ahead.id0 = ahead.id1 = 0;
     ahead.q_draft = ahead.p0 = ahead.p1 = 0.0f;
-    split_finalize(sm, a, row, n, in.top_p, in.min_p, u, 0u, in.seed, false, 0u, ahead);
+    split_finalize<false>(sm, a, row, n, in.top_p, in.min_p, u, 0u, in.seed, false, 0u, ahead);
     if (lane == 0u && sm->err) {
         atomicOr(a.status_word, 1u << (sm->err & 31u));
     }

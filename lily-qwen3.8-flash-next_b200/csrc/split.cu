@@ -1,62 +1,13 @@
-// The row kernel's and the merge kernel's translation unit: instantiations and launches.
+// The row kernel for up to 8 rows' parameters, and the merge kernel.
 #include <atomic>
 
 #include "merge_kernel.cuh"
+#include "split_launch.cuh"
 
 namespace lily {
 
-namespace {
-
-template <typename T, uint32_t MAXR, int BPS>
-cudaError_t launch_one(const SplitArgs<MAXR> &a, uint32_t rows, size_t smem, int max_smem, uint32_t *attr_mask,
-                       cudaStream_t stream) {
-    auto kernel = split_rows_kernel<T, MAXR, BPS>;
-    const uint32_t bit = 1u << ((sizeof(T) == 4 ? 16 : 17) + (MAXR == INLINE_ROWS ? 0 : MAXR == INLINE_ROWS_MID ? 2 : 4) + (BPS == 1 ? 0 : 7));
-    if (!(*attr_mask & bit)) {
-        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
-        if (e != cudaSuccess) {
-            return e;
-        }
-        *attr_mask |= bit;
-    }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(1u << a.log_blocks, rows, 1);
-    cfg.blockDim = dim3(NT, 1, 1);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = 1u << a.log_blocks;
-    attr[1].val.clusterDim.y = 1;
-    attr[1].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = a.log_blocks ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, kernel, a);
-}
-
-}  // namespace
-
-template <uint32_t MAXR>
-cudaError_t split_launch(const SplitArgs<MAXR> &a, uint32_t rows, uint32_t dtype, size_t smem, int max_smem,
-                         uint32_t *attr_mask, cudaStream_t stream) {
-    if constexpr (MAXR == INLINE_ROWS) {
-        if (a.two_per_sm) {
-            return dtype == LILY_F32 ? launch_one<float, MAXR, 2>(a, rows, smem, max_smem, attr_mask, stream)
-                                     : launch_one<__nv_bfloat16, MAXR, 2>(a, rows, smem, max_smem, attr_mask, stream);
-        }
-    }
-    return dtype == LILY_F32 ? launch_one<float, MAXR, 1>(a, rows, smem, max_smem, attr_mask, stream)
-                             : launch_one<__nv_bfloat16, MAXR, 1>(a, rows, smem, max_smem, attr_mask, stream);
-}
-
-template cudaError_t split_launch<INLINE_ROWS>(const SplitArgs<INLINE_ROWS> &, uint32_t, uint32_t, size_t, int, uint32_t *,
-                                               cudaStream_t);
-template cudaError_t split_launch<INLINE_ROWS_MID>(const SplitArgs<INLINE_ROWS_MID> &, uint32_t, uint32_t, size_t, int,
-                                                   uint32_t *, cudaStream_t);
-template cudaError_t split_launch<INLINE_ROWS_MAX>(const SplitArgs<INLINE_ROWS_MAX> &, uint32_t, uint32_t, size_t, int,
-                                                   uint32_t *, cudaStream_t);
+template cudaError_t split_launch<INLINE_ROWS>(const SplitArgs<INLINE_ROWS> &, uint32_t, uint32_t, uint32_t, size_t, int,
+                                               uint64_t *, cudaStream_t);
 
 uint32_t split_rows_at_once(int device, int sm_count, int max_smem, uint32_t log_blocks) {
     if (log_blocks == 0u) {
@@ -68,7 +19,7 @@ uint32_t split_rows_at_once(int device, int sm_count, int max_smem, uint32_t log
     std::atomic<uint32_t> *at = device >= 0 && device < DEVICES ? &known[device][log_blocks] : nullptr;
     uint32_t n = at ? at->load(std::memory_order_relaxed) : 0u;
     if (n == 0u) {
-        auto kernel = split_rows_kernel<float, INLINE_ROWS, 1>;
+        auto kernel = split_rows_kernel<float, INLINE_ROWS, 1, HAS_ALL>;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(1u << log_blocks, 1, 1);
         cfg.blockDim = dim3(NT, 1, 1);

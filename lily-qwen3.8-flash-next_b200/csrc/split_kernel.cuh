@@ -668,6 +668,7 @@ __device__ __forceinline__ void rank_sums(const float *w, uint32_t n, float &c0,
 // softmax weights, the prefix sums in rank order (tests/unit/kernels/sample.rs:37-46),
 // the cut, the draw (speculative: tests/unit/kernels/sample.rs:264-283, src/kernels/
 // metal/sample.metal:597-658), the outputs. lane i holds ranks i and i + 32.
+template <bool SPEC>
 __device__ __forceinline__ void split_finalize(SmemFixed *sm, const KArgs &a, uint32_t row, uint32_t n, float top_p, float min_p,
                                                float u, uint32_t step, uint64_t seed, bool counts_draw, uint32_t slot,
                                                const SpecAhead &ahead) {
@@ -677,7 +678,7 @@ __device__ __forceinline__ void split_finalize(SmemFixed *sm, const KArgs &a, ui
     const bool in0 = lane < n, in1 = lane + 32u < n;
     const uint32_t i0 = in0 ? sm->id[lane] : 0xFFFFFFFFu, i1 = in1 ? sm->id[lane + 32u] : 0xFFFFFFFFu;
     const float top = float_of_key(sm->key[0]);
-    const bool spec = row < a.spec.n_spec;
+    const bool spec = SPEC && row < a.spec.n_spec;
     float q0 = 0.0f, q1 = 0.0f;
     if (spec && a.spec.q_dense) {  // (for the residual, if it comes to that: on their way meanwhile)
         const float *q = a.spec.q_dense + (uint64_t)row * a.spec.q_ld;
@@ -1019,8 +1020,9 @@ static __device__ __noinline__ void wait_for_the_end(const SplitArgs<MAXR> &ca) 
 
 // Grid (blocks per row, rows), clusters of (blocks per row), NT threads, of which
 // SPL_NT do the work. BPS: blocks per SM the registers are cut for; with one, a
-// block whose share fits one bucket keeps it in registers.
-template <typename T, uint32_t MAXR, int BPS>
+// block whose share fits one bucket keeps it in registers. HAS: what the launch's rows may bring (split_args.cuh);
+// what they do not is not in the code.
+template <typename T, uint32_t MAXR, int BPS, uint32_t HAS>
 __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_constant__ SplitArgs<MAXR> ca) {
     constexpr unsigned FULL = 0xFFFFFFFFu;
     constexpr uint32_t NONE = 0xFFFFFFFFu;
@@ -1160,7 +1162,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
     RowIn in;
     uint32_t hist_len = 0, slot = 0;
     int32_t forced = -1;
-    if (a.force_greedy) {
+    if (HAS == HAS_ARGMAX || a.force_greedy) {
         in.temp = 1.0f;
         in.rep = in.top_p = 1.0f;
         in.presence = in.frequency = in.min_p = in.u = 0.0f;
@@ -1185,15 +1187,16 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         P.seed = (uint64_t)w4.x | ((uint64_t)w4.y << 32);
         in = row_in(P, (!a.uniforms && a.steps) ? __ldg(a.steps + row) : 0u);
     }
-    if (a.history_ids) {
+    if (HAS != HAS_ARGMAX && a.history_ids) {
         hist_len = ca.inline_history ? ca.inline_history - 1u : a.history_len ? __ldg(a.history_len + row) : 0u;
     }
-    const uint32_t n_bias = (a.bias_ids && a.bias_len) ? __ldg(a.bias_len + row) : 0u;
-    const uint32_t n_ban = (a.ban_ids && a.ban_len) ? __ldg(a.ban_len + row) : 0u;
-    if (a.forced_ids) {
+    constexpr bool LISTS = (HAS & HAS_LISTS) != 0u;
+    const uint32_t n_bias = (LISTS && a.bias_ids && a.bias_len) ? __ldg(a.bias_len + row) : 0u;
+    const uint32_t n_ban = (LISTS && a.ban_ids && a.ban_len) ? __ldg(a.ban_len + row) : 0u;
+    if (HAS != HAS_ARGMAX && a.forced_ids) {
         forced = __ldg(a.forced_ids + row);
     }
-    const bool table_mode = ca.inline_slots != 0u || a.count_slots != nullptr;
+    const bool table_mode = HAS != HAS_ARGMAX && (ca.inline_slots != 0u || a.count_slots != nullptr);
     if (table_mode) {
         slot = ca.inline_slots ? ca.slots[row] : __ldg(a.count_slots + row);
     }
@@ -1208,7 +1211,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
                n_ban > a.max_list || (a.ban_ld != 0u && n_ban > a.ban_ld)) {
         status = LILY_ROW_LIST;
     }
-    const bool use_pen = (in.flags & ROW_PEN) != 0u, need_counts = (in.flags & ROW_COUNTS) != 0u;
+    const bool use_pen = HAS != HAS_ARGMAX && (in.flags & ROW_PEN) != 0u, need_counts = (in.flags & ROW_COUNTS) != 0u;
     const bool list_mode = use_pen && !table_mode;
     if (!list_mode) {
         hist_len = 0;
@@ -1216,13 +1219,13 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
     const uint32_t extra_len = list_mode ? a.extra_len : 0u;
     // A vocabulary shard's launch ends in the row's record, not in a draw: the best shard_k
     // logits (a greedy row's best one) and, if asked for, the sum of exponentials.
-    const bool shard = a.cand_out != nullptr;
+    const bool shard = (HAS & HAS_SHARD) != 0u && a.cand_out != nullptr;
     const uint32_t k = shard && !(in.flags & ROW_GREEDY) ? a.shard_k : in.k;
-    const bool wide = k > SPL_SMALL_K;
+    const bool wide = (HAS & HAS_WIDE) != 0u && k > SPL_SMALL_K;
     const uint32_t mark_mode = ca.mark_mode;
     const bool marked = hist_len + extra_len != 0u;
     const bool counted = marked && need_counts;  // (a list whose multiplicities matter)
-    const bool raises = (in.flags & ROW_RAISES) != 0u;
+    const bool raises = (HAS & HAS_RAISES) != 0u && (in.flags & ROW_RAISES) != 0u;
     const bool emitted = raises && (table_mode || marked);
     // A row that keeps many takes its bound from at most SPL_MAX_BLOCKS * SPL_NT maxima: one of
     // every thread, or, of a short row over four or eight blocks, those of `groups` parts of a
@@ -1245,7 +1248,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
     const bool general = n_sp > SP_SMEM || (raises && marked && mark_mode == MARK_BITS) ||
                          (n_sp != 0u && mark_mode == MARK_BITS) ||
                          (list_mode && need_counts && mark_mode != MARK_COUNTS) ||
-                         (wide && (row < a.spec.n_spec || !wide_fits));
+                         (wide && (((HAS & HAS_SPEC) != 0u && row < a.spec.n_spec) || !wide_fits));
     if (status != LILY_ROW_OK || general) {
         if (status != LILY_ROW_OK && rank == 0u && tid == 0) {
             a.out_ids[row] = status == LILY_ROW_FORCED ? (uint32_t)forced : 0xFFFFFFFFu;
@@ -1266,10 +1269,10 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         }
         return;
     }
-    const bool argmax_mode = (in.flags & ROW_GREEDY) && !use_pen && n_sp == 0u;
+    const bool argmax_mode = HAS == HAS_ARGMAX || ((in.flags & ROW_GREEDY) && !use_pen && n_sp == 0u);
     const bool draws = rank == 0u && warp == 0u;  // the warp that ends up with the row
     SpecAhead ahead;
-    ahead.draft = draws && row < a.spec.n_spec ? __ldg(a.spec.draft_ids + row) : 0u;
+    ahead.draft = (HAS & HAS_SPEC) != 0u && draws && row < a.spec.n_spec ? __ldg(a.spec.draft_ids + row) : 0u;
     const float u_row = !draws ? 0.0f : a.uniforms ? __ldg(a.uniforms + row) : in.u;
 
     // ---- 1. the stream: maxima and marks
@@ -1666,7 +1669,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
     if (marked || n_sp != 0u) {
         asm volatile("bar.sync 3, %0;" ::"n"(NT) : "memory");
     }
-    if (draws && row < a.spec.n_spec) {
+    if ((HAS & HAS_SPEC) != 0u && draws && row < a.spec.n_spec) {
         spec_ahead(a.spec, row, vocab, ahead);
     }
     LILY_STAMP(PH_PASS1);
@@ -2227,8 +2230,8 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         if (shard) {
             write_record(n_ranked);
         } else {
-            split_finalize(sm, a, row, n_ranked, in.top_p, in.min_p, u_row, a.uniforms ? 0u : in.step, in.seed, counts_draw,
-                           slot, ahead);
+            split_finalize<(HAS & HAS_SPEC) != 0u>(sm, a, row, n_ranked, in.top_p, in.min_p, u_row, a.uniforms ? 0u : in.step,
+                                                   in.seed, counts_draw, slot, ahead);
         }
     }
     LILY_STAMP(PH_END);

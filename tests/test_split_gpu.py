@@ -397,3 +397,43 @@ def test_sums_of_many_weights_bit_for_bit(cuda, lily, W, kind):
                 assert np.array_equal(res.kept_probs[r, :len(bits)].view(np.uint32), bits), f"{kind} k={k} row {r}"
     assert s.status() == lily.OK
     s.close()
+
+
+@pytest.mark.parametrize("bf16", [False, True])
+@pytest.mark.parametrize("rows,vocab", [(2, 5_000), (7, 40_003), (9, 20_000), (63, 9_001), (65, 9_001), (147, 9_001)])
+def test_a_row_does_not_depend_on_what_the_others_bring(cuda, lily, W, rows, vocab, bf16):
+    """The kernel is compiled for what a launch's rows bring: the same rows drawn among themselves, beside
+    one that keeps many, one whose penalties can raise a logit, with (empty) lists, with their
+    parameters on the device, the greedy ones by the argmax call too. (Shards and proposals have tests of
+    their own.)"""
+    rng = np.random.default_rng([rows, vocab, bf16])
+    b = make_batch(W, rng, rows, vocab, 20, bf16, kind="zipf", history=600, presence=0.4, frequency=0.1)
+    for r in range(0, rows, 3):  # every third is greedy, without penalties
+        b.params[r].update(temperature=0.0, presence_penalty=0.0, frequency_penalty=0.0)
+    want = oracle_rows(b)
+    s = lily.SamplerScratch(vocab, max_rows=rows + 1, max_list=8)
+
+    def drawn(b, extra, **kw):
+        res = run_batch(cuda, lily, s, b, **kw)
+        cut = W.Batch(b.logits[:rows], bf16, b.params[:rows], b.uniforms[:rows])
+        res.ids, res.status = res.ids[:rows], res.status[:rows]
+        assert_parity(cut, res, want, label=extra)
+
+    drawn(b, "among themselves")
+    drawn(b, "parameters on the device", params_on_device=True)
+    for extra, more in (("keeps many", dict(top_k=0, temperature=1.1)), ("raises", dict(repetition_penalty=0.9, top_k=5))):
+        one = make_batch(W, rng, 1, vocab, 20, bf16, kind="zipf", history=600)
+        both = W.Batch(np.concatenate([b.logits, one.logits]), bf16, b.params + [dict(one.params[0], **more)],
+                       np.concatenate([b.uniforms, one.uniforms]))
+        both.history = np.concatenate([b.history, one.history])
+        both.history_len = np.concatenate([b.history_len, one.history_len])
+        drawn(both, extra)
+    b.bias_ids, b.bias_vals = np.zeros((rows, 4), np.uint32), np.zeros((rows, 4), np.float32)
+    b.bias_len = np.zeros(rows, np.uint32)
+    drawn(b, "empty lists")
+    ids = cuda.zeros(rows, dtype=cuda.int32, device="cuda")
+    s.argmax_batch(t_logits(cuda, b), ids)
+    greedy = np.arange(0, rows, 3)
+    assert np.array_equal(np_u32(ids)[greedy], np.array([want[r].token for r in greedy], np.uint32))
+    assert s.status() == lily.OK
+    s.close()
