@@ -453,8 +453,8 @@ int32_t launch(lily_sampler *h, cudaStream_t stream, const lily::KArgs &a, uint3
         lily::SplitArgs<INLINE_ROWS> sa;
         sa.a = a;
         sa.inline_params = sa.inline_slots = sa.inline_history = 0;
-        // (Parameters on the device: what their rows keep is not known here.)
-        return launch_split(h, stream, sa, plan, a.force_greedy && a.cand_out == nullptr ? lily::HAS_ARGMAX : lily::HAS_ALL, rows,
+        const bool plain = a.cand_out == nullptr && a.spec.n_spec == 0u && a.bias_ids == nullptr && a.ban_ids == nullptr;
+        return launch_split(h, stream, sa, plan, !plain ? lily::HAS_ALL : a.force_greedy ? lily::HAS_ARGMAX : lily::HAS_UNKNOWN, rows,
                             dtype);
     }
     const size_t esize = dtype == LILY_F32 ? 4 : 2;

@@ -1,4 +1,4 @@
-// The row kernel for up to 8 rows' parameters, and the merge kernel.
+// The row kernel for f32 logits and up to 8 rows' parameters, and the merge kernel.
 #include <atomic>
 
 #include "merge_kernel.cuh"
@@ -6,8 +6,27 @@
 
 namespace lily {
 
+LILY_SPLIT_LAUNCH_FOR(float, INLINE_ROWS);
+// (In units of their own.)
+extern LILY_SPLIT_LAUNCH_FOR(__nv_bfloat16, INLINE_ROWS);
+extern LILY_SPLIT_LAUNCH_FOR(float, INLINE_ROWS_MID);
+extern LILY_SPLIT_LAUNCH_FOR(__nv_bfloat16, INLINE_ROWS_MID);
+extern LILY_SPLIT_LAUNCH_FOR(float, INLINE_ROWS_MAX);
+extern LILY_SPLIT_LAUNCH_FOR(__nv_bfloat16, INLINE_ROWS_MAX);
+
+template <uint32_t MAXR>
+cudaError_t split_launch(const SplitArgs<MAXR> &a, uint32_t has, uint32_t rows, uint32_t dtype, size_t smem, int max_smem,
+                         uint64_t *attr_mask, cudaStream_t stream) {
+    return dtype == LILY_F32 ? split_launch_for<float>(a, has, rows, smem, max_smem, attr_mask, stream)
+                             : split_launch_for<__nv_bfloat16>(a, has, rows, smem, max_smem, attr_mask, stream);
+}
+
 template cudaError_t split_launch<INLINE_ROWS>(const SplitArgs<INLINE_ROWS> &, uint32_t, uint32_t, uint32_t, size_t, int,
                                                uint64_t *, cudaStream_t);
+template cudaError_t split_launch<INLINE_ROWS_MID>(const SplitArgs<INLINE_ROWS_MID> &, uint32_t, uint32_t, uint32_t, size_t,
+                                                   int, uint64_t *, cudaStream_t);
+template cudaError_t split_launch<INLINE_ROWS_MAX>(const SplitArgs<INLINE_ROWS_MAX> &, uint32_t, uint32_t, uint32_t, size_t,
+                                                   int, uint64_t *, cudaStream_t);
 
 uint32_t split_rows_at_once(int device, int sm_count, int max_smem, uint32_t log_blocks) {
     if (log_blocks == 0u) {

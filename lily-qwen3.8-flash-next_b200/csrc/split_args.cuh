@@ -156,20 +156,28 @@ __host__ __device__ inline uint32_t split_buckets(uint32_t pieces_of_block, uint
 
 // What the rows of a launch may bring beside a narrow draw: rows that keep more than SPL_SMALL_K; shards' records
 // in place of draws; bias or ban lists; penalties that can raise a logit; a proposal to verify. The kernel is
-// compiled for nothing of this, for one of them (SPEC, WIDE, SHARD), for an argmax of every row alone, and for
-// everything; a launch takes the smallest that has what its rows bring, as far as the host knows them.
-// Code that a row never runs slows down the chain of steps it does run: with everything, with nothing of
-// this, 1 x 151936 f32 8.75 -> 7.70 us, with 4096 ids 9.26 -> 8.25; 3 x 151936 bf16 8.82 -> 7.57;
-// 8 x 248320 f32 11.4 -> 10.2.
+// compiled for some sets of these and for everything; a launch takes a variant that has what its rows bring, as
+// far as the host knows them. (With parameters on the device it does not know what they keep, nor whether
+// they raise a logit.) Code that a row never runs slows down the chain of steps it does run: with everything, with
+// nothing of this, and so for rows over several blocks alone, 1 x 151936 f32 8.75, 7.66 and 7.44 us, with 4096 ids
+// 9.26, 8.18 and 7.96; 3 x 151936 bf16 with ids 8.82, 7.48 and 7.32; 8 x 248320 f32 11.4, 10.2 and 10.0.
 enum : uint32_t {
     HAS_WIDE = 1, HAS_SHARD = 2, HAS_LISTS = 4, HAS_RAISES = 8, HAS_SPEC = 16, HAS_ALL = 31,
     HAS_ARGMAX = 32  // (nothing but: parameters, lists, slots and forced ids are not looked at)
 };
+constexpr uint32_t HAS_UNKNOWN = HAS_WIDE | HAS_RAISES;  // parameters on the device, no lists
+// Variants whose rows' parameters all lie in the arguments, and whose rows all lie over two blocks or more.
+__host__ __device__ constexpr bool variant_inline(uint32_t has) {
+    return has != HAS_ALL && has != HAS_ARGMAX && has != HAS_UNKNOWN;
+}
+__host__ __device__ constexpr bool variant_many(uint32_t has, uint32_t max_rows) {
+    return variant_inline(has) && max_rows != 148u;
+}
 
 // Launches the kernel for a.a.rows rows from row0 on: logits of `dtype`, `smem` bytes of
 // dynamic shared memory (at most max_smem); `has`: what the rows may bring, HAS_ALL if that is not known.
-// `attr_mask`: bits of the kernels whose limit has been raised, the caller's to keep per device. Instantiated for
-// INLINE_ROWS, INLINE_ROWS_MID and INLINE_ROWS_MAX rows in split.cu, split_mid.cu and split_max.cu.
+// `attr_mask`: bits of the kernels whose limit has been raised, the caller's to keep per device. Instantiated in
+// split*.cu.
 template <uint32_t MAXR>
 cudaError_t split_launch(const SplitArgs<MAXR> &a, uint32_t has, uint32_t rows, uint32_t dtype, size_t smem, int max_smem,
                          uint64_t *attr_mask, cudaStream_t stream);
@@ -177,6 +185,7 @@ cudaError_t split_launch(const SplitArgs<MAXR> &a, uint32_t has, uint32_t rows, 
 // Rows whose parameters travel in the kernel's arguments: sizes of the argument block (a
 // larger one takes longer to launch), the last one as many rows as the chip has SMs.
 constexpr uint32_t INLINE_ROWS = 8, INLINE_ROWS_MID = 64, INLINE_ROWS_MAX = 148;
+static_assert(!variant_many(0u, INLINE_ROWS_MAX), "75 rows and more lie in one block each");
 
 // The most rows that clusters of 1 << log_blocks blocks run at once, one block per SM. Less
 // than the SMs would hold (15 clusters of eight on 148 SMs, 33 of four): a cluster lies in

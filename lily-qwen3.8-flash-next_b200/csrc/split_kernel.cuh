@@ -1035,6 +1035,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
     float *bmax = reinterpret_cast<float *>(marks + ca.mark_words);  // [buckets][SPL_NT]
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t rank = blockIdx.x, log_blocks = ca.log_blocks, blocks = 1u << log_blocks;
+    const bool many = variant_many(HAS, MAXR) || blocks > 1u;
     const uint32_t row = a.row0 + blockIdx.y;
     const uint32_t vocab = a.vocab;
     LILY_STAMP(PH_ENTRY);
@@ -1050,7 +1051,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         ss->bound_key = 0;
         ss->late = 0;
     }
-    if (blocks > 1u && tid < MEETS) {
+    if (many && tid < MEETS) {
         const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&ss->mbar[tid]);
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar),
                      "r"((tid == MEET_POOL || tid == MEET_SUMS ? 1u : blocks) + (ca.lost == (rank << 8 | (tid + 1u)) ? 1u : 0u))
@@ -1061,7 +1062,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         reinterpret_cast<uint4 *>(marks)[w] = make_uint4(0, 0, 0, 0);
     }
     __syncthreads();
-    if (blocks > 1u) {
+    if (many) {
         // (Waited for before the first store into another block.)
         asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     }
@@ -1170,7 +1171,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         in.flags = ROW_GREEDY;
         in.step = 0;
         in.seed = 0;
-    } else if (ca.inline_params) {
+    } else if (variant_inline(HAS) || ca.inline_params) {
         in = ca.in[row];
     } else {
         const uint2 *pp = reinterpret_cast<const uint2 *>(a.params + row);
@@ -1332,7 +1333,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
             sum += __shfl_xor_sync(FULL, sum, o);
         }
         uint2 *place = &ss->sums[rank * SPL_WARPS + warp - SPL_WARPS];
-        if (blocks > 1u) {
+        if (many) {
             asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
             if (lane == 0) {
                 put_2u32(peer_smem(place, 0), __float_as_uint(top), __float_as_uint(sum), peer_smem(&ss->mbar[MEET_SUMS], 0));
@@ -1343,7 +1344,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         if (rank != 0u) {
             return;
         }
-        if (blocks == 1u) {
+        if (!many) {
             asm volatile("bar.sync 6, %0;" ::"n"(SPL_NT) : "memory");
         }
         float total = 0.0f;
@@ -1351,7 +1352,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         bool late = false;
         if (warp == SPL_WARPS) {
             // (Collected before the verdict: the general code uses this memory for its own.)
-            if (blocks > 1u) {
+            if (many) {
                 if (lane == 0) {
                     arrive_expect(peer_smem(&ss->mbar[MEET_SUMS], 0), blocks * SPL_WARPS * 8u);
                 }
@@ -1599,7 +1600,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         }
         const uint32_t m = __reduce_max_sync(FULL, key);
         const uint32_t mi = __reduce_min_sync(FULL, key == m ? id : NONE);
-        if (blocks > 1u) {
+        if (many) {
             asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
             if (lane == 0) {
                 put_2u32(peer_smem(&ss->pool[2u * (rank * SPL_WARPS + warp)], 0), m, mi, peer_smem(&ss->mbar[MEET_POOL], 0));
@@ -1614,7 +1615,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
             return;
         }
         bool ok = true;
-        if (blocks > 1u) {
+        if (many) {
             if (tid == 0) {
                 arrive_expect(peer_smem(&ss->mbar[MEET_POOL], 0), blocks * SPL_WARPS * 8u);
             }
@@ -1731,7 +1732,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
     if (bad) {
         ss->hard = 1;  // (read after the next barrier)
     }
-    if (blocks > 1u) {
+    if (many) {
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     }
     uint32_t bound_key = 0;
@@ -1749,7 +1750,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
             // (The place in the pool takes the key's last eight bits: no two keys are the same, and
             // a bound may be a little lower than it could be.)
             const uint32_t to = (rank * SPL_WARPS + warp) * rounds + r, placed = (m & ~255u) | to;
-            if (blocks > 1u) {
+            if (many) {
                 if (lane < blocks) {
                     put_u32(peer_smem(&ss->pool[to], lane), placed, peer_smem(&ss->mbar[MEET_POOL], lane));
                 }
@@ -1757,7 +1758,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
                 ss->pool[to] = placed;
             }
         }
-        if (blocks > 1u) {
+        if (many) {
             if (tid == 0) {
                 arrive_expect(peer_smem(&ss->mbar[MEET_POOL], rank), n * 4u);
             }
@@ -1801,7 +1802,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         bound_key &= ~255u;
     } else {
         // The maxima of the whole cluster, 32 bins per unit under the largest.
-        if (blocks > 1u) {
+        if (many) {
             if (tid == 0) {
                 arrive_expect(peer_smem(&ss->mbar[MEET_POOL], rank), (blocks * groups << log_live) * 4u);
             }
@@ -1821,7 +1822,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
                 key = m_at == NONE ? 0u : adjusted(m, warp + SPL_WARPS * (m_at / PER), m_at % PER);
             }
             const uint32_t to = ((rank * groups + g) << log_live) + tid;
-            if (blocks > 1u) {
+            if (many) {
                 for (uint32_t r = 0; r < blocks; ++r) {
                     put_u32(peer_smem(&ss->tmax[to], r), key, peer_smem(&ss->mbar[MEET_POOL], r));
                 }
@@ -1835,7 +1836,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         if (tid == 0) {
             ss->bin = NONE;
         }
-        if (blocks > 1u && !wait_first_phase(&ss->mbar[MEET_POOL], ca.wait_ns >> 2)) {
+        if (many && !wait_first_phase(&ss->mbar[MEET_POOL], ca.wait_ns >> 2)) {
             ss->hard = ss->late = 1;
         }
         spl_sync();
@@ -1996,12 +1997,12 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
     const uint32_t cap = CAP >> log_blocks;
     const uint32_t n_hits = ss->n_hits;
     uint2 *cand = reinterpret_cast<uint2 *>(sm->key);  // over key and id: CAP of them, a region per block
-    const uint32_t bar = blocks > 1u ? peer_smem(&ss->mbar[MEET_CANDIDATES], 0) : 0u;
-    const uint32_t cand_at = blocks > 1u ? peer_smem(cand + rank * cap, 0) : 0u;
+    const uint32_t bar = many ? peer_smem(&ss->mbar[MEET_CANDIDATES], 0) : 0u;
+    const uint32_t cand_at = many ? peer_smem(cand + rank * cap, 0) : 0u;
     // (Wide rows: first here, over the pool, which has served.)
     // (A block alone: where the others' lists would be.)
     unsigned long long *own = wide_own(sm, ss, blocks);
-    const uint32_t most = wide ? (blocks > 1u ? min(cap, WIDE_OWN) : SPL_SORTED) : cap;
+    const uint32_t most = wide ? (many ? min(cap, WIDE_OWN) : SPL_SORTED) : cap;
     // f(id, logit, whether it comes from the bias list) for every one that may be among
     // the best: a thread per vector, mostly with one such logit.
     const uint32_t n_vecs = n_hits <= SPL_HITS && ss->hard == 0u ? n_hits : 0u;
@@ -2049,7 +2050,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
                 const uint32_t key_q = key_of(quot);
                 if (wide) {
                     own[to] = ((unsigned long long)key_q << 32) | (uint32_t)~id;
-                } else if (blocks > 1u) {
+                } else if (many) {
                     put_2u32(cand_at + to * 8u, key_q, id, bar);
                 } else {
                     cand[to] = make_uint2(key_q, id);
@@ -2083,7 +2084,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         return;
     }
     if (tid == 0) {
-        if (blocks > 1u) {
+        if (many) {
             put_4u32(peer_smem(&ss->head[rank], 0), sent, hard, __float_as_uint(least), 0u, bar);
             arrive_expect(bar, sent * 8u + 16u);
         } else {
@@ -2099,7 +2100,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
     }
 
     // ---- 4. ranks and the draw
-    if (blocks == 1u) {
+    if (!many) {
         spl_sync();  // (head[0] and the candidates are this block's own)
     }
     // Hardly more candidates than the row keeps: one warp does the rest.
@@ -2109,7 +2110,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
             return;
         }
     } else {
-        const bool late = blocks > 1u && !wait_first_phase(&ss->mbar[MEET_CANDIDATES], ca.wait_ns);
+        const bool late = many && !wait_first_phase(&ss->mbar[MEET_CANDIDATES], ca.wait_ns);
         if (late) {
             ss->late = 1;
         }
@@ -2168,7 +2169,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
     }
     const bool alone = n_ranked != 0u;  // (the warp that has ranked them)
     if (!alone) {
-        if (blocks > 1u && !wait_first_phase(&ss->mbar[MEET_CANDIDATES], ca.wait_ns)) {
+        if (many && !wait_first_phase(&ss->mbar[MEET_CANDIDATES], ca.wait_ns)) {
             ss->hard = 2;
             ss->late = 1;
         }

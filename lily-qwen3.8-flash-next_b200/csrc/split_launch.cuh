@@ -1,6 +1,8 @@
-// The row kernel's launches: one translation unit for each size of the argument block includes this and
-// instantiates split_launch.
+// The row kernel's launches. Translation units for the sizes of the argument block and the types include this and
+// instantiate split_launch_for.
 #pragma once
+
+#include <type_traits>
 
 #include "split_kernel.cuh"
 
@@ -11,7 +13,7 @@ cudaError_t split_launch_one(const SplitArgs<MAXR> &a, uint32_t rows, size_t sme
                              cudaStream_t stream) {
     auto kernel = split_rows_kernel<T, MAXR, BPS, HAS>;
     constexpr uint32_t variant = HAS == HAS_ALL ? (BPS == 1 ? 0u : 1u) : HAS == 0u ? 2u : HAS == HAS_SPEC ? 3u : HAS == HAS_WIDE ? 4u
-                                 : HAS == HAS_SHARD ? 5u : 6u;
+                                 : HAS == HAS_SHARD ? 5u : HAS == HAS_ARGMAX ? 6u : HAS == HAS_UNKNOWN ? 7u : 8u;
     constexpr uint32_t size = MAXR == INLINE_ROWS ? 0u : MAXR == INLINE_ROWS_MID ? 1u : 2u;
     constexpr uint64_t bit = 1ull << ((variant * 3u + size) * 2u + (sizeof(T) == 4 ? 0u : 1u));
     if (!(*attr_mask & bit)) {
@@ -38,48 +40,63 @@ cudaError_t split_launch_one(const SplitArgs<MAXR> &a, uint32_t rows, size_t sme
     return cudaLaunchKernelEx(&cfg, kernel, a);
 }
 
-// One block per SM: the variants beside the general one are compiled where calls of that kind are
-// common (proposals have at most 8 rows; shards' logits are a head's, f32; an argmax brings no parameters, so its
-// launches all have the smallest argument block).
+// One block per SM. The variants beside the general one are compiled where calls of that kind are common:
+// proposals have at most 8 rows; shards' logits are a head's, f32; where no parameters travel in the arguments, the
+// smallest argument block is used for any number of rows.
 template <typename T, uint32_t MAXR>
 cudaError_t split_launch_sole(const SplitArgs<MAXR> &a, uint32_t has, uint32_t rows, size_t smem, int max_smem,
                               uint64_t *attr_mask, cudaStream_t stream) {
-    if (has == 0u) {
-        return split_launch_one<T, MAXR, 1, 0u>(a, rows, smem, max_smem, attr_mask, stream);
-    }
+    auto launch = [&](auto set) {
+        return split_launch_one<T, MAXR, 1, decltype(set)::value>(a, rows, smem, max_smem, attr_mask, stream);
+    };
     if constexpr (MAXR == INLINE_ROWS) {
-        if (has == HAS_SPEC) {
-            return split_launch_one<T, MAXR, 1, HAS_SPEC>(a, rows, smem, max_smem, attr_mask, stream);
-        }
         if (has == HAS_ARGMAX) {
-            return split_launch_one<T, MAXR, 1, HAS_ARGMAX>(a, rows, smem, max_smem, attr_mask, stream);
+            return launch(std::integral_constant<uint32_t, HAS_ARGMAX>());
+        }
+        if (has == HAS_UNKNOWN) {
+            return launch(std::integral_constant<uint32_t, HAS_UNKNOWN>());
         }
     }
-    if constexpr (MAXR != INLINE_ROWS_MAX) {
-        if (has == HAS_WIDE) {
-            return split_launch_one<T, MAXR, 1, HAS_WIDE>(a, rows, smem, max_smem, attr_mask, stream);
+    if (a.inline_params && (a.log_blocks != 0u || !variant_many(0u, MAXR))) {
+        if (has == 0u) {
+            return launch(std::integral_constant<uint32_t, 0u>());
         }
-        if constexpr (sizeof(T) == 4) {
-            if (has == HAS_SHARD) {
-                return split_launch_one<T, MAXR, 1, HAS_SHARD>(a, rows, smem, max_smem, attr_mask, stream);
+        if constexpr (MAXR == INLINE_ROWS) {
+            if (has == HAS_SPEC) {
+                return launch(std::integral_constant<uint32_t, HAS_SPEC>());
+            }
+        }
+        if constexpr (MAXR != INLINE_ROWS_MAX) {
+            if (has == HAS_WIDE) {
+                return launch(std::integral_constant<uint32_t, HAS_WIDE>());
+            }
+            if ((has & ~(uint32_t)(HAS_WIDE | HAS_LISTS)) == 0u) {
+                return launch(std::integral_constant<uint32_t, HAS_WIDE | HAS_LISTS>());
+            }
+            if constexpr (sizeof(T) == 4) {
+                if (has == HAS_SHARD) {
+                    return launch(std::integral_constant<uint32_t, HAS_SHARD>());
+                }
             }
         }
     }
-    return split_launch_one<T, MAXR, 1, HAS_ALL>(a, rows, smem, max_smem, attr_mask, stream);
+    return launch(std::integral_constant<uint32_t, HAS_ALL>());
 }
 
-template <uint32_t MAXR>
-cudaError_t split_launch(const SplitArgs<MAXR> &a, uint32_t has, uint32_t rows, uint32_t dtype, size_t smem, int max_smem,
-                         uint64_t *attr_mask, cudaStream_t stream) {
+// Everything for logits of one type.
+template <typename T, uint32_t MAXR>
+cudaError_t split_launch_for(const SplitArgs<MAXR> &a, uint32_t has, uint32_t rows, size_t smem, int max_smem,
+                             uint64_t *attr_mask, cudaStream_t stream) {
     if constexpr (MAXR == INLINE_ROWS) {
         if (a.two_per_sm) {
-            return dtype == LILY_F32
-                       ? split_launch_one<float, MAXR, 2, HAS_ALL>(a, rows, smem, max_smem, attr_mask, stream)
-                       : split_launch_one<__nv_bfloat16, MAXR, 2, HAS_ALL>(a, rows, smem, max_smem, attr_mask, stream);
+            return split_launch_one<T, MAXR, 2, HAS_ALL>(a, rows, smem, max_smem, attr_mask, stream);
         }
     }
-    return dtype == LILY_F32 ? split_launch_sole<float>(a, has, rows, smem, max_smem, attr_mask, stream)
-                             : split_launch_sole<__nv_bfloat16>(a, has, rows, smem, max_smem, attr_mask, stream);
+    return split_launch_sole<T>(a, has, rows, smem, max_smem, attr_mask, stream);
 }
+
+#define LILY_SPLIT_LAUNCH_FOR(T, MAXR)                                                                            \
+    template cudaError_t split_launch_for<T, MAXR>(const SplitArgs<MAXR> &, uint32_t, uint32_t, size_t, int, uint64_t *, \
+                                                   cudaStream_t)
 
 }  // namespace lily

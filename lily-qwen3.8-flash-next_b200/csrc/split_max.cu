@@ -3,7 +3,7 @@
 
 namespace lily {
 
-template cudaError_t split_launch<INLINE_ROWS_MAX>(const SplitArgs<INLINE_ROWS_MAX> &, uint32_t, uint32_t, uint32_t, size_t,
-                                                   int, uint64_t *, cudaStream_t);
+LILY_SPLIT_LAUNCH_FOR(float, INLINE_ROWS_MAX);
+LILY_SPLIT_LAUNCH_FOR(__nv_bfloat16, INLINE_ROWS_MAX);
 
 }  // namespace lily

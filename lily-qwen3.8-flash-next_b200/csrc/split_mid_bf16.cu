@@ -1,0 +1,8 @@
+// The row kernel for bf16 logits and up to 64 rows' parameters.
+#include "split_launch.cuh"
+
+namespace lily {
+
+LILY_SPLIT_LAUNCH_FOR(__nv_bfloat16, INLINE_ROWS_MID);
+
+}  // namespace lily
