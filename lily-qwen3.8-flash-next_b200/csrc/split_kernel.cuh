@@ -1938,11 +1938,26 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
             }
         }
     } else {
-        for (uint32_t b0 = 0; b0 < buckets; b0 += 32u) {
+        uint32_t listed = buckets;
+        if (HAS == HAS_WIDE && BPS == 1 && buckets == 2u && k > CHAIN_MAX) {
+            // (A row of two buckets that keeps many looks at most of its vectors again: the second
+            // bucket's are still in registers. 1 x 151936 f32, 1024 kept: 14.62 -> 13.84 us; rows that
+            // keep 100 lose 0.25 us by it, rows of four buckets 0.2.)
+            listed = 1u;
+            if (bm >= least) {
+#pragma unroll
+                for (uint32_t i = 0; i < SPL_U; ++i) {
+                    if (vec_max<T>(q[i]) >= least) {
+                        hit(q[i], id_at(warp + SPL_WARPS * (SPL_U + i), 0u));
+                    }
+                }
+            }
+        }
+        for (uint32_t b0 = 0; b0 < listed; b0 += 32u) {
             uint32_t over = buckets == 1u && bm >= least ? 1u : 0u;
             if (buckets != 1u) {
                 const float *mine = bmax + b0 * SPL_NT + tid;
-                const uint32_t end = min(buckets - b0, 32u);
+                const uint32_t end = min(listed - b0, 32u);
 #pragma unroll 4
                 for (uint32_t b = 0; b < end; ++b) {
                     over |= mine[b * SPL_NT] >= least ? 1u << b : 0u;
@@ -1960,12 +1975,13 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         if (n_flagged > SPL_FLAGGED) {
             ss->hard = 1;
         } else {
-            // (Each of them again, from L2: four vectors per thread at a time.)
-            for (uint32_t i0 = tid; i0 < n_flagged * SPL_U; i0 += 4u * SPL_NT) {
-                uint4 x[4];
-                uint32_t v[4];
+            // (Each of them again, from L2: a narrow row has hardly more than one vector per thread.)
+            constexpr uint32_t AGAIN = (HAS & HAS_WIDE) != 0u ? 4u : 2u;
+            for (uint32_t i0 = tid; i0 < n_flagged * SPL_U; i0 += AGAIN * SPL_NT) {
+                uint4 x[AGAIN];
+                uint32_t v[AGAIN];
 #pragma unroll
-                for (uint32_t h = 0; h < 4u; ++h) {
+                for (uint32_t h = 0; h < AGAIN; ++h) {
                     const uint32_t i = i0 + h * SPL_NT;
                     v[h] = NONE;
                     if (i < n_flagged * SPL_U) {
@@ -1978,7 +1994,7 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
                     }
                 }
 #pragma unroll
-                for (uint32_t h = 0; h < 4u; ++h) {
+                for (uint32_t h = 0; h < AGAIN; ++h) {
                     if (v[h] != NONE && vec_max<T>(x[h]) >= least) {
                         hit(x[h], v[h] * PER - skip);
                     }
