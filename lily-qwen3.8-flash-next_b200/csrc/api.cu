@@ -243,16 +243,11 @@ int32_t launch_one(lily_sampler *h, cudaStream_t stream_, const lily::KArgs &a, 
         lily::KArgs whole = a;
         whole.n_slices = 1;
         const size_t smem1 = smem_bytes(a.vocab, 1);
-        if (rows > (uint32_t)h->sm_count) {
-            auto kernel = lily::stream_rows_kernel<T, 2>;
-            const int32_t st = raise_smem_limit(h, kernel, 1u << (sizeof(T) == 4 ? 4 : 5));
-            if (st != LILY_OK) {
-                return st;
-            }
-            return launch_serialised(h, stream_, kernel, dim3(rows, 1, 1), smem1, whole);
-        }
-        auto kernel = lily::stream_rows_kernel<T, 3>;
-        const int32_t st = raise_smem_limit(h, kernel, 1u << (sizeof(T) == 4 ? 6 : 7));
+        const bool plain = a.cand_out == nullptr && a.count_slots == nullptr;
+        const bool many = rows > (uint32_t)h->sm_count;
+        auto kernel = plain ? (many ? lily::stream_rows_kernel<T, 2, true> : lily::stream_rows_kernel<T, 3, true>)
+                            : (many ? lily::stream_rows_kernel<T, 2, false> : lily::stream_rows_kernel<T, 3, false>);
+        const int32_t st = raise_smem_limit(h, kernel, 1u << (4 + (sizeof(T) == 4 ? 0 : 1) + (many ? 0 : 2) + (plain ? 4 : 0)));
         if (st != LILY_OK) {
             return st;
         }

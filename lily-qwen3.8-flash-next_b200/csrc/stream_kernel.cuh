@@ -246,7 +246,9 @@ __device__ __forceinline__ uint32_t small_select(SmemFixed *sm, uint32_t n, uint
     return min(live, k);
 }
 
-template <typename T, uint32_t AHEAD>
+// PLAIN: a launch without histogram slots whose rows are drawn, not shards' records. (What such a launch does not
+// run is not in its code.)
+template <typename T, uint32_t AHEAD, bool PLAIN>
 __global__ void __launch_bounds__(NT, 2) stream_rows_kernel(const __grid_constant__ KArgs a) {
     static_assert(AHEAD < STREAM_STAGES, "rounds in flight");
     constexpr uint32_t NS = STREAM_STAGES, HQ = STREAM_HQ;
@@ -284,7 +286,8 @@ __global__ void __launch_bounds__(NT, 2) stream_rows_kernel(const __grid_constan
     const int32_t forced = a.forced_ids ? __ldg(a.forced_ids + row) : -1;
     const uint32_t bias_len_row = (a.bias_ids && a.bias_len) ? __ldg(a.bias_len + row) : 0u;
     const uint32_t ban_len_row = (a.ban_ids && a.ban_len) ? __ldg(a.ban_len + row) : 0u;
-    const uint32_t slot = a.count_slots ? __ldg(a.count_slots + row) : 0u;
+    const bool shard = !PLAIN && a.cand_out != nullptr;
+    const uint32_t slot = !PLAIN && a.count_slots ? __ldg(a.count_slots + row) : 0u;
     const float u_row = a.uniforms ? __ldg(a.uniforms + row) : 0.0f;
     const uint32_t step_row = (!a.uniforms && a.steps) ? __ldg(a.steps + row) : 0u;
     lily_sampling_params_t P;
@@ -338,7 +341,7 @@ __global__ void __launch_bounds__(NT, 2) stream_rows_kernel(const __grid_constan
         }
     };
     auto refuse = [&](uint32_t status) {
-        if (a.cand_out) {
+        if (shard) {
             empty_record(status);
         } else if (tid == 0) {
             a.out_ids[row] = status == LILY_ROW_FORCED ? (uint32_t)forced : 0xFFFFFFFFu;
@@ -383,14 +386,14 @@ __global__ void __launch_bounds__(NT, 2) stream_rows_kernel(const __grid_constan
                          P.repetition_penalty != 1.0f;
     // (A shard keeps shard_k candidates of a sampled row, whatever its top_k: the
     // host made sure that top_k fits.)
-    const uint32_t k = greedy ? 1u : a.cand_out ? a.shard_k : (P.top_k == 0u ? KCAP : min(P.top_k, KCAP));
+    const uint32_t k = greedy ? 1u : shard ? a.shard_k : (P.top_k == 0u ? KCAP : min(P.top_k, KCAP));
     // (A shard's record: the sum of exponentials in the same pass, if asked for.)
-    const bool sums = a.cand_out != nullptr && a.shard_sums != 0u;
+    const bool sums = shard && a.shard_sums != 0u;
     const float sum_scale = 1.4426950408889634f / (greedy ? 1.0f : P.temperature);
     const bool monotone = P.repetition_penalty >= 1.0f && !(__float_as_uint(P.presence_penalty) >> 31) &&
                           !(__float_as_uint(P.frequency_penalty) >> 31);
     const bool need_counts = use_pen && P.frequency_penalty != 0.0f;
-    const bool table_mode = a.count_slots != nullptr;
+    const bool table_mode = !PLAIN && a.count_slots != nullptr;
     // A row this path does not take, or cannot finish (below), gets the general
     // code on the whole row, from the start.
     bool mine = !(k > STREAM_K_MAX || bias_len_row + ban_len_row != 0u || (use_pen && !monotone) ||
@@ -755,7 +758,7 @@ __global__ void __launch_bounds__(NT, 2) stream_rows_kernel(const __grid_constan
     if (stamps && tid == 0) {
         stamps[PH_LOCAL_SELECT] = global_ns();
     }
-    if (a.cand_out) {
+    if (shard) {
         float total = 0.0f;
         if (sums && n != 0u) {
             total = running_sum_total(sm, rs, float_of_key(sm->key[0]) * 1.4426950408889634f);
@@ -798,8 +801,8 @@ __global__ void __launch_bounds__(NT, 2) stream_rows_kernel(const __grid_constan
     }
     if (tid < 32u) {
         if (tid == 0) {
-            sm->ctx.count_draw = a.count_slots != nullptr && sm->ctx.use_pen;
-            sm->ctx.slot = a.count_slots ? a.count_slots[row] : 0u;
+            sm->ctx.count_draw = table_mode && use_pen;
+            sm->ctx.slot = table_mode ? slot : 0u;
         }
         __syncwarp();
         finalize_warp(sm, a, row, n, P.seed);
