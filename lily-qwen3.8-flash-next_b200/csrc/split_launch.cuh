@@ -13,7 +13,7 @@ cudaError_t split_launch_one(const SplitArgs<MAXR> &a, uint32_t rows, size_t sme
                              cudaStream_t stream) {
     auto kernel = split_rows_kernel<T, MAXR, BPS, HAS>;
     constexpr uint32_t variant = HAS == HAS_ALL ? (BPS == 1 ? 0u : 1u) : HAS == 0u ? 2u : HAS == HAS_SPEC ? 3u : HAS == HAS_WIDE ? 4u
-                                 : HAS == HAS_SHARD ? 5u : HAS == HAS_ARGMAX ? 6u : HAS == HAS_UNKNOWN ? 7u : 8u;
+                                 : HAS == HAS_SHARD ? 5u : HAS == HAS_ARGMAX ? 6u : HAS == HAS_UNKNOWN ? (BPS == 1 ? 7u : 8u) : 9u;
     constexpr uint32_t size = MAXR == INLINE_ROWS ? 0u : MAXR == INLINE_ROWS_MID ? 1u : 2u;
     constexpr uint64_t bit = 1ull << ((variant * 3u + size) * 2u + (sizeof(T) == 4 ? 0u : 1u));
     if (!(*attr_mask & bit)) {
@@ -89,7 +89,8 @@ cudaError_t split_launch_for(const SplitArgs<MAXR> &a, uint32_t has, uint32_t ro
                              uint64_t *attr_mask, cudaStream_t stream) {
     if constexpr (MAXR == INLINE_ROWS) {
         if (a.two_per_sm) {
-            return split_launch_one<T, MAXR, 2, HAS_ALL>(a, rows, smem, max_smem, attr_mask, stream);
+            return has == HAS_UNKNOWN ? split_launch_one<T, MAXR, 2, HAS_UNKNOWN>(a, rows, smem, max_smem, attr_mask, stream)
+                                      : split_launch_one<T, MAXR, 2, HAS_ALL>(a, rows, smem, max_smem, attr_mask, stream);
         }
     }
     return split_launch_sole<T>(a, has, rows, smem, max_smem, attr_mask, stream);
