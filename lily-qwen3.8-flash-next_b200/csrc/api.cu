@@ -372,10 +372,10 @@ SplitPlan split_plan(const lily_sampler *h, const lily::KArgs &a, uint32_t rows,
     p.smem = fixed + (size_t)p.mark_words * 4u;
     p.smem = p.smem > general ? p.smem : general;
     // More rows than SMs: two blocks to an SM, unless the kernel of one block per row takes the
-    // call (aligned logits), which reads further ahead. 256 rows x 151936 bf16: 30.6 us here,
-    // 27.6 there. What only the general kernel took, 256 rows with ids of a power law: x 151937
-    // bf16 without lists 31.6, with 4096 ids a row 35.0, with 32768 49.5; x 50257 f32 with 8192
-    // ids 28.5 (the general kernel, by its first measurement: 117, 122, 128 and 55.5).
+    // call (aligned logits), which reads further ahead. 256 rows x 151936 bf16 with 1024 ids a row: 31.0 us here,
+    // 27.0 there; 200 x 100352 f32 33.7 and 26.2; 256 x 50304 f32 22.3 and 20.0. What only the general kernel took,
+    // 256 rows: x 151937 bf16 with 4096 ids a row 31.0, with 32768 39.1; x 50257 f32 with 8192 ids 24.0
+    // (the general kernel, by its first measurement, with ids of a power law: 122, 128 and 55.5).
     p.take = p.smem <= (size_t)h->max_smem && (p.sole || !stream_route(a, rows, dtype));
     return p;
 }

@@ -87,14 +87,16 @@ cudaError_t launch_for(const Args &a, Format format, uint32_t sms, cudaStream_t 
 // their scaling all go with it. Measured per call, both launches, back to back (before:
 // 64 always, one pipeline for both halves of a tile, bf16 only, the affine term in a kernel
 // of its own, whole tiles only):
-//   262144 x 4096, symmetric:     64 tokens 325 -> 245 us, 32 tokens 194, 16 tokens 180
-//   248320 x 4096, affine 8 bits: 64 tokens 430 -> 285 us,  4 tokens 435 -> 172
-//   151936 x 2048, affine 4 bits: 64 tokens 90 us, 32 tokens 160 -> 61, 4 tokens 50
+//   262144 x 4096, symmetric:     64 tokens 325 -> 240 us, 32 tokens 193, 16 tokens 179
+//   248320 x 4096, affine 8 bits: 64 tokens 430 -> 280 us,  4 tokens 435 -> 170
+//   151936 x 2048, affine 4 bits: 64 tokens 89 us, 32 tokens 160 -> 57, 4 tokens 48
 // (4 bits, 32 tokens, step by step: 80; two groups per hand-over and fewer stages 70; codes
 // as subnormals 61; sums of shared tiles handed on through the logits' place instead of a
-// workspace: + 0.6 to 1.2 at 4 bits, nothing elsewhere.) At 16 tokens the weights' stream bounds bytes (5.9 TB/s of 6.6
-// measured for a copy); the rest is bound by issue slots (67 % busy before the last step):
-// widening a weight, and one FMA per logit and group.
+// workspace: + 0.6 to 1.2 at 4 bits, nothing elsewhere; scales through shared memory 58.4; a warp's waits as one
+// 57.3.) At 16 tokens the weights' stream bounds bytes (5.9 TB/s of 6.6
+// measured for a copy); the rest is bound by what its warps issue (slots 62 to 65 % busy; 4 % more
+// instructions take 3.6 % longer): widening a weight, one FMA per logit and group, and the waits. In calls
+// that go on for a tenth of a second the power limit lowers the clock: 64 tokens 240 -> 275 us.
 cudaError_t launch_head(const Args &a, Format format, uint32_t sms, cudaStream_t stream) {
     switch (padded_tokens(a.tokens)) {
         case 16: return launch_for<16>(a, format, sms, stream);

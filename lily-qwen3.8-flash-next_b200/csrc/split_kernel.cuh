@@ -20,17 +20,18 @@
 //      in rank order, the cut and the draw (or writes a shard's record).
 //
 // What bounds it is latency, not memory: a call of a few rows is a chain of some ten
-// dependent steps: from the share read to the bound known, with the pool's meeting in between, 1.4 to
-// 1.65 us, from the candidates sent to all of them there 0.1 to 0.25. So blocks meet by stores
+// dependent steps: from the share read to the bound known, with the pool's meeting in between, 1.05 to
+// 1.45 us, from the candidates sent to all of them there 0.1 to 0.25. So blocks meet by stores
 // that complete a barrier in the receiver, no warp waits for one that it does not need, and the
-// draw's adds run in two chains of 32 lanes. Measured back to back: 1 row x 151936 f32 with a history of 4096 ids 50 -> 9.35 us, 64 rows x
-// 151936 bf16 with histories 32 -> 14.4, argmax of 1 x 32768 9.2 -> 3.25 (before: cut in
+// draw's adds run in two chains of 32 lanes. Measured back to back: 1 row x 151936 f32 with a history of 4096 ids 50 -> 7.7 us, 64 rows x
+// 151936 bf16 with histories 32 -> 12.8, argmax of 1 x 32768 9.2 -> 2.55 (before: cut in
 // slices through global memory, or a cluster that kept the row in shared memory). Code that the
 // warps run once is slow code: of the 21 clocks between two instructions of a warp 6 to 7.5 wait for the
 // instruction itself and 7.5 at barriers. So what stands on the way counts: functions
 // that take the launch's arguments by address load each of them from memory (1 us), an
 // arrival that releases waits for the thread's stores (0.3 us each), and code that a call never
-// runs still slows it where it stands between what it does run.
+// runs still slows it where it stands between what it does run: the kernel is compiled for what a
+// launch's rows bring (split_args.cuh).
 //
 // A row that keeps more than 64 candidates takes its bound from the maxima of all
 // threads of the cluster, and all blocks rank its candidates. Where penalties can raise a

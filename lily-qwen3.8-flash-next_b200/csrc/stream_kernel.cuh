@@ -36,7 +36,7 @@ constexpr uint32_t STREAM_MIN_ROUNDS = 8;  // shorter rows go to the row kernel,
 constexpr uint32_t STREAM_K_MAX = 64;      // finalize_warp holds two candidates per lane
 // AHEAD (template argument of the kernel): rounds of the ring in flight beyond the
 // one being read. With a block slot's worth of rows two measured faster than
-// three (33.4 against 34.0 us per 256-row launch; asking L2 for further rounds
+// three (34.6 against 34.9 us per 256-row launch; asking L2 for further rounds
 // ahead of the ring was slower still: the stream is not short of requests).
 constexpr uint32_t STREAM_STAGES = 4;      // of the ring
 constexpr uint32_t STREAM_HQ = 2;          // 16-byte loads of history ids per thread and round
