@@ -437,3 +437,15 @@ def test_a_row_does_not_depend_on_what_the_others_bring(cuda, lily, W, rows, voc
     assert np.array_equal(np_u32(ids)[greedy], np.array([want[r].token for r in greedy], np.uint32))
     assert s.status() == lily.OK
     s.close()
+
+
+@pytest.mark.parametrize("rows,vocab", [(75, 327_680), (75, 330_003), (149, 197_003)])
+def test_more_buckets_than_a_word_has_bits(cuda, lily, W, rows, vocab):
+    # A row in one block whose thread has 32 buckets, 33, and 33 with two blocks to an SM: those that reach the
+    # bound are listed 32 at a time.
+    rng = np.random.default_rng(rows + vocab)
+    b = make_batch(W, rng, rows, vocab, 20, False, history=30, rep=1.1)
+    for r in range(rows):  # (the best ones all over the row, its last bucket among them)
+        b.logits[r, rng.integers(0, vocab, 12)] += 3.0
+        b.logits[r, vocab - 1 - rng.integers(0, 400, 4)] += 4.0
+    check(cuda, lily, W, b, vocab, f"B={rows} V={vocab}")
