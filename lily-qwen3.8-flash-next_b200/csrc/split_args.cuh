@@ -93,11 +93,15 @@ struct alignas(16) SplitSmem {
     uint4 head[SPL_MAX_BLOCKS];      // first block: a block's number of candidates, flag, bound
     uint2 sums[SPL_MAX_BLOCKS * SPL_WARPS];  // first block, a shard's record: (reference, sum) of every warp
     union {
-        alignas(16) uint32_t pool[SPL_POOL];     // the best keys of every warp of the cluster
+        struct {
+            alignas(16) uint32_t pool[SPL_POOL];  // the best keys of every warp of the cluster
+            // Buckets that reach the bound. (The maxima have served by then; the pool may still be read. By itself
+            // this list kept a second block of 151937 f32 logits off an SM: 256 rows 77 us, so 48.)
+            uint16_t flagged[SPL_FLAGGED];
+        };
         uint32_t tmax[SPL_MAX_BLOCKS * SPL_NT];  // wide rows: the keys of all its threads
     };
     uint32_t hit_at[SPL_HITS];       // vectors that reach the bound: the id of their first logit (mod 2^32)
-    uint16_t flagged[SPL_FLAGGED];
     uint32_t n_flagged;
     uint32_t n_hits;
     uint32_t n_listed;               // ids on the row's bias list that are this block's
