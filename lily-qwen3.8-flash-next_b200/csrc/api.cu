@@ -70,8 +70,6 @@ struct lily_sampler {
     cudaEvent_t ev[RING] = {};
     int ring_pos = 0;
     uint32_t *h_status = nullptr;
-    uint32_t attr_mask = 0;  // kernel variants whose shared-memory limit is raised
-    uint64_t split_mask = 0;  // likewise, of the row kernel
     long long *phase_clocks = nullptr;
     // The parameters a sharded call staged last: a decode step stages the same
     // rows for its candidate call and its merge call, and usually again next step.
@@ -211,22 +209,13 @@ int32_t launch_accept(lily_sampler *h, cudaStream_t stream, const uint32_t *draw
     return LILY_OK;
 }
 
-template <typename Kernel>
-int32_t raise_smem_limit(lily_sampler *h, Kernel kernel, uint32_t bit) {
-    if (!(h->attr_mask & bit)) {
-        CU(h, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, h->max_smem));
-        h->attr_mask |= bit;
-    }
-    return LILY_OK;
-}
-
 // Whether a call goes to the kernel of one block per row (see launch_one).
 bool stream_route(const lily::KArgs &a, uint32_t rows, uint32_t dtype) {
     const size_t esize = dtype == LILY_F32 ? 4 : 2;
     const bool vec = (reinterpret_cast<uintptr_t>(a.logits) % 16u == 0u) && ((a.logits_ld * esize) % 16u == 0u);
     const uint32_t round = dtype == LILY_F32 ? lily::Geo<float>::ROUND : lily::Geo<__nv_bfloat16>::ROUND;
     return vec && a.vocab / round >= lily::STREAM_MIN_ROUNDS && a.merge_in == nullptr && a.spec.n_spec == 0u &&
-           a.extra_len == 0u && rows >= 16u && (a.cand_out == nullptr || a.shard_k <= lily::STREAM_K_MAX);
+           a.extra_len == 0u && rows >= lily::STREAM_MIN_ROWS && (a.cand_out == nullptr || a.shard_k <= lily::STREAM_K_MAX);
 }
 
 template <typename T, bool VEC>
@@ -247,18 +236,9 @@ int32_t launch_one(lily_sampler *h, cudaStream_t stream_, const lily::KArgs &a, 
         const bool many = rows > (uint32_t)h->sm_count;
         auto kernel = plain ? (many ? lily::stream_rows_kernel<T, 2, true> : lily::stream_rows_kernel<T, 3, true>)
                             : (many ? lily::stream_rows_kernel<T, 2, false> : lily::stream_rows_kernel<T, 3, false>);
-        const int32_t st = raise_smem_limit(h, kernel, 1u << (4 + (sizeof(T) == 4 ? 0 : 1) + (many ? 0 : 2) + (plain ? 4 : 0)));
-        if (st != LILY_OK) {
-            return st;
-        }
         return launch_serialised(h, stream_, kernel, dim3(rows, 1, 1), smem1, whole);
     }
-    auto kernel = lily::sample_rows_kernel<T, VEC>;
-    const int32_t st = raise_smem_limit(h, kernel, 1u << ((sizeof(T) == 4 ? 0 : 2) + (VEC ? 1 : 0)));
-    if (st != LILY_OK) {
-        return st;
-    }
-    return launch_serialised(h, stream_, kernel, dim3(a.n_slices, rows, 1), smem, a);
+    return launch_serialised(h, stream_, lily::sample_rows_kernel<T, VEC>, dim3(a.n_slices, rows, 1), smem, a);
 }
 
 // Parameters of more rows than a launch's own arguments take go to the device in the
@@ -391,7 +371,7 @@ int32_t launch_split(lily_sampler *h, cudaStream_t stream, lily::SplitArgs<MAXR>
     sa.wait_ns = h->wait_ns;
     sa.lost = h->lost_arrival;
     h->lost_arrival = 0;  // one launch only
-    CU(h, lily::split_launch<MAXR>(sa, has, rows, dtype, p.smem, h->max_smem, &h->split_mask, stream));
+    CU(h, lily::split_launch<MAXR>(sa, has, rows, dtype, p.smem, stream));
     return LILY_OK;
 }
 
@@ -461,6 +441,55 @@ int32_t launch(lily_sampler *h, cudaStream_t stream, const lily::KArgs &a, uint3
     }
     return vec ? launch_one<__nv_bfloat16, true>(h, stream, a, rows, smem)
                : launch_one<__nv_bfloat16, false>(h, stream, a, rows, smem);
+}
+
+// Every kernel that the handle's calls can come to is on the device, with its shared-memory limit raised, before the
+// first of them: which one a call takes depends on what its rows bring, and loading it there (an allocation on
+// the device) would hold up one step in the middle of serving, or fall into a capture. (Not the LM head's: its
+// first call loads them.)
+cudaError_t load_kernels(const lily_sampler *h) {
+    cudaError_t e = lily::split_ready(h->max_rows, (uint32_t)h->sm_count, h->max_smem);
+    if (e == cudaSuccess) {
+        e = lily::merge_ready();
+    }
+    for (uint32_t log_blocks = 1; log_blocks <= 3u; ++log_blocks) {
+        lily::split_rows_at_once(h->device, h->sm_count, h->max_smem, log_blocks);  // (asked of the device once)
+    }
+    auto load = [&](auto kernel, int smem) {
+        cudaFuncAttributes fa;
+        if (e == cudaSuccess) {
+            e = cudaFuncGetAttributes(&fa, kernel);  // (this loads it)
+        }
+        if (e == cudaSuccess && smem != 0) {
+            e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        }
+    };
+    auto of_type = [&](auto logit) {
+        using T = decltype(logit);
+        load(lily::sample_rows_kernel<T, true>, h->max_smem);
+        load(lily::sample_rows_kernel<T, false>, h->max_smem);
+        if (h->max_rows >= lily::STREAM_MIN_ROWS) {
+            load(lily::stream_rows_kernel<T, 3, true>, h->max_smem);
+            load(lily::stream_rows_kernel<T, 3, false>, h->max_smem);
+        }
+        if (h->max_rows > (uint32_t)h->sm_count) {
+            load(lily::stream_rows_kernel<T, 2, true>, h->max_smem);
+            load(lily::stream_rows_kernel<T, 2, false>, h->max_smem);
+        }
+        load(lily::shard_sums_kernel<T>, 0);
+    };
+    of_type(0.0f);
+    of_type(__nv_bfloat16());
+    load(put_kernel<4096>, 0);
+    load(put_kernel<16384>, 0);
+    load(put_kernel<32000>, 0);
+    load(lily::spec_accept_kernel, 0);
+    load(lily::shard_publish_kernel, 0);
+    if (h->flags & LILY_FLAG_COUNTS_TABLE) {
+        load(lily::uncount_kernel, 0);
+        load(lily::rebuild_seen_kernel, 0);
+    }
+    return e;
 }
 
 uint32_t choose_slices(const lily_sampler *h, uint32_t rows) {
@@ -594,6 +623,9 @@ int32_t lily_sampler_create(int32_t device, uint32_t vocab, uint32_t max_rows,
     if ((e = cudaDeviceGetAttribute(&h->max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin,
                                     device)) != cudaSuccess) {
         return bail(e, "shared memory limit");
+    }
+    if ((e = load_kernels(h)) != cudaSuccess) {
+        return bail(e, "kernels");
     }
     // One device allocation, one pinned one: an allocation takes some 0.3 ms, whatever
     // its size. What has to start from zero comes first, cleared by one call.
@@ -1472,7 +1504,7 @@ int32_t merge_draw(lily_sampler_t *h, void *stream_, const void *gathered, uint3
     if (peer != nullptr) {
         a.peer = *peer;
     }
-    CU(h, lily::merge_launch(ma, g.rows, &h->attr_mask, stream));
+    CU(h, lily::merge_launch(ma, g.rows, stream));
     if (!in_args) {
         CU(h, cudaEventRecord(h->ev[slot], stream));
     }

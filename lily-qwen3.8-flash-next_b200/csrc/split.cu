@@ -6,27 +6,42 @@
 
 namespace lily {
 
-LILY_SPLIT_LAUNCH_FOR(float, INLINE_ROWS);
+LILY_SPLIT_LAUNCH_FOR(, float, INLINE_ROWS);
 // (In units of their own.)
-extern LILY_SPLIT_LAUNCH_FOR(__nv_bfloat16, INLINE_ROWS);
-extern LILY_SPLIT_LAUNCH_FOR(float, INLINE_ROWS_MID);
-extern LILY_SPLIT_LAUNCH_FOR(__nv_bfloat16, INLINE_ROWS_MID);
-extern LILY_SPLIT_LAUNCH_FOR(float, INLINE_ROWS_MAX);
-extern LILY_SPLIT_LAUNCH_FOR(__nv_bfloat16, INLINE_ROWS_MAX);
+LILY_SPLIT_LAUNCH_FOR(extern, __nv_bfloat16, INLINE_ROWS);
+LILY_SPLIT_LAUNCH_FOR(extern, float, INLINE_ROWS_MID);
+LILY_SPLIT_LAUNCH_FOR(extern, __nv_bfloat16, INLINE_ROWS_MID);
+LILY_SPLIT_LAUNCH_FOR(extern, float, INLINE_ROWS_MAX);
+LILY_SPLIT_LAUNCH_FOR(extern, __nv_bfloat16, INLINE_ROWS_MAX);
 
 template <uint32_t MAXR>
-cudaError_t split_launch(const SplitArgs<MAXR> &a, uint32_t has, uint32_t rows, uint32_t dtype, size_t smem, int max_smem,
-                         uint64_t *attr_mask, cudaStream_t stream) {
-    return dtype == LILY_F32 ? split_launch_for<float>(a, has, rows, smem, max_smem, attr_mask, stream)
-                             : split_launch_for<__nv_bfloat16>(a, has, rows, smem, max_smem, attr_mask, stream);
+cudaError_t split_launch(const SplitArgs<MAXR> &a, uint32_t has, uint32_t rows, uint32_t dtype, size_t smem,
+                         cudaStream_t stream) {
+    return dtype == LILY_F32 ? split_launch_for<float>(a, has, rows, smem, stream)
+                             : split_launch_for<__nv_bfloat16>(a, has, rows, smem, stream);
 }
 
-template cudaError_t split_launch<INLINE_ROWS>(const SplitArgs<INLINE_ROWS> &, uint32_t, uint32_t, uint32_t, size_t, int,
-                                               uint64_t *, cudaStream_t);
+template cudaError_t split_launch<INLINE_ROWS>(const SplitArgs<INLINE_ROWS> &, uint32_t, uint32_t, uint32_t, size_t,
+                                               cudaStream_t);
 template cudaError_t split_launch<INLINE_ROWS_MID>(const SplitArgs<INLINE_ROWS_MID> &, uint32_t, uint32_t, uint32_t, size_t,
-                                                   int, uint64_t *, cudaStream_t);
+                                                   cudaStream_t);
 template cudaError_t split_launch<INLINE_ROWS_MAX>(const SplitArgs<INLINE_ROWS_MAX> &, uint32_t, uint32_t, uint32_t, size_t,
-                                                   int, uint64_t *, cudaStream_t);
+                                                   cudaStream_t);
+
+cudaError_t split_ready(uint32_t max_rows, uint32_t sms, int max_smem) {
+    cudaError_t e = split_ready_for<float, INLINE_ROWS>(max_rows > sms, max_smem);
+    auto and_then = [&](bool needed, auto ready) {
+        if (e == cudaSuccess && needed) {
+            e = ready(max_rows > sms, max_smem);
+        }
+    };
+    and_then(true, split_ready_for<__nv_bfloat16, INLINE_ROWS>);
+    and_then(max_rows > INLINE_ROWS, split_ready_for<float, INLINE_ROWS_MID>);
+    and_then(max_rows > INLINE_ROWS, split_ready_for<__nv_bfloat16, INLINE_ROWS_MID>);
+    and_then(max_rows > INLINE_ROWS_MID, split_ready_for<float, INLINE_ROWS_MAX>);
+    and_then(max_rows > INLINE_ROWS_MID, split_ready_for<__nv_bfloat16, INLINE_ROWS_MAX>);
+    return e;
+}
 
 uint32_t split_rows_at_once(int device, int sm_count, int max_smem, uint32_t log_blocks) {
     if (log_blocks == 0u) {
@@ -64,16 +79,15 @@ uint32_t split_rows_at_once(int device, int sm_count, int max_smem, uint32_t log
     return n - 1u;
 }
 
-cudaError_t merge_launch(const MergeArgs &a, uint32_t rows, uint32_t *attr_mask, cudaStream_t stream) {
-    constexpr uint32_t bit = 1u << 22;
-    if (!(*attr_mask & bit)) {
-        const cudaError_t e =
-            cudaFuncSetAttribute(merge_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemFixed));
-        if (e != cudaSuccess) {
-            return e;
-        }
-        *attr_mask |= bit;
-    }
+cudaError_t merge_ready() {
+    cudaFuncAttributes fa;
+    const cudaError_t e = cudaFuncGetAttributes(&fa, merge_rows_kernel);
+    return e != cudaSuccess ? e
+                            : cudaFuncSetAttribute(merge_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)sizeof(SmemFixed));
+}
+
+cudaError_t merge_launch(const MergeArgs &a, uint32_t rows, cudaStream_t stream) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(rows, 1, 1);
     cfg.blockDim = dim3(NT, 1, 1);

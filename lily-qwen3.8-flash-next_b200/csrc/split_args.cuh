@@ -179,12 +179,16 @@ __host__ __device__ constexpr bool variant_many(uint32_t has, uint32_t max_rows)
 }
 
 // Launches the kernel for a.a.rows rows from row0 on: logits of `dtype`, `smem` bytes of
-// dynamic shared memory (at most max_smem); `has`: what the rows may bring, HAS_ALL if that is not known.
-// `attr_mask`: bits of the kernels whose limit has been raised, the caller's to keep per device. Instantiated in
-// split*.cu.
+// dynamic shared memory (at most what split_ready was given); `has`: what the rows may bring, HAS_ALL if that is not
+// known. Instantiated in split*.cu.
 template <uint32_t MAXR>
-cudaError_t split_launch(const SplitArgs<MAXR> &a, uint32_t has, uint32_t rows, uint32_t dtype, size_t smem, int max_smem,
-                         uint64_t *attr_mask, cudaStream_t stream);
+cudaError_t split_launch(const SplitArgs<MAXR> &a, uint32_t has, uint32_t rows, uint32_t dtype, size_t smem,
+                         cudaStream_t stream);
+
+// Loads every variant that launches of up to max_rows rows can take on the current device, and lets it have max_smem
+// bytes of shared memory. (Left to the launches, the first request of another kind would wait 0.2 to 1 ms for
+// its kernel in the middle of serving, or 4 to 19 where it is the first of its translation unit.)
+cudaError_t split_ready(uint32_t max_rows, uint32_t sms, int max_smem);
 
 // Rows whose parameters travel in the kernel's arguments: sizes of the argument block (a
 // larger one takes longer to launch), the last one as many rows as the chip has SMs.
@@ -202,6 +206,7 @@ struct MergeArgs {
     KArgs a;
     RowIn in[INLINE_ROWS_MID];
 };
-cudaError_t merge_launch(const MergeArgs &a, uint32_t rows, uint32_t *attr_mask, cudaStream_t stream);
+cudaError_t merge_launch(const MergeArgs &a, uint32_t rows, cudaStream_t stream);
+cudaError_t merge_ready();
 
 }  // namespace lily

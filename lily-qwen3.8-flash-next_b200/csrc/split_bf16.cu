@@ -3,6 +3,6 @@
 
 namespace lily {
 
-LILY_SPLIT_LAUNCH_FOR(__nv_bfloat16, INLINE_ROWS);
+LILY_SPLIT_LAUNCH_FOR(, __nv_bfloat16, INLINE_ROWS);
 
 }  // namespace lily

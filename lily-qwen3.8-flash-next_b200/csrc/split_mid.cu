@@ -3,6 +3,6 @@
 
 namespace lily {
 
-LILY_SPLIT_LAUNCH_FOR(float, INLINE_ROWS_MID);
+LILY_SPLIT_LAUNCH_FOR(, float, INLINE_ROWS_MID);
 
 }  // namespace lily

@@ -3,6 +3,6 @@
 
 namespace lily {
 
-LILY_SPLIT_LAUNCH_FOR(__nv_bfloat16, INLINE_ROWS_MID);
+LILY_SPLIT_LAUNCH_FOR(, __nv_bfloat16, INLINE_ROWS_MID);
 
 }  // namespace lily

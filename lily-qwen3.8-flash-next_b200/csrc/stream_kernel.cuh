@@ -33,6 +33,7 @@
 namespace lily {
 
 constexpr uint32_t STREAM_MIN_ROUNDS = 8;  // shorter rows go to the row kernel, or in slices
+constexpr uint32_t STREAM_MIN_ROWS = 16;   // fewer rows of long vocabularies are cut into slices
 constexpr uint32_t STREAM_K_MAX = 64;      // finalize_warp holds two candidates per lane
 // AHEAD (template argument of the kernel): rounds of the ring in flight beyond the
 // one being read. With a block slot's worth of rows two measured faster than
