@@ -170,12 +170,17 @@ enum : uint32_t {
     HAS_ARGMAX = 32  // (nothing but: parameters, lists, slots and forced ids are not looked at)
 };
 constexpr uint32_t HAS_UNKNOWN = HAS_WIDE | HAS_RAISES;  // parameters on the device, no lists
-// Variants whose rows' parameters all lie in the arguments, and whose rows all lie over two blocks or more.
+// Rows whose parameters travel in the kernel's arguments: sizes of the argument block (a
+// larger one takes longer to launch), the last one as many rows as the chip has SMs.
+constexpr uint32_t INLINE_ROWS = 8, INLINE_ROWS_MID = 64, INLINE_ROWS_MAX = 148;
+// Variants whose rows' parameters all lie in the arguments, and those of them whose rows all lie over two blocks or
+// more: not of the largest argument block, whose launches have one block a row from 75 rows on. (No launch of
+// other rows takes them: split_takes in split_launch.cuh.)
 __host__ __device__ constexpr bool variant_inline(uint32_t has) {
     return has != HAS_ALL && has != HAS_ARGMAX && has != HAS_UNKNOWN;
 }
 __host__ __device__ constexpr bool variant_many(uint32_t has, uint32_t max_rows) {
-    return variant_inline(has) && max_rows != 148u;
+    return variant_inline(has) && max_rows != INLINE_ROWS_MAX;
 }
 
 // Launches the kernel for a.a.rows rows from row0 on: logits of `dtype`, `smem` bytes of
@@ -189,11 +194,6 @@ cudaError_t split_launch(const SplitArgs<MAXR> &a, uint32_t has, uint32_t rows, 
 // bytes of shared memory. (Left to the launches, the first request of another kind would wait 0.2 to 1 ms for
 // its kernel in the middle of serving, or 4 to 19 where it is the first of its translation unit.)
 cudaError_t split_ready(uint32_t max_rows, uint32_t sms, int max_smem);
-
-// Rows whose parameters travel in the kernel's arguments: sizes of the argument block (a
-// larger one takes longer to launch), the last one as many rows as the chip has SMs.
-constexpr uint32_t INLINE_ROWS = 8, INLINE_ROWS_MID = 64, INLINE_ROWS_MAX = 148;
-static_assert(!variant_many(0u, INLINE_ROWS_MAX), "75 rows and more lie in one block each");
 
 // The most rows that clusters of 1 << log_blocks blocks run at once, one block per SM. Less
 // than the SMs would hold (15 clusters of eight on 148 SMs, 33 of four): a cluster lies in
