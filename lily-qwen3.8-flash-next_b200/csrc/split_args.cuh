@@ -169,7 +169,10 @@ enum : uint32_t {
     HAS_WIDE = 1, HAS_SHARD = 2, HAS_LISTS = 4, HAS_RAISES = 8, HAS_SPEC = 16, HAS_ALL = 31,
     HAS_ARGMAX = 32  // (nothing but: parameters, lists, slots and forced ids are not looked at)
 };
-constexpr uint32_t HAS_UNKNOWN = HAS_WIDE | HAS_RAISES;  // parameters on the device, no lists
+// Parameters on the device, no lists; and of up to 8 rows what else needs no more than this: rows whose penalties
+// raise a logit (4 x 151936 bf16, 4096 ids: 14.85 us with everything, 13.45 so; 8 x 151936 f32 12.7, 11.95), and rows in
+// one block (1 x 1000 f32: 8.24, 7.60).
+constexpr uint32_t HAS_UNKNOWN = HAS_WIDE | HAS_RAISES;
 // Rows whose parameters travel in the kernel's arguments: sizes of the argument block (a
 // larger one takes longer to launch), the last one as many rows as the chip has SMs.
 constexpr uint32_t INLINE_ROWS = 8, INLINE_ROWS_MID = 64, INLINE_ROWS_MAX = 148;

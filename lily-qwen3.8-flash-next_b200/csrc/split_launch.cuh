@@ -63,10 +63,10 @@ void split_variants(F f) {
         };
         (void)(one(set) || ...);
     };
-    each(std::integral_constant<uint32_t, HAS_ARGMAX>(), std::integral_constant<uint32_t, HAS_UNKNOWN>(),
-         std::integral_constant<uint32_t, 0u>(), std::integral_constant<uint32_t, HAS_SPEC>(),
-         std::integral_constant<uint32_t, HAS_WIDE>(), std::integral_constant<uint32_t, HAS_WIDE | HAS_LISTS>(),
-         std::integral_constant<uint32_t, HAS_SHARD>(), std::integral_constant<uint32_t, HAS_ALL>());
+    each(std::integral_constant<uint32_t, HAS_ARGMAX>(), std::integral_constant<uint32_t, 0u>(),
+         std::integral_constant<uint32_t, HAS_SPEC>(), std::integral_constant<uint32_t, HAS_WIDE>(),
+         std::integral_constant<uint32_t, HAS_WIDE | HAS_LISTS>(), std::integral_constant<uint32_t, HAS_SHARD>(),
+         std::integral_constant<uint32_t, HAS_UNKNOWN>(), std::integral_constant<uint32_t, HAS_ALL>());
 }
 
 // Whether a launch whose rows may bring `has` may take the variant.
@@ -78,7 +78,8 @@ bool split_takes(const SplitArgs<MAXR> &a, uint32_t variant, uint32_t has) {
     if ((variant_inline(variant) && !a.inline_params) || (variant_many(variant, MAXR) && a.log_blocks == 0u)) {
         return false;
     }
-    return has == variant || (variant == (HAS_WIDE | HAS_LISTS) && (has & ~variant) == 0u);
+    // (HAS_UNKNOWN serves whatever it has, with parameters in the arguments or not.)
+    return has == variant || ((variant == (HAS_WIDE | HAS_LISTS) || variant == HAS_UNKNOWN) && (has & ~variant) == 0u);
 }
 
 // Everything for logits of one type.
