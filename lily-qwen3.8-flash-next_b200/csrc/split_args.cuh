@@ -95,8 +95,8 @@ struct alignas(16) SplitSmem {
     union {
         struct {
             alignas(16) uint32_t pool[SPL_POOL];  // the best keys of every warp of the cluster
-            // Buckets that reach the bound. (The maxima have served by then; the pool may still be read. By itself
-            // this list kept a second block of 151937 f32 logits off an SM: 256 rows 77 us, so 48.)
+            // Buckets that reach the bound. (The maxima have served by then, and a block that waited for them in vain
+            // lists none; the pool may still be read. By itself this list kept a second block of 151937 f32 logits off an SM: 256 rows 77 us, so 48.)
             uint16_t flagged[SPL_FLAGGED];
         };
         uint32_t tmax[SPL_MAX_BLOCKS * SPL_NT];  // wide rows: the keys of all its threads
