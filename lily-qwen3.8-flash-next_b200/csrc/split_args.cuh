@@ -20,6 +20,7 @@ constexpr uint32_t SPL_SMALL_K = 64;     // up to here a row's bound comes from 
 constexpr uint32_t SPL_POOL = 256;       // keys in the pool a narrow row's bound is taken from
 constexpr uint32_t SPL_HITS = 512;       // vectors of a block that may reach the bound
 constexpr uint32_t SPL_FLAGGED = 2048;   // buckets that may reach the bound
+constexpr uint32_t HELD_MIN = 320;       // a row of two buckets that keeps more does not read the second one again
 constexpr uint32_t SPL_SORTED = 2048;    // candidates of a wide row
 // Pieces of a block, at least: half of its warps have one. (With a piece for every warp, and
 // so fewer blocks, 4096 bf16 that keep 64 took 14.2 us instead of 12.9.)

@@ -1941,10 +1941,17 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         }
     } else {
         uint32_t listed = buckets;
-        if (HAS == HAS_WIDE && BPS == 1 && buckets == 2u && k > CHAIN_MAX) {
+        if (HAS == HAS_WIDE && BPS == 1 && buckets == 2u && k > HELD_MIN) {
             // (A row of two buckets that keeps many looks at most of its vectors again: the second
-            // bucket's are still in registers. 1 x 151936 f32, 1024 kept: 14.62 -> 13.84 us; rows that
-            // keep 100 lose 0.25 us by it, rows of four buckets 0.2.)
+            // bucket's are still in registers. It pays where the read again would take a thread more than a
+            // round or two. From L2 and so, by the number kept: 3 x 151936 f32, eight blocks, 100 10.74 and 10.99 us,
+            // 256 11.49 and 11.54, 320 11.80 and 11.87, 384 12.18 and 12.18, 512 12.40 and 12.29, 1024 14.71 and 13.88;
+            // 3 x 248320 bf16 384 12.49 and 12.35, 1024 15.33 and 14.37; 24 x 100352 bf16, four blocks, 192 12.03 and 12.01,
+            // 256 12.60 and 12.46, 384 14.23 and 13.58; 50 x 40000 f32, two, 128 12.77 and 12.81, 192 13.99 and 13.59. So the
+            // line lies where neither side loses more than 0.15 us, but for two blocks. Of three buckets, two read
+            // again: 1 x 200064 f32, 100 11.36 and 11.52, 512 12.89 and 12.83, 1024 15.24 and 14.83: left out. In
+            // the variants for lists and for parameters on the device it gains as much (4 x 151936 f32, 1024 kept
+            // 15.48 and 14.36), and their other rows lose 0.1: left out.)
             listed = 1u;
             if (bm >= least) {
 #pragma unroll

@@ -449,3 +449,23 @@ def test_more_buckets_than_a_word_has_bits(cuda, lily, W, rows, vocab):
         b.logits[r, rng.integers(0, vocab, 12)] += 3.0
         b.logits[r, vocab - 1 - rng.integers(0, 400, 4)] += 4.0
     check(cuda, lily, W, b, vocab, f"B={rows} V={vocab}")
+
+
+@pytest.mark.parametrize("rows,vocab,bf16", [
+    (4, 81_920, False), (4, 81_921, False), (4, 82_304, False), (5, 151_937, False), (4, 163_840, False), (4, 163_843, False),
+    (4, 163_840, True), (4, 163_841, True), (5, 262_143, True),
+    (24, 40_960, False), (24, 41_003, False), (24, 100_353, True), (50, 20_483, False), (50, 40_001, False), (50, 60_007, True)])
+def test_rows_that_keep_many_and_hold_their_second_bucket(cuda, lily, W, rows, vocab, bf16):
+    """Rows without lists that keep more than 320 do not read the second of two
+    buckets again: kept counts around that, shares of one, two and three buckets (in one cluster too: a
+    bucket is 80 pieces of 512 bytes), rows over eight, four and two blocks that do not start on 16 bytes."""
+    rng = np.random.default_rng([rows, vocab, bf16])
+    ks = [65, 319, 320, 321, 384, 385, 1024, 640, 0]
+    for kw in ({}, dict(history=700, rep=1.2)):
+        b = make_batch(W, rng, rows, vocab, 0, bf16, kind="zipf", **kw)
+        for r in range(rows):
+            b.params[r].update(top_k=ks[(r + len(kw)) % len(ks)], top_p=1.0, min_p=0.0)
+        check(cuda, lily, W, b, vocab, f"B={rows} V={vocab} {kw}")
+        for p in b.params:  # (all of them on one side)
+            p["top_k"] = 448
+        check(cuda, lily, W, b, vocab, f"B={rows} V={vocab} {kw} 448 kept")
