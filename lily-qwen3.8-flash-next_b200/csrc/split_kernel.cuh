@@ -1839,6 +1839,8 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         }
         if (many && !wait_first_phase(&ss->mbar[MEET_POOL], ca.wait_ns >> 2)) {
             ss->hard = ss->late = 1;
+            // (Others may still put their maxima where the list of buckets would lie: it is full.)
+            ss->n_flagged = SPL_FLAGGED + 1u;
         }
         spl_sync();
         uint32_t keys[SPL_MAX_BLOCKS], m = 0;
@@ -1895,10 +1897,9 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
             cum += c[j];
         }
         spl_sync();
-        // The lower edge of the k-th maximum's bin (the rounding of d is covered below). None if the maxima are
-        // not all there: others may still put theirs where the list of buckets would lie.
+        // The lower edge of the k-th maximum's bin (the rounding of d is covered below).
         const uint32_t bin = ss->bin;
-        bound_key = bin == NONE || ss->late != 0u ? 0u : key_of(__fsub_rn(top, __fdiv_rn((float)(bin + 1u), BINS_PER_UNIT)));
+        bound_key = bin == NONE ? 0u : key_of(__fsub_rn(top, __fdiv_rn((float)(bin + 1u), BINS_PER_UNIT)));
     }
     LILY_STAMP(PH_FIRST_THRESHOLD);
     // At least k logits of the row have a value (before the division) of `bound`

@@ -33,17 +33,20 @@ def test_the_lists_meeting_releases_what_the_block_has_read():
 
 def test_no_list_of_buckets_lies_where_a_late_block_may_store():
     # `flagged` lies over `tmax`, into which the other blocks of a wide row put their maxima. A block whose wait for
-    # them ran out goes on to the later meetings, but has no bound: it is `hopeless`, and lists and reads nothing.
+    # them ran out goes on to the later meetings, but its list counts as full: nothing is written to it or read
+    # from it. (Nothing but the list's own adds changes its length after that.)
     with open(os.path.join(CSRC, "split_args.cuh")) as f:
         union = re.search(r"union \{(.*?)\n    \};", f.read(), re.S).group(1)
     assert "flagged[" in union and "tmax[" in union
     with open(os.path.join(CSRC, "split_kernel.cuh")) as f:
         source = f.read()
     wait = source.index("wait_first_phase(&ss->mbar[MEET_POOL], ca.wait_ns >> 2)", source.index("ss->bin = NONE;"))
-    bound = re.search(r"bound_key = ([^;]*?)\? 0u", source[wait:])
-    assert re.search(r"\{\s*ss->hard = ss->late = 1;", source[wait:wait + 200])
-    assert "ss->late != 0u" in bound.group(1)
-    # (The barrier between the two makes it one value for all threads: other blocks' waits set their own.)
-    assert "spl_sync();" in source[wait:wait + bound.start()]
-    hopeless = source.index("const bool hopeless = bound_key == 0u", wait)
-    assert hopeless < source.index("if (hopeless) {", hopeless) < source.index("ss->flagged[at++]", hopeless)
+    out = source[wait:source.index("spl_sync();", wait)]
+    assert "ss->hard = ss->late = 1;" in out and "ss->n_flagged = SPL_FLAGGED + 1u;" in out
+    listed = source.index("atomicAdd(&ss->n_flagged", wait)
+    assert not re.search(r"n_flagged\s*=[^=]", source[wait + len(out):listed])
+    write = source.index("ss->flagged[at++] =", listed)
+    assert "at < SPL_FLAGGED" in source[listed:write]
+    refuse = source.index("if (n_flagged > SPL_FLAGGED) {", write)
+    assert refuse < source.index("ss->flagged[i / SPL_U]", refuse)
+    assert source.count("ss->flagged[") == 2
