@@ -127,7 +127,7 @@ uint32_t lily_residual_step(uint32_t step);
  * Every kernel that a draw of up to `max_rows` rows may take is loaded here, so
  * that no request of a new kind waits for one later, or loads it inside a
  * stream capture. The first handle of a process on a device takes 65 ms for that with
- * one row and 115 to 190 ms with 160 (13 and 29 MB on the device); another one of the
+ * one row and 115 to 340 ms with 160 (13 and 29 MB on the device); another one of the
  * same size 0.02 to 0.4 ms. (The first LM head call loads the head's kernels: 2 ms.)
  */
 int32_t lily_sampler_create(int32_t device, uint32_t vocab, uint32_t max_rows,

@@ -94,7 +94,7 @@ cudaError_t launch_for(const Args &a, Format format, uint32_t sms, cudaStream_t 
 // as subnormals 61; sums of shared tiles handed on through the logits' place instead of a
 // workspace: + 0.6 to 1.2 at 4 bits, nothing elsewhere; scales through shared memory 58.4; a warp's waits as one
 // 57.3.) At 16 tokens the weights' stream bounds bytes (5.9 TB/s of 6.6
-// measured for a copy); the rest is bound by what its warps issue (slots 62 to 65 % busy; 4 % more
+// measured for a copy); the rest is bound by what its warps issue (slots 58 to 63 % busy; 4 % more
 // instructions take 3.6 % longer): widening a weight, one FMA per logit and group, and the waits. In calls
 // that go on for a tenth of a second the power limit lowers the clock: 64 tokens 240 -> 275 us.
 cudaError_t launch_head(const Args &a, Format format, uint32_t sms, cudaStream_t stream) {

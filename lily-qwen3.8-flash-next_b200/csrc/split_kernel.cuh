@@ -24,10 +24,10 @@
 // 1.45 us, from the candidates sent to all of them there 0.1 to 0.25. So blocks meet by stores
 // that complete a barrier in the receiver, no warp waits for one that it does not need, and the
 // draw's adds run in two chains of 32 lanes. Measured back to back: 1 row x 151936 f32 with a history of 4096 ids 50 -> 7.7 us, 64 rows x
-// 151936 bf16 with histories 32 -> 12.8, argmax of 1 x 32768 9.2 -> 2.55 (before: cut in
+// 151936 bf16 with histories 32 -> 12.8, argmax of 1 x 32768 9.2 -> 2.55 to 2.7 (before: cut in
 // slices through global memory, or a cluster that kept the row in shared memory). Code that the
-// warps run once is slow code: of the 21 clocks between two instructions of a warp 6 to 7.5 wait for the
-// instruction itself and 7.5 at barriers. So what stands on the way counts: functions
+// warps run once is slow code: of the 18 and 15.5 clocks between two instructions of a warp (the first two of
+// these) 5.7 and 3.2 wait for the instruction itself and 5.4 and 4.2 at barriers. So what stands on the way counts: functions
 // that take the launch's arguments by address load each of them from memory (1 us), an
 // arrival that releases waits for the thread's stores (0.3 us each), and code that a call never
 // runs still slows it where it stands between what it does run: the kernel is compiled for what a
@@ -1985,7 +1985,9 @@ __global__ void __launch_bounds__(NT, BPS) split_rows_kernel(const __grid_consta
         if (n_flagged > SPL_FLAGGED) {
             ss->hard = 1;
         } else {
-            // (Each of them again, from L2: a narrow row has hardly more than one vector per thread.)
+            // (Each of them again, from L2: a narrow row has hardly more than one vector per thread. Four and two at
+            // a time: 1 x 151936 f32 with 4096 ids 7.88 and 7.77 us, 8 x 248320 f32 from slots 13.32 and 13.54, 24 x 50257
+            // f32 and 64 x 151936 bf16 the same.)
             constexpr uint32_t AGAIN = (HAS & HAS_WIDE) != 0u ? 4u : 2u;
             for (uint32_t i0 = tid; i0 < n_flagged * SPL_U; i0 += AGAIN * SPL_NT) {
                 uint4 x[AGAIN];
